@@ -78,7 +78,7 @@ __device__ __forceinline__ D3 move_exact_f(D3 p, D3 v, double R) {
     D3 q{__dadd_rn(p.x, __dsub_rn(v.x, __dmul_rn(s, p.x))), __dadd_rn(p.y, __dsub_rn(v.y, __dmul_rn(s, p.y))),
          __dadd_rn(p.z, __dsub_rn(v.z, __dmul_rn(s, p.z)))};
     const double qq = __dadd_rn(__dadd_rn(__dmul_rn(q.x, q.x), __dmul_rn(q.y, q.y)), __dmul_rn(q.z, q.z));
-    const double inv = f64_div(1.0, f64_sqrt(qq));
+    const double inv = f64_div_root(1.0, qq);
     return D3{__dmul_rn(R, __dmul_rn(inv, q.x)), __dmul_rn(R, __dmul_rn(inv, q.y)), __dmul_rn(R, __dmul_rn(inv, q.z))};
 }
 

@@ -32,7 +32,7 @@ __device__ __forceinline__ int comp(const int4& a, int s) { return s == 0 ? a.x 
 // (any radius), from the raw position difference d.
 __device__ __forceinline__ D3 grad_geo_vec(D3 a, D3 d) {
     const D3 t = sub3(d, scl3(dot3(d, a), a));
-    return scl3(f64_div(-1.0, f64_sqrt(dot3(t, t))), t);
+    return scl3(f64_div_root(-1.0, dot3(t, t)), t);
 }
 // Gradient w.r.t. v = |v| a of the signed spherical triangle area R^2 E(a, a + beta, a + gamma),
 // beta and gamma the raw differences to the other corners over |v|: tan(E/2) = N/D (Van Oosterom
@@ -47,67 +47,12 @@ __device__ __forceinline__ D3 grad_tri_vec(D3 a, D3 beta, D3 gamma, double R) {
     return scl3(R, sub3(g, scl3(dot3(g, a), a)));
 }
 
-// The geodesic-length gradient at v towards its ring predecessor in cell slot s, in Cartesian
-// form.  Each neighbour of v is the predecessor in one of its cells and the successor in another,
-// so the three of them cover both geodesic terms of every slot, each evaluated once.
-__device__ __forceinline__ D3 slot_geodesic(const ForceArgs& A, int v, int s) {
-    const double4_32a sv = A.vsph[v];
-    return from_basis(sv, grad_geodesic(sv, A.vsph[comp(A.vlast[v], s)]));
-}
-
-// The contribution of cell slot s to the force on vertex v: the fSet term of the header's sum for
-// the vertex's cell s, which block_slot_force adds in slot order, skipping a NaN term, as the
-// reference's loop over the three cells does.  Three threads share a vertex (more warps in flight
-// when the vertex count is small).  gG: the vertex's three slot_geodesic values (reference form
-// only).  The vector form (A.vec: the exact gradient as vectors, well conditioned where the
-// reference's closed forms lose digits -- short edges, thin fan triangles) uses grad_geo_vec and
-// grad_tri_vec on the position differences instead.
 // The force form of a kernel: chosen per launch from A.vec (kFormAny), or fixed at compile time, which
 // lets a kernel that runs one form drop the other's registers.
 constexpr int kFormAny = 0, kFormVector = 1, kFormReference = 2;
-template <int kForm = kFormAny>
-__device__ __forceinline__ D3 slot_force(const ForceArgs& A, int v, int s, const D3* gG) {
-    const int4 cells = A.vcell[v], lasts = A.vlast[v], nexts = A.vnext[v];
-    const int c = comp(cells, s), L = comp(lasts, s), X = comp(nexts, s);
-    if (kForm == kFormVector || (kForm == kFormAny && A.vec)) {
-        const D3 P = ld3(A.pos, v);
-        const double inv = f64_div(1.0, f64_sqrt(dot3(P, P)));
-        const D3 a = scl3(inv, P);
-        const D3 dc = sub3(ld3(A.cellPos, c), P);
-        const D3 dl = sub3(ld3(A.pos, L), P), dx = sub3(ld3(A.pos, X), P);
-        const double2 apc = A.ap[c], pr = A.pref[c];
-        const double pp = 2.0 * (apc.y - pr.y), aa = 2.0 * A.Kr * (apc.x - pr.x);
-        const D3 bl = scl3(inv, dl), bc = scl3(inv, dc), bx = scl3(inv, dx);
-        return add3(scl3(-pp, add3(grad_geo_vec(a, dl), grad_geo_vec(a, dx))),
-                    scl3(-aa, add3(grad_tri_vec(a, bl, bc, A.R), grad_tri_vec(a, bc, bx, A.R))));
-    }
-    const D3 p = ld3(A.pos, v);
-    const double4_32a sv = A.vsph[v];
-    const D3 cp = ld3(A.cellPos, c);
-    const double4_32a sc = A.cellSph[c];
-    const double2 apc = A.ap[c], pr = A.pref[c];
-    const double dA = apc.x - pr.x, dP = apc.y - pr.y;
-    const D3 pl = ld3(A.pos, L), px = ld3(A.pos, X);
-    const double4_32a sl = A.vsph[L], sx = A.vsph[X];
-    const double pp = 2.0 * dP;
-    const double aa = 2.0 * A.Kr * dA;
-    const int jx = X == lasts.x ? 0 : (X == lasts.y ? 1 : (X == lasts.z ? 2 : -1));
-    D3 fs{0.0, 0.0, 0.0}, t;
-    t = pick3(gG, s);
-    fs = sub3(fs, scl3(pp, t));
-    t = jx >= 0 ? pick3(gG, jx) : from_basis(sv, grad_geodesic(sv, sx));
-    fs = sub3(fs, scl3(pp, t));
-    t = from_basis(sv, grad_triangle(sv, sl, sc, p, pl, cp, A.R));
-    fs = sub3(fs, scl3(aa, t));
-    t = from_basis(sv, grad_triangle(sv, sc, sx, p, cp, px, A.R));
-    fs = sub3(fs, scl3(aa, t));
-    return fs;
-}
 
 // Block-level force of kSlotVerts vertices by 3 kSlotVerts threads (thread 3 i + s computes slot s
-// of vertex i of the block); threads i < kSlotVerts receive vertex i's force in slot order.  The
-// geodesic gradients of the reference form are evaluated once per neighbour (thread 3 i + s for
-// the predecessor in slot s) and shared through the block.
+// of vertex i of the block); threads i < kSlotVerts receive vertex i's force in slot order.
 constexpr int kSlotVerts = 64;
 // Resident blocks per SM the slot-force kernels are compiled for: three blocks of 3 kSlotVerts
 // threads (the register budget falls from 120 to 96 with a few bytes of spill), whose 18 warps hide
@@ -115,29 +60,102 @@ constexpr int kSlotVerts = 64;
 // Brownian step's force kernel at 100k cells: 0.49 -> 0.475 ms per launch; FIRE's at 20k cells
 // likewise).  Blocks of 32 vertices (six per SM) measured no faster at 20k or 100k cells.
 constexpr int kSlotMinBlocks = 3;
-struct SlotShared { double x[3 * kSlotVerts], y[3 * kSlotVerts], z[3 * kSlotVerts]; };
+struct SlotShared {
+    double x[3 * kSlotVerts], y[3 * kSlotVerts], z[3 * kSlotVerts];  // edge gradients, then slot forces
+    double sP[3 * kSlotVerts], s[3 * kSlotVerts], d[3 * kSlotVerts];  // pair terms towards the predecessor
+};
+
+// The contribution of cell slot s to the force on vertex v in the reference form: the fSet term of the
+// header's sum for the vertex's cell s.  Three threads share a vertex (more warps in flight when the
+// vertex count is small).  Each neighbour of v is the predecessor in one of its cells and the successor
+// in another, so the three threads' predecessors cover all of the vertex's edges: each thread
+// evaluates its predecessor's pair terms and edge gradient, and takes its successor's from the thread
+// that has it, through the block's shared memory.  Every thread of the block calls it.
+__device__ __forceinline__ D3 slot_force_reference(const ForceArgs& A, int v, int vi, int s, bool live, SlotShared& sh) {
+    const int t = threadIdx.x;
+    int4 cells, lasts, nexts;
+    double4_32a sv, sl;
+    PairTerms pL;
+    D3 gL;
+    if (live) {
+        cells = A.vcell[v]; lasts = A.vlast[v]; nexts = A.vnext[v];
+        sv = A.vsph[v];
+        sl = A.vsph[comp(lasts, s)];
+        pL = pair_terms(sv, sl);
+        gL = from_basis(sv, grad_geodesic(pL, sl.y));
+        sh.x[t] = gL.x; sh.y[t] = gL.y; sh.z[t] = gL.z;
+        sh.sP[t] = pL.sP; sh.s[t] = pL.s; sh.d[t] = pL.d;
+    }
+    __syncthreads();
+    D3 fs;
+    if (live) {
+        const int c = comp(cells, s), L = comp(lasts, s), X = comp(nexts, s);
+        const double2 apc = A.ap[c], pr = A.pref[c];
+        const double dA = apc.x - pr.x, dP = apc.y - pr.y;
+        const double pp = sf::twice(dP), aa = 2.0 * A.Kr * dA;
+        const double4_32a sx = A.vsph[X], sc = A.cellSph[c];
+        const int jx = X == lasts.x ? 0 : (X == lasts.y ? 1 : (X == lasts.z ? 2 : -1));
+        PairTerms pX;
+        D3 gX;
+        if (jx >= 0) {
+            const int tx = 3 * vi + jx;
+            gX = D3{sh.x[tx], sh.y[tx], sh.z[tx]};
+            pX.sP = sh.sP[tx]; pX.s = sh.s[tx]; pX.d = sh.d[tx];
+            pX.ss = __dmul_rn(pX.s, pX.s);
+            pX.q = -1. + pX.ss;
+        } else {  // inconsistent lists
+            pX = pair_terms(sv, sx);
+            gX = from_basis(sv, grad_geodesic(pX, sx.y));
+        }
+        fs = sub3(scl3(-pp, gL), scl3(pp, gX));
+        const PairTerms pC = pair_terms(sv, sc);
+        double2 g1 = grad_triangle(pL, pC, pair_cos(sl, sc), sl.y, sc.y, A.R);
+        double2 g2 = grad_triangle(pC, pX, pair_cos(sc, sx), sc.y, sx.y, A.R);
+        // the sign of each triangle's det: FP32 where that is certain (all but nearly flat triangles)
+        const D3 p = ld3(A.pos, v), pl = ld3(A.pos, L), px = ld3(A.pos, X), cp = ld3(A.cellPos, c);
+        const svm_det::F3 v32 = svm_det::near3(p.x, p.y, p.z);
+        const svm_det::F3 c32 = svm_det::diff(svm_det::near3(cp.x, cp.y, cp.z), v32);
+        int n1 = svm_det::below_zero(v32, svm_det::diff(svm_det::near3(pl.x, pl.y, pl.z), v32), c32);
+        int n2 = svm_det::below_zero(v32, c32, svm_det::diff(svm_det::near3(px.x, px.y, px.z), v32));
+        if (n1 < 0) n1 = det3(p, pl, cp) < 0 ? 1 : 0;
+        if (n2 < 0) n2 = det3(p, cp, px) < 0 ? 1 : 0;
+        if (n1) g1 = make_double2(-g1.x, -g1.y);
+        if (n2) g2 = make_double2(-g2.x, -g2.y);
+        fs = sub3(fs, scl3(aa, from_basis(sv, g1)));
+        fs = sub3(fs, scl3(aa, from_basis(sv, g2)));
+    }
+    __syncthreads();
+    return fs;
+}
+
+// The same in the vector form (A.vec: the exact gradient as vectors, well conditioned where the
+// reference's closed forms lose digits -- short edges, thin fan triangles).
+__device__ __forceinline__ D3 slot_force_vector(const ForceArgs& A, int v, int s) {
+    const int4 cells = A.vcell[v], lasts = A.vlast[v], nexts = A.vnext[v];
+    const int c = comp(cells, s), L = comp(lasts, s), X = comp(nexts, s);
+    const D3 P = ld3(A.pos, v);
+    const double inv = f64_div_root(1.0, dot3(P, P));
+    const D3 a = scl3(inv, P);
+    const D3 dc = sub3(ld3(A.cellPos, c), P);
+    const D3 dl = sub3(ld3(A.pos, L), P), dx = sub3(ld3(A.pos, X), P);
+    const double2 apc = A.ap[c], pr = A.pref[c];
+    const double pp = 2.0 * (apc.y - pr.y), aa = 2.0 * A.Kr * (apc.x - pr.x);
+    const D3 bl = scl3(inv, dl), bc = scl3(inv, dc), bx = scl3(inv, dx);
+    return add3(scl3(-pp, add3(grad_geo_vec(a, dl), grad_geo_vec(a, dx))),
+                scl3(-aa, add3(grad_tri_vec(a, bl, bc, A.R), grad_tri_vec(a, bc, bx, A.R))));
+}
+
+// The slots' contributions are added in slot order, a NaN term skipped, as the reference's loop over
+// the three cells does.
 template <int kForm = kFormAny>
 __device__ __forceinline__ D3 block_slot_force(const ForceArgs& A, int nV, SlotShared& sh) {
     const bool vec = kForm == kFormVector || (kForm == kFormAny && A.vec);
     const int t = threadIdx.x, base = blockIdx.x * kSlotVerts;
     const int vi = t / 3, s = t - 3 * (t / 3);
     const int v = base + vi;
-    if (!vec) {
-        if (v < nV) {
-            const D3 g = slot_geodesic(A, v, s);
-            sh.x[t] = g.x; sh.y[t] = g.y; sh.z[t] = g.z;
-        }
-        __syncthreads();
-    }
     D3 fs{0.0, 0.0, 0.0};
-    if (v < nV) {
-        D3 gG[3];
-        if (!vec)
-#pragma unroll
-            for (int j = 0; j < 3; ++j) gG[j] = D3{sh.x[3 * vi + j], sh.y[3 * vi + j], sh.z[3 * vi + j]};
-        fs = slot_force<kForm>(A, v, s, gG);
-    }
-    __syncthreads();
+    if (!vec) fs = slot_force_reference(A, v, vi, s, v < nV, sh);
+    else if (v < nV) fs = slot_force_vector(A, v, s);
     if (v < nV) { sh.x[t] = fs.x; sh.y[t] = fs.y; sh.z[t] = fs.z; }
     __syncthreads();
     D3 f{0.0, 0.0, 0.0};
@@ -239,7 +257,7 @@ __device__ __forceinline__ D3 move_exact(D3 p, D3 v, double R) {
     D3 q{__dadd_rn(p.x, __dsub_rn(v.x, __dmul_rn(s, p.x))), __dadd_rn(p.y, __dsub_rn(v.y, __dmul_rn(s, p.y))),
          __dadd_rn(p.z, __dsub_rn(v.z, __dmul_rn(s, p.z)))};
     const double qq = __dadd_rn(__dadd_rn(__dmul_rn(q.x, q.x), __dmul_rn(q.y, q.y)), __dmul_rn(q.z, q.z));
-    const double inv = f64_div(1.0, f64_sqrt(qq));
+    const double inv = f64_div_root(1.0, qq);
     return D3{__dmul_rn(R, __dmul_rn(inv, q.x)), __dmul_rn(R, __dmul_rn(inv, q.y)), __dmul_rn(R, __dmul_rn(inv, q.z))};
 }
 

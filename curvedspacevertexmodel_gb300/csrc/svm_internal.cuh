@@ -23,6 +23,7 @@
 #include "svm_acos.h"
 #include "svm_softf64.cuh"
 #include "svm_edge_filter.h"
+#include "svm_det_filter.h"
 
 namespace svm {
 
@@ -56,6 +57,25 @@ __device__ __forceinline__ double f64_sqrt(double a) {
     if constexpr (kHw) return __dsqrt_rn(a);
     else return sf::sqrt(a);
 #endif
+}
+
+// A divisor used more than once, and a square root used as a divisor: the quotients are f64_div's.
+#ifdef SVM_NATIVE_FP64_DIV
+struct F64Divisor { double d; };
+__device__ __forceinline__ F64Divisor f64_divisor(double b) { return F64Divisor{b}; }
+__device__ __forceinline__ F64Divisor f64_root_divisor(double a) { return F64Divisor{__dsqrt_rn(a)}; }
+__device__ __forceinline__ double f64_div(double a, const F64Divisor& b) { return __ddiv_rn(a, b.d); }
+#else
+using F64Divisor = sf::Divisor;
+__device__ __forceinline__ F64Divisor f64_divisor(double b) { return sf::divisor(b); }
+__device__ __forceinline__ F64Divisor f64_root_divisor(double a) { return sf::sqrt_divisor(a); }
+__device__ __forceinline__ double f64_div(double a, const F64Divisor& b) { return sf::div(a, b); }
+#endif
+// a / sqrt(b)
+template <bool kHw = false>
+__device__ __forceinline__ double f64_div_root(double a, double b) {
+    if constexpr (kHw) return __ddiv_rn(a, __dsqrt_rn(b));
+    else return f64_div(a, f64_root_divisor(b));
 }
 
 // The arccosine of the FP64 geometry (arcs, included angles, triangle areas, T1 length tests).
@@ -138,7 +158,7 @@ __device__ __forceinline__ double det3(D3 a, D3 b, D3 c) {    // a . (b x c), sp
 
 // putInBoxReal (sphericalDomain.h:183-187): p <- R p / |p|
 __device__ __forceinline__ D3 renorm(D3 p, double R) {
-    double inv = f64_div(1.0, f64_sqrt(dot3e(p, p)));
+    double inv = f64_div_root(1.0, dot3e(p, p));
     return scl3(R, scl3(inv, p));
 }
 // move(p, v) (sphericalDomain.h:203-209): project v onto the tangent plane at p, add, renormalise
@@ -267,7 +287,7 @@ __device__ __forceinline__ double included_angle_clamped(D3 p1, D3 p2, D3 p3) {
 }
 // sphericalTriangleArea (sphericalDomain.h:135-166)
 // q / |q| as sphericalTriangleArea normalises each corner
-__device__ __forceinline__ D3 unit_corner(D3 q) { return scl3(f64_div(1.0, f64_sqrt(dot3e(q, q))), q); }
+__device__ __forceinline__ D3 unit_corner(D3 q) { return scl3(f64_div_root(1.0, dot3e(q, q)), q); }
 __device__ __forceinline__ double triangle_area_unit(D3 p1, D3 p2, D3 p3, double R);
 __device__ __forceinline__ double triangle_area(D3 q1, D3 q2, D3 q3, double R) {
     return triangle_area_unit(unit_corner(q1), unit_corner(q2), unit_corner(q3), R);
@@ -289,69 +309,86 @@ template <bool kHw = false>
 __device__ __forceinline__ double4_32a sph_coords_n(D3 p, double r) {  // r = pos_norm(p)
     double cosT = f64_div<kHw>(p.z, r);
     double sinT = f64_sqrt<kHw>(1. - cosT * cosT);
-    double rxy = f64_sqrt<kHw>(early_mul<kHw>(p.x, p.x) + early_mul<kHw>(p.y, p.y));
-    return make_double4_32a(cosT, sinT, f64_div<kHw>(p.x, rxy), f64_div<kHw>(p.y, rxy));
+    const double rxy2 = early_mul<kHw>(p.x, p.x) + early_mul<kHw>(p.y, p.y);
+    if constexpr (kHw) {
+        const double rxy = f64_sqrt<kHw>(rxy2);
+        return make_double4_32a(cosT, sinT, f64_div<kHw>(p.x, rxy), f64_div<kHw>(p.y, rxy));
+    } else {
+        const F64Divisor rxy = f64_root_divisor(rxy2);
+        return make_double4_32a(cosT, sinT, f64_div(p.x, rxy), f64_div(p.y, rxy));
+    }
 }
 template <bool kHw = false>
 __device__ __forceinline__ double4_32a sph_coords(D3 p) { return sph_coords_n<kHw>(p, pos_norm<kHw>(p)); }
 
-// gradientGeodesicDistance (sphericalDomain.h:248-273) in the (theta, phi) basis of v1:
-// returns (d/dtheta, d/dphi) components.
-__device__ __forceinline__ double2 grad_geodesic(double4_32a s1, double4_32a s2) {
+// The terms of a pair of points (a, b), in spherical coordinates, that the gradients at a of both
+// gradientGeodesicDistance (sphericalDomain.h:248-273) and gradientTriangleArea (347-411) evaluate:
+// sin(phi_a - phi_b), s = cos of the arc, d = its derivative by theta_a, s s and s s - 1.  A pair is
+// evaluated once and serves its edge and both triangles it is a side of.
+struct PairTerms { double sP, s, d, ss, q; };
+__device__ __forceinline__ PairTerms pair_terms(const double4_32a& a, const double4_32a& b) {
     const auto E = [](double x, double y) { return early_mul(x, y); };
-    double sP12 = E(s1.w, s2.z) - E(s1.z, s2.w);
-    double cP12 = E(s1.z, s2.z) + E(s1.w, s2.w);
-    double dp = E(s1.x, s2.x) + E(E(cP12, s1.y), s2.y);
-    double dinv = f64_div(1., f64_sqrt(1 - dp * dp));
-    double gT = 1.0 * (E(s2.x, s1.y) - E(E(s1.x, cP12), s2.y)) * dinv;
-    double gP = E(s2.y, sP12) * dinv;
-    return make_double2(gT, gP);
+    PairTerms p;
+    p.sP = E(a.w, b.z) - E(a.z, b.w);
+    const double cP = E(a.z, b.z) + E(a.w, b.w);
+    p.s = E(a.x, b.x) + E(E(cP, a.y), b.y);
+    p.d = E(E(a.x, cP), b.y) - E(b.x, a.y);
+    p.ss = __dmul_rn(p.s, p.s);
+    p.q = -1. + p.ss;
+    return p;
+}
+// cos of the arc between b and c alone (the third side of a triangle at a)
+__device__ __forceinline__ double pair_cos(const double4_32a& b, const double4_32a& c) {
+    const auto E = [](double x, double y) { return early_mul(x, y); };
+    const double cP = E(b.z, c.z) + E(b.w, c.w);
+    return E(b.x, c.x) + E(E(cP, b.y), c.y);
+}
+
+// gradientGeodesicDistance (sphericalDomain.h:248-273) in the (theta, phi) basis of v1, from the
+// pair's terms and sin(theta) of the other point: returns (d/dtheta, d/dphi) components.
+__device__ __forceinline__ double2 grad_geodesic(const PairTerms& p, double sinT2) {
+    const double dinv = f64_div_root(1., -p.q);   // 1 - s s = -(s s - 1) exactly
+    return make_double2(-p.d * dinv, early_mul(sinT2, p.sP) * dinv);
 }
 
 // The other products of grad_triangle: the hardware multiply, spelled out.
 __device__ __forceinline__ double tri_mul(double x, double y) { return __dmul_rn(x, y); }
-
-// gradientTriangleArea (sphericalDomain.h:347-411) in the (theta, phi) basis of v1; the sign
-// follows det(v1, v2, v3).  Returns (d/dtheta, d/dphi) components.  Every product and sum in the
-// order the reference's expressions evaluate them (left to right, products first).
-__device__ __forceinline__ double2 grad_triangle(double4_32a a, double4_32a b, double4_32a c, D3 v1, D3 v2, D3 v3, double R) {
+// gradientTriangleArea (sphericalDomain.h:347-411) in the (theta, phi) basis of v1 for the triangle
+// (v1, v2, v3), without the sign of det(v1, v2, v3), from the terms of the pairs (v1, v2) and
+// (v1, v3), s23 = pair_cos(v2, v3) and sin(theta) of v2 and v3.  Returns (d/dtheta, d/dphi)
+// components.  Every product and sum rounds as the reference's expressions evaluate them (left to
+// right, products first); equal subexpressions, and those that differ by an exact sign or a power
+// of two, are evaluated once.  Each denominator is a square root and divides two numerators: its
+// reciprocal comes with the root (f64_root_divisor) and serves both.
+__device__ __forceinline__ double2 grad_triangle(const PairTerms& p12, const PairTerms& p13, double s23, double sinT2,
+                                                 double sinT3, double R) {
     const auto M = tri_mul;
     const auto E = [](double x, double y) { return early_mul(x, y); };
-    const double sP12 = E(a.w, b.z) - E(a.z, b.w);
-    const double sP13 = E(a.w, c.z) - E(a.z, c.w);
-    const double cP12 = E(a.z, b.z) + E(a.w, b.w);
-    const double cP13 = E(a.z, c.z) + E(a.w, c.w);
-    const double cP23 = E(b.z, c.z) + E(b.w, c.w);
-    const double s12 = E(a.x, b.x) + E(E(cP12, a.y), b.y);
-    const double s13 = E(a.x, c.x) + E(E(cP13, a.y), c.y);
-    const double s23 = E(b.x, c.x) + E(E(cP23, b.y), c.y);
-    const double d12 = E(E(a.x, cP12), b.y) - E(b.x, a.y);
-    const double d13 = E(E(a.x, cP13), c.y) - E(c.x, a.y);
-    const double s12s12 = M(s12, s12), s13s13 = M(s13, s13), s12s13 = M(s12, s13);
-    const double g = (((1 - s12s12) - s13s13) - M(s23, s23)) + M(M(M(2.0, s12), s13), s23);
-    const double q12 = -1. + s12s12, q13 = -1. + s13s13;
-    const double den1 = f64_sqrt(M(M(q12, q12), g));
-    const double den2 = f64_sqrt(M(M(q13, q13), g));
-    const double a12 = s12s12 - 1., a13 = s13s13 - 1.;
-    const double den3 = f64_sqrt(M(M(M(M(a12, a13), a12), a13), g));
-    const double s12s23 = M(s12, s23), s13s23 = M(s13, s23);
+    const double s12s13 = M(p12.s, p13.s);
+    // 2 s12 s13 s23 = 2 ((s12 s13) s23): the factor two is exact wherever it is applied
+    const double g = ((-p12.q - p13.ss) - M(s23, s23)) + sf::twice(M(s12s13, s23));
+    const F64Divisor den1 = f64_root_divisor(M(M(p12.q, p12.q), g));
+    const F64Divisor den2 = f64_root_divisor(M(M(p13.q, p13.q), g));
+    const F64Divisor den3 = f64_root_divisor(M(M(M(M(p12.q, p13.q), p12.q), p13.q), g));
+    const double t = s23 - s12s13, u = p13.s - M(p12.s, s23), w = p12.s - M(p13.s, s23);
     // the d/dtheta numerators are formed while the square roots of the denominators run: integer pipes
-    double gT = f64_div(E(d13, a12) + E(d12, s23 - s12s13), den1)
-              + f64_div(E(d12, a13) + E(d13, s23 - s12s13), den2)
-              - f64_div(E(E(d12, a13), s13 - s12s23) + E(E(d13, a12), s12 - s13s23), den3);
+    const double d12q13 = E(p12.d, p13.q), d13q12 = E(p13.d, p12.q);
+    double gT = f64_div(d13q12 + E(p12.d, t), den1) + f64_div(d12q13 + E(p13.d, t), den2)
+              - f64_div(E(d12q13, u) + E(d13q12, w), den3);
     gT = M(gT, R);
-    double gP = f64_div(M(M(s12s13 - s23, sP12), b.y) - M(M(-1 + s12s12, sP13), c.y), den1)
-              - f64_div(M(M(-1 + s13s13, sP12), b.y) + M(M(-s12s13 + s23, sP13), c.y), den2)
-              + f64_div(M(M(M(-1 + s13s13, s13 - s12s23), sP12), b.y) + M(M(M(-1 + s12s12, s12 - s13s23), sP13), c.y), den3);
+    double gP = f64_div(-M(M(t, p12.sP), sinT2) - M(M(p12.q, p13.sP), sinT3), den1)
+              - f64_div(M(M(p13.q, p12.sP), sinT2) + M(M(t, p13.sP), sinT3), den2)
+              + f64_div(M(M(M(p13.q, u), p12.sP), sinT2) + M(M(M(p12.q, w), p13.sP), sinT3), den3);
     gP = M(gP, R);
-    if (det3(v1, v2, v3) < 0) { gT = -gT; gP = -gP; }
     return make_double2(gT, gP);
 }
 
 // (theta, phi) components to Cartesian with the basis of sphericalDomain.h:218-232:
 // thetaHat = (cos t cos p, cos t sin p, -sin t), phiHat = (-sin p, cos p, 0).
 __device__ __forceinline__ D3 from_basis(double4_32a s, double2 g) {
-    return D3{g.x * (s.x * s.z) + g.y * (-s.w), g.x * (s.x * s.w) + g.y * s.z, g.x * (-s.y) + g.y * 0};
+    double z = g.x * (-s.y);   // + g.y * 0, which changes it only for an infinite or NaN g.y
+    if ((((unsigned)__double2hiint(g.y) >> 20) & 0x7ffu) == 0x7ffu) z += g.y * 0;
+    return D3{g.x * (s.x * s.z) + g.y * (-s.w), g.x * (s.x * s.w) + g.y * s.z, z};
 }
 
 // ---- host-side state -----------------------------------------------------------------------
