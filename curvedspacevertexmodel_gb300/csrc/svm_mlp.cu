@@ -16,16 +16,23 @@
 // W3[2][64], b3[2], row-major (out, in).  The forward pass uses their BF16 roundings; gradients
 // are taken with respect to those (straight-through) and applied to the master copy by Adam.
 //
-// Training runs one thread per sample in blocks of kTB samples: the forward activations and the
-// backward deltas are staged in shared memory, and each block writes its partial gradient sums
-// (products summed over its samples in a fixed order); a second kernel sums the block partials in
-// block order, so gradients are deterministic.
+// Every layer runs as register tiles over shared memory: a block of kTT threads takes kTS samples, a
+// thread four samples by two units, each output one chain of FP32 multiply-adds over the inputs in
+// ascending order.  Training takes kTB samples per cluster of four such blocks: each block runs its
+// quarter of the samples forward and back, then, with the cluster's activations and deltas gathered
+// through distributed shared memory, sums a quarter of the parameters' gradients over all kTB samples
+// in sample order; a second kernel sums the clusters' partials in order and applies Adam, so gradients
+// are deterministic and do not depend on how the work is spread.
+// What bounds it: FP32 multiply-adds (35k per sample and step, 2 us for 4096 samples at 128 a clock on
+// 152 SMs) and the latency of the chains; a batch of 4096 is 128 blocks.  The batch's loss stays on the
+// device until the epoch ends.
 #include <algorithm>
 #include <cmath>
 #include <mutex>
 #include <cstdio>
 #include <random>
 #include <vector>
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include "svm_internal.cuh"
 
@@ -35,8 +42,18 @@ using namespace svm;
 constexpr int kIn = 24, kH = 64, kOut = 2;
 constexpr int oW1 = 0, oB1 = oW1 + kH * kIn, oW2 = oB1 + kH, oB2 = oW2 + kH * kH, oW3 = oB2 + kH,
               oB3 = oW3 + kOut * kH, kParams = oB3 + kOut;
-constexpr int kTB = 128;       // samples per training block
-constexpr int kPad = kH + 1;   // shared-memory row stride of the activations (bank-conflict free)
+constexpr int kTB = 128;       // samples per training cluster (one partial gradient)
+constexpr int kTC = 4;         // blocks per training cluster
+constexpr int kTS = 32;        // samples per tile
+constexpr int kTT = 256;       // threads per tile
+constexpr int kQ = kH / kTC;   // hidden units whose gradients one block of a cluster sums
+static_assert(kTS * kTC == kTB, "a cluster's tiles cover its samples");
+// Shared-memory row strides (floats): 16-byte rows whose starts fall on distinct banks, so that a
+// warp's 8 sample rows and 4 unit rows load as 16-byte vectors without conflicts.
+constexpr int kSX = kIn + 4, kSH = kH + 4, kSQ = kQ + 4;
+// the weights in shared memory: W1[64][kSX] | W2[64][kSH] | W3[2][64] | b1 | b2 | b3
+constexpr int sW1 = 0, sW2 = sW1 + kH * kSX, sW3 = sW2 + kH * kSH, sB1 = sW3 + kOut * kH, sB2 = sB1 + kH, sB3 = sB2 + kH,
+              kWeights = sB3 + 4;
 
 __device__ __forceinline__ int c3(const int4& a, int s) { return s == 0 ? a.x : (s == 1 ? a.y : a.z); }
 
@@ -93,161 +110,259 @@ __global__ void k_features(FeatArgs A, int nV, float* __restrict__ X, double* __
     }
 }
 
-// BF16 weights -> FP32 in shared memory
+// BF16 weights -> FP32 in shared memory, rows at their strides
 __device__ void load_weights(const __nv_bfloat16* __restrict__ wb, float* w) {
-    for (int i = threadIdx.x; i < kParams; i += blockDim.x) w[i] = __bfloat162float(wb[i]);
-    __syncthreads();
+    for (int i = threadIdx.x; i < kParams; i += blockDim.x) {
+        int at;
+        if (i < oB1) at = sW1 + (i / kIn) * kSX + i % kIn;
+        else if (i < oW2) at = sB1 + (i - oB1);
+        else if (i < oB2) at = sW2 + ((i - oW2) / kH) * kSH + (i - oW2) % kH;
+        else if (i < oW3) at = sB2 + (i - oB2);
+        else if (i < oB3) at = sW3 + (i - oW3);
+        else at = sB3 + (i - oB3);
+        w[at] = __bfloat162float(wb[i]);
+    }
 }
 
-// y = W3 relu(W2 relu(W1 x + b1) + b2) + b3 for one sample, activations into h1, h2 (may be null)
-__device__ void forward1(const float* w, const float* x, float* y, float* h1, float* h2) {
-    float a1[kH];
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+// s + a . b over four consecutive inputs, one multiply-add after the other
+__device__ __forceinline__ float chain4(float4 a, float4 b, float s) {
+    return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, s))));
+}
+
+// One hidden layer of a tile: out[s][j] = relu(b[j] + sum_k W[j][k] in[s][k]).  Thread t computes
+// samples t % 8 + 8 i (i < 4) of units t / 8 + 32 u (u < 2) and keeps them in h.  Samples from `count`
+// on are written as zeros.
+template <int kK, int kSIn>
+__device__ __forceinline__ void tile_layer(const float* W, const float* b, const float* in, float* out, int count,
+                                           float (&h)[4][2]) {
+    const int sg = threadIdx.x & 7, jg = threadIdx.x >> 3;
+    float acc[4][2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[i][u] = b[jg + 32 * u];
 #pragma unroll 4
-    for (int j = 0; j < kH; ++j) {
-        float s = w[oB1 + j];
-        for (int k = 0; k < kIn; ++k) s = fmaf(w[oW1 + j * kIn + k], x[k], s);
-        a1[j] = fmaxf(s, 0.f);
-        if (h1) h1[j] = a1[j];
+    for (int k = 0; k < kK; k += 4) {
+        const float4 w0 = ld4(W + jg * kSIn + k), w1 = ld4(W + (jg + 32) * kSIn + k);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 x = ld4(in + (sg + 8 * i) * kSIn + k);
+            acc[i][0] = chain4(w0, x, acc[i][0]);
+            acc[i][1] = chain4(w1, x, acc[i][1]);
+        }
     }
-    float o0 = w[oB3], o1 = w[oB3 + 1];
-    for (int j = 0; j < kH; ++j) {
-        float s = w[oB2 + j];
-        for (int k = 0; k < kH; ++k) s = fmaf(w[oW2 + j * kH + k], a1[k], s);
-        s = fmaxf(s, 0.f);
-        if (h2) h2[j] = s;
-        o0 = fmaf(w[oW3 + j], s, o0);
-        o1 = fmaf(w[oW3 + kH + j], s, o1);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            h[i][u] = sg + 8 * i < count ? fmaxf(acc[i][u], 0.f) : 0.f;
+            out[(sg + 8 * i) * kSH + jg + 32 * u] = h[i][u];
+        }
+}
+// The network on a tile of kTS samples (x: rows of kSX in shared memory; every thread of the block
+// calls it, after a barrier): activations to h1, h2 (rows of kSH; this thread's in a1, a2), and the
+// outputs y[s][o] held by threads t < 2 kTS (s = t / 2, o = t % 2) as the return value.
+__device__ __forceinline__ float tile_forward(const float* w, const float* x, float* h1, float* h2, int count,
+                                              float (&a1)[4][2], float (&a2)[4][2]) {
+    tile_layer<kIn, kSX>(w + sW1, w + sB1, x, h1, count, a1);
+    __syncthreads();
+    tile_layer<kH, kSH>(w + sW2, w + sB2, h1, h2, count, a2);
+    __syncthreads();
+    float y = 0.f;
+    if (threadIdx.x < 2 * kTS) {
+        const int s = threadIdx.x >> 1, o = threadIdx.x & 1;
+        y = w[sB3 + o];
+#pragma unroll
+        for (int j = 0; j < kH; j += 4) y = chain4(ld4(w + sW3 + o * kH + j), ld4(h2 + s * kSH + j), y);
     }
-    y[0] = o0;
-    y[1] = o1;
+    return y;
 }
 
-// Forward + backward of one block of samples; per-block partial gradients and loss.
-// Dynamic shared memory: w[kParams] | X[kTB][kIn] | H1[kTB][kPad] | H2[kTB][kPad] | D2[kTB][kPad] | DY[kTB][2]
-__global__ void __launch_bounds__(kTB) k_train_block(const __nv_bfloat16* __restrict__ wb, const float* __restrict__ X,
-                                                     const float* __restrict__ Y, const int* __restrict__ order,
-                                                     int first, int count, float invBatch,
-                                                     float* __restrict__ partials, double* __restrict__ lossPartials) {
-    extern __shared__ float sm[];
-    float* w = sm;
-    float* sx = w + kParams;
-    float* h1 = sx + kTB * kIn;
-    float* h2 = h1 + kTB * kPad;
-    float* d2 = h2 + kTB * kPad;
-    float* dy = d2 + kTB * kPad;
-    __shared__ double lossSh[kTB / 32];
-    load_weights(wb, w);
-    const int t = threadIdx.x;
-    const int local = blockIdx.x * kTB + t;
-    const bool live = local < count;
-    float x[kIn], y[kOut];
-    double loss = 0.0;
-    if (live) {
-        const int sIdx = order ? order[first + local] : first + local;
-        for (int k = 0; k < kIn; ++k) x[k] = X[(long)sIdx * kIn + k];
-        forward1(w, x, y, h1 + t * kPad, h2 + t * kPad);
-        const float r0 = y[0] - Y[2L * sIdx], r1 = y[1] - Y[2L * sIdx + 1];
-        loss = (double)r0 * r0 + (double)r1 * r1;
-        dy[2 * t] = 2.f * r0 * invBatch;
-        dy[2 * t + 1] = 2.f * r1 * invBatch;
-        // delta of layer 2 pre-activations
-        for (int j = 0; j < kH; ++j) {
-            const float g = w[oW3 + j] * dy[2 * t] + w[oW3 + kH + j] * dy[2 * t + 1];
-            d2[t * kPad + j] = h2[t * kPad + j] > 0.f ? g : 0.f;
-        }
-    } else {
-        for (int k = 0; k < kIn; ++k) x[k] = 0.f;
-        for (int j = 0; j < kH; ++j) { h1[t * kPad + j] = 0.f; h2[t * kPad + j] = 0.f; d2[t * kPad + j] = 0.f; }
-        dy[2 * t] = dy[2 * t + 1] = 0.f;
+// Shared memory of a training block: the weights, this tile's x | h1 | h2 | d2 | d1 | dy, and the
+// cluster's H1 | X and, of the block's kQ units, D2 | D1 | H2, and DY.
+constexpr int tX = kWeights, tH1 = tX + kTS * kSX, tH2 = tH1 + kTS * kSH, tD2 = tH2 + kTS * kSH, tD1 = tD2 + kTS * kSH,
+              tDY = tD1 + kTS * kSH, gH1 = tDY + kTS * 2, gX = gH1 + kTB * kSH, gD2 = gX + kTB * kSX, gD1 = gD2 + kTB * kSQ,
+              gH2 = gD1 + kTB * kSQ, gDY = gH2 + kTB * kSQ, kTrainFloats = gDY + kTB * 2;
+
+// Forward + backward of kTB samples per cluster of kTC blocks; the cluster's partial gradients and each
+// tile's loss.
+__global__ void __cluster_dims__(kTC, 1, 1) __launch_bounds__(kTT)
+    k_train_block(const __nv_bfloat16* __restrict__ wb, const float* __restrict__ X, const float* __restrict__ Y,
+                  const int* __restrict__ order, int first, int count, float invBatch, float* __restrict__ partials,
+                  double* __restrict__ lossPartials) {
+    namespace cg = cooperative_groups;
+    extern __shared__ float4 smem4[];
+    float* sm = reinterpret_cast<float*>(smem4);
+    cg::cluster_group cluster = cg::this_cluster();
+    const int t = threadIdx.x, rank = (int)cluster.block_rank();
+    const int base = blockIdx.x * kTS;                 // tiles of a cluster are consecutive
+    const int live = max(0, min(kTS, count - base));
+    load_weights(wb, sm);
+    for (int e = t; e < kTS * kIn; e += kTT) {
+        const int s = e / kIn, k = e - s * kIn;
+        float v = 0.f;
+        if (s < live) v = X[(long)(order ? order[first + base + s] : first + base + s) * kIn + k];
+        sm[tX + s * kSX + k] = v;
     }
-    for (int k = 0; k < kIn; ++k) sx[t * kIn + k] = x[k];
-    // block loss
-    for (int o = 16; o > 0; o >>= 1) loss += __shfl_down_sync(0xffffffffu, loss, o);
-    if ((t & 31) == 0) lossSh[t >> 5] = loss;
     __syncthreads();
-    float* out = partials + (long)blockIdx.x * kParams;
-    if (t == 0) {
-        double l = 0.0;
-        for (int i = 0; i < kTB / 32; ++i) l += lossSh[i];
-        lossPartials[blockIdx.x] = l;
+    float a1[4][2], a2[4][2];
+    const float y = tile_forward(sm, sm + tX, sm + tH1, sm + tH2, live, a1, a2);
+    if (t < 2 * kTS) {
+        const int s = t >> 1, o = t & 1;
+        float r = 0.f;
+        if (s < live) {
+            const int sIdx = order ? order[first + base + s] : first + base + s;
+            r = y - Y[2L * sIdx + o];
+        }
+        sm[tDY + t] = 2.f * r * invBatch;
+        // (y0 - t0)^2 + (y1 - t1)^2 of sample s on its even thread, summed over the tile as a warp's
+        // shuffle tree over its samples does: the even threads of two warps hold 16 samples each
+        const double rd = (double)r * r;
+        const double ro = __shfl_xor_sync(0xffffffffu, rd, 1);
+        double* lossSh = reinterpret_cast<double*>(sm + gDY);   // (not yet in use)
+        if (o == 0) lossSh[s] = rd + ro;
     }
-    // dW3, db3 (needs H2 and DY)
-    for (int e = t; e < kOut * kH; e += kTB) {
-        const int o = e / kH, j = e % kH;
-        float s = 0.f;
-        for (int q = 0; q < kTB; ++q) s = fmaf(dy[2 * q + o], h2[q * kPad + j], s);
-        out[oW3 + e] = s;
+    __syncthreads();
+    if (t < 32) {
+        double loss = reinterpret_cast<const double*>(sm + gDY)[t];
+        for (int o = 16; o > 0; o >>= 1) loss += __shfl_down_sync(0xffffffffu, loss, o);
+        if (t == 0) lossPartials[blockIdx.x] = loss;
     }
-    if (t < kOut) {
+    const int sg = t & 7, jg = t >> 3;
+    // deltas of layer 2's pre-activations
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int s = sg + 8 * i;
+        const float dy0 = sm[tDY + 2 * s], dy1 = sm[tDY + 2 * s + 1];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int j = jg + 32 * u;
+            const float g = sm[sW3 + j] * dy0 + sm[sW3 + kH + j] * dy1;
+            sm[tD2 + s * kSH + j] = a2[i][u] > 0.f ? g : 0.f;
+        }
+    }
+    __syncthreads();
+    // deltas of layer 1's pre-activations
+    {
+        float g[4][2] = {};
+#pragma unroll 4
+        for (int i = 0; i < kH; i += 4) {
+            float4 d[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) d[q] = ld4(sm + tD2 + (sg + 8 * q) * kSH + i);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const float* w = sm + sW2 + i * kSH + jg + 32 * u;
+                const float4 wv = make_float4(w[0], w[kSH], w[2 * kSH], w[3 * kSH]);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) g[q][u] = chain4(wv, d[q], g[q][u]);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int u = 0; u < 2; ++u) sm[tD1 + (sg + 8 * q) * kSH + jg + 32 * u] = a1[q][u] > 0.f ? g[q][u] : 0.f;
+    }
+    cluster.sync();
+    // the cluster's activations and deltas, in sample order
+    const int u0 = rank * kQ;
+    for (int p = 0; p < kTC; ++p) {
+        const float* src = cluster.map_shared_rank(sm, p);
+        for (int e = t; e < kTS * (kH / 4); e += kTT) {
+            const int s = e / (kH / 4), k = 4 * (e % (kH / 4));
+            *reinterpret_cast<float4*>(sm + gH1 + (p * kTS + s) * kSH + k) = ld4(src + tH1 + s * kSH + k);
+        }
+        if (t < kTS * (kIn / 4)) {
+            const int s = t / (kIn / 4), k = 4 * (t % (kIn / 4));
+            *reinterpret_cast<float4*>(sm + gX + (p * kTS + s) * kSX + k) = ld4(src + tX + s * kSX + k);
+        }
+        for (int e = t; e < 3 * kTS * (kQ / 4); e += kTT) {
+            const int a = e / (kTS * (kQ / 4)), r = e % (kTS * (kQ / 4)), s = r / (kQ / 4), k = 4 * (r % (kQ / 4));
+            const int from = a == 0 ? tD2 : (a == 1 ? tD1 : tH2), to = a == 0 ? gD2 : (a == 1 ? gD1 : gH2);
+            *reinterpret_cast<float4*>(sm + to + (p * kTS + s) * kSQ + k) = ld4(src + from + s * kSH + u0 + k);
+        }
+        if (t < 2 * kTS) sm[gDY + p * 2 * kTS + t] = src[tDY + t];
+    }
+    cluster.sync();  // (no block leaves while another still reads its shared memory)
+    float* out = partials + (long)(blockIdx.x / kTC) * kParams;
+    {   // dW2 rows u0 .. u0 + kQ: thread (column j, four rows)
+        const int j = t & (kH - 1), ig = 4 * (t >> 6);
+        float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll 8
+        for (int q = 0; q < kTB; ++q) {
+            const float4 d = ld4(sm + gD2 + q * kSQ + ig);
+            const float h = sm[gH1 + q * kSH + j];
+            s0 = fmaf(d.x, h, s0); s1 = fmaf(d.y, h, s1); s2 = fmaf(d.z, h, s2); s3 = fmaf(d.w, h, s3);
+        }
+        float* o = out + oW2 + (u0 + ig) * kH + j;
+        o[0] = s0; o[kH] = s1; o[2 * kH] = s2; o[3 * kH] = s3;
+    }
+    if (t < 192) {  // dW1 rows u0 .. u0 + kQ: thread (column k, two rows)
+        const int k = t % kIn, ig = 2 * (t / kIn);
+        float s0 = 0.f, s1 = 0.f;
+#pragma unroll 8
+        for (int q = 0; q < kTB; ++q) {
+            const float x = sm[gX + q * kSX + k];
+            s0 = fmaf(sm[gD1 + q * kSQ + ig], x, s0);
+            s1 = fmaf(sm[gD1 + q * kSQ + ig + 1], x, s1);
+        }
+        out[oW1 + (u0 + ig) * kIn + k] = s0;
+        out[oW1 + (u0 + ig + 1) * kIn + k] = s1;
+    } else if (t < 224) {  // dW3 columns u0 .. u0 + kQ
+        const int o = (t - 192) / kQ, j = (t - 192) % kQ;
         float s = 0.f;
-        for (int q = 0; q < kTB; ++q) s += dy[2 * q + t];
+#pragma unroll 8
+        for (int q = 0; q < kTB; ++q) s = fmaf(sm[gDY + 2 * q + o], sm[gH2 + q * kSQ + j], s);
+        out[oW3 + o * kH + u0 + j] = s;
+    } else {  // db2, db1 of the kQ units
+        const int i = (t - 224) % kQ, which = (t - 224) / kQ;
+        const float* d = sm + (which ? gD1 : gD2) + i;
+        float s = 0.f;
+#pragma unroll 8
+        for (int q = 0; q < kTB; ++q) s += d[q * kSQ];
+        out[(which ? oB1 : oB2) + u0 + i] = s;
+    }
+    if (rank == 0 && t < kOut) {
+        float s = 0.f;
+        for (int q = 0; q < kTB; ++q) s += sm[gDY + 2 * q + t];
         out[oB3 + t] = s;
     }
-    // dW2, db2 (D2 and H1)
-    for (int e = t; e < kH * kH; e += kTB) {
-        const int i = e / kH, j = e % kH;
-        float s = 0.f;
-        for (int q = 0; q < kTB; ++q) s = fmaf(d2[q * kPad + i], h1[q * kPad + j], s);
-        out[oW2 + e] = s;
-    }
-    if (t < kH) {
-        float s = 0.f;
-        for (int q = 0; q < kTB; ++q) s += d2[q * kPad + t];
-        out[oB2 + t] = s;
-    }
-    __syncthreads();
-    // delta of layer 1 pre-activations, into H2's rows (H2 no longer needed)
-    float* d1 = h2;
-    for (int j = 0; j < kH; ++j) {
-        float g = 0.f;
-        for (int i = 0; i < kH; ++i) g = fmaf(w[oW2 + i * kH + j], d2[t * kPad + i], g);
-        d1[t * kPad + j] = h1[t * kPad + j] > 0.f ? g : 0.f;
-    }
-    __syncthreads();
-    // dW1, db1 (D1 and X)
-    for (int e = t; e < kH * kIn; e += kTB) {
-        const int i = e / kIn, k = e % kIn;
-        float s = 0.f;
-        for (int q = 0; q < kTB; ++q) s = fmaf(d1[q * kPad + i], sx[q * kIn + k], s);
-        out[oW1 + e] = s;
-    }
-    if (t < kH) {
-        float s = 0.f;
-        for (int q = 0; q < kTB; ++q) s += d1[q * kPad + t];
-        out[oB1 + t] = s;
-    }
 }
 
-// grad[i] = sum over blocks (in block order) of the partials
+struct AdamStep { float lr, b1, b2, eps, c1, c2; };
+// grad[i] = sum over clusters (in order) of the partials; with kAdam the update of the FP32 master
+// weights (Adam, Kingma and Ba, 2015) and their BF16 copy follows.  loss: the samples' sum, each
+// cluster's four tiles in order, then the clusters; added to *loss with kAdam, else stored there.
+template <bool kAdam>
 __global__ void k_reduce_grad(const float* __restrict__ partials, int nBlocks, float* __restrict__ grad,
-                              const double* __restrict__ lossPartials, double* __restrict__ loss) {
+                              const double* __restrict__ lossPartials, double* __restrict__ loss, float* __restrict__ w,
+                              float* __restrict__ m, float* __restrict__ v, __nv_bfloat16* __restrict__ wb, AdamStep A) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < kParams) {
-        float s = 0.f;
-        for (int b = 0; b < nBlocks; ++b) s += partials[(long)b * kParams + i];
-        grad[i] = s;
-    }
-    if (i == 0 && loss) {
+        float gi = 0.f;
+#pragma unroll 8
+        for (int b = 0; b < nBlocks; ++b) gi += partials[(long)b * kParams + i];
+        grad[i] = gi;
+        if (kAdam) {
+            const float mi = A.b1 * m[i] + (1.f - A.b1) * gi;
+            const float vi = A.b2 * v[i] + (1.f - A.b2) * gi * gi;
+            m[i] = mi;
+            v[i] = vi;
+            const float wi = w[i] - A.lr * (mi / A.c1) / (sqrtf(vi / A.c2) + A.eps);
+            w[i] = wi;
+            wb[i] = __float2bfloat16_rn(wi);
+        }
+    } else if (i == kParams) {
         double l = 0.0;
-        for (int b = 0; b < nBlocks; ++b) l += lossPartials[b];
-        *loss = l;
+#pragma unroll 4
+        for (int b = 0; b < nBlocks; ++b) {
+            double lb = 0.0;
+            for (int q = 0; q < kTC; ++q) lb += lossPartials[b * kTC + q];
+            l += lb;
+        }
+        *loss = kAdam ? *loss + l : l;
     }
-}
-
-// Adam (Kingma and Ba, 2015) on the FP32 master weights, then the BF16 copy.
-__global__ void k_adam(float* __restrict__ w, float* __restrict__ m, float* __restrict__ v,
-                       const float* __restrict__ g, __nv_bfloat16* __restrict__ wb, float lr, float b1, float b2,
-                       float eps, float c1, float c2) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kParams) return;
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.f - b1) * gi;
-    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    w[i] = wi;
-    wb[i] = __float2bfloat16_rn(wi);
 }
 
 __global__ void k_to_bf16(const float* __restrict__ w, __nv_bfloat16* __restrict__ wb) {
@@ -255,37 +370,73 @@ __global__ void k_to_bf16(const float* __restrict__ w, __nv_bfloat16* __restrict
     if (i < kParams) wb[i] = __float2bfloat16_rn(w[i]);
 }
 
-__global__ void k_predict(const __nv_bfloat16* __restrict__ wb, const float* __restrict__ X, int n,
-                          float* __restrict__ Y) {
-    __shared__ float w[kParams];
-    load_weights(wb, w);
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float x[kIn], y[kOut];
-    for (int k = 0; k < kIn; ++k) x[k] = X[(long)i * kIn + k];
-    forward1(w, x, y, nullptr, nullptr);
-    Y[2L * i] = y[0];
-    Y[2L * i + 1] = y[1];
+// Dynamic shared memory of the inference kernels: the weights, x[kSamples] rows, h1, h2 of one tile.
+constexpr size_t infer_floats(int samples) { return kWeights + (size_t)samples * kSX + 2 * kTS * kSH; }
+
+// Outputs of n samples, a tile at a time per block.
+__global__ void __launch_bounds__(kTT) k_predict(const __nv_bfloat16* __restrict__ wb, const float* __restrict__ X,
+                                                 int n, float* __restrict__ Y) {
+    extern __shared__ float4 smem4[];
+    float* sm = reinterpret_cast<float*>(smem4);
+    float *x = sm + kWeights, *h1 = x + kTS * kSX, *h2 = h1 + kTS * kSH;
+    load_weights(wb, sm);
+    for (int base = blockIdx.x * kTS; base < n; base += gridDim.x * kTS) {
+        const int live = min(kTS, n - base);
+        __syncthreads();  // (the weights; the previous tile's x)
+        for (int e = threadIdx.x; e < kTS * kIn; e += kTT) {
+            const int s = e / kIn, k = e - s * kIn;
+            x[s * kSX + k] = s < live ? X[(long)base * kIn + e] : 0.f;
+        }
+        __syncthreads();
+        float a1[4][2], a2[4][2];
+        const float y = tile_forward(sm, x, h1, h2, live, a1, a2);
+        if (threadIdx.x < 2 * live) Y[2L * base + threadIdx.x] = y;
+    }
 }
 
-// Fused inference: features of the current state, the network, and the move of every vertex by
-// scale * (y0 e1 + y1 e2) onto the sphere (sphericalDomain::move), written to the other buffer.
-__global__ void k_warm_start(const __nv_bfloat16* __restrict__ wb, FeatArgs A, int nV, double scale, double R,
-                             double4_32a* __restrict__ posOut) {
-    __shared__ float w[kParams];
-    load_weights(wb, w);
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= nV) return;
-    float x[kIn], y[kOut];
+// Fused inference: features of the current state (a thread per vertex), the network (kTT / kTS tiles),
+// and the move of every vertex by scale * (y0 e1 + y1 e2) onto the sphere (sphericalDomain::move),
+// written to the other buffer.
+__global__ void __launch_bounds__(kTT) k_warm_start(const __nv_bfloat16* __restrict__ wb, FeatArgs A, int nV, double scale,
+                                                    double R, double4_32a* __restrict__ posOut) {
+    extern __shared__ float4 smem4[];
+    float* sm = reinterpret_cast<float*>(smem4);
+    float *x = sm + kWeights, *h1 = x + kTT * kSX, *h2 = h1 + kTS * kSH;
+    __shared__ float ySh[2 * kTT];
+    load_weights(wb, sm);
+    const int v = blockIdx.x * kTT + threadIdx.x;
     D3 e1, e2, p;
-    vertex_features(A, v, x, e1, e2, p);
-    forward1(w, x, y, nullptr, nullptr);
-    const D3 d = add3(scl3(scale * y[0], e1), scl3(scale * y[1], e2));
+    float f[kIn] = {};
+    if (v < nV) vertex_features(A, v, f, e1, e2, p);
+#pragma unroll
+    for (int k = 0; k < kIn; ++k) x[threadIdx.x * kSX + k] = f[k];
+    const int live = min(kTT, nV - (int)blockIdx.x * kTT);
+    for (int base = 0; base < live; base += kTS) {
+        __syncthreads();
+        float a1[4][2], a2[4][2];
+        const float y = tile_forward(sm, x + base * kSX, h1, h2, min(kTS, live - base), a1, a2);
+        if (threadIdx.x < 2 * kTS) ySh[2 * base + threadIdx.x] = y;
+    }
+    __syncthreads();
+    if (v >= nV) return;
+    const float y0 = ySh[2 * threadIdx.x], y1 = ySh[2 * threadIdx.x + 1];
+    const D3 d = add3(scl3(scale * y0, e1), scl3(scale * y1, e2));
     st3(posOut, v, sphere_move(p, d, R));
 }
 
-size_t train_smem() {
-    return sizeof(float) * (kParams + kTB * kIn + 3 * kTB * kPad + 2 * kTB);
+// The kernels' dynamic shared memory, above the default 48 KB: opted in once per device.
+int mlp_opt_in() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return SVM_ERR_CUDA;
+    static std::once_flag once[64];
+    static cudaError_t err[64];
+    std::call_once(once[dev], [&] {
+        const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+        err[dev] = cudaFuncSetAttribute(k_train_block, a, (int)(kTrainFloats * sizeof(float)));
+        if (err[dev] == cudaSuccess) err[dev] = cudaFuncSetAttribute(k_predict, a, (int)(infer_floats(kTS) * sizeof(float)));
+        if (err[dev] == cudaSuccess) err[dev] = cudaFuncSetAttribute(k_warm_start, a, (int)(infer_floats(kTT) * sizeof(float)));
+    });
+    return err[dev] == cudaSuccess ? SVM_OK : SVM_ERR_CUDA;
 }
 
 }  // namespace
@@ -312,31 +463,30 @@ static int mlp_reserve(svm_mlp* M, int blocks) {
     if (M->lossPartials) cudaFree(M->lossPartials);
     M->partials = nullptr; M->lossPartials = nullptr;
     if (cudaMalloc(&M->partials, sizeof(float) * (size_t)blocks * kParams) != cudaSuccess ||
-        cudaMalloc(&M->lossPartials, sizeof(double) * blocks) != cudaSuccess)
+        cudaMalloc(&M->lossPartials, sizeof(double) * kTC * blocks) != cudaSuccess)
         return SVM_ERR_CUDA;
     M->maxBlocks = blocks;
     return SVM_OK;
 }
 
-// forward + backward over samples [first, first + count) of `order` (or of X directly); gradient
-// of sum (y - t)^2 * invBatch into M->g, loss sum into M->loss
+// forward + backward over samples [first, first + count) of `order` (or of X directly): the gradient
+// of sum (y - t)^2 * invBatch into M->g and the loss sum into M->loss, or, with an Adam step, the
+// step taken and the loss added to M->loss
 static int mlp_grad(svm_mlp* M, const float* X, const float* Y, const int* order, int first, int count,
-                    float invBatch) {
+                    float invBatch, const AdamStep* adam) {
     const int blocks = (count + kTB - 1) / kTB;
     int rc = mlp_reserve(M, blocks);
-    if (rc) return rc;
-    // the training kernel's shared memory exceeds the default 48 KB: opt in (per device)
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return SVM_ERR_CUDA;
-    static std::once_flag once[64];
-    static cudaError_t attrErr[64];
-    std::call_once(once[dev], [&] {
-        attrErr[dev] = cudaFuncSetAttribute(k_train_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)train_smem());
-    });
-    if (attrErr[dev] != cudaSuccess) return SVM_ERR_CUDA;
-    k_train_block<<<blocks, kTB, train_smem(), M->stream>>>(M->wb, X, Y, order, first, count, invBatch, M->partials,
-                                                          M->lossPartials);
-    k_reduce_grad<<<(kParams + 255) / 256, 256, 0, M->stream>>>(M->partials, blocks, M->g, M->lossPartials, M->loss);
+    if (rc || (rc = mlp_opt_in())) return rc;
+    k_train_block<<<kTC * blocks, kTT, kTrainFloats * sizeof(float), M->stream>>>(M->wb, X, Y, order, first, count, invBatch,
+                                                                               M->partials, M->lossPartials);
+    // 64-thread blocks: the sums are chains over the partials, and 93 blocks reach most SMs
+    const int nb = kParams / 64 + 1;
+    if (adam)
+        k_reduce_grad<true><<<nb, 64, 0, M->stream>>>(M->partials, blocks, M->g, M->lossPartials, M->loss, M->w, M->m, M->v,
+                                                      M->wb, *adam);
+    else
+        k_reduce_grad<false><<<nb, 64, 0, M->stream>>>(M->partials, blocks, M->g, M->lossPartials, M->loss, nullptr, nullptr,
+                                                       nullptr, nullptr, AdamStep{});
     return check_launch();
 }
 
@@ -427,7 +577,7 @@ int svm_mlp_features(svm_model* m, float* X, double* frames) {
 
 int svm_mlp_gradient(svm_mlp* M, const float* X, const float* Y, int n, float* grad, double* loss) {
     if (!M || !X || !Y || n <= 0 || !grad) return SVM_ERR_ARG;
-    int rc = mlp_grad(M, X, Y, nullptr, 0, n, 1.f / n);
+    int rc = mlp_grad(M, X, Y, nullptr, 0, n, 1.f / n, nullptr);
     if (rc) return rc;
     if (cudaMemcpyAsync(grad, M->g, sizeof(float) * kParams, cudaMemcpyDeviceToHost, M->stream) != cudaSuccess)
         return SVM_ERR_CUDA;
@@ -439,35 +589,32 @@ int svm_mlp_gradient(svm_mlp* M, const float* X, const float* Y, int n, float* g
     return SVM_OK;
 }
 
-int svm_mlp_train(svm_mlp* M, const float* X, const float* Y, const int* order, int n, int batch, float lr,
+int svm_mlp_train(svm_mlp* M, const float* X, const float* Y, const int* order, int n, int batch, float learningRate,
                   double* meanLoss) {
     if (!M || !X || !Y || !order || n <= 0 || batch <= 0) return SVM_ERR_ARG;
-    double total = 0.0;
+    if (cudaMemsetAsync(M->loss, 0, sizeof(double), M->stream) != cudaSuccess) return SVM_ERR_CUDA;
     for (int first = 0; first < n; first += batch) {
         const int count = std::min(batch, n - first);
-        int rc = mlp_grad(M, X, Y, order, first, count, 1.f / count);
-        if (rc) return rc;
         M->adamStep++;
-        const float c1 = 1.f - std::pow(M->beta1, (float)M->adamStep);
-        const float c2 = 1.f - std::pow(M->beta2, (float)M->adamStep);
-        k_adam<<<(kParams + 255) / 256, 256, 0, M->stream>>>(M->w, M->m, M->v, M->g, M->wb, lr, M->beta1, M->beta2,
-                                                            M->eps, c1, c2);
-        if (check_launch()) return SVM_ERR_CUDA;
-        if (meanLoss) {
-            double l = 0.0;
-            if (cudaMemcpyAsync(&l, M->loss, sizeof(double), cudaMemcpyDeviceToHost, M->stream) != cudaSuccess ||
-                cudaStreamSynchronize(M->stream) != cudaSuccess)
-                return SVM_ERR_CUDA;
-            total += l;
-        }
+        AdamStep A{learningRate, M->beta1, M->beta2, M->eps, 0.f, 0.f};
+        A.c1 = 1.f - std::pow(M->beta1, (float)M->adamStep);
+        A.c2 = 1.f - std::pow(M->beta2, (float)M->adamStep);
+        if (int rc = mlp_grad(M, X, Y, order, first, count, 1.f / count, &A)) return rc;
     }
+    double total = 0.0;
+    if (meanLoss && cudaMemcpyAsync(&total, M->loss, sizeof(double), cudaMemcpyDeviceToHost, M->stream) != cudaSuccess)
+        return SVM_ERR_CUDA;
+    if (cudaStreamSynchronize(M->stream) != cudaSuccess) return SVM_ERR_CUDA;
     if (meanLoss) *meanLoss = total / n;
-    return cudaStreamSynchronize(M->stream) == cudaSuccess ? SVM_OK : SVM_ERR_CUDA;
+    return SVM_OK;
 }
 
 int svm_mlp_predict(svm_mlp* M, const float* X, int n, float* Y) {
     if (!M || !X || !Y || n <= 0) return SVM_ERR_ARG;
-    k_predict<<<(n + 255) / 256, 256, 0, M->stream>>>(M->wb, X, n, Y);
+    if (int rc = mlp_opt_in()) return rc;
+    // four resident blocks per SM (47 KB of shared memory each), each over several tiles at large n
+    const int tiles = (n + kTS - 1) / kTS;
+    k_predict<<<std::min(tiles, 4 * 152), kTT, infer_floats(kTS) * sizeof(float), M->stream>>>(M->wb, X, n, Y);
     if (check_launch()) return SVM_ERR_CUDA;
     return cudaStreamSynchronize(M->stream) == cudaSuccess ? SVM_OK : SVM_ERR_CUDA;
 }
@@ -479,8 +626,9 @@ int svm_mlp_warm_start(svm_mlp* M, svm_model* m) {
     int rc = svm_model_compute_forces(m);
     if (rc) return rc;
     const int nxt = 1 - m->cur;
-    k_warm_start<<<(m->nVertices + 255) / 256, 256, 0, m->stream>>>(M->wb, feat_args(m), m->nVertices, M->outScale,
-                                                                    m->R, m->pos[nxt]);
+    if ((rc = mlp_opt_in())) return rc;
+    k_warm_start<<<(m->nVertices + kTT - 1) / kTT, kTT, infer_floats(kTT) * sizeof(float), m->stream>>>(
+        M->wb, feat_args(m), m->nVertices, M->outScale, m->R, m->pos[nxt]);
     if (check_launch()) return SVM_ERR_CUDA;
     m->cur = nxt;
     m->cornersValid = false;
