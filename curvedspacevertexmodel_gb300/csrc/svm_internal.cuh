@@ -406,22 +406,25 @@ struct UndoEntry {
 // Counters of one parallel T1 pass: in shared memory for a single-block pass, in global memory
 // (T1Scratch::ctl) for a pass spread over a cooperative grid, with the grid barrier's words.
 struct T1Ctl {
-    int nCur, flag, nWordsHit, undo, late, rollback, exec, flips, next[2];
+    int undo, late, rollback, exec, flips, next[2];
     unsigned barCount, barGen;
 };
 constexpr int kT1CtlInts = sizeof(T1Ctl) / sizeof(int);
 
 struct T1Scratch {
     unsigned* bits = nullptr;      // one bit per (vertex, slot) position, 3*Nv bits
-    unsigned* summary = nullptr;   // one bit per word of `bits`
-    int* count = nullptr;          // number of candidate positions found by the test
+    unsigned* summary = nullptr;   // one bit per word of `bits`: set only for k_t1_apply's replay
+    int* count = nullptr;          // positions a rolled-back segment left to k_t1_apply
+    int* segCount = nullptr;       // per segment (the sphere, or each replica): positions the test flagged
+    const int* segOff = nullptr;   // first vertex of each segment [segments + 1] (null: one sphere)
+    int listPad = 0;               // list slack per segment
     int* flipLog = nullptr;        // (pass, position, v1, v2) per flip, capacity flipLogCap
     int* flipCount = nullptr;
     int* pass = nullptr;           // T1 passes so far (orders the flip log across passes)
-    int* touched = nullptr;        // cells whose rings changed during the apply kernel
+    int* touched = nullptr;        // cells whose rings changed (batches, and k_t1_apply's replay)
     int nWords = 0, nSummary = 0, flipLogCap = 0, touchedCap = 0;
     // parallel pass (deterministic reservations), capacity `cap` pending positions
-    int* listA = nullptr;          // pending positions of this round
+    int* listA = nullptr;          // pending positions of this round (the first: as the test flags them)
     int* listB = nullptr;          // pending positions of the next round
     int* listOrig = nullptr;       // the candidates as flagged by the test (for a rollback)
     int* fp = nullptr;             // footprint of each pending position, kFootprint ints
@@ -442,6 +445,34 @@ constexpr int kFootprint = 14;     // 8 vertex slots + 6 cell slots (duplicates 
 constexpr int kListPad = 1024;     // list slack of a single-sphere parallel pass
 constexpr int kListPadBatch = 64;  // list slack per replica of a batch's parallel pass
 constexpr int kResFree = 0x7f7f7f7f;
+
+#ifdef __CUDACC__
+// Footprint of the edge (v1, v2): every vertex and cell that testing, flipping and re-testing after
+// the flip can read or write (v1, v2 and their neighbours; the cells of v1 and v2).  Two positions
+// with disjoint footprints commute.
+__device__ __forceinline__ void t1_footprint(int v1, int v2, const int4& n1, const int4& n2, const int4& c1, const int4& c2,
+                                             int* f) {
+    f[0] = v1; f[1] = v2; f[2] = n1.x; f[3] = n1.y; f[4] = n1.z; f[5] = n2.x; f[6] = n2.y; f[7] = n2.z;
+    f[8] = c1.x; f[9] = c1.y; f[10] = c1.z; f[11] = c2.x; f[12] = c2.y; f[13] = c2.z;
+}
+// The T1 test's record of a short edge (position p = 3 v + slot, neighbour u, replica seg): its flag, its
+// place in the pass's first list, its footprint, and its reservation of it -- so that the pass starts
+// with its first round's reservations made.  Short edges are a few in ten thousand.
+inline __device__ __noinline__ void t1_flag(const T1Scratch& t1, int p, int v, int u, int seg, const int4* __restrict__ vnbr,
+                                     const int4* __restrict__ vcell) {
+    atomicOr(&t1.bits[p >> 5], 1u << (p & 31));
+    const int lo = t1.segOff ? 3 * t1.segOff[seg] : 0;
+    const int i = atomicAdd(t1.segCount + seg, 1);
+    const int at = lo / 2 + t1.listPad * seg + i;
+    // (a segment's slice holds one position per edge and more: the bounds only guard a broken state)
+    if (at >= t1.cap || (t1.segOff && i >= 3 * (t1.segOff[seg + 1] - t1.segOff[seg]) / 2 + t1.listPad)) return;
+    t1.listA[at] = p;
+    int* f = t1.fp + (long)at * kFootprint;
+    t1_footprint(v, u, vnbr[v], vnbr[u], vcell[v], vcell[u], f);
+    for (int k = 0; k < 8; ++k) atomicMin(t1.resV + f[k], p);
+    for (int k = 8; k < kFootprint; ++k) atomicMin(t1.resC + f[k], p);
+}
+#endif
 
 }  // namespace svm
 

@@ -168,10 +168,7 @@ __global__ void k32_corners(const float4* __restrict__ pos, const int4* __restri
         for (int s = 0; s < 3; ++s) {
             const int u = comp(nb, s);
             if (v < u && arc[s] < t1Threshold) {
-                const int q = 3 * v + s;
-                atomicOr(&t1.bits[q >> 5], 1u << (q & 31));
-                atomicOr(&t1.summary[q >> 10], 1u << ((q >> 5) & 31));
-                atomicAdd(t1.count, 1);
+                t1_flag(t1, 3 * v + s, v, u, rep_of(p), vnbr, vcell);
             }
         }
     }

@@ -135,7 +135,7 @@ __device__ __forceinline__ int nth_set(unsigned m, int n) {
 // warp's owned edges (about half of its 96 slots) are compacted over its lanes first, so that the
 // FP64 work runs on full warps.
 __global__ void k_edges(const double4_32a* __restrict__ pos, const double* __restrict__ vnorm,
-                        double4_32a* __restrict__ vsph, const int4* __restrict__ vnbr,
+                        double4_32a* __restrict__ vsph, const int4* __restrict__ vnbr, const int4* __restrict__ vcell,
                         double4_32a* __restrict__ edgeC, double* __restrict__ edgeArc, int nV, double R, int t1test,
                         double t1Threshold, T1Scratch t1) {
     const int v = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
@@ -163,11 +163,7 @@ __global__ void k_edges(const double4_32a* __restrict__ pos, const double* __res
         edgeC[e] = make_double4_32a(C.x, C.y, C.z, f64_sqrt(dot3e(C, C)));
         edgeArc[e] = arc;
         // geodesic(u, p) < t is the reference's test (sphericalVertexModel.cpp:475)
-        if (t1test && arc < t1Threshold) {
-            atomicOr(&t1.bits[e >> 5], 1u << (e & 31));
-            atomicOr(&t1.summary[e >> 10], 1u << ((e >> 5) & 31));
-            atomicAdd(t1.count, 1);
-        }
+        if (t1test && arc < t1Threshold) t1_flag(t1, e, w, u, 0, vnbr, vcell);
     }
 }
 
@@ -463,8 +459,8 @@ __global__ void k_move(double4_32a* __restrict__ pos, const double* __restrict__
 
 // Standalone T1 edge test (gpu_vm_test_edges_for_T1, sphericalVertexModel.cu:225-273).
 __global__ void k_t1_test(const double4_32a* __restrict__ pos, const float4* __restrict__ pos32,
-                          const double* __restrict__ repR, const int4* __restrict__ vnbr, int nV, double R,
-                          double t1Threshold, double cosLo, double cosHi, double s2Lo, double s2Hi, T1Scratch t1) {
+                          const double* __restrict__ repR, const int4* __restrict__ vnbr,
+                          const int4* __restrict__ vcell, int nV, double R, double t1Threshold, double cosLo, double cosHi, double s2Lo, double s2Hi, T1Scratch t1) {
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nV) return;
     const int4 nb = vnbr[v];
@@ -474,12 +470,7 @@ __global__ void k_t1_test(const double4_32a* __restrict__ pos, const float4* __r
         if (!(v < u)) continue;
         const bool shortEdge = pos32 ? arc32(pos32[v], pos32[u], (float)repR[rep_of(pos32[v])]) < (float)t1Threshold
                                      : shorter_than<true>(ld3(pos, v), ld3(pos, u), R, t1Threshold, cosLo, cosHi, s2Lo, s2Hi);
-        if (shortEdge) {
-            const int q = 3 * v + s;
-            atomicOr(&t1.bits[q >> 5], 1u << (q & 31));
-            atomicOr(&t1.summary[q >> 10], 1u << ((q >> 5) & 31));
-            atomicAdd(t1.count, 1);
-        }
+        if (shortEdge) t1_flag(t1, 3 * v + s, v, u, pos32 ? rep_of(pos32[v]) : 0, vnbr, vcell);
     }
 }
 
@@ -853,16 +844,86 @@ __device__ __forceinline__ int4 shfl0(int4 a) {
     return make_int4(__shfl_sync(kFull, a.x, 0), __shfl_sync(kFull, a.y, 0), __shfl_sync(kFull, a.z, 0),
                      __shfl_sync(kFull, a.w, 0));
 }
-// t1_flip by a whole warp (every lane calls it with the same arguments; p1, p2 are the old
-// positions of v1 and v2): lane 0 plans and commits the topology, the warp moves the pair.  Same
-// writes as t1_flip; the warp's lanes see them after it returns.
-__device__ bool t1_flip_warp(const ApplyArgs& A, int v1, int v2, int4& cs, int4& vs, UndoEntry* undo, int* undoRings,
-                             D3 p1, D3 p2, int lane) {
-    int ok = 0;
-    FlipPlan16 F;
-    if (ring16_ok(A) && lane == 0) ok = t1_plan16(A, v1, v2, cs, vs, F);
-    ok = ring16_ok(A) ? __shfl_sync(kFull, ok, 0) : 2;
-    if (ok == 2) {  // other ring capacities, or rings of more than 16 entries: lane 0 alone
+// The rings of a flip as a warp holds them, entry l % 16 of two rings per lane l: `a` of v1's cells c[0]
+// (lanes 0-15) and c[1] (16-31), `b` of c[2] and of v2's fourth cell, with their counts.
+struct WarpRings { int a, b, na, nb; };
+__device__ __forceinline__ WarpRings warp_rings_load(const ApplyArgs& A, const int c[3], int cw, int lane) {
+    const int k = lane & 15, ca = lane < 16 ? c[0] : c[1], cb = lane < 16 ? c[2] : (cw >= 0 ? cw : c[2]);
+    const bool in = k < A.Wc;   // (capacities below 16 take the general path)
+    return WarpRings{in ? A.ring[(long)ca * A.Wc + k] : -1, in ? A.ring[(long)cb * A.Wc + k] : -1, A.ringCount[ca],
+                     A.ringCount[cb]};
+}
+// ring16_neighbours on the ring in the half `h` of r (count n): the entries before and after `target`
+// (of repeated entries the last of the ring first, then the lowest; none found: the ring's end).
+__device__ __forceinline__ void warp_ring_neighbours(int r, int n, int h, int target, int lane, int& vl, int& vx) {
+    const unsigned m = (__ballot_sync(kFull, (lane >> 4) == h && (lane & 15) < n && r == target) >> (16 * h)) & 0xffffu;
+    int il, ix;
+    if (!m) { il = n - 2; ix = n - 1; }
+    else {
+        const int k = (m >> (n - 1)) & 1u ? n - 1 : __ffs(m) - 1;
+        il = k == 0 ? n - 1 : k - 1;
+        ix = k + 1 == n ? 0 : k + 1;
+    }
+    vl = __shfl_sync(kFull, r, 16 * h + il);
+    vx = __shfl_sync(kFull, r, 16 * h + ix);
+}
+// ring16_remove(target) or ring16_insert_after(target, added) on the half-warp's ring r of n entries.
+__device__ __forceinline__ int warp_ring_edit(int r, int n, bool remove, int target, int added, int lane) {
+    const int k = lane & 15;
+    const unsigned m = (__ballot_sync(kFull, k < n && r == target) >> (lane & 16)) & 0xffffu;
+    const int after = __shfl_down_sync(kFull, r, 1, 16), before = __shfl_up_sync(kFull, r, 1, 16);
+    const int at = m ? __ffs(m) - 1 : n;
+    if (remove) return k >= at && k < n - 1 ? after : r;
+    return k <= at ? r : (k == at + 1 ? added : (k <= n ? before : r));
+}
+// t1_flip by a whole warp (every lane calls it with the same arguments): f, the edge's footprint (lane k
+// holds entry k); W, its rings, loaded by the caller alongside the positions p1, p2 of v1 and v2.  The
+// rings are searched, edited and stored 16 lanes each, so a flip waits for memory twice after its
+// loads (the outer neighbours; the re-test), and its serial work is the pair's rotation.  Same writes
+// as t1_flip; the warp's lanes see them after it returns.
+__device__ bool t1_flip_warp(const ApplyArgs& A, int f, const WarpRings& W, int4& cs, int4& vs, UndoEntry* undo,
+                             int* undoRings, D3 p1, D3 p2, int lane) {
+    const int v1 = __shfl_sync(kFull, f, 0), v2 = __shfl_sync(kFull, f, 1);
+    int4 n1 = make_int4(__shfl_sync(kFull, f, 2), __shfl_sync(kFull, f, 3), __shfl_sync(kFull, f, 4), -1);
+    int4 n2 = make_int4(__shfl_sync(kFull, f, 5), __shfl_sync(kFull, f, 6), __shfl_sync(kFull, f, 7), -1);
+    int4 c1 = make_int4(__shfl_sync(kFull, f, 8), __shfl_sync(kFull, f, 9), __shfl_sync(kFull, f, 10), -1);
+    int4 c2 = make_int4(__shfl_sync(kFull, f, 11), __shfl_sync(kFull, f, 12), __shfl_sync(kFull, f, 13), -1);
+    cs = make_int4(-1, -1, -1, -1);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const int t = comp(c2, q);
+        if (t != c1.x && t != c1.y && t != c1.z) cs.w = t;
+    }
+    // counts of the four rings: c1.x, c1.y, c1.z, cs.w
+    const int cnt[4] = {__shfl_sync(kFull, W.na, 0), __shfl_sync(kFull, W.na, 16), __shfl_sync(kFull, W.nb, 0),
+                        __shfl_sync(kFull, W.nb, 16)};
+    bool general = !ring16_ok(A) || cnt[0] > 16 || cnt[1] > 16 || cnt[2] > 16 || (cs.w >= 0 && cnt[3] > 16);
+    int qx = 0, qy = 0, qz = 0, ok = 0;
+    vs = make_int4(-1, -1, -1, -1);
+    if (!general) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            int vl, vx;
+            warp_ring_neighbours(q < 2 ? W.a : W.b, cnt[q], q & 1, v1, lane, vl, vx);
+            const int c = comp(c1, q);
+            if (vl == v2) { cs.x = c; qx = q; }
+            else if (vx == v2) { cs.z = c; qz = q; }
+            else { cs.y = c; qy = q; vs.x = vl; vs.y = vx; }
+        }
+        if (cs.x < 0 || cs.y < 0 || cs.z < 0 || cs.w < 0) {
+            if (lane == 0) atomicOr(A.status, SVM_DEV_BAD_TOPOLOGY);
+            return false;
+        }
+        int vl, vx;
+        warp_ring_neighbours(W.b, cnt[3], 1, v2, lane, vl, vx);
+        vs.w = vl; vs.z = vx;
+        const int nx = qx == 0 ? cnt[0] : (qx == 1 ? cnt[1] : cnt[2]), nz = qz == 0 ? cnt[0] : (qz == 1 ? cnt[1] : cnt[2]);
+        const int ny = qy == 0 ? cnt[0] : (qy == 1 ? cnt[1] : cnt[2]);
+        // forbid a T1 that would shrink a triangular cell (sphericalVertexModel.cpp:485-487)
+        if (nx == 3 || nz == 3) return false;
+        general = ny + 1 > 16 || cnt[3] + 1 > 16;
+    }
+    if (general) {  // other ring capacities, or rings of more than 16 entries: lane 0 alone
         if (lane == 0) ok = t1_flip_any(A, v1, v2, cs, vs, undo, undoRings) ? 1 : 0;
         ok = __shfl_sync(kFull, ok, 0);
         cs = shfl0(cs);
@@ -870,47 +931,73 @@ __device__ bool t1_flip_warp(const ApplyArgs& A, int v1, int v2, int4& cs, int4&
         __syncwarp();
         return ok != 0;
     }
-    if (!ok) return false;
-    cs = shfl0(cs);
-    vs = shfl0(vs);
-    t1_move_pair_warp(A, v1, v2, p1, p2, apos(A, vs.z), lane);
-    if (lane == 0) t1_commit16(A, v1, v2, cs, vs, F, undo, undoRings, p1, p2);
+    int4 ny = A.vnbr[vs.y], nz = A.vnbr[vs.z];
+    const D3 pC = apos(A, vs.z);
+    // the edited rings, 16 lanes each (slots 0-2: v1's cells; 3: cs.w)
+    const int sa = lane >> 4, sb = 2 + (lane >> 4);
+    const bool ra = sa == qx || sa == qz, rb = sb != 3 && (sb == qx || sb == qz);
+    const int ea = warp_ring_edit(W.a, W.na, ra, sa == qx ? v2 : v1, v2, lane);
+    const int eb = warp_ring_edit(W.b, W.nb, rb, sb == 3 || sb == qx ? v2 : v1, sb == 3 ? v1 : v2, lane);
+    const int ma = W.na + (ra ? -1 : 1), mb = W.nb + (rb ? -1 : 1);
+    const int ca = sa == 0 ? c1.x : c1.y, cb = sb == 2 ? c1.z : cs.w, k16 = lane & 15;
+    if (undo) {
+        // (the undo entry lists its cells as cs does)
+        const int ua = sa == qx ? 0 : (sa == qy ? 1 : 2), ub = sb == 3 ? 3 : (sb == qx ? 0 : (sb == qy ? 1 : 2));
+        undoRings[ua * A.Wc + k16] = W.a;
+        undoRings[ub * A.Wc + k16] = W.b;
+        if (k16 == 0) {
+            undo->cells[ua] = ca; undo->counts[ua] = W.na;
+            undo->cells[ub] = cb; undo->counts[ub] = W.nb;
+        }
+        if (lane == 1) {
+            undo->v1 = v1; undo->v2 = v2; undo->b = vs.y; undo->c = vs.z;
+            undo->p1 = make_double4_32a(p1.x, p1.y, p1.z, 0.0); undo->p2 = make_double4_32a(p2.x, p2.y, p2.z, 0.0);
+        }
+        if (lane == 2) {
+            undo->vc1 = c1; undo->vc2 = c2;
+            undo->vn[0] = n1; undo->vn[1] = n2; undo->vn[2] = ny; undo->vn[3] = nz;
+        }
+    }
+    __syncwarp();   // (every lane has read the outer neighbours' lists and positions)
+    A.ring[(long)ca * A.Wc + k16] = ea;
+    A.ring[(long)cb * A.Wc + k16] = eb;
+    if (k16 == 0) { A.ringCount[ca] = ma; A.ringCount[cb] = mb; }
+    // the slot rewiring of t1_flip_positions, slot by slot in the same order (for a shared outer
+    // neighbour both of its replacements apply, the first one first)
+    const bool yz = vs.y == vs.z;
+    slots_replace(c1, cs.z, cs.w);
+    slots_replace(c2, cs.x, cs.y);
+    slots_replace(ny, v1, v2);
+    if (yz) slots_replace(ny, v2, v1);
+    else slots_replace(nz, v2, v1);
+    slots_replace(n1, vs.y, vs.z);
+    slots_replace(n2, vs.z, vs.y);
+    if (lane == 0) {
+        A.vcell[v1] = c1; A.vcell[v2] = c2; A.vnbr[v1] = n1; A.vnbr[v2] = n2; A.vnbr[vs.y] = ny;
+        if (!yz) A.vnbr[vs.z] = nz;
+        const int gy = qy == 0 ? cnt[0] : (qy == 1 ? cnt[1] : cnt[2]);
+        atomicMax(A.ringMax, max(gy, cnt[3]) + 1);
+    }
+    t1_move_pair_warp(A, v1, v2, p1, p2, pC, lane);
     __syncwarp();
     return true;
 }
 
 // Ring bookkeeping (vrpos/vlast/vnext) and corners of the cells whose rings a T1 pass changed,
-// and fresh spherical coordinates of their vertices.  Grid-stride over (touched cell, ring
-// position); every written value depends only on the final rings and positions, so duplicate
-// entries and concurrent writers of the same vertex agree.
-__global__ void k_t1_patch(ApplyArgs A, T1Scratch t1) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) {  // the pass's largest ring, for the host's capacity check
-        *(volatile int*)A.ringMaxOut = *(volatile int*)A.ringMax;
-        __threadfence_system();
-    }
-    // appends past the list's capacity roll the pass back; a pass cut short by an exhausted barrier
-    // wait may leave the counter above it, and only the stored entries are read
-    const int ntRaw = *(volatile int*)(t1.ctr + 5);
-    const int nt = min(ntRaw, t1.touchedCap);
-    const long gs = (long)gridDim.x * blockDim.x, g0 = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    // A host-buffer step's output: the force kernel wrote the moved positions; the flips moved
-    // vertices of the touched cells, whose ring entries below rewrite them.  A list that may have
-    // lost entries (full) rewrites every vertex instead.
-    const bool hostAll = A.hostOut && ntRaw > t1.touchedCap - 4;
-    if (hostAll)
-        for (long v = g0; v < A.nV; v += gs) {
-            const D3 p = ld3(A.pos, (int)v);
-            A.hostOut[3 * v] = p.x; A.hostOut[3 * v + 1] = p.y; A.hostOut[3 * v + 2] = p.z;
-        }
-    // The touched cells go round-robin over the blocks (cell i to block i mod gridDim, 32 of a
-    // block's at a time), and each block packs its cells' ring entries onto consecutive threads: the
-    // few hundred cells of a pass then spread over all SMs, with every lane of a busy warp on a real
-    // entry (a flat index over (cell, slot < capacity) leaves most lanes and most SMs idle).
+// and fresh spherical coordinates of their vertices, over (touched cell, ring position); every written
+// value depends only on the final rings and positions, so duplicate entries and concurrent writers of
+// the same vertex agree.
+// The cells are cellOf(i), i < count (-1: none), shared out round-robin over `blocks` blocks (cell i to
+// block i mod blocks, 32 of a block's at a time), and each block packs its cells' ring entries onto
+// consecutive threads: the few hundred cells of a pass then spread over many SMs, with every lane of a
+// busy warp on a real entry.  Every thread of the block calls it.
+template <class CellOf>
+__device__ __forceinline__ void patch_cells(const ApplyArgs& A, int count, int block, int blocks, bool hostOut, CellOf cellOf) {
     __shared__ int patchCell[32], patchOff[33];
-    for (int base = blockIdx.x; base < nt; base += 32 * gridDim.x) {
+    for (int base = block; base < count; base += 32 * blocks) {
         if (threadIdx.x < 32) {
-            const int i = base + (int)gridDim.x * (int)threadIdx.x;
-            const int cell = i < nt ? t1.touched[i] : -1;
+            const int i = base + blocks * (int)threadIdx.x;
+            const int cell = i < count ? cellOf(i) : -1;
             const int cnt = cell >= 0 ? A.ringCount[cell] : 0;
             int incl = cnt;
             for (int o = 1; o < 32; o <<= 1) {
@@ -937,7 +1024,7 @@ __global__ void k_t1_patch(ApplyArgs A, T1Scratch t1) {
                     compRef(A.vnext, u, s) = next;
                 }
             const D3 pl = apos(A, last), p = apos(A, u), px = apos(A, next);
-            if (A.hostOut && !hostAll) { A.hostOut[3L * u] = p.x; A.hostOut[3L * u + 1] = p.y; A.hostOut[3L * u + 2] = p.z; }
+            if (hostOut) { A.hostOut[3L * u] = p.x; A.hostOut[3L * u + 1] = p.y; A.hostOut[3L * u + 2] = p.z; }
             if (A.pos32) {
                 A.corner[(long)cell * A.Wc + k] =
                     make_double2((double)arc32(A.pos32[last], A.pos32[u], (float)aR(A, u)), included_angle_clamped<true>(pl, p, px));
@@ -948,6 +1035,30 @@ __global__ void k_t1_patch(ApplyArgs A, T1Scratch t1) {
         }
         __syncthreads();
     }
+}
+// The pass's largest ring, for the host's capacity check.
+__device__ __forceinline__ void publish_ring_max(const ApplyArgs& A) {
+    *(volatile int*)A.ringMaxOut = *(volatile int*)A.ringMax;
+    __threadfence_system();
+}
+// The cells of the touched list (batches, and k_t1_apply's replay of a sphere's pass).  A host-buffer
+// step's output: the force kernel wrote the moved positions; the flips moved vertices of the touched
+// cells, whose ring entries rewrite them.  A list that may have lost entries (full) rewrites every
+// vertex instead.  (Appends past the list's capacity roll the pass back; a pass cut short by an
+// exhausted barrier wait may leave the counter above it, and only the stored entries are read.)
+__device__ __forceinline__ void patch_touched(const ApplyArgs& A, const T1Scratch& t1, int ntRaw, int block, int blocks) {
+    const bool hostAll = A.hostOut && ntRaw > t1.touchedCap - 4;
+    if (hostAll)
+        for (long v = block * (long)blockDim.x + threadIdx.x; v < A.nV; v += (long)blocks * blockDim.x) {
+            const D3 p = ld3(A.pos, (int)v);
+            A.hostOut[3 * v] = p.x; A.hostOut[3 * v + 1] = p.y; A.hostOut[3 * v + 2] = p.z;
+        }
+    patch_cells(A, min(ntRaw, t1.touchedCap), block, blocks, A.hostOut && !hostAll, [&](int i) { return t1.touched[i]; });
+}
+// Batches: the patch over all replicas' touched cells, after k_t1_apply.
+__global__ void k_t1_patch(ApplyArgs A, T1Scratch t1) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) publish_ring_max(A);
+    patch_touched(A, t1, *(volatile int*)(t1.ctr + 5), blockIdx.x, gridDim.x);
 }
 
 // Restores everything a committed flip overwrote.
@@ -994,8 +1105,14 @@ __device__ __forceinline__ bool t1_candidate(const ApplyArgs& A, int q) {
 // re-testing each edge against the current state when it is reached and re-testing, after every
 // flip, the edges of the six vertices whose slots or positions the flip changed.  Flags ahead of
 // the extracted window live in the bitmap; flags inside it in a small heap.  Afterwards every
-// cell whose ring changed gets its ring bookkeeping (vrpos/vlast/vnext) and corners rebuilt.
-__global__ void __launch_bounds__(kApplyThreads) k_t1_apply(ApplyArgs A, T1Scratch t1) {
+// cell whose ring changed gets its ring bookkeeping (vrpos/vlast/vnext) and corners rebuilt (here for
+// one sphere, by k_t1_patch for a batch).  For one sphere it is the pass's last kernel and leaves the
+// counters of the next pass cleared.
+__device__ void t1_reset(const T1Scratch& t1) {
+    int* c = t1.ctr + 5;   // touched cells, round maximum, ticket, and the pass's T1Ctl
+    for (int k = 0; k < 3 + kT1CtlInts; ++k) c[k] = 0;
+}
+__global__ void __launch_bounds__(kApplyThreads) k_t1_apply(ApplyArgs A, T1Scratch t1, bool sphere) {
     __shared__ int buf[kExtractCap];
     __shared__ int heap[kHeapCap];
     __shared__ int nbuf, head, nheap, extractWord, nTouched;
@@ -1007,10 +1124,14 @@ __global__ void __launch_bounds__(kApplyThreads) k_t1_apply(ApplyArgs A, T1Scrat
             *t1.pass += 1;
             t1.stats[0] += 1;
             if (A.bumpStep) *A.stepCounter += 1ull;
+            if (sphere) {
+                publish_ring_max(A);
+                t1_reset(t1);
+            }
         }
         return;
     }
-    // touched cells are appended after those of the parallel pass's segments that succeeded
+    // (a batch's touched cells are appended after those of the segments that succeeded)
     if (tid == 0) { nbuf = 0; head = 0; nheap = 0; extractWord = 0; nTouched = t1.ctr[5]; t1.stats[6] = *t1.flipCount; }
     __syncthreads();
     int lastProcessed = -1;
@@ -1113,10 +1234,15 @@ __global__ void __launch_bounds__(kApplyThreads) k_t1_apply(ApplyArgs A, T1Scrat
         }
         __syncthreads();
     }
-    // ring bookkeeping and corners of the touched cells: k_t1_patch
+    // ring bookkeeping and corners of the touched cells
     __syncthreads();
+    if (sphere) patch_touched(A, t1, nTouched, 0, 1);
     if (tid == 0) {
         t1.ctr[5] = nTouched;
+        if (sphere) {
+            publish_ring_max(A);
+            t1_reset(t1);
+        }
         *t1.count = 0;
         *t1.pass += 1;
         t1.stats[0] += 1;
@@ -1127,14 +1253,10 @@ __global__ void __launch_bounds__(kApplyThreads) k_t1_apply(ApplyArgs A, T1Scrat
 
 
 // ---- parallel T1 pass -------------------------------------------------------------------------
-// Footprint of the edge at position p: every vertex and cell that testing, flipping and
-// re-testing after the flip can read or write (v1, v2 and their neighbours; the cells of v1 and
-// v2).  Two positions with disjoint footprints commute.
-__device__ __forceinline__ void t1_footprint(const ApplyArgs& A, int p, int* f) {
+// Footprint of the edge at position p.
+__device__ __forceinline__ void t1_footprint_of(const ApplyArgs& A, int p, int* f) {
     const int v1 = p / 3, v2 = compRef(A.vnbr, v1, p - 3 * v1);
-    const int4 n1 = A.vnbr[v1], n2 = A.vnbr[v2], c1 = A.vcell[v1], c2 = A.vcell[v2];
-    f[0] = v1; f[1] = v2; f[2] = n1.x; f[3] = n1.y; f[4] = n1.z; f[5] = n2.x; f[6] = n2.y; f[7] = n2.z;
-    f[8] = c1.x; f[9] = c1.y; f[10] = c1.z; f[11] = c2.x; f[12] = c2.y; f[13] = c2.z;
+    t1_footprint(v1, v2, A.vnbr[v1], A.vnbr[v2], A.vcell[v1], A.vcell[v2], f);
 }
 
 // Vertex a of (v1, v2, vs.x, vs.y, vs.z, vs.w): the six whose slots a flip re-tests.
@@ -1146,39 +1268,12 @@ constexpr int kParThreads = 512;        // one segment: the whole sphere
 constexpr int kParThreadsBatch = 128;   // one segment per replica (4 resident blocks per SM at 128 registers)
 constexpr int kCoopThreads = 256;       // per block of a cooperative single-sphere pass
 
-// Block-wide exclusive scan of one int per thread; returns the block total in *total.
-__device__ int block_excl_scan(int v, int* total) {
-    __shared__ int warpTot[32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int incl = v;
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-    }
-    if (lane == 31) warpTot[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        const int nw = blockDim.x >> 5;
-        int t = lane < nw ? warpTot[lane] : 0;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, t, o);
-            if (lane >= o) t += y;
-        }
-        if (lane < nw) warpTot[lane] = t;  // inclusive over warps
-    }
-    __syncthreads();
-    const int before = (warp == 0 ? 0 : warpTot[warp - 1]) + incl - v;
-    *total = warpTot[(blockDim.x >> 5) - 1];
-    __syncthreads();
-    return before;
-}
-
 // Barrier of all blocks of a cooperative launch (co-resident by construction): the last block
 // to arrive resets the count and advances the generation; the others poll the generation, at most
-// kBarrierSpins times, after which the wait gives up and the barrier returns false.  Fences before
+// spinLimit times (svm_model_set_t1_wait_limit; the default 2^20 is at least 67 ms with 64 ns naps), after
+// which the wait gives up and the barrier returns false.  Fences before
 // the arrival and after the wait order every block's writes before the barrier with every read
 // after it.
-constexpr int kBarrierSpins = 1 << 20;  // at least 67 ms with 64 ns naps (svm_model_set_t1_wait_limit)
 __device__ bool grid_barrier(T1Ctl* ctl, int spinLimit) {
     __shared__ int ok;
     __syncthreads();
@@ -1207,33 +1302,38 @@ __device__ bool grid_barrier(T1Ctl* ctl, int spinLimit) {
 // deterministic reservations: every pending position writes its own value into the footprint
 // cells (atomicMin); a position whose whole footprint holds its value runs (test, flip,
 // re-test of the affected edges), the others wait for the next round.  Overlapping positions
-// therefore run in ascending order and disjoint ones commute.  A position created by a re-test
-// that overlaps a higher position which has already run would need the CPU order broken; that is
-// detected through the per-vertex/per-cell record of the highest position that ran, and then
-// every flip of the pass is undone and the bitmap restored for k_t1_apply, which then applies
-// the flips one by one.  On success *t1.count is cleared so k_t1_apply returns at once.
+// therefore run in ascending order and disjoint ones commute, whatever the order of the list.  The
+// first round's list, footprints and reservations come from the T1 test (t1_flag), so the pass starts
+// running at once.  A position created by a re-test that overlaps a higher position which has already
+// run would need the CPU order broken; that is detected through the per-vertex/per-cell record of the
+// highest position that ran, and then every flip of the pass is undone and the bitmap restored for
+// k_t1_apply, which then applies the flips one by one (it finds nothing to do otherwise).
 //
 // kCoop = false: one block per segment of the position space: the whole sphere, or one replica
 // of a batch (whose flagged edges share no vertex or cell with another replica's, and whose
 // positions are a contiguous range).  A block's lists, footprints, commit list and undo log are
-// its own slices of the scratch arrays; the touched-cell list and the flip log are shared (atomic
+// its own slices of the scratch arrays; a batch's touched-cell list and the flip log are shared (atomic
 // appends).  A block whose pass is not the sequential order undoes its own flips, marks their log
-// entries invalid (pass -1) and restores its segment's flags, which k_t1_apply then replays; the
-// counter of flagged positions drops by the positions of every block that succeeded.  The last
-// block to finish (ticket) folds the round count into the statistics and clears summary bits
-// whose bitmap words are empty.
+// entries invalid (pass -1) and restores its segment's flags, which k_t1_apply then replays.  The last
+// block to finish (ticket) folds the round count into the statistics.
 // kCoop = true: one segment (the whole sphere) over all blocks of a cooperative launch, so that the
-// flips' FP64 work spreads over many SMs instead of one: block 0 extracts the flagged positions,
-// position i of a round runs on block i mod gridDim.x, the phases are separated by grid barriers
-// instead of block barriers, the counters live in global memory (t1.ctl), and block 0 alone
-// finishes the pass (rollback, statistics, cleanup).  Same decisions, same results.
+// flips spread over many SMs instead of one: position i of a round runs on block i mod gridDim.x, the
+// phases are separated by grid barriers instead of block barriers, the counters live in global memory
+// (t1.ctl, cleared by the last pass's k_t1_apply), and block 0 alone finishes a rollback and the
+// statistics.  Same decisions, same results.
+// A sphere's pass also rebuilds the corners of the cells its flips changed (patch_cells over the undo
+// entries): a batch leaves them to k_t1_patch, which spreads its hottest replicas' cells over all SMs.
+//
+// What bounds it is latency: a few tens of flips, each a chain of loads and the pair's FP64 rotation.  A
+// flip runs on a warp (t1_flip_warp).  100k cells, 1.3 rounds and 75 flips a pass on average: see the
+// figures at launch_t1_apply.
 template <bool kCoop>
-__global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_parallel(ApplyArgs A, T1Scratch t1, const int* __restrict__ segOff,
-                                                             int listPad, int undoPer) {
+__global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_parallel(ApplyArgs A, T1Scratch t1, int undoPer) {
     __shared__ T1Ctl sctl;
     T1Ctl* ctl = kCoop ? t1.ctl : &sctl;
     const int tid = threadIdx.x, seg = kCoop ? 0 : blockIdx.x;
-    const bool leader = !kCoop || blockIdx.x == 0;  // extracts the positions and finishes the pass
+    const bool leader = !kCoop || blockIdx.x == 0;  // finishes the pass
+    const bool sphere = kCoop || t1.segOff == nullptr;
     // this thread's first position of a round and the stride (reserve and release phases), and
     // this warp's (run phase: one warp per position).  Consecutive positions go to different
     // blocks of a cooperative grid.
@@ -1242,20 +1342,21 @@ __global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_paral
     const int gs = kCoop ? gridDim.x * blockDim.x : blockDim.x;
     const int wi = kCoop ? blockIdx.x + gridDim.x * (tid >> 5) : (tid >> 5);
     const int ws = kCoop ? gridDim.x * warps : warps;
+    const int qLo = sphere ? 0 : 3 * t1.segOff[seg];
+    const int qHi = sphere ? 3 * A.nV : 3 * t1.segOff[seg + 1];
+    const int base = qLo / 2 + t1.listPad * seg;
+    const int capB = (qHi - qLo) / 2 + t1.listPad;
+    // The count is read by every block before the first grid barrier, so before block 0 can change it.
+    const int nOrig = min(*(volatile int*)(t1.segCount + seg), capB);
     // one segment and nothing flagged: nothing to do.  (With several segments every block runs:
-    // the last one to finish does the pass's cleanup.)  The count is read by every block before
-    // the first grid barrier, so before block 0 can change it.
-    if ((kCoop || gridDim.x == 1) && *t1.count == 0) return;
+    // the last one to finish does the pass's cleanup.)
+    if (sphere && nOrig == 0) return;
     auto group_sync = [&]() -> bool {
         if (!kCoop) { __syncthreads(); return true; }
         if (grid_barrier(ctl, A.barrierSpins)) return true;
         if (tid == 0) atomicOr(A.status, SVM_DEV_T1_TIMEOUT);
         return false;
     };
-    const int qLo = segOff ? 3 * segOff[seg] : 0;
-    const int qHi = segOff ? 3 * segOff[seg + 1] : 3 * A.nV;
-    const int base = qLo / 2 + listPad * seg;
-    const int capB = (qHi - qLo) / 2 + listPad;
     int* cur = t1.listA + base;
     int* nxt = t1.listB + base;
     int* orig = t1.listOrig + base;
@@ -1263,13 +1364,11 @@ __global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_paral
     int* comB = t1.comList + (long)base * kFootprint;
     UndoEntry* undoB = t1.undo + (long)seg * undoPer;
     int* undoRingsB = t1.undoRings + (long)seg * undoPer * 4 * A.Wc;
-    // a cooperative pass starts from zeroed counters (cleared with the launch's memset)
-    if (!kCoop && tid == 0) {
-        sctl.nCur = 0; sctl.flag = 0; sctl.nWordsHit = 0; sctl.undo = 0; sctl.rollback = 0; sctl.exec = 0;
-        sctl.flips = 0; sctl.next[0] = 0; sctl.next[1] = 0; sctl.late = 0;
+    if (!kCoop) {
+        if (tid == 0) { sctl.undo = 0; sctl.rollback = 0; sctl.exec = 0; sctl.flips = 0; sctl.next[0] = 0; sctl.next[1] = 0; sctl.late = 0; }
+        __syncthreads();
     }
-    __syncthreads();
-    // phase clocks (block 0, thread 0; svm_model_t1_clocks): extraction, reserve, run, release, end
+    // phase clocks (block 0, thread 0; svm_model_t1_clocks): (none), reserve, run, release, end
     const bool clk = t1.clocks && seg == 0 && blockIdx.x == 0 && tid == 0;
     long long c0 = clk ? clock64() : 0, c1 = c0;
     auto lap = [&](int slot) {
@@ -1278,105 +1377,51 @@ __global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_paral
         atomicAdd(t1.clocks + slot, (unsigned long long)(c1 - c0));
         c0 = c1;
     };
-    // 1. the segment's flagged positions, ascending: the bitmap words whose summary bit is set
-    //    (a superset of the non-empty words) into `nxt`, then their set bits inside [qLo, qHi)
-    const int wLo = qLo >> 5, wHi = (qHi + 31) >> 5;  // words [wLo, wHi)
-    if (leader) {
-        for (int base2 = wLo >> 5; base2 < ((wHi + 31) >> 5); base2 += blockDim.x) {
-            const int sw = base2 + tid;
-            unsigned sword = sw < ((wHi + 31) >> 5) && sw < t1.nSummary ? t1.summary[sw] : 0u;
-            // keep the summary bits of words inside [wLo, wHi)
-            if (sw == (wLo >> 5)) sword &= ~0u << (wLo & 31);
-            if (sw == ((wHi - 1) >> 5) && (wHi & 31)) sword &= (1u << (wHi & 31)) - 1u;
-            int tot;
-            const int off = block_excl_scan(__popc(sword), &tot);
-            unsigned x = sword;
-            int at = ctl->nWordsHit + off;
-            while (x) {
-                const int b = __ffs(x) - 1;
-                x &= x - 1u;
-                const int w = sw * 32 + b;
-                if (w < t1.nWords && at < capB) nxt[at] = w;
-                ++at;
-            }
-            __syncthreads();
-            if (tid == 0) ctl->nWordsHit = min(ctl->nWordsHit + tot, capB);
-            __syncthreads();
-        }
-        const int nHit = ctl->nWordsHit;
-        for (int b0 = 0; b0 < nHit; b0 += blockDim.x) {
-            const int i = b0 + tid;
-            const int w = i < nHit ? nxt[i] : -1;
-            unsigned word = (w >= 0 && w < t1.nWords) ? t1.bits[w] : 0u;
-            if (w == (qLo >> 5)) word &= ~0u << (qLo & 31);
-            if (w >= 0 && w == ((qHi - 1) >> 5) && (qHi & 31)) word &= (1u << (qHi & 31)) - 1u;
-            int tot;
-            const int off = block_excl_scan(__popc(word), &tot);
-            const int n0 = ctl->nCur;
-            if (n0 + tot > capB) { if (tid == 0) ctl->flag = 1; __syncthreads(); break; }
-            unsigned x = word;
-            int at = n0 + off;
-            while (x) {
-                const int b = __ffs(x) - 1;
-                x &= x - 1u;
-                cur[at] = w * 32 + b;
-                orig[at] = w * 32 + b;
-                ++at;
-            }
-            __syncthreads();
-            if (tid == 0) ctl->nCur = n0 + tot;
-            __syncthreads();
-        }
-    }
-    if (!group_sync()) return;
-    // uniform over the group from here on: every thread reads the same counters after a barrier
-    const int nOrig = *(volatile int*)&ctl->nCur;
+    // counters below are uniform over the group: every thread reads the same values after a barrier
     int nCur = nOrig;
     int par = 0;  // the round's next-list counter: ctl->next[par]
-    int rounds = 0;
-    bool rollback = *(volatile int*)&ctl->flag != 0;  // more candidates than the slice holds: k_t1_apply takes them all
-    lap(0);
-    // 2. rounds
-    while (!rollback && nCur > 0) {
+    int rounds = 0, lastRan = 0;
+    bool rollback = false;
+    while (nCur > 0) {
         ++rounds;
-        // reserve
-        for (int i = gi; i < nCur; i += gs) {
-            const int p = cur[i];
-            int* f = fpB + (long)i * kFootprint;
-            t1_footprint(A, p, f);
-            bool late = false;
-            for (int k = 0; k < 8; ++k) { late |= t1.comV[f[k]] > p; atomicMin(t1.resV + f[k], p); }
-            for (int k = 8; k < kFootprint; ++k) { late |= t1.comC[f[k]] > p; atomicMin(t1.resC + f[k], p); }
-            if (late) atomicExch(&ctl->late, 1);
-        }
-        if (!group_sync()) return;
-        lap(1);
-        // `late` is written only while reserving and `rollback` only while running, so each is
-        // read after the barrier that ends its phase, by every block alike
-        if (*(volatile int*)&ctl->late) {
-            // release this round's reservations before leaving
+        if (rounds > 1) {  // reserve (the first round's reservations are the test's)
             for (int i = gi; i < nCur; i += gs) {
-                const int* f = fpB + (long)i * kFootprint;
-                for (int k = 0; k < 8; ++k) t1.resV[f[k]] = kResFree;
-                for (int k = 8; k < kFootprint; ++k) t1.resC[f[k]] = kResFree;
+                const int p = cur[i];
+                int* f = fpB + (long)i * kFootprint;
+                t1_footprint_of(A, p, f);
+                bool late = false;
+                for (int k = 0; k < 8; ++k) { late |= t1.comV[f[k]] > p; atomicMin(t1.resV + f[k], p); }
+                for (int k = 8; k < kFootprint; ++k) { late |= t1.comC[f[k]] > p; atomicMin(t1.resC + f[k], p); }
+                if (late) atomicExch(&ctl->late, 1);
             }
-            rollback = true;
-            break;
+            if (!group_sync()) return;
+            lap(1);
+            // `late` is written only while reserving and `rollback` only while running, so each is
+            // read after the barrier that ends its phase, by every block alike
+            rollback = *(volatile int*)&ctl->late != 0;
         }
-        // run the positions that hold their whole footprint.  While the round's positions fit the
-        // warps: one warp per position, its lanes sharing the reservation checks, the pair's
-        // rotation and the 18 re-tests (an FP64 warp instruction costs the same for 1 or 32 lanes,
-        // so a flip's FP64 chain shortens ~2.6x); beyond that (segments with many flips in a
-        // round): one thread per position.  The same decisions and writes either way.
-        if (nCur <= ws) {
+        // run the positions that hold their whole footprint, one warp per position: its lanes share the
+        // reservation checks, the rings, the pair's rotation and the 18 re-tests.  Beyond 16 positions a
+        // warp (passes with very many flips): one thread per position.  The same decisions and writes
+        // either way.
+        if (!rollback && nCur <= 16 * ws) {
         for (int i = wi; i < nCur; i += ws) {
             const int p = cur[i];
+            if (rounds == 1 && lane == 0) orig[i] = p;
             const int* f = fpB + (long)i * kFootprint;
-            // the edge (f[0], f[1]) is p's; its positions load alongside the reservation words (if
-            // p does not hold its footprint they may be changing, and are not used)
-            const int v1 = f[0], v2 = f[1];
-            const TPos P1 = tpos(A, v1), P2 = tpos(A, v2);
+            // the edge (f[0], f[1]) is p's; its positions and rings load alongside the reservation words
+            // (if p does not hold its footprint they may be changing, and are not used)
             const int fk = lane < kFootprint ? f[lane] : 0;
+            const int v1 = __shfl_sync(kFull, fk, 0), v2 = __shfl_sync(kFull, fk, 1);
+            const int c[3] = {__shfl_sync(kFull, fk, 8), __shfl_sync(kFull, fk, 9), __shfl_sync(kFull, fk, 10)};
+            int cw = -1;
+#pragma unroll
+            for (int q = 11; q < 14; ++q) {
+                const int t = __shfl_sync(kFull, fk, q);
+                if (t != c[0] && t != c[1] && t != c[2]) cw = t;
+            }
+            const WarpRings W = warp_rings_load(A, c, cw, lane);
+            const TPos P1 = tpos(A, v1), P2 = tpos(A, v2);
             bool held = true;
             if (lane < kFootprint) held = (lane < 8 ? t1.resV[fk] : t1.resC[fk]) == p;
             if (!__all_sync(kFull, held)) {
@@ -1387,23 +1432,29 @@ __global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_paral
                 }
                 continue;
             }
-            int ci = 0;
-            if (lane == 0) ci = atomicAdd(&ctl->exec, 1);
-            ci = __shfl_sync(kFull, ci, 0);
-            if (ci >= capB) { if (lane == 0) atomicExch(&ctl->rollback, 1); continue; }
+            // lanes 0 and 1 take the position's places in the commit and undo lists together
+            const bool isShort = v1 < v2 && t1_short(A, P1, P2);  // t1_candidate(A, p), on every lane alike
+            int got = 0;
+            if (lane == 0) got = atomicAdd(&ctl->exec, 1);
+            if (lane == 1 && isShort) got = atomicAdd(&ctl->undo, 1);
+            const int ci = __shfl_sync(kFull, got, 0), ui = __shfl_sync(kFull, got, 1);
+            if (ci >= capB) {
+                if (lane == 0) {
+                    if (isShort && ui < undoPer) undoB[ui].v1 = -1;
+                    atomicExch(&ctl->rollback, 1);
+                }
+                continue;
+            }
             if (lane < kFootprint) {
                 comB[(long)ci * kFootprint + lane] = fk;
                 atomicMax((lane < 8 ? t1.comV : t1.comC) + fk, p);
             }
             if (lane == 0) atomicAnd(t1.bits + (p >> 5), ~(1u << (p & 31)));
-            if (!(v1 < v2 && t1_short(A, P1, P2))) continue;  // t1_candidate(A, p), on every lane alike
-            int ui = 0;
-            if (lane == 0) ui = atomicAdd(&ctl->undo, 1);
-            ui = __shfl_sync(kFull, ui, 0);
+            if (!isShort) continue;
             if (ui >= undoPer) { if (lane == 0) atomicExch(&ctl->rollback, 1); continue; }
             int4 cs, vs;
             UndoEntry* u = undoB + ui;
-            if (!t1_flip_warp(A, v1, v2, cs, vs, u, undoRingsB + (long)ui * 4 * A.Wc, D3{P1.x, P1.y, P1.z},
+            if (!t1_flip_warp(A, fk, W, cs, vs, u, undoRingsB + (long)ui * 4 * A.Wc, D3{P1.x, P1.y, P1.z},
                               D3{P2.x, P2.y, P2.z}, lane)) {
                 if (lane == 0) u->v1 = -1;  // nothing was written
                 continue;
@@ -1416,6 +1467,8 @@ __global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_paral
                     int* e = t1.flipLog + 4 * fc;
                     e[0] = *t1.pass; e[1] = p; e[2] = v1; e[3] = v2;
                 }
+            }
+            if (lane == 1 && !sphere) {
                 const int tc = atomicAdd(t1.ctr + 5, 4);
                 if (tc + 4 <= t1.touchedCap) {
                     t1.touched[tc] = cs.x; t1.touched[tc + 1] = cs.y; t1.touched[tc + 2] = cs.z; t1.touched[tc + 3] = cs.w;
@@ -1425,33 +1478,30 @@ __global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_paral
             }
             // re-test the 18 slots of the six vertices whose slots or positions the flip changed
             // (t1_candidate on each): lane l < 18 tests slot l % 3 of vertex l / 3 of
-            // (v1, v2, vs.x, vs.y, vs.z, vs.w); lane 0 then flags the new candidates in that order
+            // (v1, v2, vs.x, vs.y, vs.z, vs.w) and flags it when it is a new candidate
             bool again = false;
+            int r = 0;
             if (lane < 18) {
                 const int a = lane / 3, sl = lane - 3 * (lane / 3);
                 const int v = pick_aff(a, v1, v2, vs);
-                const int r = 3 * v + sl;
+                r = 3 * v + sl;
                 const int w = compRef(A.vnbr, v, sl);
                 again = r > p && r < qHi && v < w && t1_short(A, tpos(A, v), tpos(A, w));
             }
-            const unsigned hits = __ballot_sync(kFull, again);
-            if (lane == 0) {
-                for (unsigned m = hits; m; m &= m - 1u) {
-                    const int l = __ffs(m) - 1;
-                    const int r = 3 * pick_aff(l / 3, v1, v2, vs) + (l - 3 * (l / 3));
-                    const unsigned bit = 1u << (r & 31);
-                    if (!(atomicOr(t1.bits + (r >> 5), bit) & bit)) {
-                        atomicOr(t1.summary + (r >> 10), 1u << ((r >> 5) & 31));
-                        const int ni = atomicAdd(&ctl->next[par], 1);
-                        if (ni < capB) nxt[ni] = r;
-                        else atomicExch(&ctl->rollback, 1);
-                    }
+            if (again) {
+                const unsigned bit = 1u << (r & 31);
+                if (!(atomicOr(t1.bits + (r >> 5), bit) & bit)) {
+                    const int ni = atomicAdd(&ctl->next[par], 1);
+                    if (ni < capB) nxt[ni] = r;
+                    else atomicExch(&ctl->rollback, 1);
                 }
             }
+            __syncwarp();
         }
-        } else {
+        } else if (!rollback) {
         for (int i = gi; i < nCur; i += gs) {
             const int p = cur[i];
+            if (rounds == 1) orig[i] = p;
             const int* f = fpB + (long)i * kFootprint;
             bool ready = true;
             for (int k = 0; k < 8; ++k) ready &= t1.resV[f[k]] == p;
@@ -1485,11 +1535,13 @@ __global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_paral
                 int* e = t1.flipLog + 4 * fc;
                 e[0] = *t1.pass; e[1] = p; e[2] = v1; e[3] = v2;
             }
-            const int tc = atomicAdd(t1.ctr + 5, 4);
-            if (tc + 4 <= t1.touchedCap) {
-                t1.touched[tc] = cs.x; t1.touched[tc + 1] = cs.y; t1.touched[tc + 2] = cs.z; t1.touched[tc + 3] = cs.w;
-            } else {
-                atomicExch(&ctl->rollback, 1);
+            if (!sphere) {
+                const int tc = atomicAdd(t1.ctr + 5, 4);
+                if (tc + 4 <= t1.touchedCap) {
+                    t1.touched[tc] = cs.x; t1.touched[tc + 1] = cs.y; t1.touched[tc + 2] = cs.z; t1.touched[tc + 3] = cs.w;
+                } else {
+                    atomicExch(&ctl->rollback, 1);
+                }
             }
             const int aff[6] = {v1, v2, vs.x, vs.y, vs.z, vs.w};
             for (int a = 0; a < 6; ++a)
@@ -1498,7 +1550,6 @@ __global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_paral
                     if (!(r > p && r < qHi && t1_candidate(A, r))) continue;
                     const unsigned bit = 1u << (r & 31);
                     if (!(atomicOr(t1.bits + (r >> 5), bit) & bit)) {
-                        atomicOr(t1.summary + (r >> 10), 1u << ((r >> 5) & 31));
                         const int ni = atomicAdd(&ctl->next[par], 1);
                         if (ni < capB) nxt[ni] = r;
                         else atomicExch(&ctl->rollback, 1);
@@ -1506,28 +1557,44 @@ __global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_paral
                 }
         }
         }
-        if (!group_sync()) return;
+        if (!rollback && !group_sync()) return;
         lap(2);
-        // release this round's reservations; the other next-list counter starts the next round at 0
+        // release this round's reservations
         for (int i = gi; i < nCur; i += gs) {
             const int* f = fpB + (long)i * kFootprint;
             for (int k = 0; k < 8; ++k) t1.resV[f[k]] = kResFree;
             for (int k = 8; k < kFootprint; ++k) t1.resC[f[k]] = kResFree;
         }
+        // (the lowest position always runs; a round that ran nothing means reservations left by a pass that
+        // gave up waiting, and the positions go to the replay)
+        const int ran = *(volatile int*)&ctl->exec;
+        if (rollback || *(volatile int*)&ctl->rollback || ran == lastRan) { rollback = true; break; }
+        lastRan = ran;
+        nCur = min(*(volatile int*)&ctl->next[par], capB);
+        if (nCur == 0) break;
+        // the other next-list counter starts the next round at 0
         if (leader && tid == 0) ctl->next[par ^ 1] = 0;
         if (!group_sync()) return;
-        nCur = min(*(volatile int*)&ctl->next[par], capB);
         par ^= 1;
         int* t = cur; cur = nxt; nxt = t;
         lap(3);
-        if (*(volatile int*)&ctl->rollback) rollback = true;
     }
-    if (!group_sync()) return;
+    // the record of what ran, cleared over the group
+    const int ne = min(*(volatile int*)&ctl->exec, capB);
+    for (int i = gi; i < ne; i += gs) {
+        const int* f = comB + (long)i * kFootprint;
+        for (int k = 0; k < 8; ++k) t1.comV[f[k]] = -1;
+        for (int k = 8; k < kFootprint; ++k) t1.comC[f[k]] = -1;
+    }
+    const int nu = min(*(volatile int*)&ctl->undo, undoPer);
+    if (sphere && !rollback)
+        patch_cells(A, 4 * nu, kCoop ? blockIdx.x : 0, kCoop ? gridDim.x : 1, A.hostOut != nullptr,
+                    [&](int i) { return undoB[i >> 2].v1 < 0 ? -1 : undoB[i >> 2].cells[i & 3]; });
     if (!leader) return;
     if (rollback) {
+        __syncthreads();
         if (tid == 0) {
             // undo this segment's flips, newest first, and invalidate their log entries
-            const int nu = min(*(volatile int*)&ctl->undo, undoPer);
             for (int i = nu - 1; i >= 0; --i) {
                 const UndoEntry& u = undoB[i];
                 if (u.v1 < 0) continue;
@@ -1536,7 +1603,9 @@ __global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_paral
             }
         }
         __syncthreads();
-        // the segment's flags back to the ones the test set: clear, then set the originals
+        // the segment's flags back to the ones the test set: clear, then set the originals, with the
+        // summary bits that k_t1_apply finds them by
+        const int wLo = qLo >> 5, wHi = (qHi + 31) >> 5;  // words [wLo, wHi)
         for (int w = wLo + tid; w < wHi; w += blockDim.x) {
             unsigned keep = 0u;  // bits of other segments in a shared boundary word
             if (w == (qLo >> 5)) keep |= ~(~0u << (qLo & 31));
@@ -1551,41 +1620,23 @@ __global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_paral
         }
     }
     __syncthreads();
-    const int ne = min(*(volatile int*)&ctl->exec, capB);
-    for (int i = tid; i < ne; i += blockDim.x) {
-        const int* f = comB + (long)i * kFootprint;
-        for (int k = 0; k < 8; ++k) t1.comV[f[k]] = -1;
-        for (int k = 8; k < kFootprint; ++k) t1.comC[f[k]] = -1;
-    }
-    __shared__ bool amLast;
     if (tid == 0) {
-        atomicAdd(t1.stats + 1, nOrig);
-        atomicAdd(t1.stats + 2, ne);
-        atomicMax(t1.ctr + 6, rounds);
-        if (rollback) atomicAdd(t1.stats + 5, 1);
-        else {
-            atomicAdd(t1.stats + 3, *(volatile int*)&ctl->flips);
-            atomicSub(t1.count, nOrig);
+        t1.segCount[seg] = 0;   // (read by every block before the pass's first barrier)
+        if (nOrig > 0) {
+            atomicAdd(t1.stats + 1, nOrig);
+            atomicAdd(t1.stats + 2, ne);
+            atomicMax(t1.ctr + 6, rounds);
+            if (rollback) {
+                atomicAdd(t1.stats + 5, 1);
+                atomicAdd(t1.count, nOrig);
+            } else {
+                atomicAdd(t1.stats + 3, *(volatile int*)&ctl->flips);
+            }
         }
         __threadfence();
-        amLast = kCoop || atomicAdd(t1.ctr + 7, 1) == (int)gridDim.x - 1;
+        if (sphere || atomicAdd(t1.ctr + 7, 1) == (int)gridDim.x - 1) t1.stats[4] += *(volatile int*)(t1.ctr + 6);
     }
-    __syncthreads();
     lap(4);
-    if (!amLast) return;
-    if (tid == 0) t1.stats[4] += *(volatile int*)(t1.ctr + 6);
-    // summary bits of words that are now empty
-    for (int sw = tid; sw < t1.nSummary; sw += blockDim.x) {
-        unsigned sword = *(volatile unsigned*)(t1.summary + sw);
-        unsigned keep = sword;
-        while (sword) {
-            const int b = __ffs(sword) - 1;
-            sword &= sword - 1u;
-            const int w = sw * 32 + b;
-            if (w >= t1.nWords || *(volatile unsigned*)(t1.bits + w) == 0u) keep &= ~(1u << b);
-        }
-        t1.summary[sw] = keep;
-    }
 }
 
 // Ring bookkeeping for all vertices after a topology upload: for each cell and ring position,
@@ -1812,7 +1863,7 @@ int launch_corners(svm_model* m, bool t1test, bool vnormReady) {
     if (!m->edgeC) return SVM_ERR_ARG;  // FP64 corners exist for single spheres only
     const int bv = spread_block(m, m->nVertices);
     if (!vnormReady) k_vnorm<<<blocksFor(m->nVertices, bv), bv, 0, m->stream>>>(m->pos[m->cur], m->vnorm, m->nVertices);
-    k_edges<<<blocksFor(m->nVertices, bv), bv, 0, m->stream>>>(m->pos[m->cur], m->vnorm, m->vsph, m->vnbr, m->edgeC,
+    k_edges<<<blocksFor(m->nVertices, bv), bv, 0, m->stream>>>(m->pos[m->cur], m->vnorm, m->vsph, m->vnbr, m->vcell, m->edgeC,
                                                               m->edgeArc, m->nVertices, m->R, t1test ? 1 : 0,
                                                               m->t1Threshold, m->t1);
     // both corner kernels write the same values; the three-thread one is faster below ~100k vertices
@@ -1982,14 +2033,13 @@ static int mark_pass(svm_model* m) {
 
 int launch_t1_apply(svm_model* m, int bump) {
     if (int rc = ensure_ring_headroom(m)) return rc;
-    PhaseTimer pt(m, SVM_PHASE_T1APPLY, 3);
-    // touched-cell count (ctr[5]), per-pass round maximum (ctr[6]), block ticket (ctr[7]) and the
-    // cooperative pass's counters and barrier (t1.ctl, after them)
-    if (cudaMemsetAsync(m->t1.ctr + 5, 0, (3 + kT1CtlInts) * sizeof(int), m->stream) != cudaSuccess)
-        return SVM_ERR_CUDA;
     const bool batch = m->nRep > 1;
+    PhaseTimer pt(m, SVM_PHASE_T1APPLY, batch ? 3 : 2);
     const int nSeg = batch ? m->nRep : 1;
     const int coop = batch ? 1 : t1_coop_blocks(m);
+    // a batch's touched-cell count (ctr[5]), per-pass round maximum (ctr[6]) and block ticket (ctr[7]);
+    // one sphere's k_t1_apply leaves them cleared
+    if (batch && cudaMemsetAsync(m->t1.ctr + 5, 0, 3 * sizeof(int), m->stream) != cudaSuccess) return SVM_ERR_CUDA;
     if (coop > 1) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(coop);
@@ -2000,17 +2050,14 @@ int launch_t1_apply(svm_model* m, int bump) {
         attr[0].val.cooperative = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        const int* noSeg = nullptr;
-        if (cudaLaunchKernelEx(&cfg, k_t1_parallel<true>, apply_args(m, bump), m->t1, noSeg, kListPad,
-                               m->t1.undoCap) != cudaSuccess)
+        if (cudaLaunchKernelEx(&cfg, k_t1_parallel<true>, apply_args(m, bump), m->t1, m->t1.undoCap) != cudaSuccess)
             return SVM_ERR_CUDA;
     } else {
-        k_t1_parallel<false><<<nSeg, batch ? kParThreadsBatch : kParThreads, 0, m->stream>>>(
-            apply_args(m, bump), m->t1, batch ? m->repVertOff : nullptr, batch ? kListPadBatch : kListPad,
-            m->t1.undoCap / nSeg);
+        k_t1_parallel<false><<<nSeg, batch ? kParThreadsBatch : kParThreads, 0, m->stream>>>(apply_args(m, bump), m->t1,
+                                                                                             m->t1.undoCap / nSeg);
     }
-    k_t1_apply<<<1, kApplyThreads, 0, m->stream>>>(apply_args(m, bump), m->t1);
-    k_t1_patch<<<2 * m->sms, 256, 0, m->stream>>>(apply_args(m, bump), m->t1);
+    k_t1_apply<<<1, kApplyThreads, 0, m->stream>>>(apply_args(m, bump), m->t1, !batch);
+    if (batch) k_t1_patch<<<2 * m->sms, 256, 0, m->stream>>>(apply_args(m, bump), m->t1);
     if (int rc = check_launch()) return rc;
     return mark_pass(m);
 }
@@ -2023,7 +2070,7 @@ int launch_t1_test(svm_model* m) {
     t1_bracket(m->t1Threshold, m->R, &lo, &hi);
     t1_sin2_bracket(m->t1Threshold, m->R, &s2lo, &s2hi);
     k_t1_test<<<blocksFor(m->nVertices), kBlock, 0, m->stream>>>(
-        m->pos[m->cur], m->precision == SVM_PRECISION_MIXED ? m->pos32[m->cur] : nullptr, m->repR, m->vnbr,
+        m->pos[m->cur], m->precision == SVM_PRECISION_MIXED ? m->pos32[m->cur] : nullptr, m->repR, m->vnbr, m->vcell,
         m->nVertices, m->R, m->t1Threshold, lo, hi, s2lo, s2hi, m->t1);
     return check_launch();
 }
@@ -2214,6 +2261,8 @@ int svm::model_alloc(int nCells, int nVertices, int Wc, const double* radius, in
     alloc((void**)&m->t1.bits, (size_t)m->t1.nSummary * 32 * sizeof(unsigned));
     alloc((void**)&m->t1.summary, (size_t)m->t1.nSummary * sizeof(unsigned));
     alloc((void**)&m->t1.count, sizeof(int));
+    alloc((void**)&m->t1.segCount, nRep * sizeof(int));
+    m->t1.listPad = nRep > 1 ? svm::kListPadBatch : svm::kListPad;
     alloc((void**)&m->t1.flipLog, 4 * (size_t)m->t1.flipLogCap * sizeof(int));
     alloc((void**)&m->t1.pass, sizeof(int));
     alloc((void**)&m->t1.listA, (size_t)m->t1.cap * sizeof(int));
@@ -2238,6 +2287,7 @@ int svm::model_alloc(int nCells, int nVertices, int Wc, const double* radius, in
     alloc((void**)&m->repVertOff, (nRep + 1) * sizeof(int));
     alloc((void**)&m->repFlag, nRep * sizeof(int));
     alloc((void**)&m->repScal, 3 * nRep * sizeof(double));
+    if (nRep > 1) m->t1.segOff = m->repVertOff;
     alloc((void**)&m->ringMax, sizeof(int));
     if (ok && cudaHostAlloc((void**)&m->ringMaxHost, sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
         m->ringMaxHost = nullptr;
@@ -2270,7 +2320,7 @@ int svm_model_destroy(svm_model* m) {
     void* ptrs[] = {m->pos[0], m->pos[1], m->vsph, m->vnorm, m->dir, m->dirTarget, m->cellRef, m->edgeC, m->edgeArc, m->vcell, m->vnbr, m->vlast, m->vnext, m->vrpos, m->ring,
                     m->ringCount, m->corner, m->cellPos, m->cellSph, m->ap, m->pref, m->force, m->vel, m->noiseBuf,
                     m->dispBuf, m->partials, m->ticket, m->scalars, m->fallbackFlag, m->status, m->stepCounter,
-                    m->t1.bits, m->t1.summary, m->t1.count, m->t1.flipLog, m->t1.flipCount, m->t1.touched,
+                    m->t1.bits, m->t1.summary, m->t1.count, m->t1.segCount, m->t1.flipLog, m->t1.flipCount, m->t1.touched,
                     m->t1.pass, m->t1.listA, m->t1.listB, m->t1.listOrig, m->t1.fp, m->t1.comList, m->t1.resV,
                     m->t1.resC, m->t1.comV, m->t1.comC, m->t1.undo, m->t1.undoRings, m->t1.ctr, m->t1.stats,
                     m->pos32[0], m->pos32[1], m->cellPos32, m->force32, m->dap32, m->repR, m->repNp, m->repCellOff,
