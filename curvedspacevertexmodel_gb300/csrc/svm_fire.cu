@@ -7,7 +7,7 @@
 //                  disp = dt v + dt^2/2 F, v += dt/2 F / m, move onto the sphere (in place), and
 //                  the moved vertex's norm for the corner pass
 //   corners + T1   unless motion is restricted: k_edges (edge terms and the T1 length test),
-//                  k_corner or k_corner_s, then the T1 pass (k_t1_parallel, k_t1_apply, k_t1_patch)
+//                  k_corner or k_corner_s, then the T1 pass (k_t1_parallel, k_t1_apply)
 //   geometry       k_cells, k_fallback_fan (the corners too when motion is restricted)
 //   k_fire_force   per vertex: F, v += dt/2 F / m, block partials of F.v, F.F, v.v, max |F|^2;
 //                  the last block reduces them in a fixed order and runs the FIRE control
@@ -45,6 +45,7 @@ struct svm_fire {
 namespace {
 
 constexpr int kB = 256;
+constexpr int kFireVerts = kSlotVerts;   // vertices per block of the reductions (k_fire_force, k_fire_sums)
 
 // Block sum (bmax: maximum) in a fixed order, valid in thread 0.  Warps from `live` on hold zeros and
 // skip their shuffles (their +0.0 leaves the sum's bits unchanged).
@@ -160,7 +161,7 @@ template <bool kControl, bool kCount>
 __device__ void fire_reduce_tail(FireState* __restrict__ Sp, double P, double FF, double VV, int nV,
                                  double* __restrict__ partials, unsigned* __restrict__ ticket, double* __restrict__ out4,
                                  double* sh, bool& amLast) {
-    constexpr int kLive = kSlotVerts / 32;  // the warps of the block's vertex threads
+    constexpr int kLive = (kFireVerts + 31) / 32;  // the warps of the block's vertex threads
     const double bP = bsum(P, sh, kLive), bF = bsum(FF, sh, kLive), bV = bsum(VV, sh, kLive), bM = bmax(FF, sh, kLive);
     if (threadIdx.x == 0) {
         double* q = partials + 4 * blockIdx.x;
@@ -211,24 +212,23 @@ __device__ void fire_reduce_tail(FireState* __restrict__ Sp, double P, double FF
     *Sp = S;
 }
 
-// Blocks of 3 kSlotVerts threads: three per vertex for the force (one per cell slot), then the
-// first kSlotVerts threads finish their vertex.  One instantiation per force form: the vector form
-// alone fits 78 registers without spill, so four blocks per SM (a 40k-vertex sphere's 625 blocks in
-// 1.03 waves of them instead of 1.37 waves of three; measured 0.171 against 0.172 ms per FIRE
-// iteration at 20k cells).
+// Blocks of kFireVerts vertices (block_slot_force); its first kFireVerts threads then finish their
+// vertex.  One instantiation per force form, which lets each drop the other's registers: six blocks of
+// the vector form per SM.  FIRE iteration in the vector form against three threads a vertex and separate
+// products and sums: 20k cells 163 -> 121 us, 100k cells 432 us.
 template <int kForm>
-__global__ void __launch_bounds__(3 * kSlotVerts, kForm == kFormVector ? 4 : kSlotMinBlocks)
+__global__ void __launch_bounds__(slot_threads(kFireVerts), kForm == kFormVector ? 6 : kSlotMinBlocks)
     k_fire_force(ForceArgs A, FireState* __restrict__ Sp, int nV, double4_32a* __restrict__ force,
                  double4_32a* __restrict__ vel, double* __restrict__ partials, unsigned* __restrict__ ticket) {
     __shared__ double sh[32];
     __shared__ bool amLast;
-    __shared__ SlotShared slots;
+    __shared__ SlotShared<kFireVerts> slots;
     if (Sp->done) return;
     const double dt = Sp->dt;
-    const D3 fv = block_slot_force<kForm>(A, nV, slots);
-    const int i = blockIdx.x * kSlotVerts + threadIdx.x;
+    const D3 fv = block_slot_force<kForm, kFireVerts>(A, nV, slots, NoSide());
+    const int i = blockIdx.x * kFireVerts + threadIdx.x;
     double P = 0.0, FF = 0.0, VV = 0.0;
-    if (threadIdx.x < kSlotVerts && i < nV) {
+    if (threadIdx.x < kFireVerts && i < nV) {
         const D3 f = fv;
         st3(force, i, f);
         const D3 v = vv_kick(ld3(vel, i), f, dt);
@@ -239,20 +239,19 @@ __global__ void __launch_bounds__(3 * kSlotVerts, kForm == kFormVector ? 4 : kSl
 }
 
 // fireStep (energyMinimizerFIRE.h:56, fireStepCPU cpp:122-174) on the current forces and
-// velocities: the sums and the control, in blocks of 3 kSlotVerts threads whose first kSlotVerts
-// hold one vertex each, which is k_fire_force's layout, so the sums are bitwise those of a
-// minimize iteration.  With kControl false: the four totals to out4 (gpu_dVec_dot_products).
+// velocities: the sums and the control, in blocks whose first kFireVerts threads hold one vertex each,
+// which is k_fire_force's layout, so the sums are bitwise those of a minimize iteration.  With kControl false: the four totals to out4 (gpu_dVec_dot_products).
 template <bool kControl>
-__global__ void __launch_bounds__(3 * kSlotVerts) k_fire_sums(FireState* __restrict__ Sp, int nV,
+__global__ void __launch_bounds__(slot_threads(kFireVerts)) k_fire_sums(FireState* __restrict__ Sp, int nV,
                                                               const double4_32a* __restrict__ force,
                                                               const double4_32a* __restrict__ vel,
                                                               double* __restrict__ partials,
                                                               unsigned* __restrict__ ticket, double* __restrict__ out4) {
     __shared__ double sh[32];
     __shared__ bool amLast;
-    const int i = blockIdx.x * kSlotVerts + threadIdx.x;
+    const int i = blockIdx.x * kFireVerts + threadIdx.x;
     double P = 0.0, FF = 0.0, VV = 0.0;
-    if (threadIdx.x < kSlotVerts && i < nV) fire_dots(ld3(force, i), ld3(vel, i), P, FF, VV);
+    if (threadIdx.x < kFireVerts && i < nV) fire_dots(ld3(force, i), ld3(vel, i), P, FF, VV);
     fire_reduce_tail<kControl, false>(Sp, P, FF, VV, nV, partials, ticket, out4, sh, amLast);
 }
 
@@ -287,12 +286,12 @@ int fire_iteration(svm_fire* F) {
     rc = launch_geometry(m);
     if (rc) return rc;
     PhaseTimer pt(m, SVM_PHASE_FORCE);
-    const int nf = (m->nVertices + kSlotVerts - 1) / kSlotVerts;
+    const int nf = (m->nVertices + kFireVerts - 1) / kFireVerts;
     if (m->precision == SVM_PRECISION_FP64_VECTOR)
-        k_fire_force<kFormVector><<<nf, 3 * kSlotVerts, 0, m->stream>>>(fargs(m), F->d, m->nVertices, m->force, m->vel,
+        k_fire_force<kFormVector><<<nf, slot_threads(kFireVerts), 0, m->stream>>>(fargs(m), F->d, m->nVertices, m->force, m->vel,
                                                                         F->partials, F->ticket);
     else
-        k_fire_force<kFormReference><<<nf, 3 * kSlotVerts, 0, m->stream>>>(fargs(m), F->d, m->nVertices, m->force,
+        k_fire_force<kFormReference><<<nf, slot_threads(kFireVerts), 0, m->stream>>>(fargs(m), F->d, m->nVertices, m->force,
                                                                            m->vel, F->partials, F->ticket);
     return check_launch();
 }
@@ -316,7 +315,7 @@ int svm_fire_create(svm_model* m, double dt, double alphaStart, double dtMax, do
     S.dt = dt; S.dtMin = dt * .01; S.alphaStart = alphaStart; S.alpha = alphaStart; S.dtMax = dtMax;
     S.dtInc = dtInc; S.dtDec = dtDec; S.alphaDec = alphaDec; S.nMin = nMin; S.cutoff = forceCutoff;
     S.alphaMin = alphaMin; S.maxIterations = maxIterations; S.rmsOverN = 100.; S.maxForce = 100.;
-    F->nBlocks = (m->nVertices + kSlotVerts - 1) / kSlotVerts;  // blocks of k_fire_force
+    F->nBlocks = (m->nVertices + kFireVerts - 1) / kFireVerts;  // blocks of k_fire_force
     bool ok = cudaMalloc(&F->d, sizeof(FireState)) == cudaSuccess &&
               cudaMalloc(&F->partials, sizeof(double) * 4 * (F->nBlocks + 1)) == cudaSuccess &&
               cudaMalloc(&F->ticket, sizeof(unsigned)) == cudaSuccess;
@@ -409,8 +408,8 @@ int svm_fire_step(svm_fire* F) {
     if (!F || !F->m) return SVM_ERR_ARG;
     svm_model* m = F->m;
     if (m->precision == SVM_PRECISION_MIXED) return SVM_ERR_ARG;
-    const int nb = (m->nVertices + kSlotVerts - 1) / kSlotVerts;
-    k_fire_sums<true><<<nb, 3 * kSlotVerts, 0, m->stream>>>(F->d, m->nVertices, m->force, m->vel, F->partials,
+    const int nb = (m->nVertices + kFireVerts - 1) / kFireVerts;
+    k_fire_sums<true><<<nb, slot_threads(kFireVerts), 0, m->stream>>>(F->d, m->nVertices, m->force, m->vel, F->partials,
                                                             F->ticket, nullptr);
     k_fire_finish<<<(m->nVertices + kB - 1) / kB, kB, 0, m->stream>>>(F->d, m->vel, m->force, m->nVertices);
     k_fire_clear_pending<<<1, 1, 0, m->stream>>>(F->d);
@@ -454,10 +453,10 @@ int svm_velocity_verlet_step(svm_model* m, double dt, int nSteps) {
 
 int svm_reduce_dots(svm_model* m, double* out4) {
     if (!m || !out4 || m->precision == SVM_PRECISION_MIXED) return SVM_ERR_ARG;
-    const int nb = (m->nVertices + kSlotVerts - 1) / kSlotVerts;
+    const int nb = (m->nVertices + kFireVerts - 1) / kFireVerts;
     if (!m->dotPartials && cudaMalloc(&m->dotPartials, sizeof(double) * 4 * (size_t)(nb + 1)) != cudaSuccess)
         return SVM_ERR_CUDA;
-    k_fire_sums<false><<<nb, 3 * kSlotVerts, 0, m->stream>>>(nullptr, m->nVertices, m->force, m->vel, m->dotPartials,
+    k_fire_sums<false><<<nb, slot_threads(kFireVerts), 0, m->stream>>>(nullptr, m->nVertices, m->force, m->vel, m->dotPartials,
                                                              m->ticket + 3, m->scalars + 8);
     if (check_launch()) return SVM_ERR_CUDA;
     double r[4];

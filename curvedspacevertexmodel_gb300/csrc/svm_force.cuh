@@ -28,146 +28,246 @@ struct ForceArgs {
 
 __device__ __forceinline__ int comp(const int4& a, int s) { return s == 0 ? a.x : (s == 1 ? a.y : a.z); }
 
-// Unit tangent at a pointing away from the neighbour at v + d: gradient of the geodesic length
-// (any radius), from the raw position difference d.
-__device__ __forceinline__ D3 grad_geo_vec(D3 a, D3 d) {
-    const D3 t = sub3(d, scl3(dot3(d, a), a));
-    return scl3(f64_div_root(-1.0, dot3(t, t)), t);
-}
-// Gradient w.r.t. v = |v| a of the signed spherical triangle area R^2 E(a, a + beta, a + gamma),
-// beta and gamma the raw differences to the other corners over |v|: tan(E/2) = N/D (Van Oosterom
-// and Strackee, 1983) differentiated, projected onto the tangent plane.
-__device__ __forceinline__ D3 grad_tri_vec(D3 a, D3 beta, D3 gamma, double R) {
-    const D3 bg = cross3(beta, gamma);
-    const D3 bxc = add3(add3(cross3(a, gamma), cross3(beta, a)), bg);
-    const double N = dot3(a, bg);
-    const double D = 4.0 - dot3(beta, beta) - dot3(gamma, gamma) + dot3(beta, gamma);
-    const double w = f64_div(2.0, N * N + D * D);
-    const D3 g = scl3(w, sub3(scl3(D, bxc), scl3(N, add3(beta, gamma))));
-    return scl3(R, sub3(g, scl3(dot3(g, a), a)));
-}
-
 // The force form of a kernel: chosen per launch from A.vec (kFormAny), or fixed at compile time, which
 // lets a kernel that runs one form drop the other's registers.
 constexpr int kFormAny = 0, kFormVector = 1, kFormReference = 2;
 
-// Block-level force of kSlotVerts vertices by 3 kSlotVerts threads (thread 3 i + s computes slot s
-// of vertex i of the block); threads i < kSlotVerts receive vertex i's force in slot order.
-constexpr int kSlotVerts = 64;
-// Resident blocks per SM the slot-force kernels are compiled for: three blocks of 3 kSlotVerts
-// threads (the register budget falls from 120 to 96 with a few bytes of spill), whose 18 warps hide
-// the latency of the integer-pipe divisions and square roots better than two blocks' 12 (the
-// Brownian step's force kernel at 100k cells: 0.49 -> 0.475 ms per launch; FIRE's at 20k cells
-// likewise).  Blocks of 32 vertices (six per SM) measured no faster at 20k or 100k cells.
-constexpr int kSlotMinBlocks = 3;
+// Block-level force of kVerts vertices by six threads a vertex: thread (role, vi, s) with s one of the
+// vertex's three cell slots and a role per triangle of the slot's fan.  Role 0 holds the slot's ring
+// predecessor L and the triangle (v, L, c), role 1 the cell's centroid c and the triangle (v, c, X), X
+// the successor.  Each thread first evaluates its point's terms -- every neighbour of v is the
+// predecessor in one of its cells, so the six threads cover the vertex's six pairs once -- and then,
+// with the other's through shared memory, its triangle.  The roles are whole warps.
+//
+// What bounds it: at large N the FP64 pipe (2 lanes per clock per SM) and the instruction caches; at
+// small N one warp's chain of dependent operations, which two threads a slot halve.  Measured for the
+// Brownian kernel (k_force_bd) against three threads a vertex, 64 vertices a block, three blocks per SM
+// and every product but the chains' first ones on the FP64 pipe:
+//   100k cells  265 us -> 266 (six threads) -> 251 (all of the triangle's products but the roots'
+//               arguments on the integer pipes, FP64 pipe 67% busy) -> 226 (those products out of
+//               line, normals drawn by role 1 beside the edge gradients)
+//   20k cells   78 -> 58 us;   200 cells  28.7 -> 20.5 us.
+// Also tried at 100k cells: the roots' arguments on the integer pipes too 231 us, the quotients out of
+// line too 230, four blocks per SM 240; blocks of 10 vertices at 200 cells 20.3, at 20k cells 72.
+constexpr int kSlotVerts = 32;
+constexpr int slot_role_threads(int verts) { return (3 * verts + 31) / 32 * 32; }
+constexpr int slot_threads(int verts) { return 2 * slot_role_threads(verts); }
+// Blocks per SM the slot-force kernels are compiled for (64 registers: 30 warps per SM).
+constexpr int kSlotMinBlocks = 5;
+template <int kVerts = kSlotVerts>
 struct SlotShared {
-    double x[3 * kSlotVerts], y[3 * kSlotVerts], z[3 * kSlotVerts];  // edge gradients, then slot forces
-    double sP[3 * kSlotVerts], s[3 * kSlotVerts], d[3 * kSlotVerts];  // pair terms towards the predecessor
+    double l[7][3 * kVerts];   // predecessor terms: (sin dphi, s, d, s s, s s - 1) or (beta, a x beta, beta^2)
+    double c[7][3 * kVerts];   // centroid terms, the same
+    double g[3][3 * kVerts];   // edge gradients towards the predecessors, then the slots' forces
+    double t[3][3 * kVerts];   // role 1's triangle terms
 };
 
-// The contribution of cell slot s to the force on vertex v in the reference form: the fSet term of the
-// header's sum for the vertex's cell s.  Three threads share a vertex (more warps in flight when the
-// vertex count is small).  Each neighbour of v is the predecessor in one of its cells and the successor
-// in another, so the three threads' predecessors cover all of the vertex's edges: each thread
-// evaluates its predecessor's pair terms and edge gradient, and takes its successor's from the thread
-// that has it, through the block's shared memory.  Every thread of the block calls it.
-__device__ __forceinline__ D3 slot_force_reference(const ForceArgs& A, int v, int vi, int s, bool live, SlotShared& sh) {
-    const int t = threadIdx.x;
-    int4 cells, lasts, nexts;
-    double4_32a sv, sl;
-    PairTerms pL;
+struct SlotIndex { int v, vi, s, at, c, L, X, jx; bool live; };
+template <int kVerts>
+__device__ __forceinline__ SlotIndex slot_index(const ForceArgs& A, int nV, int k) {
+    SlotIndex q;
+    q.vi = k / 3; q.s = k - 3 * q.vi; q.at = k;
+    q.v = blockIdx.x * kVerts + q.vi;
+    q.live = q.vi < kVerts && q.v < nV;
+    q.c = q.L = q.X = q.jx = 0;
+    if (q.live) {
+        const int4 cells = A.vcell[q.v], lasts = A.vlast[q.v], nexts = A.vnext[q.v];
+        q.c = comp(cells, q.s); q.L = comp(lasts, q.s); q.X = comp(nexts, q.s);
+        // the slot whose predecessor X is (-1: inconsistent lists)
+        q.jx = q.X == lasts.x ? 0 : (q.X == lasts.y ? 1 : (q.X == lasts.z ? 2 : -1));
+    }
+    return q;
+}
+template <int kVerts>
+__device__ __forceinline__ void put_pair(double (*a)[3 * kVerts], int k, const PairTerms& p) {
+    a[0][k] = p.sP; a[1][k] = p.s; a[2][k] = p.d; a[3][k] = p.ss; a[4][k] = p.q;
+}
+template <int kVerts>
+__device__ __forceinline__ PairTerms get_pair(const double (*a)[3 * kVerts], int k) {
+    return PairTerms{a[0][k], a[1][k], a[2][k], a[3][k], a[4][k]};
+}
+template <int kVerts>
+__device__ __forceinline__ void put3(double (*a)[3 * kVerts], int k, D3 p) { a[0][k] = p.x; a[1][k] = p.y; a[2][k] = p.z; }
+template <int kVerts>
+__device__ __forceinline__ D3 get3(const double (*a)[3 * kVerts], int k) { return D3{a[0][k], a[1][k], a[2][k]}; }
+
+// det(p, a, b) < 0: in FP32 where that is certain (all but nearly flat triangles).
+__device__ __forceinline__ bool det_negative(D3 p, D3 a, D3 b) {
+    const svm_det::F3 v32 = svm_det::near3(p.x, p.y, p.z);
+    const int n = svm_det::below_zero(v32, svm_det::diff(svm_det::near3(a.x, a.y, a.z), v32),
+                                      svm_det::diff(svm_det::near3(b.x, b.y, b.z), v32));
+    return n >= 0 ? n != 0 : det3(p, a, b) < 0;
+}
+
+// The slot forces of the reference form, left in sh.g for the block: per slot
+//   -pp (grad d(v, L) + grad d(v, X)) - aa (grad A(v, L, c) + grad A(v, c, X)), pp = 2 dP, aa = 2 Kr dA,
+// each term subtracted in the reference's order.  `side(q)` is work that does not depend on the force: one
+// call per slot, by role 1's threads while role 0 evaluates the edge gradients.  Every thread of the block calls it.
+template <int kVerts, class Side>
+__device__ __forceinline__ void slot_forces_reference(const ForceArgs& A, int nV, SlotShared<kVerts>& sh, Side side) {
+    constexpr int kRole = slot_role_threads(kVerts);
+    const bool role0 = threadIdx.x < kRole;
+    const SlotIndex q = slot_index<kVerts>(A, nV, role0 ? threadIdx.x : threadIdx.x - kRole);
+    double4_32a sv, s2;   // the spherical coordinates of v and of the thread's own point
+    PairTerms own;
     D3 gL;
-    if (live) {
-        cells = A.vcell[v]; lasts = A.vlast[v]; nexts = A.vnext[v];
-        sv = A.vsph[v];
-        sl = A.vsph[comp(lasts, s)];
-        pL = pair_terms(sv, sl);
-        gL = from_basis(sv, grad_geodesic(pL, sl.y));
-        sh.x[t] = gL.x; sh.y[t] = gL.y; sh.z[t] = gL.z;
-        sh.sP[t] = pL.sP; sh.s[t] = pL.s; sh.d[t] = pL.d;
+    if (q.live) {
+        sv = A.vsph[q.v];
+        s2 = role0 ? A.vsph[q.L] : A.cellSph[q.c];
+        own = pair_terms(sv, s2);
+        if (role0) {
+            gL = from_basis(sv, grad_geodesic(own, s2.y));
+            put3<kVerts>(sh.g, q.at, gL);
+        } else {
+            side(q);
+        }
+        put_pair<kVerts>(role0 ? sh.l : sh.c, q.at, own);
     }
     __syncthreads();
     D3 fs;
-    if (live) {
-        const int c = comp(cells, s), L = comp(lasts, s), X = comp(nexts, s);
-        const double2 apc = A.ap[c], pr = A.pref[c];
-        const double dA = apc.x - pr.x, dP = apc.y - pr.y;
-        const double pp = sf::twice(dP), aa = 2.0 * A.Kr * dA;
-        const double4_32a sx = A.vsph[X], sc = A.cellSph[c];
-        const int jx = X == lasts.x ? 0 : (X == lasts.y ? 1 : (X == lasts.z ? 2 : -1));
-        PairTerms pX;
+    if (q.live) {
+        const double2 apc = A.ap[q.c], pr = A.pref[q.c];
+        const double aa = 2.0 * A.Kr * (apc.x - pr.x);
+        // the triangle's third corner: the centroid (role 0) or the successor (role 1)
+        const double4_32a s3 = role0 ? A.cellSph[q.c] : A.vsph[q.X];
+        PairTerms other;
         D3 gX;
-        if (jx >= 0) {
-            const int tx = 3 * vi + jx;
-            gX = D3{sh.x[tx], sh.y[tx], sh.z[tx]};
-            pX.sP = sh.sP[tx]; pX.s = sh.s[tx]; pX.d = sh.d[tx];
-            pX.ss = __dmul_rn(pX.s, pX.s);
-            pX.q = -1. + pX.ss;
-        } else {  // inconsistent lists
-            pX = pair_terms(sv, sx);
-            gX = from_basis(sv, grad_geodesic(pX, sx.y));
+        const int tx = 3 * q.vi + q.jx;
+        if (role0) {
+            other = get_pair<kVerts>(sh.c, q.at);
+            const double pp = sf::twice(apc.y - pr.y);
+            if (q.jx >= 0) gX = get3<kVerts>(sh.g, tx);
+            else {
+                const double4_32a sx = A.vsph[q.X];
+                gX = from_basis(sv, grad_geodesic(pair_terms(sv, sx), sx.y));
+            }
+            fs = sub3(scl3(-pp, gL), scl3(pp, gX));
+        } else {
+            other = q.jx >= 0 ? get_pair<kVerts>(sh.l, tx) : pair_terms(sv, s3);
         }
-        fs = sub3(scl3(-pp, gL), scl3(pp, gX));
-        const PairTerms pC = pair_terms(sv, sc);
-        double2 g1 = grad_triangle(pL, pC, pair_cos(sl, sc), sl.y, sc.y, A.R);
-        double2 g2 = grad_triangle(pC, pX, pair_cos(sc, sx), sc.y, sx.y, A.R);
-        // the sign of each triangle's det: FP32 where that is certain (all but nearly flat triangles)
-        const D3 p = ld3(A.pos, v), pl = ld3(A.pos, L), px = ld3(A.pos, X), cp = ld3(A.cellPos, c);
-        const svm_det::F3 v32 = svm_det::near3(p.x, p.y, p.z);
-        const svm_det::F3 c32 = svm_det::diff(svm_det::near3(cp.x, cp.y, cp.z), v32);
-        int n1 = svm_det::below_zero(v32, svm_det::diff(svm_det::near3(pl.x, pl.y, pl.z), v32), c32);
-        int n2 = svm_det::below_zero(v32, c32, svm_det::diff(svm_det::near3(px.x, px.y, px.z), v32));
-        if (n1 < 0) n1 = det3(p, pl, cp) < 0 ? 1 : 0;
-        if (n2 < 0) n2 = det3(p, cp, px) < 0 ? 1 : 0;
-        if (n1) g1 = make_double2(-g1.x, -g1.y);
-        if (n2) g2 = make_double2(-g2.x, -g2.y);
-        fs = sub3(fs, scl3(aa, from_basis(sv, g1)));
-        fs = sub3(fs, scl3(aa, from_basis(sv, g2)));
+        double2 g = grad_triangle(own, other, pair_cos(s2, s3), s2.y, s3.y, A.R);
+        const D3 p = ld3(A.pos, q.v), cp = ld3(A.cellPos, q.c), pn = ld3(A.pos, role0 ? q.L : q.X);
+        if (det_negative(p, role0 ? pn : cp, role0 ? cp : pn)) g = make_double2(-g.x, -g.y);
+        const D3 t = scl3(aa, from_basis(sv, g));
+        if (role0) fs = sub3(fs, t);
+        else put3<kVerts>(sh.t, q.at, t);
     }
     __syncthreads();
-    return fs;
-}
-
-// The same in the vector form (A.vec: the exact gradient as vectors, well conditioned where the
-// reference's closed forms lose digits -- short edges, thin fan triangles).
-__device__ __forceinline__ D3 slot_force_vector(const ForceArgs& A, int v, int s) {
-    const int4 cells = A.vcell[v], lasts = A.vlast[v], nexts = A.vnext[v];
-    const int c = comp(cells, s), L = comp(lasts, s), X = comp(nexts, s);
-    const D3 P = ld3(A.pos, v);
-    const double inv = f64_div_root(1.0, dot3(P, P));
-    const D3 a = scl3(inv, P);
-    const D3 dc = sub3(ld3(A.cellPos, c), P);
-    const D3 dl = sub3(ld3(A.pos, L), P), dx = sub3(ld3(A.pos, X), P);
-    const double2 apc = A.ap[c], pr = A.pref[c];
-    const double pp = 2.0 * (apc.y - pr.y), aa = 2.0 * A.Kr * (apc.x - pr.x);
-    const D3 bl = scl3(inv, dl), bc = scl3(inv, dc), bx = scl3(inv, dx);
-    return add3(scl3(-pp, add3(grad_geo_vec(a, dl), grad_geo_vec(a, dx))),
-                scl3(-aa, add3(grad_tri_vec(a, bl, bc, A.R), grad_tri_vec(a, bc, bx, A.R))));
-}
-
-// The slots' contributions are added in slot order, a NaN term skipped, as the reference's loop over
-// the three cells does.
-template <int kForm = kFormAny>
-__device__ __forceinline__ D3 block_slot_force(const ForceArgs& A, int nV, SlotShared& sh) {
-    const bool vec = kForm == kFormVector || (kForm == kFormAny && A.vec);
-    const int t = threadIdx.x, base = blockIdx.x * kSlotVerts;
-    const int vi = t / 3, s = t - 3 * (t / 3);
-    const int v = base + vi;
-    D3 fs{0.0, 0.0, 0.0};
-    if (!vec) fs = slot_force_reference(A, v, vi, s, v < nV, sh);
-    else if (v < nV) fs = slot_force_vector(A, v, s);
-    if (v < nV) { sh.x[t] = fs.x; sh.y[t] = fs.y; sh.z[t] = fs.z; }
+    if (q.live) {
+        if (role0) put3<kVerts>(sh.g, q.at, sub3(fs, get3<kVerts>(sh.t, q.at)));
+    }
     __syncthreads();
+}
+
+// The vector form (A.vec: the exact gradient as vectors, well conditioned where the reference's closed
+// forms lose digits -- short edges, thin fan triangles), the same way.  Products and sums contract to
+// multiply-adds here: the form's values are pinned to its formulas, not to the CPU's sequence of
+// roundings.
+__device__ __forceinline__ double dot3f(D3 a, D3 b) { return fma(a.z, b.z, fma(a.y, b.y, a.x * b.x)); }
+__device__ __forceinline__ D3 cross3f(D3 a, D3 b) {
+    return D3{fma(a.y, b.z, -(a.z * b.y)), fma(a.z, b.x, -(a.x * b.z)), fma(a.x, b.y, -(a.y * b.x))};
+}
+__device__ __forceinline__ D3 axpy3f(double s, D3 x, D3 y) { return D3{fma(s, x.x, y.x), fma(s, x.y, y.y), fma(s, x.z, y.z)}; }
+// Unit tangent at a pointing away from the neighbour at v + d: gradient of the geodesic length
+// (any radius), from the raw position difference d.
+__device__ __forceinline__ D3 grad_geo_vec(D3 a, D3 d) {
+    const D3 t = axpy3f(-dot3f(d, a), a, d);
+    return scl3(f64_div_root(-1.0, dot3f(t, t)), t);
+}
+// Gradient w.r.t. v = |v| a of the signed spherical triangle area R^2 E(a, a + beta, a + gamma), over R
+// and without its projection onto the tangent plane: tan(E/2) = N/D (Van Oosterom and Strackee, 1983)
+// differentiated, beta and gamma the raw differences to the other corners over |v|, ab = a x beta,
+// ag = a x gamma, and the squares of beta and gamma given.
+__device__ __forceinline__ D3 grad_tri_vec(D3 a, D3 beta, D3 gamma, D3 ab, D3 ag, double beta2, double gamma2) {
+    const D3 bg = cross3f(beta, gamma);
+    const D3 bxc = add3(sub3(ag, ab), bg);
+    const double N = dot3f(a, bg);
+    const double D = 4.0 - beta2 - gamma2 + dot3f(beta, gamma);
+    const double w = f64_div(2.0, fma(N, N, D * D));
+    return scl3(w, axpy3f(-N, add3(beta, gamma), scl3(D, bxc)));
+}
+template <int kVerts, class Side>
+__device__ __forceinline__ void slot_forces_vector(const ForceArgs& A, int nV, SlotShared<kVerts>& sh, Side side) {
+    constexpr int kRole = slot_role_threads(kVerts);
+    const bool role0 = threadIdx.x < kRole;
+    const SlotIndex q = slot_index<kVerts>(A, nV, role0 ? threadIdx.x : threadIdx.x - kRole);
+    D3 a, b, ab, gL;
+    double b2, inv;
+    if (q.live) {
+        const D3 P = ld3(A.pos, q.v), d = sub3(role0 ? ld3(A.pos, q.L) : ld3(A.cellPos, q.c), P);
+        inv = f64_div_root(1.0, dot3f(P, P));
+        a = scl3(inv, P);
+        b = scl3(inv, d);
+        ab = cross3f(a, b);
+        b2 = dot3f(b, b);
+        double (*o)[3 * kVerts] = role0 ? sh.l : sh.c;
+        put3<kVerts>(o, q.at, b);
+        put3<kVerts>(o + 3, q.at, ab);
+        o[6][q.at] = b2;
+        if (role0) {
+            gL = grad_geo_vec(a, d);
+            put3<kVerts>(sh.g, q.at, gL);
+        } else {
+            side(q);
+        }
+    }
+    __syncthreads();
+    D3 fs;
+    if (q.live) {
+        const double2 apc = A.ap[q.c], pr = A.pref[q.c];
+        const double aaR = 2.0 * A.Kr * (apc.x - pr.x) * A.R;
+        D3 o, ao, gX;   // the triangle's third corner: the centroid (role 0) or the successor (role 1)
+        double o2;
+        const int tx = 3 * q.vi + q.jx;
+        if (role0 || q.jx >= 0) {
+            const double (*p)[3 * kVerts] = role0 ? sh.c : sh.l;
+            const int k = role0 ? q.at : tx;
+            o = get3<kVerts>(p, k);
+            ao = get3<kVerts>(p + 3, k);
+            o2 = p[6][k];
+        } else {  // inconsistent lists
+            o = scl3(inv, sub3(ld3(A.pos, q.X), ld3(A.pos, q.v)));
+            ao = cross3f(a, o);
+            o2 = dot3f(o, o);
+        }
+        const D3 t = scl3(aaR, grad_tri_vec(a, b, o, ab, ao, b2, o2));
+        if (role0) {
+            const double pp = 2.0 * (apc.y - pr.y);
+            gX = q.jx >= 0 ? get3<kVerts>(sh.g, tx) : grad_geo_vec(a, sub3(ld3(A.pos, q.X), ld3(A.pos, q.v)));
+            fs = sub3(scl3(-pp, add3(gL, gX)), t);
+        } else {
+            put3<kVerts>(sh.t, q.at, t);
+        }
+    }
+    __syncthreads();
+    if (q.live) {
+        if (role0) {   // the slot's sum, projected onto the tangent plane (the edge gradients lie in it)
+            const D3 f = sub3(fs, get3<kVerts>(sh.t, q.at));
+            put3<kVerts>(sh.g, q.at, axpy3f(-dot3f(f, a), a, f));
+        }
+    }
+    __syncthreads();
+}
+
+// The force of vertex threadIdx.x of the block's kVerts vertices (threads from kVerts on: zero).  The
+// slots' contributions are added in slot order, a NaN term skipped, as the reference's loop over the
+// three cells does.
+template <int kForm, int kVerts, class Side>
+__device__ __forceinline__ D3 block_slot_force(const ForceArgs& A, int nV, SlotShared<kVerts>& sh, Side side) {
+    if (kForm == kFormVector || (kForm == kFormAny && A.vec)) slot_forces_vector<kVerts>(A, nV, sh, side);
+    else slot_forces_reference<kVerts>(A, nV, sh, side);
+    const int t = threadIdx.x;
     D3 f{0.0, 0.0, 0.0};
-    if (t < kSlotVerts && base + t < nV) {
+    if (t < kVerts && blockIdx.x * kVerts + t < nV) {
 #pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            const D3 fq{sh.x[3 * t + q], sh.y[3 * t + q], sh.z[3 * t + q]};
+        for (int k = 0; k < 3; ++k) {
+            const D3 fq = get3<kVerts>(sh.g, 3 * t + k);
             if (!isnan(fq.x)) f = add3(f, fq);
         }
     }
     return f;
 }
+struct NoSide { __device__ void operator()(const SlotIndex&) const {} };
 
 // Philox4x32-10 (Salmon, Moraes, Dror, Shaw, "Parallel random numbers: as easy as 1, 2, 3",
 // SC'11): ten rounds of two 32x32->64 multiplies with a Weyl-sequence key schedule.
@@ -218,7 +318,10 @@ static __device__ __noinline__ double zig_slow(const ZigTable* __restrict__ Z, i
             continue;
         }
         const double y = __ldg(Z->f + i) + u53(r.x, r.y) * (__ldg(Z->f + i + 1) - __ldg(Z->f + i));
-        if (y < exp(-0.5 * x * x)) return neg ? -x : x;
+        // y < exp(-x^2 / 2) in FP32 where that is certain: the FP32 exponential is within 2e-6 of it
+        const float xf = svm_det::near32(x), yf = svm_det::near32(y), ef = expf(-0.5f * xf * xf);
+        const bool under = fabsf(yf - ef) > 2e-5f * ef ? yf < ef : y < exp(-0.5 * x * x);
+        if (under) return neg ? -x : x;
         x = zig_draw(Z, r.z, r.w, i, neg);
         if (x < __ldg(Z->x + i + 1)) return neg ? -x : x;
     }
@@ -231,16 +334,15 @@ __device__ __forceinline__ double zig_normal(const ZigTable* __restrict__ Z, uns
     if (x < __ldg(Z->x + i + 1)) return neg ? -x : x;
     return zig_slow(Z, i, x, neg, ctr, key);
 }
-// Three standard normals for (vertex, step): two Philox draws (counter words 0 and 1) give the
-// three fast-path draws; normal j retries on counter words 64 (j + 1) + 1, 2, ...
-__device__ __forceinline__ D3 philox_normals3(const ZigTable* __restrict__ Z, uint64_t seed, unsigned long long step, int v) {
+// Component k of the three standard normals for (vertex, step): two Philox draws (counter words 0 and 1)
+// give the three fast-path draws; normal k retries on counter words 64 (k + 1) + 1, 2, ...
+__device__ __forceinline__ double philox_normal(const ZigTable* __restrict__ Z, uint64_t seed, unsigned long long step, int v,
+                                                int k) {
     const uint2 key = make_uint2((unsigned)seed, (unsigned)(seed >> 32));
-    const uint4 c0 = make_uint4((unsigned)v, (unsigned)step, (unsigned)(step >> 32), 0u);
-    const uint4 r0 = philox4x32_10(c0, key);
-    const uint4 r1 = philox4x32_10(make_uint4(c0.x, c0.y, c0.z, 1u), key);
-    return D3{zig_normal(Z, r0.x, r0.y, make_uint4(c0.x, c0.y, c0.z, 64u), key),
-              zig_normal(Z, r0.z, r0.w, make_uint4(c0.x, c0.y, c0.z, 128u), key),
-              zig_normal(Z, r1.x, r1.y, make_uint4(c0.x, c0.y, c0.z, 192u), key)};
+    uint4 c = make_uint4((unsigned)v, (unsigned)step, (unsigned)(step >> 32), k == 2 ? 1u : 0u);
+    const uint4 r = philox4x32_10(c, key);
+    c.w = 64u * (unsigned)(k + 1);
+    return zig_normal(Z, k == 1 ? r.z : r.x, k == 1 ? r.w : r.y, c, key);
 }
 
 // disp_d = xi_d sqrt(2 dt mu T) + F_d dt mu (brownianDynamics.cpp:37-44), products rounded

@@ -37,49 +37,49 @@ __global__ void k_zig_init() {
 namespace {
 using namespace svm;
 
-// Blocks of 3 kSlotVerts threads, three per vertex (one per cell slot), kSlotVerts vertices each.
-__global__ void __launch_bounds__(3 * kSlotVerts, kSlotMinBlocks) k_force(ForceArgs A, int nV,
-                                                                         double4_32a* __restrict__ force) {
-    __shared__ SlotShared sh;
-    const D3 f = block_slot_force(A, nV, sh);
+__global__ void __launch_bounds__(slot_threads(kSlotVerts), kSlotMinBlocks)
+    k_force(ForceArgs A, int nV, double4_32a* __restrict__ force) {
+    __shared__ SlotShared<> sh;
+    const D3 f = block_slot_force<kFormAny>(A, nV, sh, NoSide());
     const int v = blockIdx.x * kSlotVerts + threadIdx.x;
     if (threadIdx.x >= kSlotVerts || v >= nV) return;
     st3(force, v, f);
 }
 
-// Fused Brownian step for one vertex: force, displacement, move; reads `A.pos`, writes posNext (and
-// hostOut, when non-null).  (Writing the moved vertex's norm here as well, which would spare the
-// corner pass its k_vnorm, made this FP64-bound kernel as much slower as the corner pass got faster.)
+// Fused Brownian step: force, displacement, move; reads `A.pos`, writes posNext (and hostOut, when
+// non-null).  Role 1's threads draw the vertex's three normals, one each, while role 0 evaluates the
+// edge gradients.
+// (Writing the moved vertex's norm here as well, which would spare the corner pass its k_vnorm, made
+// this FP64-bound kernel as much slower as the corner pass got faster.)
 template <int kNoise>
-__global__ void __launch_bounds__(3 * kSlotVerts, kSlotMinBlocks) k_force_bd(
-                                                             ForceArgs A, int nV, double4_32a* __restrict__ force,
-                                                             double4_32a* __restrict__ posNext,
-                                                             const double* __restrict__ noise, uint64_t seed,
-                                                             const unsigned long long* __restrict__ stepCounter,
-                                                             double np, double fp, const ZigTable* __restrict__ zig,
-                                                             double* __restrict__ hostOut) {
-    __shared__ SlotShared sh;
-    const D3 f = block_slot_force(A, nV, sh);
-    const int v = blockIdx.x * kSlotVerts + threadIdx.x;
-    if (threadIdx.x >= kSlotVerts || v >= nV) return;
+__global__ void __launch_bounds__(slot_threads(kSlotVerts), kSlotMinBlocks)
+    k_force_bd(ForceArgs A, int nV, double4_32a* __restrict__ force, double4_32a* __restrict__ posNext,
+               const double* __restrict__ noise, uint64_t seed, const unsigned long long* __restrict__ stepCounter,
+               double np, double fp, const ZigTable* __restrict__ zig, double* __restrict__ hostOut) {
+    __shared__ SlotShared<> sh;
+    __shared__ double xi[3 * kSlotVerts];
+    const D3 f = block_slot_force<kFormAny>(A, nV, sh, [&](const SlotIndex& q) {
+        xi[q.at] = kNoise == SVM_NOISE_BUFFER ? noise[3 * q.v + q.s] : philox_normal(zig, seed, *stepCounter, q.v, q.s);
+    });
+    const int t = threadIdx.x, v = blockIdx.x * kSlotVerts + t;
+    if (t >= kSlotVerts || v >= nV) return;
     st3(force, v, f);
-    D3 xi;
-    if (kNoise == SVM_NOISE_BUFFER) xi = D3{noise[3 * v], noise[3 * v + 1], noise[3 * v + 2]};
-    else xi = philox_normals3(zig, seed, *stepCounter, v);
-    const D3 d{bd_disp(xi.x, np, f.x, fp), bd_disp(xi.y, np, f.y, fp), bd_disp(xi.z, np, f.z, fp)};
-    const D3 q = move_exact(ld3(A.pos, v), d, A.R);
-    st3(posNext, v, q);
+    const D3 d{bd_disp(xi[3 * t], np, f.x, fp), bd_disp(xi[3 * t + 1], np, f.y, fp), bd_disp(xi[3 * t + 2], np, f.z, fp)};
+    const D3 p = move_exact(ld3(A.pos, v), d, A.R);
+    st3(posNext, v, p);
     // a host-buffer step's output, straight into the caller's mapped page-locked array (AoS)
-    if (hostOut) { hostOut[3 * v] = q.x; hostOut[3 * v + 1] = q.y; hostOut[3 * v + 2] = q.z; }
+    if (hostOut) { hostOut[3 * v] = p.x; hostOut[3 * v + 1] = p.y; hostOut[3 * v + 2] = p.z; }
 }
+
+int slot_blocks(int nV) { return (nV + kSlotVerts - 1) / kSlotVerts; }
 
 }  // namespace
 
 namespace svm {
 
 int launch_force_fp64(svm_model* m) {
-    const int nb = (m->nVertices + kSlotVerts - 1) / kSlotVerts;
-    k_force<<<nb, 3 * kSlotVerts, 0, m->stream>>>(force_args(m, m->cur), m->nVertices, m->force);
+    k_force<<<slot_blocks(m->nVertices), slot_threads(kSlotVerts), 0, m->stream>>>(force_args(m, m->cur), m->nVertices,
+                                                                                  m->force);
     return check_launch();
 }
 
@@ -101,18 +101,15 @@ int zig_init() {
 
 int launch_force_bd_fp64(svm_model* m, double np, double fp, int noiseMode, const double* noise, uint64_t seed,
                          int nxt) {
-    const int nb = (m->nVertices + kSlotVerts - 1) / kSlotVerts;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || !gZigAddr[dev]) return SVM_ERR_CUDA;
     const ZigTable* zig = gZigAddr[dev];
-    if (noiseMode == SVM_NOISE_BUFFER)
-        k_force_bd<SVM_NOISE_BUFFER><<<nb, 3 * kSlotVerts, 0, m->stream>>>(
+    const auto go = [&](auto kernel) {
+        kernel<<<slot_blocks(m->nVertices), slot_threads(kSlotVerts), 0, m->stream>>>(
             force_args(m, m->cur), m->nVertices, m->force, m->pos[nxt], noise, seed, m->stepCounter, np, fp, zig,
             m->ioHostOut);
-    else
-        k_force_bd<SVM_NOISE_PHILOX><<<nb, 3 * kSlotVerts, 0, m->stream>>>(
-            force_args(m, m->cur), m->nVertices, m->force, m->pos[nxt], noise, seed, m->stepCounter, np, fp, zig,
-            m->ioHostOut);
+    };
+    noiseMode == SVM_NOISE_BUFFER ? go(k_force_bd<SVM_NOISE_BUFFER>) : go(k_force_bd<SVM_NOISE_PHILOX>);
     return check_launch();
 }
 

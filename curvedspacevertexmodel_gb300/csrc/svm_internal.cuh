@@ -62,12 +62,10 @@ __device__ __forceinline__ double f64_sqrt(double a) {
 // A divisor used more than once, and a square root used as a divisor: the quotients are f64_div's.
 #ifdef SVM_NATIVE_FP64_DIV
 struct F64Divisor { double d; };
-__device__ __forceinline__ F64Divisor f64_divisor(double b) { return F64Divisor{b}; }
 __device__ __forceinline__ F64Divisor f64_root_divisor(double a) { return F64Divisor{__dsqrt_rn(a)}; }
 __device__ __forceinline__ double f64_div(double a, const F64Divisor& b) { return __ddiv_rn(a, b.d); }
 #else
 using F64Divisor = sf::Divisor;
-__device__ __forceinline__ F64Divisor f64_divisor(double b) { return sf::divisor(b); }
 __device__ __forceinline__ F64Divisor f64_root_divisor(double a) { return sf::sqrt_divisor(a); }
 __device__ __forceinline__ double f64_div(double a, const F64Divisor& b) { return sf::div(a, b); }
 #endif
@@ -119,19 +117,11 @@ __device__ __forceinline__ double dot3(D3 a, D3 b) { double s = a.x * b.x; s += 
 __device__ __forceinline__ D3 cross3(D3 p1, D3 p2) {          // inc/functions.h:160-167
     return D3{p1.y * p2.z - p1.z * p2.y, p1.z * p2.x - p1.x * p2.z, p1.x * p2.y - p1.y * p2.x};
 }
-// A product on the integer pipes (sf::mul: the same bits as the hardware multiply) for the products
-// that start the FP64 kernels' dependency chains -- the pair terms of the geodesic and triangle-area
-// gradients, which depend only on the spherical coordinates, and the cross and dot products ahead of
-// the geometry's divisions and arccosines.  The FP64 pipe, which bounds the force
-// kernel, keeps the rest; the integer pipes, otherwise busy only with the divisions and square
-// roots, take these early, mutually independent products, whose latency the resident warps hide.
-// Measured at 100k cells: 0.476 -> 0.447 ms per force launch, and 0.442 with grad_triangle's
-// d/dtheta numerators, which are formed while the denominators' square roots run.  Moving the
-// d/dphi numerators too (chains of three products: 0.487 ms), the products at the end of
-// grad_triangle's chains (0.509 ms), all its products, or the pair terms' sums (0.531 ms) was slower.
-// The corner phase (k_edges' cross products and arcs, the included angles' products): 0.159 -> 0.151 ms;
-// the norms ahead of the centroids', vertices' and fan triangles' square roots: cells and fallback
-// phases 2-3% shorter.
+// A product on the integer pipes (sf::mul: the same bits as the hardware multiply), for products the
+// FP64 pipe -- the bound of these kernels -- can be spared: the cross and dot products ahead of the
+// geometry's divisions and arccosines (corner phase 0.159 -> 0.151 ms at 100k cells when they moved), the
+// norms ahead of the centroids', vertices' and fan triangles' square roots (cells and fallback phases
+// 2-3% shorter).  The gradients' products are grad_mul.
 // (kHw: the hardware multiply, for the T1 pass's latency-bound chains.)
 template <bool kHw = false>
 __device__ __forceinline__ double early_mul(double x, double y) {
@@ -321,25 +311,29 @@ __device__ __forceinline__ double4_32a sph_coords_n(D3 p, double r) {  // r = po
 template <bool kHw = false>
 __device__ __forceinline__ double4_32a sph_coords(D3 p) { return sph_coords_n<kHw>(p, pos_norm<kHw>(p)); }
 
+// The gradients' products on the integer pipes, out of line: some sixty to a slot, whose inlined code
+// (56 KB for the Brownian force kernel) did not fit the instruction caches.
+__device__ __forceinline__ double grad_mul(double x, double y) { return sf::mul_call(x, y); }
+
 // The terms of a pair of points (a, b), in spherical coordinates, that the gradients at a of both
 // gradientGeodesicDistance (sphericalDomain.h:248-273) and gradientTriangleArea (347-411) evaluate:
 // sin(phi_a - phi_b), s = cos of the arc, d = its derivative by theta_a, s s and s s - 1.  A pair is
 // evaluated once and serves its edge and both triangles it is a side of.
 struct PairTerms { double sP, s, d, ss, q; };
 __device__ __forceinline__ PairTerms pair_terms(const double4_32a& a, const double4_32a& b) {
-    const auto E = [](double x, double y) { return early_mul(x, y); };
+    const auto E = [](double x, double y) { return grad_mul(x, y); };
     PairTerms p;
     p.sP = E(a.w, b.z) - E(a.z, b.w);
     const double cP = E(a.z, b.z) + E(a.w, b.w);
     p.s = E(a.x, b.x) + E(E(cP, a.y), b.y);
     p.d = E(E(a.x, cP), b.y) - E(b.x, a.y);
-    p.ss = __dmul_rn(p.s, p.s);
+    p.ss = E(p.s, p.s);
     p.q = -1. + p.ss;
     return p;
 }
 // cos of the arc between b and c alone (the third side of a triangle at a)
 __device__ __forceinline__ double pair_cos(const double4_32a& b, const double4_32a& c) {
-    const auto E = [](double x, double y) { return early_mul(x, y); };
+    const auto E = [](double x, double y) { return grad_mul(x, y); };
     const double cP = E(b.z, c.z) + E(b.w, c.w);
     return E(b.x, c.x) + E(E(cP, b.y), c.y);
 }
@@ -348,10 +342,11 @@ __device__ __forceinline__ double pair_cos(const double4_32a& b, const double4_3
 // pair's terms and sin(theta) of the other point: returns (d/dtheta, d/dphi) components.
 __device__ __forceinline__ double2 grad_geodesic(const PairTerms& p, double sinT2) {
     const double dinv = f64_div_root(1., -p.q);   // 1 - s s = -(s s - 1) exactly
-    return make_double2(-p.d * dinv, early_mul(sinT2, p.sP) * dinv);
+    return make_double2(-p.d * dinv, grad_mul(sinT2, p.sP) * dinv);
 }
 
-// The other products of grad_triangle: the hardware multiply, spelled out.
+// grad_triangle's products that stay on the FP64 pipe, which balances the two: the roots' arguments
+// (chains of up to five products, ahead of everything else) and the last scaling.
 __device__ __forceinline__ double tri_mul(double x, double y) { return __dmul_rn(x, y); }
 // gradientTriangleArea (sphericalDomain.h:347-411) in the (theta, phi) basis of v1 for the triangle
 // (v1, v2, v3), without the sign of det(v1, v2, v3), from the terms of the pairs (v1, v2) and
@@ -363,22 +358,22 @@ __device__ __forceinline__ double tri_mul(double x, double y) { return __dmul_rn
 __device__ __forceinline__ double2 grad_triangle(const PairTerms& p12, const PairTerms& p13, double s23, double sinT2,
                                                  double sinT3, double R) {
     const auto M = tri_mul;
-    const auto E = [](double x, double y) { return early_mul(x, y); };
-    const double s12s13 = M(p12.s, p13.s);
+    const auto E = [](double x, double y) { return grad_mul(x, y); };
+    const double s12s13 = E(p12.s, p13.s);
     // 2 s12 s13 s23 = 2 ((s12 s13) s23): the factor two is exact wherever it is applied
     const double g = ((-p12.q - p13.ss) - M(s23, s23)) + sf::twice(M(s12s13, s23));
     const F64Divisor den1 = f64_root_divisor(M(M(p12.q, p12.q), g));
     const F64Divisor den2 = f64_root_divisor(M(M(p13.q, p13.q), g));
     const F64Divisor den3 = f64_root_divisor(M(M(M(M(p12.q, p13.q), p12.q), p13.q), g));
-    const double t = s23 - s12s13, u = p13.s - M(p12.s, s23), w = p12.s - M(p13.s, s23);
+    const double t = s23 - s12s13, u = p13.s - E(p12.s, s23), w = p12.s - E(p13.s, s23);
     // the d/dtheta numerators are formed while the square roots of the denominators run: integer pipes
     const double d12q13 = E(p12.d, p13.q), d13q12 = E(p13.d, p12.q);
     double gT = f64_div(d13q12 + E(p12.d, t), den1) + f64_div(d12q13 + E(p13.d, t), den2)
               - f64_div(E(d12q13, u) + E(d13q12, w), den3);
     gT = M(gT, R);
-    double gP = f64_div(-M(M(t, p12.sP), sinT2) - M(M(p12.q, p13.sP), sinT3), den1)
-              - f64_div(M(M(p13.q, p12.sP), sinT2) + M(M(t, p13.sP), sinT3), den2)
-              + f64_div(M(M(M(p13.q, u), p12.sP), sinT2) + M(M(M(p12.q, w), p13.sP), sinT3), den3);
+    double gP = f64_div(-E(E(t, p12.sP), sinT2) - E(E(p12.q, p13.sP), sinT3), den1)
+              - f64_div(E(E(p13.q, p12.sP), sinT2) + E(E(t, p13.sP), sinT3), den2)
+              + f64_div(E(E(E(p13.q, u), p12.sP), sinT2) + E(E(E(p12.q, w), p13.sP), sinT3), den3);
     gP = M(gP, R);
     return make_double2(gT, gP);
 }

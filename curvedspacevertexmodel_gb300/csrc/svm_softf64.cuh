@@ -235,6 +235,9 @@ SF_HD double mul(double a, double b) {
     return hw_mul(a, b);
 }
 
+// mul out of line, for kernels with dozens of products, whose code would not fit the instruction caches.
+SF_SLOW double mul_call(double a, double b) { return mul(a, b); }
+
 // 2 x (exact; zeros, subnormals, the largest binade, infinities and NaN take the hardware)
 SF_HD double twice(double x) {
     const unsigned long long u = bits(x);
