@@ -39,6 +39,7 @@ __device__ double rep_block_sum(double v) {
 // one block per replica: total area, excess over 4 pi R^2, fallback flag
 __global__ void k_rep_check(const double2* __restrict__ ap, const int* __restrict__ cellOff,
                             const double* __restrict__ repR, int* __restrict__ repFlag, double* __restrict__ repScal) {
+    step_begin();
     const int r = blockIdx.x;
     double s = 0.0;
     for (int c = cellOff[r] + threadIdx.x; c < cellOff[r + 1]; c += blockDim.x) s += ap[c].x;
@@ -95,7 +96,7 @@ struct BatchTuners {
 namespace svm {
 
 int launch_rep_check(svm_model* m) {
-    k_rep_check<<<m->nRep, kRB, 0, m->stream>>>(m->ap, m->repCellOff, m->repR, m->repFlag, m->repScal);
+    launch_next(m, k_rep_check, m->nRep, kRB, m->ap, m->repCellOff, m->repR, m->repFlag, m->repScal);
     return check_launch();
 }
 

@@ -118,6 +118,7 @@ __device__ __forceinline__ D3 vv_kick(D3 v, D3 f, double dt) {
 __global__ void k_fire_vv1(const FireState* __restrict__ Sp, double4_32a* __restrict__ pos,
                            double4_32a* __restrict__ vel, const double4_32a* __restrict__ force,
                            double* __restrict__ vnorm, int nV, double R) {
+    step_begin();
     const FireState S = *Sp;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nV) return;
@@ -135,11 +136,13 @@ __global__ void k_fire_vv1(const FireState* __restrict__ Sp, double4_32a* __rest
 __global__ void k_vv_drift(double4_32a* __restrict__ pos, double4_32a* __restrict__ vel,
                            const double4_32a* __restrict__ force, double* __restrict__ vnorm, int nV, double dt,
                            double R) {
+    step_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nV) return;
     vv_drift(pos, vel, vnorm, i, ld3(vel, i), ld3(force, i), dt, R);
 }
 __global__ void k_vv_half(double4_32a* __restrict__ vel, const double4_32a* __restrict__ force, int nV, double dt) {
+    step_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nV) return;
     st3(vel, i, vv_kick(ld3(vel, i), ld3(force, i), dt));
@@ -220,6 +223,7 @@ template <int kForm>
 __global__ void __launch_bounds__(slot_threads(kFireVerts), kForm == kFormVector ? 6 : kSlotMinBlocks)
     k_fire_force(ForceArgs A, FireState* __restrict__ Sp, int nV, double4_32a* __restrict__ force,
                  double4_32a* __restrict__ vel, double* __restrict__ partials, unsigned* __restrict__ ticket) {
+    step_begin();
     __shared__ double sh[32];
     __shared__ bool amLast;
     __shared__ SlotShared<kFireVerts> slots;
@@ -273,7 +277,7 @@ int fire_iteration(svm_fire* F) {
     const int bs = spread_block(m, m->nVertices), nb = (m->nVertices + bs - 1) / bs;
     {
         PhaseTimer pt(m, SVM_PHASE_MOVE);
-        k_fire_vv1<<<nb, bs, 0, m->stream>>>(F->d, m->pos[m->cur], m->vel, m->force, m->vnorm, m->nVertices, m->R);
+        launch_next(m, k_fire_vv1, nb, bs, F->d, m->pos[m->cur], m->vel, m->force, m->vnorm, m->nVertices, m->R);
     }
     m->cornersValid = false;
     int rc;
@@ -288,10 +292,10 @@ int fire_iteration(svm_fire* F) {
     PhaseTimer pt(m, SVM_PHASE_FORCE);
     const int nf = (m->nVertices + kFireVerts - 1) / kFireVerts;
     if (m->precision == SVM_PRECISION_FP64_VECTOR)
-        k_fire_force<kFormVector><<<nf, slot_threads(kFireVerts), 0, m->stream>>>(fargs(m), F->d, m->nVertices, m->force, m->vel,
+        launch_next(m, k_fire_force<kFormVector>, nf, slot_threads(kFireVerts), fargs(m), F->d, m->nVertices, m->force, m->vel,
                                                                         F->partials, F->ticket);
     else
-        k_fire_force<kFormReference><<<nf, slot_threads(kFireVerts), 0, m->stream>>>(fargs(m), F->d, m->nVertices, m->force,
+        launch_next(m, k_fire_force<kFormReference>, nf, slot_threads(kFireVerts), fargs(m), F->d, m->nVertices, m->force,
                                                                            m->vel, F->partials, F->ticket);
     return check_launch();
 }
@@ -418,7 +422,7 @@ int svm_fire_step(svm_fire* F) {
 
 int svm_vv_half(svm_model* m, double dt) {
     if (!m || !(dt == dt) || m->precision == SVM_PRECISION_MIXED) return SVM_ERR_ARG;
-    k_vv_half<<<(m->nVertices + kB - 1) / kB, kB, 0, m->stream>>>(m->vel, m->force, m->nVertices, dt);
+    launch_next(m, k_vv_half, (m->nVertices + kB - 1) / kB, kB, m->vel, m->force, m->nVertices, dt);
     return check_launch();
 }
 
@@ -428,7 +432,7 @@ int svm_velocity_verlet_step(svm_model* m, double dt, int nSteps) {
     for (int k = 0; k < nSteps; ++k) {
         {
             PhaseTimer pt(m, SVM_PHASE_MOVE);
-            k_vv_drift<<<nb, bs, 0, m->stream>>>(m->pos[m->cur], m->vel, m->force, m->vnorm, m->nVertices, dt, m->R);
+            launch_next(m, k_vv_drift, nb, bs, m->pos[m->cur], m->vel, m->force, m->vnorm, m->nVertices, dt, m->R);
         }
         m->cornersValid = false;
         int rc;
@@ -445,7 +449,7 @@ int svm_velocity_verlet_step(svm_model* m, double dt, int nSteps) {
             rc = launch_force_fp64(m);
             if (rc) return rc;
         }
-        k_vv_half<<<nb, bs, 0, m->stream>>>(m->vel, m->force, m->nVertices, dt);
+        launch_next(m, k_vv_half, nb, bs, m->vel, m->force, m->nVertices, dt);
         if (check_launch()) return SVM_ERR_CUDA;
     }
     return SVM_OK;

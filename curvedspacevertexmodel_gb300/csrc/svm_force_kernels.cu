@@ -39,6 +39,7 @@ using namespace svm;
 
 __global__ void __launch_bounds__(slot_threads(kSlotVerts), kSlotMinBlocks)
     k_force(ForceArgs A, int nV, double4_32a* __restrict__ force) {
+    step_begin();
     __shared__ SlotShared<> sh;
     const D3 f = block_slot_force<kFormAny>(A, nV, sh, NoSide());
     const int v = blockIdx.x * kSlotVerts + threadIdx.x;
@@ -56,6 +57,7 @@ __global__ void __launch_bounds__(slot_threads(kSlotVerts), kSlotMinBlocks)
     k_force_bd(ForceArgs A, int nV, double4_32a* __restrict__ force, double4_32a* __restrict__ posNext,
                const double* __restrict__ noise, uint64_t seed, const unsigned long long* __restrict__ stepCounter,
                double np, double fp, const ZigTable* __restrict__ zig, double* __restrict__ hostOut) {
+    step_begin();
     __shared__ SlotShared<> sh;
     __shared__ double xi[3 * kSlotVerts];
     const D3 f = block_slot_force<kFormAny>(A, nV, sh, [&](const SlotIndex& q) {
@@ -78,7 +80,7 @@ int slot_blocks(int nV) { return (nV + kSlotVerts - 1) / kSlotVerts; }
 namespace svm {
 
 int launch_force_fp64(svm_model* m) {
-    k_force<<<slot_blocks(m->nVertices), slot_threads(kSlotVerts), 0, m->stream>>>(force_args(m, m->cur), m->nVertices,
+    launch_next(m, k_force, slot_blocks(m->nVertices), slot_threads(kSlotVerts), force_args(m, m->cur), m->nVertices,
                                                                                   m->force);
     return check_launch();
 }
@@ -105,7 +107,7 @@ int launch_force_bd_fp64(svm_model* m, double np, double fp, int noiseMode, cons
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || !gZigAddr[dev]) return SVM_ERR_CUDA;
     const ZigTable* zig = gZigAddr[dev];
     const auto go = [&](auto kernel) {
-        kernel<<<slot_blocks(m->nVertices), slot_threads(kSlotVerts), 0, m->stream>>>(
+        launch_next(m, kernel, slot_blocks(m->nVertices), slot_threads(kSlotVerts),
             force_args(m, m->cur), m->nVertices, m->force, m->pos[nxt], noise, seed, m->stepCounter, np, fp, zig,
             m->ioHostOut);
     };

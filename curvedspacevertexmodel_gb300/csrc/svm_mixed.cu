@@ -132,6 +132,7 @@ __global__ void k32_corners(const float4* __restrict__ pos, const int4* __restri
                             const int4* __restrict__ vrpos, const int4* __restrict__ vnbr,
                             double2* __restrict__ corner, int Wc, int nV, const double* __restrict__ repR,
                             int t1test, float t1Threshold, T1Scratch t1) {
+    step_begin();
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nV) return;
     const float4 p = pos[v];
@@ -175,6 +176,7 @@ __global__ void k32_corners(const float4* __restrict__ pos, const int4* __restri
 }
 
 __global__ void k32_force(Args32 A, int nV, float4* __restrict__ force) {
+    step_begin();
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nV) return;
     const F3 f = vertex_force32(A, v, sf::narrow(A.repR[rep_of(A.pos[v])]));
@@ -187,6 +189,7 @@ __global__ void k32_force_bd(Args32 A, int nV, float4* __restrict__ force, float
                              const double* __restrict__ noise, uint64_t seed,
                              const unsigned long long* __restrict__ stepCounter, float np,
                              const float* __restrict__ repNp, float fp) {
+    step_begin();
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nV) return;
     const float4 p = A.pos[v];
@@ -240,14 +243,14 @@ namespace svm {
 
 int mixed_launch_corners(svm_model* m, bool t1test) {
     const int bs = m->blkCorners;
-    k32_corners<<<(m->nVertices + bs - 1) / bs, bs, 0, m->stream>>>(m->pos32[m->cur], m->vcell, m->vlast, m->vnext,
+    launch_next(m, k32_corners, (m->nVertices + bs - 1) / bs, bs, m->pos32[m->cur], m->vcell, m->vlast, m->vnext,
                                                                   m->vrpos, m->vnbr, m->corner, m->Wc, m->nVertices,
                                                                   m->repR, t1test ? 1 : 0, (float)m->t1Threshold, m->t1);
     return check_launch();
 }
 
 int mixed_launch_force(svm_model* m) {
-    k32_force<<<blocksFor(m->nVertices), kB, 0, m->stream>>>(args32(m, m->cur), m->nVertices, m->force32);
+    launch_next(m, k32_force, blocksFor(m->nVertices), kB, args32(m, m->cur), m->nVertices, m->force32);
     return check_launch();
 }
 
@@ -257,11 +260,11 @@ int mixed_launch_force_bd(svm_model* m, double T, double dt, double mu, int nois
     const float* repNp = m->nRep > 1 ? m->repNp : nullptr;
     const int bs = m->blkForce, nb = (m->nVertices + bs - 1) / bs;
     if (noiseMode == SVM_NOISE_BUFFER)
-        k32_force_bd<SVM_NOISE_BUFFER><<<nb, bs, 0, m->stream>>>(args32(m, m->cur), m->nVertices, m->force32,
+        launch_next(m, k32_force_bd<SVM_NOISE_BUFFER>, nb, bs, args32(m, m->cur), m->nVertices, m->force32,
                                                                 m->pos32[nxt], noise, seed, m->stepCounter, (float)np,
                                                                 repNp, (float)fp);
     else
-        k32_force_bd<SVM_NOISE_PHILOX><<<nb, bs, 0, m->stream>>>(args32(m, m->cur), m->nVertices, m->force32,
+        launch_next(m, k32_force_bd<SVM_NOISE_PHILOX>, nb, bs, args32(m, m->cur), m->nVertices, m->force32,
                                                                 m->pos32[nxt], noise, seed, m->stepCounter, (float)np,
                                                                 repNp, (float)fp);
     return check_launch();

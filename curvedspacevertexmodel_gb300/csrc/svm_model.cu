@@ -110,6 +110,7 @@ __device__ double block_sum(double v) {
 // One thread per vertex (large vertex counts: keeps each vertex's shared values in registers).
 // |p| of every vertex, once per corner pass: each is read by the vertex and its three neighbours.
 __global__ void k_vnorm(const double4_32a* __restrict__ pos, double* __restrict__ vnorm, int nV) {
+    step_begin();
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v < nV) vnorm[v] = pos_norm(ld3(pos, v));
 }
@@ -138,6 +139,7 @@ __global__ void k_edges(const double4_32a* __restrict__ pos, const double* __res
                         double4_32a* __restrict__ vsph, const int4* __restrict__ vnbr, const int4* __restrict__ vcell,
                         double4_32a* __restrict__ edgeC, double* __restrict__ edgeArc, int nV, double R, int t1test,
                         double t1Threshold, T1Scratch t1) {
+    step_begin();
     const int v = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
     const bool live = v < nV;
     int4 nb = make_int4(-1, -1, -1, -1);
@@ -204,6 +206,7 @@ __global__ void __launch_bounds__(3 * kCornerVerts) k_corner_s(
     const int4* __restrict__ vnext, const int4* __restrict__ vrpos, const int4* __restrict__ vnbr,
     const double4_32a* __restrict__ edgeC, const double* __restrict__ edgeArc, double2* __restrict__ corner, int Wc,
     int nV, double R) {
+    step_begin();
     __shared__ CornerShared sh;
     const int t = threadIdx.x, vi = t / 3, j = t - 3 * (t / 3), b = 3 * vi;
     const int v = blockIdx.x * kCornerVerts + vi;
@@ -247,6 +250,7 @@ __global__ void __launch_bounds__(256, 3) k_corner(const double4_32a* __restrict
                          const int4* __restrict__ vlast, const int4* __restrict__ vnext, const int4* __restrict__ vrpos,
                          const int4* __restrict__ vnbr, const double4_32a* __restrict__ edgeC,
                          const double* __restrict__ edgeArc, double2* __restrict__ corner, int Wc, int nV, double R) {
+    step_begin();
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nV) return;
     const int4 nb = vnbr[v], cells = vcell[v], lasts = vlast[v], nexts = vnext[v], rp = vrpos[v];
@@ -287,7 +291,8 @@ __global__ void k_cells(const PT* __restrict__ pos, const int* __restrict__ ring
                         double R0, const double* __restrict__ repR, PT* __restrict__ cellPos,
                         double4_32a* __restrict__ cellSph, double2* __restrict__ ap, double* __restrict__ partials,
                         unsigned* __restrict__ ticket, double* __restrict__ scalars, int* __restrict__ fallbackFlag,
-                        const double2* __restrict__ pref = nullptr, float2* __restrict__ dap32 = nullptr) {
+                        const double2* __restrict__ pref, float2* __restrict__ dap32) {
+    step_begin();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     double area = 0.0;
     if (c < nC) {
@@ -357,7 +362,8 @@ __global__ void k_fallback(const PT* __restrict__ pos, const int* __restrict__ r
                            const int* __restrict__ ringCount, const PT* __restrict__ cellPos, int Wc, int nC,
                            double R0, const int* __restrict__ fallbackFlag, const int* __restrict__ repFlag,
                            const double* __restrict__ repR, double2* __restrict__ ap,
-                           const double2* __restrict__ pref = nullptr, float2* __restrict__ dap32 = nullptr) {
+                           const double2* __restrict__ pref, float2* __restrict__ dap32) {
+    step_begin();
     if (!repFlag && *fallbackFlag == 0) return;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nC) return;
@@ -391,7 +397,8 @@ __global__ void __launch_bounds__(kFanThreads) k_fallback_fan(
     const PT* __restrict__ pos, const int* __restrict__ ring, const int* __restrict__ ringCount,
     const PT* __restrict__ cellPos, int Wc, int nC, double R0, const int* __restrict__ fallbackFlag,
     const int* __restrict__ repFlag, const double* __restrict__ repR, double2* __restrict__ ap,
-    const double2* __restrict__ pref = nullptr, float2* __restrict__ dap32 = nullptr) {
+    const double2* __restrict__ pref, float2* __restrict__ dap32) {
+    step_begin();
     if (!repFlag && *fallbackFlag == 0) return;
     __shared__ int cnt[kFanCells], off[kFanCells + 1], owner[kFanCells * 32];
     __shared__ double radius[kFanCells];
@@ -461,6 +468,7 @@ __global__ void k_move(double4_32a* __restrict__ pos, const double* __restrict__
 __global__ void k_t1_test(const double4_32a* __restrict__ pos, const float4* __restrict__ pos32,
                           const double* __restrict__ repR, const int4* __restrict__ vnbr,
                           const int4* __restrict__ vcell, int nV, double R, double t1Threshold, double cosLo, double cosHi, double s2Lo, double s2Hi, T1Scratch t1) {
+    step_begin();
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nV) return;
     const int4 nb = vnbr[v];
@@ -1057,6 +1065,7 @@ __device__ __forceinline__ void patch_touched(const ApplyArgs& A, const T1Scratc
 }
 // Batches: the patch over all replicas' touched cells, after k_t1_apply.
 __global__ void k_t1_patch(ApplyArgs A, T1Scratch t1) {
+    step_begin();
     if (blockIdx.x == 0 && threadIdx.x == 0) publish_ring_max(A);
     patch_touched(A, t1, *(volatile int*)(t1.ctr + 5), blockIdx.x, gridDim.x);
 }
@@ -1113,6 +1122,7 @@ __device__ void t1_reset(const T1Scratch& t1) {
     for (int k = 0; k < 3 + kT1CtlInts; ++k) c[k] = 0;
 }
 __global__ void __launch_bounds__(kApplyThreads) k_t1_apply(ApplyArgs A, T1Scratch t1, bool sphere) {
+    step_begin();
     __shared__ int buf[kExtractCap];
     __shared__ int heap[kHeapCap];
     __shared__ int nbuf, head, nheap, extractWord, nTouched;
@@ -1329,6 +1339,7 @@ __device__ bool grid_barrier(T1Ctl* ctl, int spinLimit) {
 // figures at launch_t1_apply.
 template <bool kCoop>
 __global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_parallel(ApplyArgs A, T1Scratch t1, int undoPer) {
+    step_begin();
     __shared__ T1Ctl sctl;
     T1Ctl* ctl = kCoop ? t1.ctl : &sctl;
     const int tid = threadIdx.x, seg = kCoop ? 0 : blockIdx.x;
@@ -1663,6 +1674,7 @@ __global__ void k_ring_index(const int* __restrict__ ring, const int* __restrict
 
 __global__ void k_energy(const double2* __restrict__ ap, const double2* __restrict__ pref, double Kr, int nC,
                          double* partials, unsigned* ticket, double* out) {
+    step_begin();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     double e = 0.0;
     if (c < nC) {
@@ -1734,6 +1746,7 @@ __global__ void k_dynamics(const double4_32a* __restrict__ ref, const PT* __rest
 // CPU (the director n as the previous step left it).
 __global__ void k_spp_move(double4_32a* __restrict__ pos, const double4_32a* __restrict__ dir,
                            const double4_32a* __restrict__ force, double dt, double mu, double v0, int nV, double R) {
+    step_begin();
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nV) return;
     const D3 n = ld3(dir, v), f = ld3(force, v);
@@ -1751,6 +1764,7 @@ template <int kNoise>
 __global__ void k_spp_dirs(const double4_32a* __restrict__ pos, double4_32a* __restrict__ dir,
                            const double* __restrict__ r, uint64_t seed,
                            const unsigned long long* __restrict__ stepCounter, double amp, int nV) {
+    step_begin();
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nV) return;
     const D3 p = ld3(pos, v);
@@ -1788,6 +1802,7 @@ __global__ void k_vicsek_target(const double4_32a* __restrict__ pos, const doubl
                                 const int4* __restrict__ vnbr, double4_32a* __restrict__ target,
                                 const double* __restrict__ r, uint64_t seed,
                                 const unsigned long long* __restrict__ stepCounter, double eta, int nV) {
+    step_begin();
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nV) return;
     double u, w;
@@ -1825,6 +1840,7 @@ __global__ void k_vicsek_target(const double4_32a* __restrict__ pos, const doubl
 // n += (dt / tau)(target - n), projected onto the tangent plane and normalised.
 __global__ void k_vicsek_update(const double4_32a* __restrict__ pos, double4_32a* __restrict__ dir,
                                 const double4_32a* __restrict__ target, double rate, int nV) {
+    step_begin();
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nV) return;
     const D3 p = ld3(pos, v), t = ld3(target, v);
@@ -1862,17 +1878,17 @@ int launch_corners(svm_model* m, bool t1test, bool vnormReady) {
     }
     if (!m->edgeC) return SVM_ERR_ARG;  // FP64 corners exist for single spheres only
     const int bv = spread_block(m, m->nVertices);
-    if (!vnormReady) k_vnorm<<<blocksFor(m->nVertices, bv), bv, 0, m->stream>>>(m->pos[m->cur], m->vnorm, m->nVertices);
-    k_edges<<<blocksFor(m->nVertices, bv), bv, 0, m->stream>>>(m->pos[m->cur], m->vnorm, m->vsph, m->vnbr, m->vcell, m->edgeC,
+    if (!vnormReady) launch_next(m, k_vnorm, blocksFor(m->nVertices, bv), bv, m->pos[m->cur], m->vnorm, m->nVertices);
+    launch_next(m, k_edges, blocksFor(m->nVertices, bv), bv, m->pos[m->cur], m->vnorm, m->vsph, m->vnbr, m->vcell, m->edgeC,
                                                               m->edgeArc, m->nVertices, m->R, t1test ? 1 : 0,
                                                               m->t1Threshold, m->t1);
     // both corner kernels write the same values; the three-thread one is faster below ~100k vertices
     if (m->nVertices < kCornerSlotsBelow)
-        k_corner_s<<<(m->nVertices + kCornerVerts - 1) / kCornerVerts, 3 * kCornerVerts, 0, m->stream>>>(
+        launch_next(m, k_corner_s, (m->nVertices + kCornerVerts - 1) / kCornerVerts, 3 * kCornerVerts,
             m->pos[m->cur], m->vcell, m->vlast, m->vnext, m->vrpos, m->vnbr, m->edgeC, m->edgeArc, m->corner, m->Wc,
             m->nVertices, m->R);
     else
-        k_corner<<<blocksFor(m->nVertices), kBlock, 0, m->stream>>>(m->pos[m->cur], m->vcell, m->vlast, m->vnext,
+        launch_next(m, k_corner, blocksFor(m->nVertices), kBlock, m->pos[m->cur], m->vcell, m->vlast, m->vnext,
                                                                    m->vrpos, m->vnbr, m->edgeC, m->edgeArc, m->corner,
                                                                    m->Wc, m->nVertices, m->R);
     m->cornersValid = true;
@@ -1887,7 +1903,7 @@ int max_block_cells_batch() {
 
 static int launch_cells_batch(svm_model* m) {
     const int bs = m->blkCells;
-    k_cells<float4><<<(m->nCells + bs - 1) / bs, bs, 0, m->stream>>>(
+    launch_next(m, k_cells<float4>, (m->nCells + bs - 1) / bs, bs,
         m->pos32[m->cur], m->ring, m->ringCount, m->corner, m->Wc, m->nCells, m->R, m->repR, m->cellPos32, nullptr,
         m->ap, nullptr, nullptr, nullptr, nullptr, m->pref, m->dap32);
     return check_launch();
@@ -1902,13 +1918,13 @@ static int launch_cells(svm_model* m) {
             if (int rc = batch_tuned_cells(m, launch_cells_batch)) return rc;
             if (int rc = launch_rep_check(m)) return rc;
         } else if (mixed) {
-            k_cells<float4><<<blocksFor(m->nCells), kBlock, 0, m->stream>>>(
+            launch_next(m, k_cells<float4>, blocksFor(m->nCells), kBlock,
                 m->pos32[m->cur], m->ring, m->ringCount, m->corner, m->Wc, m->nCells, m->R, m->repR, m->cellPos32,
                 nullptr, m->ap, m->partials, m->ticket, m->scalars, m->fallbackFlag, m->pref, m->dap32);
         } else {
-            k_cells<double4_32a><<<blocksFor(m->nCells), kBlock, 0, m->stream>>>(
+            launch_next(m, k_cells<double4_32a>, blocksFor(m->nCells), kBlock,
                 m->pos[m->cur], m->ring, m->ringCount, m->corner, m->Wc, m->nCells, m->R, nullptr, m->cellPos,
-                m->cellSph, m->ap, m->partials, m->ticket, m->scalars, m->fallbackFlag);
+                m->cellSph, m->ap, m->partials, m->ticket, m->scalars, m->fallbackFlag, nullptr, nullptr);
         }
     }
     PhaseTimer pt(m, SVM_PHASE_FALLBACK);
@@ -1916,20 +1932,20 @@ static int launch_cells(svm_model* m) {
     if (m->Wc <= 32) {
         const int nf = (m->nCells + kFanCells - 1) / kFanCells;
         if (mixed)
-            k_fallback_fan<float4><<<nf, kFanThreads, 0, m->stream>>>(
+            launch_next(m, k_fallback_fan<float4>, nf, kFanThreads,
                 m->pos32[m->cur], m->ring, m->ringCount, m->cellPos32, m->Wc, m->nCells, m->R, m->fallbackFlag,
                 batch ? m->repFlag : nullptr, m->repR, m->ap, m->pref, m->dap32);
         else
-            k_fallback_fan<double4_32a><<<nf, kFanThreads, 0, m->stream>>>(
+            launch_next(m, k_fallback_fan<double4_32a>, nf, kFanThreads,
                 m->pos[m->cur], m->ring, m->ringCount, m->cellPos, m->Wc, m->nCells, m->R, m->fallbackFlag, nullptr,
-                nullptr, m->ap);
+                nullptr, m->ap, nullptr, nullptr);
     } else if (mixed)
-        k_fallback<float4><<<nb, kBlock, 0, m->stream>>>(m->pos32[m->cur], m->ring, m->ringCount, m->cellPos32, m->Wc,
+        launch_next(m, k_fallback<float4>, nb, kBlock, m->pos32[m->cur], m->ring, m->ringCount, m->cellPos32, m->Wc,
                                                          m->nCells, m->R, m->fallbackFlag, batch ? m->repFlag : nullptr,
                                                          m->repR, m->ap, m->pref, m->dap32);
     else
-        k_fallback<double4_32a><<<nb, kBlock, 0, m->stream>>>(m->pos[m->cur], m->ring, m->ringCount, m->cellPos, m->Wc,
-                                                              m->nCells, m->R, m->fallbackFlag, nullptr, nullptr, m->ap);
+        launch_next(m, k_fallback<double4_32a>, nb, kBlock, m->pos[m->cur], m->ring, m->ringCount, m->cellPos, m->Wc,
+                                                              m->nCells, m->R, m->fallbackFlag, nullptr, nullptr, m->ap, nullptr, nullptr);
     return check_launch();
 }
 
@@ -2053,11 +2069,11 @@ int launch_t1_apply(svm_model* m, int bump) {
         if (cudaLaunchKernelEx(&cfg, k_t1_parallel<true>, apply_args(m, bump), m->t1, m->t1.undoCap) != cudaSuccess)
             return SVM_ERR_CUDA;
     } else {
-        k_t1_parallel<false><<<nSeg, batch ? kParThreadsBatch : kParThreads, 0, m->stream>>>(apply_args(m, bump), m->t1,
+        launch_next(m, k_t1_parallel<false>, nSeg, batch ? kParThreadsBatch : kParThreads, apply_args(m, bump), m->t1,
                                                                                              m->t1.undoCap / nSeg);
     }
-    k_t1_apply<<<1, kApplyThreads, 0, m->stream>>>(apply_args(m, bump), m->t1, !batch);
-    if (batch) k_t1_patch<<<2 * m->sms, 256, 0, m->stream>>>(apply_args(m, bump), m->t1);
+    launch_next(m, k_t1_apply, 1, kApplyThreads, apply_args(m, bump), m->t1, !batch);
+    if (batch) launch_next(m, k_t1_patch, 2 * m->sms, 256, apply_args(m, bump), m->t1);
     if (int rc = check_launch()) return rc;
     return mark_pass(m);
 }
@@ -2069,7 +2085,7 @@ int launch_t1_test(svm_model* m) {
     double lo, hi, s2lo, s2hi;
     t1_bracket(m->t1Threshold, m->R, &lo, &hi);
     t1_sin2_bracket(m->t1Threshold, m->R, &s2lo, &s2hi);
-    k_t1_test<<<blocksFor(m->nVertices), kBlock, 0, m->stream>>>(
+    launch_next(m, k_t1_test, blocksFor(m->nVertices), kBlock,
         m->pos[m->cur], m->precision == SVM_PRECISION_MIXED ? m->pos32[m->cur] : nullptr, m->repR, m->vnbr, m->vcell,
         m->nVertices, m->R, m->t1Threshold, lo, hi, s2lo, s2hi, m->t1);
     return check_launch();
@@ -2467,7 +2483,7 @@ int svm_model_compute_forces(svm_model* m) {
 
 int svm_model_compute_energy(svm_model* m, double* e) {
     if (!m || !e) return SVM_ERR_ARG;
-    k_energy<<<svm::blocksFor(m->nCells), svm::kBlock, 0, m->stream>>>(m->ap, m->pref, m->Kr, m->nCells,
+    launch_next(m, k_energy, svm::blocksFor(m->nCells), svm::kBlock, m->ap, m->pref, m->Kr, m->nCells,
                                                                          m->partials + m->maxPartialBlocks,
                                                                          m->ticket + 1, m->scalars + 2);
     if (svm::check_launch()) return SVM_ERR_CUDA;
@@ -2831,7 +2847,7 @@ static int step_io_sequence(svm_model* m, double T, double dt, double mu, uint64
     m->ioHostOut = nullptr;
     if (rc) return rc;
     if (energyOut) {
-        k_energy<<<svm::blocksFor(m->nCells), svm::kBlock, 0, m->stream>>>(m->ap, m->pref, m->Kr, m->nCells,
+        launch_next(m, k_energy, svm::blocksFor(m->nCells), svm::kBlock, m->ap, m->pref, m->Kr, m->nCells,
                                                                              m->partials + m->maxPartialBlocks,
                                                                              m->ticket + 1, m->scalars + 2);
         if (svm::check_launch()) return SVM_ERR_CUDA;
@@ -2905,7 +2921,7 @@ int svm_spp_step(svm_model* m, double dt, double mu, double v0, double tau, int 
                                  m->stream));
     int rc = svm::launch_geometry(m);
     if (rc || (rc = svm::launch_force_fp64(m))) return rc;
-    k_spp_move<<<svm::blocksFor(m->nVertices), svm::kBlock, 0, m->stream>>>(m->pos[m->cur], m->dir, m->force, dt, mu,
+    launch_next(m, k_spp_move, svm::blocksFor(m->nVertices), svm::kBlock, m->pos[m->cur], m->dir, m->force, dt, mu,
                                                                             v0, m->nVertices, m->R);
     if (svm::check_launch()) return SVM_ERR_CUDA;
     m->cornersValid = false;
@@ -2913,10 +2929,10 @@ int svm_spp_step(svm_model* m, double dt, double mu, double v0, double tau, int 
     if ((rc = svm::launch_corners(m, !m->restricted)) || (rc = svm::launch_t1_apply(m, 1))) return rc;
     const double amp = sqrt(2.0 * dt * tau);
     if (noiseMode == SVM_NOISE_BUFFER)
-        k_spp_dirs<SVM_NOISE_BUFFER><<<svm::blocksFor(m->nVertices), svm::kBlock, 0, m->stream>>>(
+        launch_next(m, k_spp_dirs<SVM_NOISE_BUFFER>, svm::blocksFor(m->nVertices), svm::kBlock,
             m->pos[m->cur], m->dir, m->noiseBuf, seed, m->stepCounter, amp, m->nVertices);
     else
-        k_spp_dirs<SVM_NOISE_PHILOX><<<svm::blocksFor(m->nVertices), svm::kBlock, 0, m->stream>>>(
+        launch_next(m, k_spp_dirs<SVM_NOISE_PHILOX>, svm::blocksFor(m->nVertices), svm::kBlock,
             m->pos[m->cur], m->dir, nullptr, seed, m->stepCounter, amp, m->nVertices);
     return svm::check_launch();
 }
@@ -2931,19 +2947,19 @@ int svm_vicsek_step(svm_model* m, double dt, double mu, double v0, double eta, d
                                  m->stream));
     int rc = svm::launch_geometry(m);
     if (rc || (rc = svm::launch_force_fp64(m))) return rc;
-    k_spp_move<<<svm::blocksFor(m->nVertices), svm::kBlock, 0, m->stream>>>(m->pos[m->cur], m->dir, m->force, dt, mu,
+    launch_next(m, k_spp_move, svm::blocksFor(m->nVertices), svm::kBlock, m->pos[m->cur], m->dir, m->force, dt, mu,
                                                                             v0, m->nVertices, m->R);
     if (svm::check_launch()) return SVM_ERR_CUDA;
     m->cornersValid = false;
     if ((rc = svm::launch_corners(m, !m->restricted)) || (rc = svm::launch_t1_apply(m, 1))) return rc;
     if (noiseMode == SVM_NOISE_BUFFER)
-        k_vicsek_target<SVM_NOISE_BUFFER><<<svm::blocksFor(m->nVertices), svm::kBlock, 0, m->stream>>>(
+        launch_next(m, k_vicsek_target<SVM_NOISE_BUFFER>, svm::blocksFor(m->nVertices), svm::kBlock,
             m->pos[m->cur], m->dir, m->vnbr, m->dirTarget, m->noiseBuf, seed, m->stepCounter, eta, m->nVertices);
     else
-        k_vicsek_target<SVM_NOISE_PHILOX><<<svm::blocksFor(m->nVertices), svm::kBlock, 0, m->stream>>>(
+        launch_next(m, k_vicsek_target<SVM_NOISE_PHILOX>, svm::blocksFor(m->nVertices), svm::kBlock,
             m->pos[m->cur], m->dir, m->vnbr, m->dirTarget, nullptr, seed, m->stepCounter, eta, m->nVertices);
     if (svm::check_launch()) return SVM_ERR_CUDA;
-    k_vicsek_update<<<svm::blocksFor(m->nVertices), svm::kBlock, 0, m->stream>>>(m->pos[m->cur], m->dir, m->dirTarget,
+    launch_next(m, k_vicsek_update, svm::blocksFor(m->nVertices), svm::kBlock, m->pos[m->cur], m->dir, m->dirTarget,
                                                                                  dt / tau, m->nVertices);
     return svm::check_launch();
 }
