@@ -248,16 +248,79 @@ __device__ __forceinline__ double included_angle(D3 p1, D3 p2, D3 p3) {
 //
 // With `clamp` (the mixed form) the cosine is clamped to [-1, 1]: for a nearly straight corner its
 // rounding can leave the domain, where acos is NaN (the reference does not clamp, and the FP64
-// form keeps that behaviour).
+// form keeps that behaviour).  In two parts, around the arccosine; comparisons on the integer pipes.
+__device__ __forceinline__ bool positive(double x) {   // x > 0
+    return (unsigned long long)__double_as_longlong(x) - 1ull < 0x7ff0000000000000ull;
+}
+template <bool clamp = false>
+__device__ __forceinline__ double included_cos(D3 Cx, D3 Cl, double nx, double nl) {
+    double c = f64_div(dot3e(Cx, Cl), early_mul(nx, nl));
+    // fmin(1, fmax(-1, c)), a NaN to -1
+    if (clamp) {
+        const unsigned long long b = (unsigned long long)__double_as_longlong(c), m = b & 0x7fffffffffffffffull;
+        if (m > 0x3ff0000000000000ull) c = (b >> 63) || m > 0x7ff0000000000000ull ? -1.0 : 1.0;
+    }
+    return c;
+}
+// the angle from its arccosine a (in [0, pi], or NaN) and whether det(pl, p, px) > 0: a, or 2 pi - a
+__device__ __forceinline__ double included_finish(double a, bool detPositive) {
+    if (detPositive) a = positive(a) ? 2. * kPI - a : -a;
+    return a;
+}
 template <bool clamp = false>
 __device__ __forceinline__ double included_angle_pre(D3 Cx, D3 Cl, double nx, double nl, D3 pl) {
-    const double det = dot3e(pl, Cx);
-    double c = f64_div(dot3e(Cx, Cl), early_mul(nx, nl));
-    if (clamp) c = fmin(1.0, fmax(-1.0, c));
-    double a = svm_acos(c);
-    if (det > 0) a = -a;
-    if (a < 0) a += 2. * kPI;
-    return a;
+    const bool dp = positive(dot3e(pl, Cx));
+    return included_finish(svm_acos(included_cos<clamp>(Cx, Cl, nx, nl)), dp);
+}
+
+// Arccosines of a block's cosines with like magnitudes on the same warps.  An arccosine evaluates one of
+// two expansions by the magnitude of its argument, and the angles of a vertex model (60 to 180 degrees)
+// fall on both sides, so a warp of them in vertex order runs both: about 50 FP64 instructions instead of
+// 25.  The block's kPer values per thread are dealt out with the magnitudes below kAcosSplit first and the
+// others last (one warp's worth mixed), evaluated, and dealt back: the same value for each.
+// val: kPer blockDim.x doubles, src: as many shorts, warpHigh: an int per warp.  Every thread of the
+// block calls it.
+// The boundary is where the measured time is least; the corner phase against one arccosine per thread in
+// vertex order: FP32 positions 1M cells 800 -> 589 us, 100k 100 -> 74.5 (with the boundary at 0.5 84.4, 0.55
+// 82.7, 0.6 89.6, 0.625 94.2), FP64 100k 123 -> 102.
+constexpr unsigned kAcosSplit = 0x3fe26666u;   // high word of the boundary, 0.575
+template <int kPer>
+__device__ __forceinline__ void block_acos(double (&c)[kPer], double* val, unsigned short* src, int* warpHigh) {
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, n = blockDim.x;
+    unsigned high[kPer];
+    int before[kPer], mine = 0;   // high values of the warp ahead of this one, by (j, lane)
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        high[j] = ((unsigned)__double2hiint(c[j]) & 0x7fffffffu) >= kAcosSplit;
+        const unsigned m = __ballot_sync(0xffffffffu, high[j]);
+        before[j] = mine + __popc(m & ((1u << lane) - 1u));
+        mine += __popc(m);
+    }
+    if (lane == 0) warpHigh[warp] = mine;
+    __syncthreads();
+    int ahead = 0;   // high values of the warps ahead
+    for (int w = 0; w < warp; ++w) ahead += warpHigh[w];
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        const int h = ahead + before[j], k = 32 * kPer * warp + 32 * j + lane;
+        const int at = high[j] ? kPer * n - 1 - h : k - h;
+        val[at] = c[j];
+        src[at] = (unsigned short)(j * n + t);
+    }
+    __syncthreads();
+    double a[kPer];
+    int from[kPer];
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        a[j] = svm_acos(val[j * n + t]);
+        from[j] = src[j * n + t];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) val[from[j]] = a[j];
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) c[j] = val[j * n + t];
 }
 // element j of a three-element register array (selects, no local-memory indexing)
 template <class T>
@@ -282,14 +345,27 @@ __device__ __forceinline__ double triangle_area_unit(D3 p1, D3 p2, D3 p3, double
 __device__ __forceinline__ double triangle_area(D3 q1, D3 q2, D3 q3, double R) {
     return triangle_area_unit(unit_corner(q1), unit_corner(q2), unit_corner(q3), R);
 }
-// the same from the normalised corners
-__device__ __forceinline__ double triangle_area_unit(D3 p1, D3 p2, D3 p3, double R) {
-    double d12 = dot3e(p1, p2), d13 = dot3e(p1, p3), d23 = dot3e(p2, p3);
+// the cosines of the three angles, from the normalised corners
+__device__ __forceinline__ void triangle_cosines(D3 p1, D3 p2, D3 p3, double (&c)[3]) {
+    const double d12 = dot3e(p1, p2), d13 = dot3e(p1, p3), d23 = dot3e(p2, p3);
+    const double s12 = f64_sqrt(1 - d12 * d12), s13 = f64_sqrt(1 - d13 * d13), s23 = f64_sqrt(1 - d23 * d23);
+    c[0] = f64_div(d23 - d12 * d13, s12 * s13);
+    c[1] = f64_div(d12 - d13 * d23, s13 * s23);
+    c[2] = f64_div(d13 - d12 * d23, s12 * s23);
+}
+// the area from the three angles
+__device__ __forceinline__ double triangle_sum(const double (&a)[3], double R) {
     double area = -kPI;
-    area += svm_acos(f64_div(d23 - d12 * d13, f64_sqrt(1 - d12 * d12) * f64_sqrt(1 - d13 * d13)));
-    area += svm_acos(f64_div(d12 - d13 * d23, f64_sqrt(1 - d13 * d13) * f64_sqrt(1 - d23 * d23)));
-    area += svm_acos(f64_div(d13 - d12 * d23, f64_sqrt(1 - d12 * d12) * f64_sqrt(1 - d23 * d23)));
+    area += a[0];
+    area += a[1];
+    area += a[2];
     return area * (R * R);
+}
+__device__ __forceinline__ double triangle_area_unit(D3 p1, D3 p2, D3 p3, double R) {
+    double c[3];
+    triangle_cosines(p1, p2, p3, c);
+    const double a[3] = {svm_acos(c[0]), svm_acos(c[1]), svm_acos(c[2])};
+    return triangle_sum(a, R);
 }
 
 // Spherical coordinates of a point as the reference's gradients compute them
@@ -613,10 +689,11 @@ __device__ __forceinline__ void step_begin() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 template <class... Params, class... Args>
-inline void launch_next(const svm_model* m, void (*kernel)(Params...), int grid, int block, Args&&... args) {
+inline void launch_next_smem(const svm_model* m, void (*kernel)(Params...), int grid, int block, int smem, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = m->stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -625,6 +702,10 @@ inline void launch_next(const svm_model* m, void (*kernel)(Params...), int grid,
     cfg.numAttrs = early_launch(m) ? 1 : 0;
     // (an error stays with the runtime for check_launch)
     (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+template <class... Params, class... Args>
+inline void launch_next(const svm_model* m, void (*kernel)(Params...), int grid, int block, Args&&... args) {
+    launch_next_smem(m, kernel, grid, block, 0, static_cast<Args&&>(args)...);
 }
 #endif
 // launch helpers shared across translation units (svm_model.cu)

@@ -34,7 +34,6 @@ __device__ __forceinline__ F3 operator-(F3 a, F3 b) { return F3{a.x - b.x, a.y -
 __device__ __forceinline__ F3 operator*(float s, F3 a) { return F3{s * a.x, s * a.y, s * a.z}; }
 __device__ __forceinline__ float dotf(F3 a, F3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 __device__ __forceinline__ F3 crossf(F3 a, F3 b) { return F3{a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x}; }
-__device__ __forceinline__ F3 unit(F3 a) { return (1.0f / sqrtf(dotf(a, a))) * a; }
 
 // Unit tangent at a pointing away from the neighbour at a + d (gradient of the geodesic distance
 // at any radius).  d is the raw difference of the two FP32 positions: for nearby points it is
@@ -133,45 +132,60 @@ __global__ void k32_corners(const float4* __restrict__ pos, const int4* __restri
                             double2* __restrict__ corner, int Wc, int nV, const double* __restrict__ repR,
                             int t1test, float t1Threshold, T1Scratch t1) {
     step_begin();
+    // block_acos's arrays: 3 blockDim.x values, their sources, a count per warp
+    extern __shared__ double cornerSh[];
+    double* val = cornerSh;
+    int* warpHigh = reinterpret_cast<int*>(val + 3 * blockDim.x);
+    unsigned short* src = reinterpret_cast<unsigned short*>(warpHigh + 32);
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= nV) return;
-    const float4 p = pos[v];
-    const float R = sf::narrow(repR[rep_of(p)]);
-    const D3 pd = ld3(pos, v);
-    const int4 cells = vcell[v], lasts = vlast[v], nexts = vnext[v], rp = vrpos[v], nb = vnbr[v];
-    // per neighbour: FP64 cross product with p and its norm (for the included angles), FP32 arc
-    D3 U[3], C[3];
-    double nC[3];
-    float arc[3];
+    const bool live = v < nV;
+    float4 p;
+    float R, arcs[3];
+    double cosine[3] = {-1.0, -1.0, -1.0};
+    bool flip[3] = {false, false, false}, ok[3];
+    int4 cells, lasts, nexts;
+    if (live) {
+        p = pos[v];
+        R = sf::narrow(repR[rep_of(p)]);
+        const D3 pd = ld3(pos, v);
+        const int4 nb = vnbr[v];
+        cells = vcell[v]; lasts = vlast[v]; nexts = vnext[v];
+        // per neighbour: FP64 cross product with p and its norm (for the included angles), FP32 arc
+        D3 U[3], C[3];
+        double nC[3];
+        float arc[3];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-        const float4 q = pos[comp(nb, j)];
-        U[j] = D3{sf::widen(q.x), sf::widen(q.y), sf::widen(q.z)};
-        C[j] = cross3e(pd, U[j]);
-        nC[j] = f64_sqrt(dot3e(C[j], C[j]));
-        arc[j] = arc32(q, p, R);
-    }
-#pragma unroll
-    for (int s = 0; s < 3; ++s) {
-        const int jl = nbr_slot(nb, comp(lasts, s)), jx = nbr_slot(nb, comp(nexts, s));
-        double2 cr;
-        if (jl >= 0 && jx >= 0) {
-            cr = make_double2(sf::widen(pick3(arc, jl)), included_angle_pre<true>(pick3(C, jx), pick3(C, jl),
-                                                                               pick3(nC, jx), pick3(nC, jl), pick3(U, jl)));
-        } else {  // inconsistent lists: evaluate directly
-            const int L = comp(lasts, s), X = comp(nexts, s);
-            cr = make_double2(sf::widen(arc32(pos[L], p, R)), included_angle_clamped(ld3(pos, L), pd, ld3(pos, X)));
+        for (int j = 0; j < 3; ++j) {
+            const float4 q = pos[comp(nb, j)];
+            U[j] = D3{sf::widen(q.x), sf::widen(q.y), sf::widen(q.z)};
+            C[j] = cross3e(pd, U[j]);
+            nC[j] = f64_sqrt(dot3e(C[j], C[j]));
+            arc[j] = arc32(q, p, R);
+            const int u = comp(nb, j);
+            if (t1test && v < u && arc[j] < t1Threshold) t1_flag(t1, 3 * v + j, v, u, rep_of(p), vnbr, vcell);
         }
-        corner[(long)comp(cells, s) * Wc + comp(rp, s)] = cr;
-    }
-    if (t1test) {
 #pragma unroll
         for (int s = 0; s < 3; ++s) {
-            const int u = comp(nb, s);
-            if (v < u && arc[s] < t1Threshold) {
-                t1_flag(t1, 3 * v + s, v, u, rep_of(p), vnbr, vcell);
+            const int jl = nbr_slot(nb, comp(lasts, s)), jx = nbr_slot(nb, comp(nexts, s));
+            ok[s] = jl >= 0 && jx >= 0;
+            if (ok[s]) {
+                arcs[s] = pick3(arc, jl);
+                flip[s] = positive(dot3e(pick3(U, jl), pick3(C, jx)));
+                cosine[s] = included_cos<true>(pick3(C, jx), pick3(C, jl), pick3(nC, jx), pick3(nC, jl));
             }
         }
+    }
+    block_acos(cosine, val, src, warpHigh);
+    if (!live) return;
+    const int4 rp = vrpos[v];
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+        double2 cr = make_double2(sf::widen(arcs[s]), included_finish(cosine[s], flip[s]));
+        if (!ok[s]) {  // inconsistent lists: evaluate directly
+            const int L = comp(lasts, s), X = comp(nexts, s);
+            cr = make_double2(sf::widen(arc32(pos[L], p, R)), included_angle_clamped(ld3(pos, L), ld3(pos, v), ld3(pos, X)));
+        }
+        corner[(long)comp(cells, s) * Wc + comp(rp, s)] = cr;
     }
 }
 
@@ -241,9 +255,11 @@ Args32 args32(svm_model* m, int buf) {
 
 namespace svm {
 
+// dynamic shared memory of k32_corners (at most 31 KB, at 1024 threads)
+static int corner_smem(int threads) { return 3 * threads * (int)(sizeof(double) + sizeof(unsigned short)) + 32 * (int)sizeof(int); }
 int mixed_launch_corners(svm_model* m, bool t1test) {
     const int bs = m->blkCorners;
-    launch_next(m, k32_corners, (m->nVertices + bs - 1) / bs, bs, m->pos32[m->cur], m->vcell, m->vlast, m->vnext,
+    launch_next_smem(m, k32_corners, (m->nVertices + bs - 1) / bs, bs, corner_smem(bs), m->pos32[m->cur], m->vcell, m->vlast, m->vnext,
                                                                   m->vrpos, m->vnbr, m->corner, m->Wc, m->nVertices,
                                                                   m->repR, t1test ? 1 : 0, (float)m->t1Threshold, m->t1);
     return check_launch();

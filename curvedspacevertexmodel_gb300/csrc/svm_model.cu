@@ -210,6 +210,9 @@ __global__ void __launch_bounds__(4 * kFewVerts) k_corners_few(
     step_begin();
     __shared__ double cx[3 * kFewVerts], cy[3 * kFewVerts], cz[3 * kFewVerts], nc[3 * kFewVerts];
     __shared__ double ux[3 * kFewVerts], uy[3 * kFewVerts], uz[3 * kFewVerts], arcs[3 * kFewVerts];
+    __shared__ double val[4 * kFewVerts];
+    __shared__ unsigned short src[4 * kFewVerts];
+    __shared__ int warpHigh[4 * kFewVerts / 32];
     const int t = threadIdx.x;
     if (t >= 3 * kFewVerts) {
         const int v = blockIdx.x * kFewVerts + t - 3 * kFewVerts;
@@ -229,15 +232,26 @@ __global__ void __launch_bounds__(4 * kFewVerts) k_corners_few(
         if (t1test && v < u && arc < t1Threshold) t1_flag(t1, 3 * v + j, v, u, 0, vnbr, vcell);
     }
     __syncthreads();
+    double cosine[1] = {-1.0}, arc = 0.0;
+    bool flip = false, ok = false;
+    int4 cells, lasts, nexts;
+    if (live) {
+        cells = vcell[v]; lasts = vlast[v]; nexts = vnext[v];
+        const int jl = nbr_slot(nb, comp(lasts, j)), jx = nbr_slot(nb, comp(nexts, j));
+        ok = jl >= 0 && jx >= 0;
+        if (ok) {
+            const int l = b + jl, x = b + jx;
+            const D3 X{cx[x], cy[x], cz[x]};
+            arc = arcs[l];
+            flip = positive(dot3e(D3{ux[l], uy[l], uz[l]}, X));
+            cosine[0] = included_cos(X, D3{cx[l], cy[l], cz[l]}, nc[x], nc[l]);
+        }
+    }
+    block_acos(cosine, val, src, warpHigh);
     if (!live) return;
-    const int4 cells = vcell[v], lasts = vlast[v], nexts = vnext[v], rp = vrpos[v];
-    const int jl = nbr_slot(nb, comp(lasts, j)), jx = nbr_slot(nb, comp(nexts, j));
-    double2 cr;
-    if (jl >= 0 && jx >= 0) {
-        const int l = b + jl, x = b + jx;
-        cr = make_double2(arcs[l], included_angle_pre(D3{cx[x], cy[x], cz[x]}, D3{cx[l], cy[l], cz[l]}, nc[x], nc[l],
-                                                      D3{ux[l], uy[l], uz[l]}));
-    } else {  // inconsistent lists: evaluate directly
+    const int4 rp = vrpos[v];
+    double2 cr = make_double2(arc, included_finish(cosine[0], flip));
+    if (!ok) {  // inconsistent lists: evaluate directly
         const D3 p = ld3(pos, v), pl = ld3(pos, comp(lasts, j)), px = ld3(pos, comp(nexts, j));
         cr = make_double2(geodesic(pl, p, R), included_angle(pl, p, px));
     }
@@ -248,31 +262,49 @@ __global__ void __launch_bounds__(4 * kFewVerts) k_corners_few(
 // angle at the vertex (the per-corner terms of computeGeometryCPU, sphericalVertexModel.cpp:257-276)
 // from the edge terms of k_edges.  Compiled for six blocks of 128 per SM (80 registers, with some
 // spill).
-__global__ void __launch_bounds__(128, 6) k_corner(const double4_32a* __restrict__ pos, const int4* __restrict__ vcell,
+constexpr int kCornerThreads = 128;
+__global__ void __launch_bounds__(kCornerThreads, 6) k_corner(const double4_32a* __restrict__ pos, const int4* __restrict__ vcell,
                          const int4* __restrict__ vlast, const int4* __restrict__ vnext, const int4* __restrict__ vrpos,
                          const int4* __restrict__ vnbr, const double4_32a* __restrict__ edgeC,
                          const double* __restrict__ edgeArc, double2* __restrict__ corner, int Wc, int nV, double R) {
     step_begin();
+    __shared__ double val[3 * kCornerThreads];
+    __shared__ unsigned short src[3 * kCornerThreads];
+    __shared__ int warpHigh[kCornerThreads / 32];
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= nV) return;
-    const int4 nb = vnbr[v], cells = vcell[v], lasts = vlast[v], nexts = vnext[v], rp = vrpos[v];
-    D3 C[3], U[3];
-    double nC[3], arc[3];
-    bool ok = true;
+    const bool live = v < nV;
+    double cosine[3] = {-1.0, -1.0, -1.0}, arcs[3];
+    bool flip[3] = {false, false, false}, ok = true;
+    int4 cells, lasts, nexts;
+    if (live) {
+        const int4 nb = vnbr[v];
+        cells = vcell[v]; lasts = vlast[v]; nexts = vnext[v];
+        D3 C[3], U[3];
+        double nC[3], arc[3];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
-        const int u = comp(nb, j);
-        U[j] = ld3(pos, u);
-        ok &= edge_terms(v, j, u, vnbr, edgeC, edgeArc, C[j], nC[j], arc[j]);
+        for (int j = 0; j < 3; ++j) {
+            const int u = comp(nb, j);
+            U[j] = ld3(pos, u);
+            ok &= edge_terms(v, j, u, vnbr, edgeC, edgeArc, C[j], nC[j], arc[j]);
+        }
+#pragma unroll
+        for (int s = 0; s < 3; ++s) {
+            const int jl = nbr_slot(nb, comp(lasts, s)), jx = nbr_slot(nb, comp(nexts, s));
+            ok &= jl >= 0 && jx >= 0;
+            if (ok) {
+                arcs[s] = pick3(arc, jl);
+                flip[s] = positive(dot3e(pick3(U, jl), pick3(C, jx)));
+                cosine[s] = included_cos(pick3(C, jx), pick3(C, jl), pick3(nC, jx), pick3(nC, jl));
+            }
+        }
     }
+    block_acos(cosine, val, src, warpHigh);
+    if (!live) return;
+    const int4 rp = vrpos[v];
 #pragma unroll
     for (int s = 0; s < 3; ++s) {
-        const int jl = nbr_slot(nb, comp(lasts, s)), jx = nbr_slot(nb, comp(nexts, s));
-        double2 cr;
-        if (ok && jl >= 0 && jx >= 0) {
-            cr = make_double2(pick3(arc, jl), included_angle_pre(pick3(C, jx), pick3(C, jl), pick3(nC, jx),
-                                                                 pick3(nC, jl), pick3(U, jl)));
-        } else {  // inconsistent lists: evaluate directly
+        double2 cr = make_double2(arcs[s], included_finish(cosine[s], flip[s]));
+        if (!ok) {  // inconsistent lists: evaluate directly
             const D3 p = ld3(pos, v), pl = ld3(pos, comp(lasts, s)), px = ld3(pos, comp(nexts, s));
             cr = make_double2(geodesic(pl, p, R), included_angle(pl, p, px));
         }
@@ -439,6 +471,9 @@ __global__ void __launch_bounds__(kFanThreads) k_fallback_fan(
     __shared__ double ux[kFanCells * 32], uy[kFanCells * 32], uz[kFanCells * 32];
     __shared__ double cx[kFanCells], cy[kFanCells], cz[kFanCells];
     __shared__ double tri[kFanCells * 32];
+    __shared__ double val[3 * kFanThreads];   // block_acos
+    __shared__ unsigned short src[3 * kFanThreads];
+    __shared__ int warpHigh[kFanThreads / 32];
     const int t = threadIdx.x, c0 = blockIdx.x * kFanCells;
     if (t < kFanCells) {
         const int c = c0 + t;
@@ -472,12 +507,17 @@ __global__ void __launch_bounds__(kFanThreads) k_fallback_fan(
         ux[e] = u.x; uy[e] = u.y; uz[e] = u.z;
     }
     __syncthreads();
-    for (int e = t; e < total; e += kFanThreads) {
+    for (int base = 0; base < total; base += kFanThreads) {
         // triangle k of cell lc in the CPU's loop: (centroid, ring[k - 2], ring[k - 1]), indices mod n
-        const int lc = owner[e], b = off[lc], n = cnt[lc], k = e - b;
-        const int i2 = b + (k + n - 2) % n, i3 = b + (k + n - 1) % n;
-        tri[e] = triangle_area_unit(D3{cx[lc], cy[lc], cz[lc]}, D3{ux[i2], uy[i2], uz[i2]}, D3{ux[i3], uy[i3], uz[i3]},
-                                    radius[lc]);
+        const int e = base + t;
+        double a[3] = {-1.0, -1.0, -1.0};
+        if (e < total) {
+            const int lc = owner[e], b = off[lc], n = cnt[lc], k = e - b;
+            const int i2 = b + (k + n - 2) % n, i3 = b + (k + n - 1) % n;
+            triangle_cosines(D3{cx[lc], cy[lc], cz[lc]}, D3{ux[i2], uy[i2], uz[i2]}, D3{ux[i3], uy[i3], uz[i3]}, a);
+        }
+        block_acos(a, val, src, warpHigh);
+        if (e < total) tri[e] = triangle_sum(a, radius[owner[e]]);
     }
     __syncthreads();
     if (t >= kFanCells || cnt[t] == 0) return;
@@ -1920,7 +1960,7 @@ int launch_corners(svm_model* m, bool t1test, bool vnormReady) {
         return check_launch();
     }
     // (blocks of 256 leave the last wave short: 100k cells 133.7 against 124.7 us, 300k 322.6 against 317.4)
-    const int bv = std::min(128, spread_block(m, m->nVertices));
+    const int bv = std::min(kCornerThreads, spread_block(m, m->nVertices));
     if (!vnormReady) launch_next(m, k_vnorm, blocksFor(m->nVertices, bv), bv, m->pos[m->cur], m->vnorm, m->nVertices);
     launch_next(m, k_edges, blocksFor(m->nVertices, bv), bv, m->pos[m->cur], m->vnorm, m->vsph, m->vnbr, m->vcell, m->edgeC,
                                                               m->edgeArc, m->nVertices, m->R, t1test ? 1 : 0,
