@@ -5,8 +5,8 @@
 // vertex lists use global indices).  All per-element kernels of a step therefore run once over all
 // replicas; what differs per replica is read through the vertex's replica index, stored in the w
 // component of its FP32 position: the radius, the noise amplitude sqrt(2 dt mu T_r), and the
-// area check |sum_c A_c - 4 pi R_r^2| > 1e-6 (sphericalVertexModel.cpp:304-310), evaluated per
-// replica by one block each.  Replica r's T1 flips are the ones the single-sphere loop would do:
+// area check |sum_c A_c - 4 pi R_r^2| > mixed_area_limit (sphericalVertexModel.cpp:304-310), evaluated
+// per replica by one block each.  Replica r's T1 flips are the ones the single-sphere loop would do:
 // the flagged edges of different replicas share no vertex or cell, and within a replica the
 // global scan order is the replica's own order.
 //
@@ -49,7 +49,7 @@ __global__ void k_rep_check(const double2* __restrict__ ap, const int* __restric
         const double excess = total - 4.0 * kPI * R * R;
         repScal[3 * r] = total;
         repScal[3 * r + 1] = excess;
-        repFlag[r] = fabs(excess) > 1e-6 ? 1 : 0;
+        repFlag[r] = fabs(excess) > mixed_area_limit(cellOff[r + 1] - cellOff[r], R) ? 1 : 0;
     }
 }
 

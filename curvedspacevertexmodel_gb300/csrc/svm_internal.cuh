@@ -368,6 +368,18 @@ __device__ __forceinline__ double triangle_area_unit(D3 p1, D3 p2, D3 p3, double
     return triangle_sum(a, R);
 }
 
+// The total-area check of the mixed form (sphericalVertexModel.cpp:304-310 compares with 1e-6): the areas
+// of nC cells on a sphere of radius R sum to 4 pi R^2 plus whole turns of R^2 -- what the check is after --
+// plus the rounding of 6 nC angles, up to half an ulp of pi each if it has a bias.  That rounding passes
+// 1e-6 at about 137,000 cells, and at 1M the check failed on nearly every state and replaced the areas by
+// the triangle fan's, which there are the less accurate ones (1e-5 each: the fan's cosines cancel) and
+// took 2.1 ms of a 3.4 ms step.  The limit is therefore never below that rounding; up to 137,000 cells it
+// is the reference's.
+__host__ __device__ inline double mixed_area_limit(int nC, double R) {
+    const double rounding = 6.0 * nC * R * R * 0x1p-53;
+    return rounding > 1e-6 ? rounding : 1e-6;
+}
+
 // Spherical coordinates of a point as the reference's gradients compute them
 // (sphericalDomain.h:218-232, 251-261): cos t = z/|p|, sin t = sqrt(1 - cos^2 t),
 // cos p = x / sqrt(x^2+y^2), sin p = y / sqrt(x^2+y^2).

@@ -315,7 +315,8 @@ __global__ void __launch_bounds__(kCornerThreads, 6) k_corner(const double4_32a*
 // Per cell: centroid (sum of ring vertices in ring order, renormalised), perimeter and angle sum
 // in the CPU's order (ring positions n-2, n-1, 0, ..., n-3), area = (sum - (n-2) pi) wrapped
 // by floor(area / pi), times R^2 (sphericalVertexModel.cpp:228-303).  The last block to finish
-// totals the areas and raises the fallback flag when |sum A - 4 pi R^2| > 1e-6 (304-310).
+// totals the areas and raises the fallback flag when |sum A - 4 pi R^2| > 1e-6 (304-310; mixed form:
+// mixed_area_limit).
 //
 // kSplit: two threads a cell, in the two halves of the block: the centroid, and the area and perimeter.
 // A cell's chain -- count, ring, positions or corners, sums, roots and divisions -- is latency at small N,
@@ -412,7 +413,8 @@ __global__ void k_cells(const PT* __restrict__ pos, const int* __restrict__ ring
             const double excess = total - 4.0 * kPI * R * R;
             scalars[0] = total;
             scalars[1] = excess;
-            const int taken = fabs(excess) > 1e-6 ? 1 : 0;
+            const double limit = std::is_same<PT, float4>::value ? mixed_area_limit(nC, R) : 1e-6;
+            const int taken = fabs(excess) > limit ? 1 : 0;
             fallbackFlag[0] = taken;
             fallbackFlag[1] += taken;  // geometry passes that took the fallback (svm_model_fallback_count)
             *ticket = 0u;

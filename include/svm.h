@@ -170,7 +170,9 @@ int svm_model_ring_info(svm_model* m, int* out3);
 int svm_model_get_vertex_cells(svm_model* m, int* out);
 int svm_model_get_vertex_neighbors(svm_model* m, int* out);
 /* The last geometry pass's total-area check (sphericalVertexModel.cpp:304-310): sum of cell
- * areas, its excess over 4 pi R^2, and whether the triangle-fan fallback replaced the areas. */
+ * areas, its excess over 4 pi R^2, and whether the triangle-fan fallback replaced the areas: when the
+ * excess is above 1e-6 or, in the mixed form from about 137,000 cells on, above what the rounding of
+ * the angles can add up to (6 nCells R^2 2^-53). */
 int svm_model_area_check(svm_model* m, double* totalArea, double* excess, int* fallbackTaken);
 /* Geometry passes of a single sphere that took the triangle-fan fallback since the last call
  * (read and cleared). */
