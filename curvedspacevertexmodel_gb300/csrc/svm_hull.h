@@ -47,7 +47,20 @@ bool convexHullTriangles(const double* points, int n, std::vector<int>& triangle
 bool topologyFromTriangles(const double* points, int n, const std::vector<int>& triangles,
                            Topology& topo);
 
+struct DeviceTopology;   // the arrays of a device-built topology (svm_hull_gpu.cu)
+
 }  // namespace svm
 
-// The C ABI's topology handle (svm_topology_*), filled by the host hull or the device hull.
-struct svm_topology { svm::Topology t; };
+// The C ABI's topology handle (svm_topology_*): filled by the host hull, or, with only its sizes in t, by
+// the device hull, whose arrays are in dev.
+struct svm_topology {
+    svm::Topology t;
+    svm::DeviceTopology* dev = nullptr;
+    svm_topology() = default;
+    svm_topology(const svm_topology&) = delete;
+    svm_topology& operator=(const svm_topology&) = delete;
+    ~svm_topology();   // svm_hull_gpu.cu
+};
+namespace svm {
+int device_topology_get(const svm_topology* t, double* vp, int* rings, int stride, unsigned* counts, int* vc, int* vn);
+}

@@ -5,13 +5,15 @@
 // equals svm_topology_from_points array for array.
 //
 // A hull built point by point instead of by incremental insertion:
-//   k_hull_star   a thread per centre p.  Candidates are the centres in the bins within w of p's
+//   k_hb_*        the centres sorted into bins (counts, a scan, each bin's centres in ascending index)
+//   k_hull_star   a warp per centre p.  Candidates are the centres in the bins within w of p's
 //                 bin (a ball of radius w h around p lies inside them).  The nearest candidate q0
 //                 spans a hull edge (for points on a sphere, the plane through p and q0 with
 //                 normal p + q0 has every other point strictly below it).  Gift wrapping around p
 //                 from the edge p -> q0: the next corner s of edge p -> q is the candidate that no
-//                 other candidate lies above, i.e. the last one to win "orient(p, q, s, x) > 0",
-//                 until the wrap returns to q0.  Each triangle of the star is then certified: its
+//                 other candidate lies above, found by the lanes' scans and a tree over them with
+//                 the test "orient(p, q, s, x) > 0", the lower candidate kept in a tie, until the
+//                 wrap returns to q0.  Each triangle of the star is then certified: its
 //                 circumcircle's cap (the part of the sphere above its plane, smaller than a
 //                 hemisphere) lies within 2 rho of p, rho the triangle's circumradius, so when
 //                 2 rho < w h every point that could lie in the cap was a candidate and the
@@ -38,11 +40,13 @@
 using namespace svm;
 
 namespace {
-constexpr int kHB = 128;          // threads per block of the star kernel (local candidate arrays)
+constexpr int kHB = 128;          // threads per block of the star kernel: four centres
+constexpr int kFewCand = 128;     // candidates of a star in the first launch (about 70 at w = 1)
 constexpr int kMaxCand = 512;     // candidates a star may draw on
 constexpr int kMaxDeg = 32;       // facets around one centre
 constexpr int kMaxW = 4;          // widest search, in bins
 constexpr int kB = 256;
+constexpr int kOutside = 16;      // error bit: a centre outside the bins' grid, or not finite
 
 struct DD { double hi, lo; };
 
@@ -121,122 +125,250 @@ __device__ __forceinline__ Plane32 plane32(const float* b, const float* c) {
     return t;
 }
 
-// Centres list[0..count) (all centres when list is null) with searches of wFirst..wLast bins.  A
-// centre whose stars all fail certification in that range is queued in retry (when given) for a
-// second launch with the wider searches, so that warps of the first launch do not wait on them.
+// FP32 form of cap_within for the triangle (p, p + a, p + b), n p's offset from the centre: 1 or 0 where a
+// margin of 1e-3 makes it certain (FP32 is good to 1e-5 for triangles this far from flat), else -1.
+__device__ __forceinline__ int cap_within32(const float* p, const float* a, const float* b, float reach) {
+    const float nx = a[1] * b[2] - a[2] * b[1], ny = a[2] * b[0] - a[0] * b[2], nz = a[0] * b[1] - a[1] * b[0];
+    const float la = sqrtf(a[0] * a[0] + a[1] * a[1] + a[2] * a[2]), lb = sqrtf(b[0] * b[0] + b[1] * b[1] + b[2] * b[2]);
+    const float c0 = a[0] - b[0], c1 = a[1] - b[1], c2 = a[2] - b[2], lab = sqrtf(c0 * c0 + c1 * c1 + c2 * c2);
+    const float ln = sqrtf(nx * nx + ny * ny + nz * nz), lp = sqrtf(p[0] * p[0] + p[1] * p[1] + p[2] * p[2]);
+    const float up = nx * p[0] + ny * p[1] + nz * p[2];
+    if (!(ln > 0.02f * la * lb && lab > 0.02f * (la + lb) && fabsf(up) > 0.1f * ln * lp && la * lb > 1e-12f)) return -1;
+    if (up < 0.f) return 0;
+    const float diameter = la * lb * lab / ln;
+    return diameter * 1.001f < reach ? 1 : (diameter * 0.999f > reach ? 0 : -1);
+}
+
+// The bins: centres list[off[bin] .. off[bin + 1]) of bin x + y nside + z nside^2, side h over
+// [-radius, radius]^3.
+struct BinGrid {
+    const int* off;
+    const int* list;
+    int nside;
+    double h, radius;
+};
+
+// Centres list[0..*count) (all n centres when list is null), a warp each, with searches of wFirst..wLast
+// bins and at most kCap candidates.  A centre whose stars all fail certification in that range, or that
+// has more candidates, is queued in retry (when given) for a second launch with the wider searches and
+// kMaxCand candidates, so that warps of the first launch do not wait on them.
+// What bounds it: issue slots and shared memory (about 1,700 FP32 instructions a warp to pivot six times
+// over 70 candidates); the FP64 pipe holds only the offsets x - p.  One centre per thread, candidates in
+// local memory: 4.5 ms at 100k centres.
+template <int kCap>
 __global__ void __launch_bounds__(kHB) k_hull_star(const double* __restrict__ P, const int* __restrict__ list,
-                                                  int count, int wFirst, int wLast, CellGrid g,
+                                                  const int* __restrict__ countPtr, int n, int wFirst, int wLast, BinGrid g,
                                                   int* __restrict__ deg, int* __restrict__ star,
                                                   int* __restrict__ retry, int* __restrict__ retryCount,
                                                   int* __restrict__ err) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= count) return;
-    const int p = list ? list[t] : t;
-    // candidates and their offsets from p, fl32(x - p) of the FP64 difference (relative error
-    // within 2^-24 (1 + 2^-29) per component)
-    int cand[kMaxCand];
-    float dv[kMaxCand][3];
-    int st[kMaxDeg];
-    double pp[3];
-    load3(P, p, pp);
-    int c[3];
-    for (int d = 0; d < 3; ++d) c[d] = max(0, min(g.nside - 1, (int)floor((pp[d] + g.radius) / g.h)));
-    bool hard = false;  // a failure no wider search can repair
-    for (int w = wFirst; w <= wLast; ++w) {
-        int lo[3], hi[3];
-        bool whole = true;
-        for (int d = 0; d < 3; ++d) {
-            lo[d] = max(0, c[d] - w); hi[d] = min(g.nside - 1, c[d] + w);
-            whole &= lo[d] == 0 && hi[d] == g.nside - 1;
-        }
-        int nc = 0, iq0 = -1;
-        bool overflow = false;
-        float b1 = INFINITY, b2 = INFINITY;
-        for (int z = lo[2]; z <= hi[2]; ++z)
-            for (int y = lo[1]; y <= hi[1]; ++y)
-                for (int x = lo[0]; x <= hi[0]; ++x) {
+    constexpr int kWarps = kHB / 32;
+    constexpr unsigned kAll = 0xffffffffu;
+    __shared__ float dvS[kWarps][kCap][3];   // offsets from p, fl32(x - p) of the FP64 difference
+    __shared__ int candS[kWarps][kCap];
+    __shared__ int stS[kWarps][kMaxDeg];     // the star, as candidate indices
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float (*dv)[3] = dvS[warp];
+    int* cand = candS[warp];
+    int* st = stS[warp];
+    const int count = list ? *countPtr : n;
+    for (int t = blockIdx.x * kWarps + warp; t < count; t += gridDim.x * kWarps) {
+        const int p = list ? list[t] : t;
+        double pp[3];
+        load3(P, p, pp);
+        const float p32[3] = {(float)pp[0], (float)pp[1], (float)pp[2]};
+        int c[3];
+        for (int d = 0; d < 3; ++d) c[d] = max(0, min(g.nside - 1, (int)floor((pp[d] + g.radius) / g.h)));
+        bool hard = false, done = false;  // hard: a failure no wider search can repair
+        for (int w = wFirst; w <= wLast && !done && !hard; ++w) {
+            int lo[3], ext[3];
+            bool whole = true;
+            for (int d = 0; d < 3; ++d) {
+                lo[d] = max(0, c[d] - w);
+                ext[d] = min(g.nside - 1, c[d] + w) - lo[d] + 1;
+                whole &= ext[d] == g.nside;
+            }
+            // candidates in the order of the bins (x fastest) and of each bin's list
+            const int nb = ext[0] * ext[1] * ext[2];
+            int nc = 0;
+            __syncwarp();
+            for (int b0 = 0; b0 < nb; b0 += 32) {
+                const int b = b0 + lane;
+                int first = 0, m = 0;
+                if (b < nb) {
+                    const int x = lo[0] + b % ext[0], y = lo[1] + (b / ext[0]) % ext[1], z = lo[2] + b / (ext[0] * ext[1]);
                     const long cell = x + (long)y * g.nside + (long)z * g.nside * g.nside;
-                    const int m = min((int)g.counts[cell], g.cap);
-                    for (int k = 0; k < m; ++k) {
-                        const int j = g.slots[cell * g.cap + k];
-                        if (j == p) continue;
-                        if (nc >= kMaxCand) { overflow = true; continue; }
+                    first = g.off[cell];
+                    m = g.off[cell + 1] - first;
+                }
+                int incl = m;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(kAll, incl, o);
+                    if (lane >= o) incl += v;
+                }
+                const int excl = incl - m, total = __shfl_sync(kAll, incl, 31);
+                for (int k0 = 0; k0 < total; k0 += 32) {
+                    const int k = k0 + lane;
+                    int owner = 0;  // the last lane whose bin starts at or before k
+                    for (int step = 16; step > 0; step >>= 1) {
+                        const int e = __shfl_sync(kAll, excl, owner + step);
+                        if (e <= k) owner += step;
+                    }
+                    const int slot = k - __shfl_sync(kAll, excl, owner), from = __shfl_sync(kAll, first, owner);
+                    const int j = k < total ? g.list[from + slot] : p;
+                    const bool valid = j != p;
+                    const unsigned mask = __ballot_sync(kAll, valid);
+                    const int at = nc + __popc(mask & ((1u << lane) - 1u));
+                    if (valid && at < kCap) {
                         double xx[3];
                         load3(P, j, xx);
-                        cand[nc] = j;
-                        dv[nc][0] = (float)(xx[0] - pp[0]);
-                        dv[nc][1] = (float)(xx[1] - pp[1]);
-                        dv[nc][2] = (float)(xx[2] - pp[2]);
-                        // the nearest in FP32 (squared length within 5 2^-24 relative of the exact one)
-                        const float d2 = dv[nc][0] * dv[nc][0] + dv[nc][1] * dv[nc][1] + dv[nc][2] * dv[nc][2];
-                        if (d2 < b1) { b2 = b1; b1 = d2; iq0 = nc; }
-                        else if (d2 < b2) b2 = d2;
-                        ++nc;
+                        cand[at] = j;
+                        dv[at][0] = (float)(xx[0] - pp[0]);
+                        dv[at][1] = (float)(xx[1] - pp[1]);
+                        dv[at][2] = (float)(xx[2] - pp[2]);
+                    }
+                    nc += __popc(mask);
+                }
+            }
+            __syncwarp();
+            if (nc > kCap) { if (kCap == kMaxCand) hard = true; break; }
+            if (nc < 3) { if (whole) hard = true; continue; }
+            // the nearest in FP32 (squared length within 5 2^-24 relative of the exact one); a near tie: the
+            // FP64 squared lengths of those near it, lowest index on ties
+            float b1 = INFINITY;
+            for (int i = lane; i < nc; i += 32) b1 = fminf(b1, dv[i][0] * dv[i][0] + dv[i][1] * dv[i][1] + dv[i][2] * dv[i][2]);
+            for (int o = 16; o > 0; o >>= 1) b1 = fminf(b1, __shfl_xor_sync(kAll, b1, o));
+            int iq0 = kCap, near = 0;
+            for (int i = lane; i < nc; i += 32) {
+                const float d2 = dv[i][0] * dv[i][0] + dv[i][1] * dv[i][1] + dv[i][2] * dv[i][2];
+                if (!(d2 > b1 * (1.0f + 1e-5f))) {
+                    ++near;
+                    if (d2 == b1) iq0 = min(iq0, i);
+                }
+            }
+            near = __reduce_add_sync(kAll, near);
+            iq0 = __reduce_min_sync(kAll, iq0);
+            if (near != 1) {
+                double best = INFINITY;
+                int bi = -1;
+                for (int i = lane; i < nc; i += 32) {
+                    if (dv[i][0] * dv[i][0] + dv[i][1] * dv[i][1] + dv[i][2] * dv[i][2] > b1 * (1.0f + 1e-5f)) continue;
+                    double xx[3];
+                    load3(P, cand[i], xx);
+                    const double dx = xx[0] - pp[0], dy = xx[1] - pp[1], dz = xx[2] - pp[2];
+                    const double d2 = dx * dx + dy * dy + dz * dz;
+                    if (bi < 0 || d2 < best || (d2 == best && cand[i] < cand[bi])) { best = d2; bi = i; }
+                }
+                for (int o = 16; o > 0; o >>= 1) {
+                    const double ob = __shfl_xor_sync(kAll, best, o);
+                    const int oi = __shfl_xor_sync(kAll, bi, o);
+                    if (oi >= 0 && (bi < 0 || ob < best || (ob == best && cand[oi] < cand[bi]))) { best = ob; bi = oi; }
+                }
+                iq0 = __shfl_sync(kAll, bi, 0);   // (none at worst)
+            }
+            if (iq0 < 0 || iq0 >= nc) { hard = true; break; }
+            // gift wrapping around p from the edge to the nearest candidate.  The pivot's sign test runs in
+            // FP32: with every input within 2^-24 relative, |det32 - det| <= 8 2^-24 perm, so |det32| > 1e-5
+            // perm32 fixes the sign; anything closer (or so small that FP32 could underflow) takes the FP64
+            // test.
+            int d = 0, iq = iq0;
+            bool ok = true;
+            do {
+                if (d >= kMaxDeg) { ok = false; break; }
+                if (lane == 0) st[d] = iq;
+                ++d;
+                const float b[3] = {dv[iq][0], dv[iq][1], dv[iq][2]};
+                // whether candidate x lies above the plane of (p, q, s)
+                const auto above = [&](const Plane32& pl, int s, int x) {
+                    const float det = pl.n[0] * dv[x][0] + pl.n[1] * dv[x][1] + pl.n[2] * dv[x][2];
+                    const float perm = pl.k[0] * fabsf(dv[x][0]) + pl.k[1] * fabsf(dv[x][1]) + pl.k[2] * fabsf(dv[x][2]);
+                    if (perm > 1e-30f && fabsf(det) > 1e-5f * perm) return det > 0.f;
+                    double qq[3], ss[3], xx[3];
+                    load3(P, cand[iq], qq); load3(P, cand[s], ss); load3(P, cand[x], xx);
+                    return orient(pp, qq, ss, xx) > 0.0;
+                };
+                int is = -1;
+                Plane32 pl;
+                for (int i = lane; i < nc; i += 32) {
+                    if (i == iq) continue;
+                    if (is < 0 || above(pl, is, i)) { is = i; pl = plane32(b, dv[i]); }
+                }
+                for (int o = 16; o > 0; o >>= 1) {
+                    const int other = __shfl_xor_sync(kAll, is, o);
+                    if (other < 0 || other == is) continue;
+                    if (is < 0) { is = other; continue; }
+                    const int s = min(is, other), x = max(is, other);
+                    is = above(plane32(b, dv[s]), s, x) ? x : s;
+                }
+                is = __shfl_sync(kAll, is, 0);
+                if (is < 0) { ok = false; break; }
+                iq = is;
+            } while (iq != iq0);
+            __syncwarp();
+            if (ok && d < 3) ok = false;
+            if (ok && !whole) {
+                const double reach = w * g.h;
+                bool in = true;
+                if (lane < d) {
+                    const int i1 = st[lane], i2 = st[lane + 1 < d ? lane + 1 : 0];
+                    const int r = cap_within32(p32, dv[i1], dv[i2], (float)reach);
+                    in = r > 0;
+                    if (r < 0) {
+                        double a[3], b[3];
+                        load3(P, cand[i1], a);
+                        load3(P, cand[i2], b);
+                        in = cap_within(pp, a, b, reach);
                     }
                 }
-        if (overflow) { hard = true; break; }
-        if (nc < 3) { if (whole) { hard = true; break; } continue; }
-        if (!(b2 > b1 * (1.0f + 1e-5f))) {  // a near tie: the FP64 squared lengths, lowest index on ties
-            double best = 0.0;
-            iq0 = -1;
-            for (int i = 0; i < nc; ++i) {
-                double xx[3];
-                load3(P, cand[i], xx);
-                const double dx = xx[0] - pp[0], dy = xx[1] - pp[1], dz = xx[2] - pp[2];
-                const double d2 = dx * dx + dy * dy + dz * dz;
-                if (iq0 < 0 || d2 < best || (d2 == best && cand[i] < cand[iq0])) { best = d2; iq0 = i; }
+                ok = __all_sync(kAll, in);
+            }
+            if (ok) {
+                if (lane == 0) deg[p] = d;
+                if (lane < d) star[(long)p * kMaxDeg + lane] = cand[st[lane]];
+                done = true;
+            } else if (whole) {
+                hard = true;
             }
         }
-        // gift wrapping around p from the edge to the nearest candidate.  The pivot's sign test
-        // runs in FP32 with the plane hoisted out of the candidate loop: with every input within
-        // 2^-24 relative, |det32 - det| <= 8 2^-24 perm, so |det32| > 1e-5 perm32 fixes the sign;
-        // anything closer (or so small that FP32 could underflow) takes the FP64 test.
-        int d = 0, iq = iq0;
-        bool ok = true;
-        do {
-            if (d >= kMaxDeg) { ok = false; break; }
-            st[d++] = cand[iq];
-            const float b[3] = {dv[iq][0], dv[iq][1], dv[iq][2]};
-            int is = -1;
-            Plane32 pl;
-            for (int i = 0; i < nc; ++i) {
-                if (i == iq) continue;
-                if (is < 0) { is = i; pl = plane32(b, dv[i]); continue; }
-                const float det = pl.n[0] * dv[i][0] + pl.n[1] * dv[i][1] + pl.n[2] * dv[i][2];
-                const float perm = pl.k[0] * fabsf(dv[i][0]) + pl.k[1] * fabsf(dv[i][1]) + pl.k[2] * fabsf(dv[i][2]);
-                bool above;
-                if (perm > 1e-30f && fabsf(det) > 1e-5f * perm) {
-                    above = det > 0.f;
-                } else {
-                    double qq[3], ss[3], xx[3];
-                    load3(P, cand[iq], qq); load3(P, cand[is], ss); load3(P, cand[i], xx);
-                    above = orient(pp, qq, ss, xx) > 0.0;
-                }
-                if (above) { is = i; pl = plane32(b, dv[i]); }
-            }
-            if (is < 0) { ok = false; break; }
-            iq = is;
-        } while (iq != iq0);
-        if (ok && d < 3) ok = false;
-        if (ok && !whole) {
-            const double reach = w * g.h;
-            for (int i = 0; i < d && ok; ++i) {
-                double a[3], b[3];
-                load3(P, st[i], a);
-                load3(P, st[(i + 1) % d], b);
-                ok = cap_within(pp, a, b, reach);
-            }
+        if (!done && lane == 0) {
+            deg[p] = 0;
+            if (retry && !hard) retry[atomicAdd(retryCount, 1)] = p;
+            else atomicOr(err, 1);
         }
-        if (ok) {
-            deg[p] = d;
-            for (int i = 0; i < d; ++i) star[(long)p * kMaxDeg + i] = st[i];
-            return;
-        }
-        if (whole) { hard = true; break; }
     }
-    deg[p] = 0;
-    if (retry && !hard) { retry[atomicAdd(retryCount, 1)] = p; return; }
-    atomicOr(err, 1);
+}
+
+// Bins: the count of each, then (after the scan of the counts) each centre at a provisional place of
+// its bin, then at its rank in the bin.
+__device__ __forceinline__ int hb_bin(const double* P, int i, int nside, double h, double radius) {
+    int b[3];
+    for (int d = 0; d < 3; ++d) b[d] = max(0, min(nside - 1, (int)floor((P[3 * (long)i + d] + radius) / h)));
+    return b[0] + b[1] * nside + b[2] * nside * nside;
+}
+__global__ void k_hb_count(const double* __restrict__ P, int n, int nside, double h, double radius, int* __restrict__ binOf,
+                           int* __restrict__ off, int* __restrict__ err) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    for (int d = 0; d < 3; ++d)
+        if (!(fabs(P[3 * (long)i + d]) <= radius)) atomicOr(err, kOutside);
+    const int b = hb_bin(P, i, nside, h, radius);
+    binOf[i] = b;
+    atomicAdd(off + b, 1);
+}
+__global__ void k_hb_place(const int* __restrict__ binOf, int n, const int* __restrict__ off, int* __restrict__ cursor,
+                           int* __restrict__ tmp) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int b = binOf[i];
+    tmp[off[b] + atomicAdd(cursor + b, 1)] = i;
+}
+__global__ void k_hb_order(const int* __restrict__ binOf, int n, const int* __restrict__ off, const int* __restrict__ tmp,
+                           int* __restrict__ list) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int b = binOf[i], first = off[b], last = off[b + 1];
+    int rank = 0;
+    for (int k = first; k < last; ++k) rank += tmp[k] < i;
+    list[first + rank] = i;
 }
 
 __device__ __forceinline__ int star_next(const int* star, const int* deg, int a, int b) {
@@ -366,125 +498,169 @@ __global__ void k_scan_add(int* a, int n, const int* sums) {
     if (i + kB < n) a[i + kB] += add;
 }
 
-int exclusive_scan(int* a, int n, cudaStream_t s, int* total) {
+// (sums: scan_ints(n) ints of workspace)
+size_t scan_ints(size_t n) {
+    const size_t nb = (n + 2 * kB - 1) / (2 * kB);
+    return nb + 1 + (nb > 1 ? scan_ints(nb) : 0);
+}
+int exclusive_scan(int* a, int n, cudaStream_t s, int* sums) {
     const int nb = (n + 2 * kB - 1) / (2 * kB);
-    int* sums = nullptr;
-    if (cudaMalloc(&sums, sizeof(int) * (nb + 1)) != cudaSuccess) return SVM_ERR_CUDA;
     k_scan_block<<<nb, kB, 0, s>>>(a, n, sums);
     int rc = check_launch();
-    if (!rc && nb > 1) rc = exclusive_scan(sums, nb, s, nullptr);
+    if (!rc && nb > 1) rc = exclusive_scan(sums, nb, s, sums + nb + 1);
     else if (!rc) rc = cudaMemsetAsync(sums, 0, sizeof(int), s) == cudaSuccess ? SVM_OK : SVM_ERR_CUDA;
     if (!rc) { k_scan_add<<<nb, kB, 0, s>>>(a, n, sums); rc = check_launch(); }
-    if (!rc && total) {  // callers end the array with a zero, so its last entry is the sum
-        rc = cudaMemcpyAsync(total, a + n - 1, sizeof(int), cudaMemcpyDeviceToHost, s) == cudaSuccess ? SVM_OK : SVM_ERR_CUDA;
-    }
-    if (cudaStreamSynchronize(s) != cudaSuccess) rc = SVM_ERR_CUDA;
-    cudaFree(sums);
     return rc;
 }
 
-struct DevBuf {
-    std::vector<void*> ptrs;
-    template <typename T> T* get(size_t count) {
-        void* p = nullptr;
-        if (cudaMalloc(&p, sizeof(T) * std::max<size_t>(count, 1)) != cudaSuccess) return nullptr;
-        ptrs.push_back(p);
-        return (T*)p;
+// Each cell's ring in a row of `stride` (-1 past its end), with the counts.
+__global__ void k_hull_rows(const int* __restrict__ ringOff, const int* __restrict__ ring, int n, int stride,
+                            int* __restrict__ rows) {
+    const long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    if (e >= (long)n * stride) return;
+    const int c = (int)(e / stride), k = (int)(e % stride), b = ringOff[c], m = ringOff[c + 1] - b;
+    rows[e] = k < m ? ring[b + k] : -1;
+}
+__global__ void k_hull_max(const int* __restrict__ deg, int n, int* __restrict__ maxDeg) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int m = __reduce_max_sync(0xffffffffu, i < n ? deg[i] : 0);
+    if ((threadIdx.x & 31) == 0) atomicMax(maxDeg, m);
+}
+
+// One device allocation cut into 256-byte aligned arrays.
+struct Arena {
+    char* base = nullptr;
+    size_t used = 0;
+    template <typename T> T* cut(size_t count) {   // with base null: counts the bytes
+        T* p = reinterpret_cast<T*>(base + used);
+        used += (sizeof(T) * std::max<size_t>(count, 1) + 255) & ~(size_t)255;
+        return p;
     }
-    ~DevBuf() { for (void* p : ptrs) cudaFree(p); }
 };
 }  // namespace
+
+// The arrays stay on the device, where they were computed, until svm_topology_get copies them straight
+// into the caller's.
+struct svm::DeviceTopology {
+    void* base = nullptr;
+    const double* vpos = nullptr;
+    const int *vcells = nullptr, *vnbrs = nullptr, *rows = nullptr, *deg = nullptr;
+    ~DeviceTopology() { cudaFree(base); }
+};
+svm_topology::~svm_topology() { delete dev; }
+
+namespace svm {
+// svm_topology_get of a device-built topology.
+int device_topology_get(const svm_topology* t, double* vp, int* rings, int stride, unsigned* counts, int* vc, int* vn) {
+    const DeviceTopology& D = *t->dev;
+    const size_t nC = t->t.nCells, nV = t->t.nVertices, W = t->t.maxRing;
+    const auto copy = [](void* dst, const void* src, size_t bytes) {
+        return cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost) == cudaSuccess;
+    };
+    bool ok = (!vp || copy(vp, D.vpos, sizeof(double) * 3 * nV)) && (!vc || copy(vc, D.vcells, sizeof(int) * 3 * nV)) &&
+              (!vn || copy(vn, D.vnbrs, sizeof(int) * 3 * nV)) && (!counts || copy(counts, D.deg, sizeof(int) * nC));
+    if (ok && rings && (size_t)stride == W) ok = copy(rings, D.rows, sizeof(int) * nC * W);
+    else if (ok && rings) {   // wider rows than the rings need
+        std::vector<int> rows(nC * W);
+        ok = copy(rows.data(), D.rows, sizeof(int) * rows.size());
+        for (size_t c = 0; c < nC; ++c)
+            for (size_t k = 0; k < (size_t)stride; ++k) rings[c * stride + k] = k < W ? rows[c * W + k] : -1;
+    }
+    return ok ? SVM_OK : SVM_ERR_CUDA;
+}
+}  // namespace svm
 
 extern "C" int svm_topology_from_points_gpu(const double* pts, int n, void* stream, svm_topology** out) {
     if (!pts || n < 4 || !out) return SVM_ERR_ARG;
     cudaStream_t s = (cudaStream_t)stream;
-    DevBuf buf;
-    double* P = buf.get<double>(3 * (size_t)n);
-    int* deg = buf.get<int>(n);
-    int* star = buf.get<int>((size_t)n * kMaxDeg);
-    int* own = buf.get<int>((size_t)n + 1);
-    int* err = buf.get<int>(2);          // [0] error bits, [1] centres queued for the wider search
-    int* retry = buf.get<int>(n);
-    if (!P || !deg || !star || !own || !err || !retry) return SVM_ERR_CUDA;
-    if (cudaMemcpyAsync(P, pts, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, s) != cudaSuccess ||
-        cudaMemsetAsync(err, 0, 2 * sizeof(int), s) != cudaSuccess || cudaMemsetAsync(own + n, 0, sizeof(int), s) != cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess)  // the cell list bins on a stream of its own
-        return SVM_ERR_CUDA;
     // bins of side 2.5 mean spacings (a unit-density sphere has ~70 candidates at w = 1)
-    double rmax = 0.0;
+    double r2 = 0.0;
     for (int i = 0; i < n; ++i)
-        rmax = std::max(rmax, std::sqrt(pts[3 * i] * pts[3 * i] + pts[3 * i + 1] * pts[3 * i + 1] + pts[3 * i + 2] * pts[3 * i + 2]));
+        r2 = std::max(r2, pts[3 * i] * pts[3 * i] + pts[3 * i + 1] * pts[3 * i + 1] + pts[3 * i + 2] * pts[3 * i + 2]);
+    const double rmax = std::sqrt(r2);
     const double gridR = rmax * (1.0 + 1e-6) + 1e-3;
     const double spacing = std::sqrt(4.0 * 3.141592653589793 * rmax * rmax / n);
-    const double a = std::min(2.5 * spacing, gridR);
-    svm_cell_list* cl = nullptr;
-    int rc = svm_cell_list_create(a, gridR, n, 32, stream, &cl);
-    if (rc) return rc;
-    CellGrid g;
-    rc = cell_list_bin(cl, P, n, &g);
-    if (!rc) {
-        k_hull_star<<<(n + kHB - 1) / kHB, kHB, 0, s>>>(P, nullptr, n, 1, 1, g, deg, star, retry, err + 1, err);
-        rc = check_launch();
-    }
-    int nRetry = 0;
-    if (!rc) rc = (cudaMemcpyAsync(&nRetry, err + 1, sizeof(int), cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-                   cudaStreamSynchronize(s) == cudaSuccess) ? SVM_OK : SVM_ERR_CUDA;
-    if (!rc && nRetry > 0) {
-        k_hull_star<<<(nRetry + kHB - 1) / kHB, kHB, 0, s>>>(P, retry, nRetry, 2, kMaxW, g, deg, star, nullptr,
-                                                            nullptr, err);
-        rc = check_launch();
-    }
-    if (!rc) {
-        k_hull_check<<<(n + kB - 1) / kB, kB, 0, s>>>(star, deg, n, own, err);
-        rc = check_launch();
-    }
-    int nf = 0, e = 0;
-    if (!rc) rc = exclusive_scan(own, n + 1, s, &nf);
-    if (!rc) rc = (cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-                   cudaStreamSynchronize(s) == cudaSuccess) ? SVM_OK : SVM_ERR_CUDA;
-    svm_cell_list_destroy(cl);
-    if (rc) return rc;
-    if (e || nf != 2 * n - 4) return SVM_ERR_HULL;
-    int* F = buf.get<int>(3 * (size_t)nf);
-    double* vpos = buf.get<double>(3 * (size_t)nf);
-    int* vcells = buf.get<int>(3 * (size_t)nf);
-    int* vnbrs = buf.get<int>(3 * (size_t)nf);
-    int* ringOff = buf.get<int>((size_t)n + 1);
-    int* ring = buf.get<int>(3 * (size_t)nf);
-    if (!F || !vpos || !vcells || !vnbrs || !ringOff || !ring) return SVM_ERR_CUDA;
-    const double radius = std::sqrt(pts[0] * pts[0] + pts[1] * pts[1] + pts[2] * pts[2]);
-    k_hull_emit<<<(n + kB - 1) / kB, kB, 0, s>>>(star, deg, n, own, F);
-    if (check_launch()) return SVM_ERR_CUDA;
-    k_hull_vertex<<<(nf + kB - 1) / kB, kB, 0, s>>>(P, F, nf, own, star, deg, radius, vpos, vcells, vnbrs, err);
-    if (check_launch()) return SVM_ERR_CUDA;
-    if (cudaMemcpyAsync(ringOff, deg, sizeof(int) * n, cudaMemcpyDeviceToDevice, s) != cudaSuccess ||
-        cudaMemsetAsync(ringOff + n, 0, sizeof(int), s) != cudaSuccess)
-        return SVM_ERR_CUDA;
-    int nr = 0;
-    if (exclusive_scan(ringOff, n + 1, s, &nr)) return SVM_ERR_CUDA;
-    if (nr != 3 * nf) return SVM_ERR_HULL;
-    k_hull_ring<<<(n + kB - 1) / kB, kB, 0, s>>>(star, deg, n, own, F, ringOff, ring, err);
-    if (check_launch()) return SVM_ERR_CUDA;
+    const double side = std::min(2.5 * spacing, gridR);
+    if (!(side > 0) || !std::isfinite(gridR)) return SVM_ERR_ARG;
+    BinGrid g;
+    g.nside = (int)std::floor(2.0 * gridR / side);
+    g.nside -= g.nside % 2;
+    if (g.nside < 1 || g.nside > 1024) return SVM_ERR_ARG;
+    g.h = 2.0 * gridR / g.nside;
+    g.radius = gridR;
+    const size_t bins = (size_t)g.nside * g.nside * g.nside, nf = 2 * (size_t)n - 4;
+    // one allocation: what svm_topology_get copies (kept), and the workspace
+    Arena A;
+    double *P, *vpos;
+    int *deg, *star, *own, *ctl, *retry, *F, *vcells, *vnbrs, *ringOff, *ring, *off, *cursor, *binOf, *list, *tmp, *sums;
+    const auto lay = [&] {
+        A.used = 0;
+        vpos = A.cut<double>(3 * nf);
+        vcells = A.cut<int>(3 * nf); vnbrs = A.cut<int>(3 * nf); deg = A.cut<int>(n);
+        star = A.cut<int>((size_t)n * kMaxDeg);   // the stars, then the ring rows
+        P = A.cut<double>(3 * (size_t)n);
+        own = A.cut<int>((size_t)n + 1); retry = A.cut<int>(n); F = A.cut<int>(3 * nf);
+        ringOff = A.cut<int>((size_t)n + 1); ring = A.cut<int>(3 * nf);
+        binOf = A.cut<int>(n); list = A.cut<int>(n); tmp = A.cut<int>(n);
+        sums = A.cut<int>(scan_ints(std::max(bins + 1, (size_t)n + 1)));
+        ctl = A.cut<int>(4);   // [0] error bits, [1] centres queued for the wider search, [2] largest ring
+        off = A.cut<int>(bins + 1); cursor = A.cut<int>(bins);   // (cleared together, to the end)
+    };
+    lay();
+    const size_t bytes = A.used;
     svm_topology* t = new svm_topology();
-    Topology& T = t->t;
-    T.nCells = n;
-    T.nVertices = nf;
-    T.vertexPos.resize(3 * (size_t)nf);
-    T.vertexCells.resize(3 * (size_t)nf);
-    T.vertexNeighbors.resize(3 * (size_t)nf);
-    T.ringOffsets.resize((size_t)n + 1);
-    T.ringVertices.resize(3 * (size_t)nf);
-    std::vector<int> degs(n);
-    bool ok = cudaMemcpyAsync(T.vertexPos.data(), vpos, sizeof(double) * 3 * nf, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-              cudaMemcpyAsync(T.vertexCells.data(), vcells, sizeof(int) * 3 * nf, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-              cudaMemcpyAsync(T.vertexNeighbors.data(), vnbrs, sizeof(int) * 3 * nf, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-              cudaMemcpyAsync(T.ringOffsets.data(), ringOff, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-              cudaMemcpyAsync(T.ringVertices.data(), ring, sizeof(int) * 3 * nf, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-              cudaMemcpyAsync(degs.data(), deg, sizeof(int) * n, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-              cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, s) == cudaSuccess &&
-              cudaStreamSynchronize(s) == cudaSuccess;
-    if (!ok || e) { delete t; return ok ? SVM_ERR_HULL : SVM_ERR_CUDA; }
-    T.maxRing = *std::max_element(degs.begin(), degs.end());
+    t->dev = new DeviceTopology();
+    if (cudaMalloc(&t->dev->base, bytes) != cudaSuccess) { cudaGetLastError(); delete t; return SVM_ERR_CUDA; }
+    A.base = (char*)t->dev->base;
+    lay();
+    const auto fail = [&](int rc) { cudaStreamSynchronize(s); delete t; return rc; };
+    if (cudaMemcpyAsync(P, pts, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, s) != cudaSuccess ||
+        cudaMemsetAsync(ctl, 0, (char*)A.base + bytes - (char*)ctl, s) != cudaSuccess ||
+        cudaMemsetAsync(own + n, 0, sizeof(int), s) != cudaSuccess)
+        return fail(SVM_ERR_CUDA);
+    const int nb = (n + kB - 1) / kB;
+    k_hb_count<<<nb, kB, 0, s>>>(P, n, g.nside, g.h, g.radius, binOf, off, ctl);
+    if (check_launch() || exclusive_scan(off, (int)bins + 1, s, sums)) return fail(SVM_ERR_CUDA);
+    k_hb_place<<<nb, kB, 0, s>>>(binOf, n, off, cursor, tmp);
+    k_hb_order<<<nb, kB, 0, s>>>(binOf, n, off, tmp, list);
+    g.off = off;
+    g.list = list;
+    const int warps = kHB / 32;
+    k_hull_star<kFewCand><<<(n + warps - 1) / warps, kHB, 0, s>>>(P, nullptr, nullptr, n, 1, 1, g, deg, star, retry, ctl + 1, ctl);
+    // the queued centres, however many there are (their count stays on the device): six blocks per SM
+    k_hull_star<kMaxCand><<<std::min((n + warps - 1) / warps, 6 * 152), kHB, 0, s>>>(P, retry, ctl + 1, n, 1, kMaxW, g, deg,
+                                                                                   star, nullptr, nullptr, ctl);
+    k_hull_check<<<nb, kB, 0, s>>>(star, deg, n, own, ctl);
+    if (check_launch() || exclusive_scan(own, n + 1, s, sums)) return fail(SVM_ERR_CUDA);
+    // the stars have to close into one triangulated sphere before facets are numbered from them
+    k_hull_max<<<nb, kB, 0, s>>>(deg, n, ctl + 2);
+    int got[3], facets = 0;
+    if (check_launch() || cudaMemcpyAsync(got, ctl, sizeof(got), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaMemcpyAsync(&facets, own + n, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess)
+        return fail(SVM_ERR_CUDA);
+    if (got[0] & kOutside) return fail(SVM_ERR_DEVICE);
+    if (got[0] || (size_t)facets != nf) return fail(SVM_ERR_HULL);
+    const double radius = std::sqrt(pts[0] * pts[0] + pts[1] * pts[1] + pts[2] * pts[2]);
+    k_hull_emit<<<nb, kB, 0, s>>>(star, deg, n, own, F);
+    k_hull_vertex<<<((int)nf + kB - 1) / kB, kB, 0, s>>>(P, F, (int)nf, own, star, deg, radius, vpos, vcells, vnbrs, ctl);
+    if (check_launch() || cudaMemcpyAsync(ringOff, deg, sizeof(int) * n, cudaMemcpyDeviceToDevice, s) != cudaSuccess ||
+        cudaMemsetAsync(ringOff + n, 0, sizeof(int), s) != cudaSuccess || exclusive_scan(ringOff, n + 1, s, sums))
+        return fail(SVM_ERR_CUDA);
+    // (a triangulated sphere of nf facets has rings of 3 nf entries)
+    k_hull_ring<<<nb, kB, 0, s>>>(star, deg, n, own, F, ringOff, ring, ctl);
+    const int W = got[2];
+    k_hull_rows<<<(int)(((long)n * W + kB - 1) / kB), kB, 0, s>>>(ringOff, ring, n, W, star);
+    int e = 0, nr = 0;
+    if (check_launch() || cudaMemcpyAsync(&e, ctl, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaMemcpyAsync(&nr, ringOff + n, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess)
+        return fail(SVM_ERR_CUDA);
+    if (e || (size_t)nr != 3 * nf) return fail(SVM_ERR_HULL);
+    t->t.nCells = n;
+    t->t.nVertices = (int)nf;
+    t->t.maxRing = W;
+    t->dev->vpos = vpos; t->dev->vcells = vcells; t->dev->vnbrs = vnbrs; t->dev->rows = star; t->dev->deg = deg;
     *out = t;
     return SVM_OK;
 }

@@ -2267,6 +2267,7 @@ int svm_topology_get(const svm_topology* t, double* vp, int* rings, int stride, 
     if (!t) return SVM_ERR_ARG;
     const svm::Topology& T = t->t;
     if (rings && stride < T.maxRing) return SVM_ERR_ARG;
+    if (t->dev) return svm::device_topology_get(t, vp, rings, stride, counts, vc, vn);
     if (vp) std::memcpy(vp, T.vertexPos.data(), sizeof(double) * T.vertexPos.size());
     if (vc) std::memcpy(vc, T.vertexCells.data(), sizeof(int) * T.vertexCells.size());
     if (vn) std::memcpy(vn, T.vertexNeighbors.data(), sizeof(int) * T.vertexNeighbors.size());
