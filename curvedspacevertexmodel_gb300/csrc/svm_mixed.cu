@@ -99,7 +99,9 @@ __device__ __forceinline__ float4 move_fp64(float4 p, F3 d, double R) {
     const F3 dt = d - (dotf(d, pf) / dotf(pf, pf)) * pf;
     const double qx = sf::widen(p.x) + sf::widen(dt.x), qy = sf::widen(p.y) + sf::widen(dt.y),
                  qz = sf::widen(p.z) + sf::widen(dt.z);
-    const double k = R * rsqrt(qx * qx + qy * qy + qz * qz);
+    // (on the integer pipes: the FP64 pipe, 72% busy with CUDA's rsqrt, bounded the force kernel; 126.8 -> 120.8
+    // us at 1M cells)
+    const double k = f64_div_root(R, qx * qx + qy * qy + qz * qz);
     return make_float4(sf::narrow(k * qx), sf::narrow(k * qy), sf::narrow(k * qz), p.w);
 }
 
@@ -126,67 +128,69 @@ __device__ __forceinline__ F3 normals32(uint64_t seed, unsigned long long step, 
     return F3{a * c0, a * s0, b * cospif(2.0f * u24(r.w))};
 }
 
+// Three threads a vertex: thread (v, j) evaluates the edge to neighbour j (FP64 cross product with v and its
+// norm, FP32 arc, T1 test), then, after a block barrier, the corner of cell slot j.  A block of any size
+// takes blockDim.x / 3 vertices.  Dynamic shared memory: 46 bytes a thread (corner_smem).
+// What bounds it: the FP64 pipe (some 120 instructions per 32 vertices, more than half of them the
+// arccosines').  One thread a vertex took 106 registers (16 warps per SM, pipe 66% busy).  Corner phase
+// against that: 200 cells 21.4 -> 12.9 us, 20k 29.4 -> 22.1, 100k 73.4 -> 65.6, 1M 583 -> 562, 512 replicas
+// (646k cells) 383 -> 371.
 __global__ void k32_corners(const float4* __restrict__ pos, const int4* __restrict__ vcell,
                             const int4* __restrict__ vlast, const int4* __restrict__ vnext,
                             const int4* __restrict__ vrpos, const int4* __restrict__ vnbr,
                             double2* __restrict__ corner, int Wc, int nV, const double* __restrict__ repR,
                             int t1test, float t1Threshold, T1Scratch t1) {
     step_begin();
-    // block_acos's arrays: 3 blockDim.x values, their sources, a count per warp
     extern __shared__ double cornerSh[];
-    double* val = cornerSh;
-    int* warpHigh = reinterpret_cast<int*>(val + 3 * blockDim.x);
+    const int bs = blockDim.x, t = threadIdx.x;
+    double *cx = cornerSh, *cy = cx + bs, *cz = cy + bs, *nc = cz + bs, *val = nc + bs;
+    float* arcs = reinterpret_cast<float*>(val + bs);
+    int* warpHigh = reinterpret_cast<int*>(arcs + bs);
     unsigned short* src = reinterpret_cast<unsigned short*>(warpHigh + 32);
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = v < nV;
+    const int per = bs / 3, vi = t / 3, j = t - 3 * vi, v = blockIdx.x * per + vi;
+    const bool live = vi < per && v < nV;
     float4 p;
-    float R, arcs[3];
-    double cosine[3] = {-1.0, -1.0, -1.0};
-    bool flip[3] = {false, false, false}, ok[3];
-    int4 cells, lasts, nexts;
+    float R;
+    int4 nb;
     if (live) {
         p = pos[v];
         R = sf::narrow(repR[rep_of(p)]);
-        const D3 pd = ld3(pos, v);
-        const int4 nb = vnbr[v];
+        nb = vnbr[v];
+        const int u = comp(nb, j);
+        const float4 q = pos[u];
+        const D3 C = cross3e(D3{sf::widen(p.x), sf::widen(p.y), sf::widen(p.z)}, D3{sf::widen(q.x), sf::widen(q.y), sf::widen(q.z)});
+        const float arc = arc32(q, p, R);
+        cx[t] = C.x; cy[t] = C.y; cz[t] = C.z;
+        nc[t] = f64_sqrt(dot3e(C, C));
+        arcs[t] = arc;
+        if (t1test && v < u && arc < t1Threshold) t1_flag(t1, 3 * v + j, v, u, rep_of(p), vnbr, vcell);
+    }
+    __syncthreads();
+    double cosine[1] = {-1.0};
+    float arc = 0.f;
+    bool flip = false, ok = false;
+    int4 cells, lasts, nexts;
+    if (live) {
         cells = vcell[v]; lasts = vlast[v]; nexts = vnext[v];
-        // per neighbour: FP64 cross product with p and its norm (for the included angles), FP32 arc
-        D3 U[3], C[3];
-        double nC[3];
-        float arc[3];
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            const float4 q = pos[comp(nb, j)];
-            U[j] = D3{sf::widen(q.x), sf::widen(q.y), sf::widen(q.z)};
-            C[j] = cross3e(pd, U[j]);
-            nC[j] = f64_sqrt(dot3e(C[j], C[j]));
-            arc[j] = arc32(q, p, R);
-            const int u = comp(nb, j);
-            if (t1test && v < u && arc[j] < t1Threshold) t1_flag(t1, 3 * v + j, v, u, rep_of(p), vnbr, vcell);
-        }
-#pragma unroll
-        for (int s = 0; s < 3; ++s) {
-            const int jl = nbr_slot(nb, comp(lasts, s)), jx = nbr_slot(nb, comp(nexts, s));
-            ok[s] = jl >= 0 && jx >= 0;
-            if (ok[s]) {
-                arcs[s] = pick3(arc, jl);
-                flip[s] = positive(dot3e(pick3(U, jl), pick3(C, jx)));
-                cosine[s] = included_cos<true>(pick3(C, jx), pick3(C, jl), pick3(nC, jx), pick3(nC, jl));
-            }
+        const int last = comp(lasts, j), jl = nbr_slot(nb, last), jx = nbr_slot(nb, comp(nexts, j));
+        ok = jl >= 0 && jx >= 0;
+        if (ok) {
+            const int l = 3 * vi + jl, x = 3 * vi + jx;
+            const D3 X{cx[x], cy[x], cz[x]};
+            arc = arcs[l];
+            flip = positive(dot3e(ld3(pos, last), X));
+            cosine[0] = included_cos<true>(X, D3{cx[l], cy[l], cz[l]}, nc[x], nc[l]);
         }
     }
     block_acos(cosine, val, src, warpHigh);
     if (!live) return;
     const int4 rp = vrpos[v];
-#pragma unroll
-    for (int s = 0; s < 3; ++s) {
-        double2 cr = make_double2(sf::widen(arcs[s]), included_finish(cosine[s], flip[s]));
-        if (!ok[s]) {  // inconsistent lists: evaluate directly
-            const int L = comp(lasts, s), X = comp(nexts, s);
-            cr = make_double2(sf::widen(arc32(pos[L], p, R)), included_angle_clamped(ld3(pos, L), ld3(pos, v), ld3(pos, X)));
-        }
-        corner[(long)comp(cells, s) * Wc + comp(rp, s)] = cr;
+    double2 cr = make_double2(sf::widen(arc), included_finish(cosine[0], flip));
+    if (!ok) {  // inconsistent lists: evaluate directly
+        const int L = comp(lasts, j), X = comp(nexts, j);
+        cr = make_double2(sf::widen(arc32(pos[L], p, R)), included_angle_clamped(ld3(pos, L), ld3(pos, v), ld3(pos, X)));
     }
+    corner[(long)comp(cells, j) * Wc + comp(rp, j)] = cr;
 }
 
 __global__ void k32_force(Args32 A, int nV, float4* __restrict__ force) {
@@ -255,11 +259,13 @@ Args32 args32(svm_model* m, int buf) {
 
 namespace svm {
 
-// dynamic shared memory of k32_corners (at most 31 KB, at 1024 threads)
-static int corner_smem(int threads) { return 3 * threads * (int)(sizeof(double) + sizeof(unsigned short)) + 32 * (int)sizeof(int); }
+// dynamic shared memory of k32_corners: 46 bytes a thread and a count per warp (at most 47 KB, at 1024)
+static int corner_smem(int threads) {
+    return threads * (int)(5 * sizeof(double) + sizeof(float) + sizeof(unsigned short)) + 32 * (int)sizeof(int);
+}
 int mixed_launch_corners(svm_model* m, bool t1test) {
     const int bs = m->blkCorners;
-    launch_next_smem(m, k32_corners, (m->nVertices + bs - 1) / bs, bs, corner_smem(bs), m->pos32[m->cur], m->vcell, m->vlast, m->vnext,
+    launch_next_smem(m, k32_corners, (m->nVertices + bs / 3 - 1) / (bs / 3), bs, corner_smem(bs), m->pos32[m->cur], m->vcell, m->vlast, m->vnext,
                                                                   m->vrpos, m->vnbr, m->corner, m->Wc, m->nVertices,
                                                                   m->repR, t1test ? 1 : 0, (float)m->t1Threshold, m->t1);
     return check_launch();
