@@ -36,20 +36,25 @@ __device__ double rep_block_sum(double v) {
     return r;
 }
 
-// one block per replica: total area, excess over 4 pi R^2, fallback flag
+// one block per replica: total area, excess over 4 pi R^2, fallback flag, and the list of the flagged
 __global__ void k_rep_check(const double2* __restrict__ ap, const int* __restrict__ cellOff,
-                            const double* __restrict__ repR, int* __restrict__ repFlag, double* __restrict__ repScal) {
+                            const double* __restrict__ repR, int* __restrict__ repFlag, double* __restrict__ repScal,
+                            int* __restrict__ repList) {
     step_begin();
     const int r = blockIdx.x;
     double s = 0.0;
-    for (int c = cellOff[r] + threadIdx.x; c < cellOff[r + 1]; c += blockDim.x) s += ap[c].x;
+    const int last = cellOff[r + 1];
+#pragma unroll 4
+    for (int c = cellOff[r] + threadIdx.x; c < last; c += blockDim.x) s += ap[c].x;
     const double total = rep_block_sum(s);
     if (threadIdx.x == 0) {
         const double R = repR[r];
         const double excess = total - 4.0 * kPI * R * R;
         repScal[3 * r] = total;
         repScal[3 * r + 1] = excess;
-        repFlag[r] = fabs(excess) > mixed_area_limit(cellOff[r + 1] - cellOff[r], R) ? 1 : 0;
+        const int taken = fabs(excess) > mixed_area_limit(last - cellOff[r], R) ? 1 : 0;
+        repFlag[r] = taken;
+        if (taken) repList[1 + atomicAdd(repList, 1)] = r;   // (cleared by k_cells, which precedes this)
     }
 }
 
@@ -96,7 +101,7 @@ struct BatchTuners {
 namespace svm {
 
 int launch_rep_check(svm_model* m) {
-    launch_next(m, k_rep_check, m->nRep, kRB, m->ap, m->repCellOff, m->repR, m->repFlag, m->repScal);
+    launch_next(m, k_rep_check, m->nRep, kRB, m->ap, m->repCellOff, m->repR, m->repFlag, m->repScal, m->repList);
     return check_launch();
 }
 

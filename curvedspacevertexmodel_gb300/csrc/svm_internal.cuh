@@ -614,6 +614,7 @@ struct svm_model {
     int* repCellOff = nullptr;         // device [nRep + 1]
     int* repVertOff = nullptr;         // device [nRep + 1]
     int* repFlag = nullptr;            // device [nRep], area-check fallback flags
+    int* repList = nullptr;            // device [1 + nRep]: how many of a batch's replicas failed the check, which
     double* repScal = nullptr;         // device [3 nRep]: total area, excess, energy
     std::vector<double> repT;          // host, per-replica temperatures of a batch
     std::vector<int> hRepCellOff, hRepVertOff;

@@ -312,6 +312,22 @@ __global__ void __launch_bounds__(kCornerThreads, 6) k_corner(const double4_32a*
     }
 }
 
+// (n - 2) kPI and (n - 2) kPILo for rings of n entries up to kRingTable: the products as the reference
+// rounds them, without the conversion and the products on the FP64 pipe.
+constexpr int kRingTable = 32;
+struct PolygonAngles { double pi[kRingTable + 1], lo[kRingTable + 1]; };
+constexpr PolygonAngles polygon_angles() {
+    PolygonAngles a{};
+    for (int n = 0; n <= kRingTable; ++n) {
+        a.pi[n] = (double)(n - 2) * kPI;
+        a.lo[n] = (double)(n - 2) * kPILo;
+    }
+    return a;
+}
+__constant__ PolygonAngles kPolygon = polygon_angles();
+__device__ __forceinline__ double polygon_pi(int n) { return n <= kRingTable ? kPolygon.pi[n] : __dmul_rn((double)(n - 2), kPI); }
+__device__ __forceinline__ double polygon_lo(int n) { return n <= kRingTable ? kPolygon.lo[n] : __dmul_rn((double)(n - 2), kPILo); }
+
 // Per cell: centroid (sum of ring vertices in ring order, renormalised), perimeter and angle sum
 // in the CPU's order (ring positions n-2, n-1, 0, ..., n-3), area = (sum - (n-2) pi) wrapped
 // by floor(area / pi), times R^2 (sphericalVertexModel.cpp:228-303).  The last block to finish
@@ -331,8 +347,9 @@ __global__ void k_cells(const PT* __restrict__ pos, const int* __restrict__ ring
                         double R0, const double* __restrict__ repR, PT* __restrict__ cellPos,
                         double4_32a* __restrict__ cellSph, double2* __restrict__ ap, double* __restrict__ partials,
                         unsigned* __restrict__ ticket, double* __restrict__ scalars, int* __restrict__ fallbackFlag,
-                        const double2* __restrict__ pref, float2* __restrict__ dap32) {
+                        const double2* __restrict__ pref, float2* __restrict__ dap32, int* __restrict__ repList) {
     step_begin();
+    if (repList && blockIdx.x == 0 && threadIdx.x == 0) repList[0] = 0;   // (filled by k_rep_check, which follows)
     const int cells = kSplit ? blockDim.x >> 1 : blockDim.x;
     const bool second = kSplit && threadIdx.x >= cells;   // (split: the second half of the block)
     const int c = blockIdx.x * cells + threadIdx.x - (second ? cells : 0);
@@ -379,14 +396,17 @@ __global__ void k_cells(const PT* __restrict__ pos, const int* __restrict__ ring
                 per += x.x;
                 ang += x.y;
             }
-            area = __dsub_rn(ang, __dmul_rn((double)(n - 2), kPI));
+            area = __dsub_rn(ang, polygon_pi(n));
             // The mixed form also subtracts (n - 2) times the part of pi below the double kPI: the
             // reference's excess is biased by +(n - 2)(pi - kPI) per cell, which over a sphere sums to
             // ~4N (pi - kPI) R^2 (4e-7 at N = 100k, 4e-5 at N = 1M) and trips its absolute 1e-6 area
             // check by itself at large N.  The FP64 form keeps the reference's arithmetic.
-            if (std::is_same<PT, float4>::value) area = __dsub_rn(area, __dmul_rn((double)(n - 2), kPILo));
-            const int extra = (int)floor(f64_div(area, 1.0 * kPI));
-            if (extra > 0) area = __dsub_rn(area, __dmul_rn((double)extra, kPI));
+            if (std::is_same<PT, float4>::value) area = __dsub_rn(area, polygon_lo(n));
+            // (an area whose high word is below pi's is below pi, and floor(area / kPI) not above 0)
+            if (__double2hiint(area) >= 0x400921fb) {
+                const int extra = (int)floor(f64_div(area, 1.0 * kPI));
+                if (extra > 0) area = __dsub_rn(area, __dmul_rn((double)extra, kPI));
+            }
             area = __dmul_rn(__dmul_rn(area, R), R);
             ap[c] = make_double2(area, per);
             if (dap32) {
@@ -457,77 +477,86 @@ __global__ void k_fallback(const PT* __restrict__ pos, const int* __restrict__ r
 // FP64 acos chains, and the FP64 pipe charges a warp instruction whatever its active lanes) and
 // every corner normalised once (a ring vertex serves two triangles, the centroid all of them),
 // then each cell's triangles summed in the CPU's order by one thread: the same areas bit for bit.
-// kFanCells cells per block; ring capacity <= 32.
+// kFanCells cells at a time per block; ring capacity <= 32.  The blocks share out the sphere's cells, or,
+// for a batch, those of the replicas in repList (count first, filled by k_rep_check): a launch that finds
+// nothing to do costs its few blocks a look at the flag (a block per kFanCells cells cost a batch of 646k
+// cells 61 us a step; 6.7 now).
 constexpr int kFanCells = 32;
 constexpr int kFanThreads = 256;
 template <class PT>
 __global__ void __launch_bounds__(kFanThreads) k_fallback_fan(
     const PT* __restrict__ pos, const int* __restrict__ ring, const int* __restrict__ ringCount,
     const PT* __restrict__ cellPos, int Wc, int nC, double R0, const int* __restrict__ fallbackFlag,
-    const int* __restrict__ repFlag, const double* __restrict__ repR, double2* __restrict__ ap,
-    const double2* __restrict__ pref, float2* __restrict__ dap32) {
+    const int* __restrict__ repList, const int* __restrict__ cellOff, const double* __restrict__ repR,
+    double2* __restrict__ ap, const double2* __restrict__ pref, float2* __restrict__ dap32) {
     step_begin();
-    if (!repFlag && *fallbackFlag == 0) return;
+    if (!repList && *fallbackFlag == 0) return;
     __shared__ int cnt[kFanCells], off[kFanCells + 1], owner[kFanCells * 32];
-    __shared__ double radius[kFanCells];
     __shared__ double ux[kFanCells * 32], uy[kFanCells * 32], uz[kFanCells * 32];
     __shared__ double cx[kFanCells], cy[kFanCells], cz[kFanCells];
     __shared__ double tri[kFanCells * 32];
     __shared__ double val[3 * kFanThreads];   // block_acos
     __shared__ unsigned short src[3 * kFanThreads];
     __shared__ int warpHigh[kFanThreads / 32];
-    const int t = threadIdx.x, c0 = blockIdx.x * kFanCells;
-    if (t < kFanCells) {
-        const int c = c0 + t;
-        int n = 0;
-        if (c < nC) {
-            n = ringCount[c];
-            const int rep = rep_of(pos[ring[(long)c * Wc]]);
-            if (repFlag && repFlag[rep] == 0) n = 0;  // this replica keeps its areas
-            radius[t] = repR ? repR[rep] : R0;
-            if (n > 0) {
-                const D3 u = unit_corner(ld3(cellPos, c));
-                cx[t] = u.x; cy[t] = u.y; cz[t] = u.z;
+    const int t = threadIdx.x, nList = repList ? repList[0] : 1, G = gridDim.x;
+    int item = 0;   // groups of cells dealt out so far, group i to block i mod G
+    for (int f = 0; f < nList; ++f) {
+        const int rep = repList ? repList[1 + f] : 0;
+        const int first = repList ? cellOff[rep] : 0, last = repList ? cellOff[rep + 1] : nC;
+        const double R = repR ? repR[rep] : R0;
+        const int groups = (last - first + kFanCells - 1) / kFanCells;
+        for (int gI = ((int)blockIdx.x + G - item % G) % G; gI < groups; gI += G) {
+            const int c0 = first + gI * kFanCells;
+            if (t < kFanCells) {
+                const int c = c0 + t;
+                const int n = c < last ? ringCount[c] : 0;
+                if (n > 0) {
+                    const D3 u = unit_corner(ld3(cellPos, c));
+                    cx[t] = u.x; cy[t] = u.y; cz[t] = u.z;
+                }
+                cnt[t] = n;
+                // exclusive scan of the counts over the first warp
+                int incl = n;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (t >= o) incl += y;
+                }
+                off[t] = incl - n;
+                if (t == kFanCells - 1) off[kFanCells] = incl;
+                for (int k = 0; k < n; ++k) owner[incl - n + k] = t;
             }
+            __syncthreads();
+            const int total = off[kFanCells];
+            for (int e = t; e < total; e += kFanThreads) {  // each ring corner, normalised once
+                const int lc = owner[e];
+                const D3 u = unit_corner(ld3(pos, ring[(long)(c0 + lc) * Wc + (e - off[lc])]));
+                ux[e] = u.x; uy[e] = u.y; uz[e] = u.z;
+            }
+            __syncthreads();
+            for (int base = 0; base < total; base += kFanThreads) {
+                // triangle k of cell lc in the CPU's loop: (centroid, ring[k - 2], ring[k - 1]), indices mod n
+                const int e = base + t;
+                double a[3] = {-1.0, -1.0, -1.0};
+                if (e < total) {
+                    const int lc = owner[e], b = off[lc], n = cnt[lc], k = e - b;
+                    const int i2 = b + (k + n - 2) % n, i3 = b + (k + n - 1) % n;
+                    triangle_cosines(D3{cx[lc], cy[lc], cz[lc]}, D3{ux[i2], uy[i2], uz[i2]}, D3{ux[i3], uy[i3], uz[i3]}, a);
+                }
+                block_acos(a, val, src, warpHigh);
+                if (e < total) tri[e] = triangle_sum(a, R);
+            }
+            __syncthreads();
+            if (t < kFanCells && cnt[t] > 0) {
+                const int c = c0 + t;
+                double area = 0.0;
+                for (int k = 0; k < cnt[t]; ++k) area += tri[off[t] + k];
+                ap[c].x = area;
+                if (dap32) dap32[c].x = sf::narrow(area - pref[c].x);
+            }
+            __syncthreads();
         }
-        cnt[t] = n;
-        // exclusive scan of the counts over the first warp
-        int incl = n;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (t >= o) incl += y;
-        }
-        off[t] = incl - n;
-        if (t == kFanCells - 1) off[kFanCells] = incl;
-        for (int k = 0; k < n; ++k) owner[incl - n + k] = t;
+        item += groups;
     }
-    __syncthreads();
-    const int total = off[kFanCells];
-    for (int e = t; e < total; e += kFanThreads) {  // each ring corner, normalised once
-        const int lc = owner[e];
-        const D3 u = unit_corner(ld3(pos, ring[(long)(c0 + lc) * Wc + (e - off[lc])]));
-        ux[e] = u.x; uy[e] = u.y; uz[e] = u.z;
-    }
-    __syncthreads();
-    for (int base = 0; base < total; base += kFanThreads) {
-        // triangle k of cell lc in the CPU's loop: (centroid, ring[k - 2], ring[k - 1]), indices mod n
-        const int e = base + t;
-        double a[3] = {-1.0, -1.0, -1.0};
-        if (e < total) {
-            const int lc = owner[e], b = off[lc], n = cnt[lc], k = e - b;
-            const int i2 = b + (k + n - 2) % n, i3 = b + (k + n - 1) % n;
-            triangle_cosines(D3{cx[lc], cy[lc], cz[lc]}, D3{ux[i2], uy[i2], uz[i2]}, D3{ux[i3], uy[i3], uz[i3]}, a);
-        }
-        block_acos(a, val, src, warpHigh);
-        if (e < total) tri[e] = triangle_sum(a, radius[owner[e]]);
-    }
-    __syncthreads();
-    if (t >= kFanCells || cnt[t] == 0) return;
-    const int c = c0 + t;
-    double area = 0.0;
-    for (int k = 0; k < cnt[t]; ++k) area += tri[off[t] + k];
-    ap[c].x = area;
-    if (dap32) dap32[c].x = sf::narrow(area - pref[c].x);
 }
 
 // ---- forces and integration ------------------------------------------------------------------
@@ -1983,7 +2012,7 @@ static int launch_cells_batch(svm_model* m) {
     const int bs = m->blkCells;
     launch_next(m, k_cells<float4, false>, (m->nCells + bs - 1) / bs, bs,
         m->pos32[m->cur], m->ring, m->ringCount, m->corner, m->Wc, m->nCells, m->R, m->repR, m->cellPos32, nullptr,
-        m->ap, nullptr, nullptr, nullptr, nullptr, m->pref, m->dap32);
+        m->ap, nullptr, nullptr, nullptr, nullptr, m->pref, m->dap32, m->repList);
     return check_launch();
 }
 
@@ -2003,24 +2032,25 @@ static int launch_cells(svm_model* m) {
         } else if (mixed) {
             launch_next(m, split ? k_cells<float4, true> : k_cells<float4, false>, nb, bs,
                 m->pos32[m->cur], m->ring, m->ringCount, m->corner, m->Wc, m->nCells, m->R, m->repR, m->cellPos32,
-                nullptr, m->ap, m->partials, m->ticket, m->scalars, m->fallbackFlag, m->pref, m->dap32);
+                nullptr, m->ap, m->partials, m->ticket, m->scalars, m->fallbackFlag, m->pref, m->dap32, nullptr);
         } else {
             launch_next(m, split ? k_cells<double4_32a, true> : k_cells<double4_32a, false>, nb, bs,
                 m->pos[m->cur], m->ring, m->ringCount, m->corner, m->Wc, m->nCells, m->R, nullptr, m->cellPos,
-                m->cellSph, m->ap, m->partials, m->ticket, m->scalars, m->fallbackFlag, nullptr, nullptr);
+                m->cellSph, m->ap, m->partials, m->ticket, m->scalars, m->fallbackFlag, nullptr, nullptr, nullptr);
         }
     }
     PhaseTimer pt(m, SVM_PHASE_FALLBACK);
     if (m->Wc <= 32) {
-        const int nf = (m->nCells + kFanCells - 1) / kFanCells;
+        // (four blocks per SM are resident, by their shared memory)
+        const int nf = std::min((m->nCells + kFanCells - 1) / kFanCells, 4 * m->sms);
         if (mixed)
             launch_next(m, k_fallback_fan<float4>, nf, kFanThreads,
                 m->pos32[m->cur], m->ring, m->ringCount, m->cellPos32, m->Wc, m->nCells, m->R, m->fallbackFlag,
-                batch ? m->repFlag : nullptr, m->repR, m->ap, m->pref, m->dap32);
+                batch ? m->repList : nullptr, m->repCellOff, m->repR, m->ap, m->pref, m->dap32);
         else
             launch_next(m, k_fallback_fan<double4_32a>, nf, kFanThreads,
                 m->pos[m->cur], m->ring, m->ringCount, m->cellPos, m->Wc, m->nCells, m->R, m->fallbackFlag, nullptr,
-                nullptr, m->ap, nullptr, nullptr);
+                nullptr, nullptr, m->ap, nullptr, nullptr);
     } else if (mixed)
         launch_next(m, k_fallback<float4>, blocksFor(m->nCells), kBlock, m->pos32[m->cur], m->ring, m->ringCount, m->cellPos32, m->Wc,
                                                          m->nCells, m->R, m->fallbackFlag, batch ? m->repFlag : nullptr,
@@ -2386,6 +2416,7 @@ int svm::model_alloc(int nCells, int nVertices, int Wc, const double* radius, in
     alloc((void**)&m->repVertOff, (nRep + 1) * sizeof(int));
     alloc((void**)&m->repFlag, nRep * sizeof(int));
     alloc((void**)&m->repScal, 3 * nRep * sizeof(double));
+    if (nRep > 1) alloc((void**)&m->repList, (nRep + 1) * sizeof(int));
     if (nRep > 1) m->t1.segOff = m->repVertOff;
     alloc((void**)&m->ringMax, sizeof(int));
     if (ok && cudaHostAlloc((void**)&m->ringMaxHost, sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
@@ -2424,7 +2455,7 @@ int svm_model_destroy(svm_model* m) {
                     m->t1.resC, m->t1.comV, m->t1.comC, m->t1.undo, m->t1.undoRings, m->t1.ctr, m->t1.stats,
                     m->pos32[0], m->pos32[1], m->cellPos32, m->force32, m->dap32, m->repR, m->repNp, m->repCellOff,
                     m->repVertOff, m->t1.clocks,
-                    m->repFlag, m->repScal, m->dotPartials, m->ringMax};
+                    m->repFlag, m->repScal, m->repList, m->dotPartials, m->ringMax};
     for (void* p : ptrs) if (p) cudaFree(p);
     if (m->ringMaxHost) cudaFreeHost(m->ringMaxHost);
     for (cudaEvent_t e : m->passEv)
