@@ -6,10 +6,11 @@
 // (inc/indexer.h:170-176).  The reference GPU kernel (hyperrectangularCellList.cu:14-51) fills
 // slots in atomic order; here the slots of a bin are put in ascending point index, as the CPU
 // loop leaves them, so the table is deterministic.  Kernels:
-//   k_cl_clear   zero the counts of the bins the previous call used (not the whole grid)
-//   k_cl_bin     bin each point, take a provisional slot with an atomic
-//   k_cl_order   rank each point among its bin's entries by index, write the final slot
-//   k_cl_nmax    Nmax = max(Nmax, largest occupancy), the grow-only width of the reference
+//   k_cl_clear   zero the counts of the bins the previous call used (not the whole grid), and the
+//                call's scalars
+//   k_cl_bin     bin each point, take a provisional slot with an atomic; a neighbour list's FP32 copies
+//   k_cl_order   rank each point among its bin's entries by index, write the final slot;
+//                Nmax = max(Nmax, largest occupancy), the grow-only width of the reference
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -29,12 +30,16 @@ struct svm_cell_list {
     int* tmp = nullptr;           // [total * cap] provisional slots
     int* slots = nullptr;         // [total * cap] ordered slots
     int* binOf = nullptr;         // [nPoints]
-    int* scalars = nullptr;       // [0] max occupancy this call, [1] Nmax (grow-only), [2] overflow, [3] out of grid
+    // [0] max occupancy this call, [1] Nmax (grow-only), [2] overflow, [3] out of grid, [4] the neighbour
+    // list's longest row
+    int* scalars = nullptr;
+    int* hostScalars = nullptr;   // page-locked, what the host reads of them
     bool first = true;
 };
 
 namespace {
 constexpr int kB = 256;
+constexpr int kClScalars = 5;
 
 __device__ __forceinline__ int bin_of(double x, double y, double z, double r, double h, int n, int* bad) {
     int bx = (int)floor((x + r) / h), by = (int)floor((y + r) / h), bz = (int)floor((z + r) / h);
@@ -45,19 +50,22 @@ __device__ __forceinline__ int bin_of(double x, double y, double z, double r, do
     return bx + by * n + bz * n * n;
 }
 
-__global__ void k_cl_clear(const int* __restrict__ binOf, unsigned* counts, int np) {
+__global__ void k_cl_clear(const int* __restrict__ binOf, unsigned* counts, int np, int* __restrict__ scalars) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < kClScalars && i != 1) scalars[i] = 0;  // (np >= 1: the grid has the threads)
     if (i < np && binOf[i] >= 0) counts[binOf[i]] = 0u;
 }
 
 template <typename P>
 __global__ void k_cl_bin(P pts, int np, double r, double h, int n, int cap, int* __restrict__ binOf,
-                         unsigned* __restrict__ counts, int* __restrict__ tmp, int* __restrict__ scalars) {
+                         unsigned* __restrict__ counts, int* __restrict__ tmp, int* __restrict__ scalars,
+                         float4* __restrict__ p32) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     int occ = 0;
     if (i < np) {
         double x, y, z;
         pts(i, x, y, z);
+        if (p32) p32[i] = make_float4((float)x, (float)y, (float)z, 0.f);
         const int b = bin_of(x, y, z, r, h, n, scalars + 3);
         binOf[i] = b;
         const unsigned s = atomicAdd(counts + b, 1u);
@@ -71,8 +79,9 @@ __global__ void k_cl_bin(P pts, int np, double r, double h, int n, int cap, int*
 }
 
 __global__ void k_cl_order(const int* __restrict__ binOf, const unsigned* __restrict__ counts,
-                           const int* __restrict__ tmp, int* __restrict__ slots, int np, int cap) {
+                           const int* __restrict__ tmp, int* __restrict__ slots, int np, int cap, int* __restrict__ scalars) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) scalars[1] = max(scalars[1], scalars[0]);
     if (i >= np) return;
     const int b = binOf[i];
     const int c = min((int)counts[b], cap);
@@ -85,10 +94,6 @@ __global__ void k_cl_order(const int* __restrict__ binOf, const unsigned* __rest
         present |= j == i;
     }
     if (present) slots[(long)b * cap + rank] = i;
-}
-
-__global__ void k_cl_nmax(int* scalars) {
-    scalars[1] = max(scalars[1], scalars[0]);
 }
 
 struct ModelPoints {
@@ -104,18 +109,35 @@ struct AosPoints {
     __device__ void operator()(int i, double& x, double& y, double& z) const { x = p[3 * i]; y = p[3 * i + 1]; z = p[3 * i + 2]; }
 };
 
+// `p32`: where to leave FP32 copies of the points, or null
 template <typename P>
-int compute(svm_cell_list* cl, P pts, int np) {
+int compute(svm_cell_list* cl, P pts, int np, float4* p32 = nullptr) {
     if (np != cl->nPoints) return SVM_ERR_ARG;
     const int nb = (np + kB - 1) / kB;
-    k_cl_clear<<<nb, kB, 0, cl->stream>>>(cl->binOf, cl->counts, np);
-    cudaMemsetAsync(cl->scalars, 0, sizeof(int), cl->stream);      // occupancy of this call
-    cudaMemsetAsync(cl->scalars + 2, 0, 2 * sizeof(int), cl->stream);  // this call's error flags
+    k_cl_clear<<<nb, kB, 0, cl->stream>>>(cl->binOf, cl->counts, np, cl->scalars);
     k_cl_bin<<<nb, kB, 0, cl->stream>>>(pts, np, cl->radius, cl->h, cl->nside, cl->cap, cl->binOf, cl->counts, cl->tmp,
-                                        cl->scalars);
-    k_cl_order<<<nb, kB, 0, cl->stream>>>(cl->binOf, cl->counts, cl->tmp, cl->slots, np, cl->cap);
-    k_cl_nmax<<<1, 1, 0, cl->stream>>>(cl->scalars);
+                                        cl->scalars, p32);
+    k_cl_order<<<nb, kB, 0, cl->stream>>>(cl->binOf, cl->counts, cl->tmp, cl->slots, np, cl->cap, cl->scalars);
     return check_launch();
+}
+
+// The model's points, ordered after the model's pending work.
+int compute_model(svm_cell_list* cl, svm_model* m, float4* p32 = nullptr) {
+    if (cl->stream != m->stream) {
+        cudaEvent_t e;
+        cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+        cudaEventRecord(e, m->stream);
+        cudaStreamWaitEvent(cl->stream, e, 0);
+        cudaEventDestroy(e);
+    }
+    if (m->precision == SVM_PRECISION_MIXED) return compute(cl, ModelPoints32{m->pos32[m->cur]}, m->nVertices, p32);
+    return compute(cl, ModelPoints{m->pos[m->cur]}, m->nVertices, p32);
+}
+
+// This call's scalars, in cl->hostScalars, once the stream has finished.
+int read_scalars(svm_cell_list* cl) {
+    return cudaMemcpyAsync(cl->hostScalars, cl->scalars, sizeof(int) * kClScalars, cudaMemcpyDeviceToHost, cl->stream) == cudaSuccess &&
+                   cudaStreamSynchronize(cl->stream) == cudaSuccess ? SVM_OK : SVM_ERR_CUDA;
 }
 
 // A bin took more points than it has slots: give every bin `cap` slots, as the reference's cell
@@ -139,28 +161,35 @@ int cl_grow(svm_cell_list* cl, int cap) {
 // count exceeds it).
 //
 // FP64 issues at a sixty-fourth of the FP32 rate here, so a candidate is first classified in FP32
-// and only neighbours (and the rare borderline candidate) see FP64:
-//   phase 1, a thread per point: scan the candidates with FP32 copies of the positions.  With E
-//     a bound on |d32 - d64| per component (coordinates within the grid, |x| <= radius, rounded
-//     to FP32 and subtracted: E = radius 2^-21 covers both roundings with a factor of two), a
-//     candidate whose |d32| components all stay below radius - 2E cannot wrap in FP64, and then
+// and only neighbours (and the rare borderline candidate) see FP64.  kNlLanes threads a point:
+//   phase 1: each thread takes kNlBins consecutive bins of the mask and classifies their candidates
+//     with FP32 copies of the positions.  With E a bound on |d32 - d64| per component (coordinates
+//     within the grid, |x| <= radius, rounded to FP32 and subtracted: E = radius 2^-21 covers both
+//     roundings with a factor of two), a candidate whose |d32| components all stay below radius - 2E
+//     cannot wrap in FP64, and then
 //       dd32 > thrHi (> ((range + 2E)(1 + 2^-20))^2)  => |d64| > range      => not a neighbour
 //       dd32 < thrLo (< ((range - 2E)(1 - 2^-20))^2)  => |d64| < range      => a neighbour
 //     (dd32's own rounding is below 3 2^-24 relative, inside the 2^-20 factors).  Any other
-//     candidate takes the reference's FP64 test in place.  Neighbours are queued in order in
-//     shared memory (kNlQueue per thread; the scan resumes where it stopped when a queue fills).
-//   phase 2, the warp: the queued neighbours of its 32 points are dealt over the lanes, and each
-//     lane computes one neighbour's displacement, squared length and root in FP64 exactly as the
-//     reference does, and stores them at the owner's next row position.
+//     candidate takes the reference's FP64 test.  The point's threads add up their counts in bin
+//     order, and each writes its neighbours' indices at its place in the row.
+//   phase 2, the block: the rows of its points, an entry a thread: displacement, squared length and
+//     root in FP64 exactly as the reference does, or zeros past the row's end.
+// What bounds it: phase 1 is a chain of dependent loads (count, slot, position) per candidate, which
+// one thread a point walked for all ~25 candidates with 8 warps on an SM; eight threads a point walk
+// it for three or four candidates each, with 64 warps' loads in flight.  The call on the device, of
+// 39,996 points at two per unit area, range 1: 114 -> 69 us; of 300 points, where launches, clears and
+// the read-back of five scalars are all of it (eleven stream operations, now five): 100 -> 46 us.
 // The minimum-image loops run at most kWrapIters times: points inside the grid need one, and a
 // point outside it is an error the host reports (the cell list's flag).
-constexpr int kNlQueue = 16;
+constexpr int kNlLanes = 8;                 // threads a point
+constexpr int kNlBins = 4;                  // consecutive bins a thread: 32 a round, the usual mask has 27
+constexpr int kNlPoints = kB / kNlLanes;    // points a block
 constexpr int kWrapIters = 8;
-constexpr unsigned kNlWrapped = 0x80000000u;  // queue flag: the displacement wrapped
+constexpr unsigned kNlWrapped = 0x80000000u;  // between the phases: the displacement wrapped
 
 struct NlParams {
     int np, cap, nside, K, nmax;
-    double h, radius, range, range2Hi;
+    double radius, range, range2Hi;
     float wrapLim, thrLo, thrHi;
 };
 
@@ -172,137 +201,153 @@ __device__ __forceinline__ bool min_image(double& d, double radius) {
 }
 
 template <typename P>
-__global__ void k_nl_pack(P pts, int np, float4* __restrict__ p32) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= np) return;
-    double x, y, z;
-    pts(i, x, y, z);
-    p32[i] = make_float4((float)x, (float)y, (float)z, 0.f);
-}
-
-template <typename P>
 __global__ void __launch_bounds__(kB, 6) k_nl(P pts, const float4* __restrict__ p32, NlParams prm,
                                           const unsigned* __restrict__ counts, const int* __restrict__ slots,
-                                          const int* __restrict__ mask, unsigned* __restrict__ npp,
-                                          int* __restrict__ idx, double* __restrict__ vec,
-                                          double* __restrict__ dist, int* __restrict__ maxCount) {
-    __shared__ unsigned queue[kNlQueue * kB];
-    const int lane = threadIdx.x & 31, wbase = threadIdx.x & ~31;
-    const int pp = blockIdx.x * kB + threadIdx.x;
+                                          const int* __restrict__ binOf, const int* __restrict__ mask,
+                                          unsigned* __restrict__ npp, int* __restrict__ idx,
+                                          double* __restrict__ vec, double* __restrict__ dist,
+                                          int* __restrict__ maxCount) {
+    __shared__ double own[kNlPoints][3];
+    __shared__ int stored[kNlPoints];
+    const int sub = threadIdx.x % kNlLanes, row = threadIdx.x / kNlLanes;
+    const int p0 = blockIdx.x * kNlPoints, pp = p0 + row;
     const bool active = pp < prm.np;
-    float t32[3] = {0.f, 0.f, 0.f};
+    float4 t32 = make_float4(0.f, 0.f, 0.f, 0.f);
     int c[3] = {0, 0, 0};
     if (active) {
-        double t[3];
-        pts(pp, t[0], t[1], t[2]);
-        const float4 f = p32[pp];
-        t32[0] = f.x; t32[1] = f.y; t32[2] = f.z;
-        for (int d = 0; d < 3; ++d) c[d] = max(0, min(prm.nside - 1, (int)floor((t[d] + prm.radius) / prm.h)));
+        t32 = p32[pp];
+        const int b = binOf[pp], q = b / prm.nside;  // the (clamped) bin the cell list found
+        c[0] = b - q * prm.nside; c[2] = q / prm.nside; c[1] = q - c[2] * prm.nside;
+        if (sub == 0) pts(pp, own[row][0], own[row][1], own[row][2]);
     }
-    auto cell_at = [&](int k) {
-        int nb[3];
-        for (int d = 0; d < 3; ++d) {
-            nb[d] = (c[d] + mask[3 * k + d]) % prm.nside;
-            if (nb[d] < 0) nb[d] += prm.nside;
+    int have = 0;
+    for (int k0 = 0; k0 < prm.K; k0 += kNlLanes * kNlBins) {
+        // this thread's bins: their first slots and, running, the candidates up to each one's end
+        long first[kNlBins];
+        int end[kNlBins], n[kNlBins];
+#pragma unroll
+        for (int i = 0; i < kNlBins; ++i) {
+            const int k = k0 + sub * kNlBins + i;
+            first[i] = 0;
+            n[i] = 0;
+            if (active && k < prm.K) {
+                int nb[3];
+                for (int d = 0; d < 3; ++d) {
+                    nb[d] = c[d] + mask[3 * k + d];
+                    // the mask's offsets may exceed the grid's side (few bins): the true remainder then
+                    if (nb[d] < 0 || nb[d] >= prm.nside) {
+                        nb[d] %= prm.nside;
+                        if (nb[d] < 0) nb[d] += prm.nside;
+                    }
+                }
+                const long cell = nb[0] + (long)nb[1] * prm.nside + (long)nb[2] * prm.nside * prm.nside;
+                first[i] = cell * prm.cap;
+                n[i] = min((int)counts[cell], prm.cap);
+            }
         }
-        return nb[0] + (long)nb[1] * prm.nside + (long)nb[2] * prm.nside * prm.nside;
-    };
-    // the next bin's count is loaded one bin ahead, off the scan's dependent-load chain
-    int cc = 0, p1 = 0, n = 0, count = 0, stored = 0;
-    long cell = 0, cellNext = 0;
-    unsigned nNext = 0;
-    if (active) { cellNext = cell_at(0); nNext = counts[cellNext]; }
-    bool more = active;
-    while (__any_sync(0xffffffffu, more)) {
-        int nq = 0;
-        // ---- phase 1: queue up to kNlQueue neighbours of this thread's point, in scan order
-        while (more && nq < kNlQueue) {
-            if (p1 >= n) {
-                if (cc >= prm.K) { more = false; break; }
-                cell = cellNext;
-                n = min((int)nNext, prm.cap);
-                p1 = 0;
-                if (++cc < prm.K) { cellNext = cell_at(cc); nNext = counts[cellNext]; }
-                continue;
-            }
-            const int j = slots[cell * prm.cap + p1];
-            ++p1;
-            if (j == pp) continue;
-            const float4 q = p32[j];
-            const float d0 = t32[0] - q.x, d1 = t32[1] - q.y, d2 = t32[2] - q.z;
-            int verdict = 0;  // 1 neighbour, -1 not, 0 decide in FP64
-            if (fabsf(d0) <= prm.wrapLim && fabsf(d1) <= prm.wrapLim && fabsf(d2) <= prm.wrapLim) {
+        int total = 0;
+#pragma unroll
+        for (int i = 0; i < kNlBins; ++i) {
+            first[i] -= total;
+            total += n[i];
+            end[i] = total;
+        }
+        const auto candidate = [&](int t) {
+            long at = first[0];
+#pragma unroll
+            for (int i = 1; i < kNlBins; ++i)
+                if (t >= end[i - 1]) at = first[i];
+            return slots[at + t];
+        };
+        // the neighbours among candidates [t0, t0 + 32), and which of them wrapped
+        const auto classify = [&](int t0, unsigned& yes, unsigned& wrapped) {
+            const int m = min(32, total - t0);
+            unsigned open = 0;
+            yes = wrapped = 0;
+#pragma unroll 4
+            for (int t = 0; t < m; ++t) {
+                const int j = candidate(t0 + t);
+                const float4 q = p32[j];
+                const float d0 = t32.x - q.x, d1 = t32.y - q.y, d2 = t32.z - q.z;
+                const bool inside = fabsf(d0) <= prm.wrapLim && fabsf(d1) <= prm.wrapLim && fabsf(d2) <= prm.wrapLim;
                 const float dd32 = d0 * d0 + d1 * d1 + d2 * d2;
-                verdict = dd32 > prm.thrHi ? -1 : (dd32 < prm.thrLo ? 1 : 0);
+                const bool no = (inside && dd32 > prm.thrHi) || j == pp, is = inside && dd32 < prm.thrLo && !no;
+                yes |= (unsigned)is << t;
+                open |= (unsigned)(!is && !no) << t;
             }
-            unsigned entry = (unsigned)j;
-            if (verdict == 0) {  // the reference's test, in FP64 (rare: the point is reloaded)
-                double t[3], qd[3], disp[3];
-                pts(pp, t[0], t[1], t[2]);
-                pts(j, qd[0], qd[1], qd[2]);
+            while (open) {  // the reference's test, in FP64 (rare: the points are reloaded)
+                const int t = __ffs(open) - 1;
+                open &= open - 1;
+                double a[3], b[3], disp[3];
+                pts(pp, a[0], a[1], a[2]);
+                pts(candidate(t0 + t), b[0], b[1], b[2]);
                 bool w = false;
                 for (int d = 0; d < 3; ++d) {
-                    disp[d] = t[d] - qd[d];
+                    disp[d] = a[d] - b[d];
                     w |= min_image(disp[d], prm.radius);
                 }
                 const double dd = disp[0] * disp[0] + disp[1] * disp[1] + disp[2] * disp[2];
-                verdict = (dd > prm.range2Hi || sqrt(dd) >= prm.range) ? -1 : 1;
-                if (w) entry |= kNlWrapped;
+                if (dd > prm.range2Hi || sqrt(dd) >= prm.range) continue;
+                yes |= 1u << t;
+                if (w) wrapped |= 1u << t;
             }
-            if (verdict < 0) continue;
-            if (count < prm.nmax) queue[nq++ * kB + threadIdx.x] = entry;
-            ++count;
+        };
+        // counts first (a thread past 32 candidates classifies the later ones twice), then the places
+        unsigned yes, wrapped;
+        classify(0, yes, wrapped);
+        int cnt = __popc(yes);
+        for (int t0 = 32; t0 < total; t0 += 32) {
+            unsigned y, w;
+            classify(t0, y, w);
+            cnt += __popc(y);
         }
-        // ---- phase 2: the warp's queued neighbours over its lanes, in FP64
-        int incl = nq;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
+        __syncwarp();
+        int incl = cnt;
+#pragma unroll
+        for (int o = 1; o < kNlLanes; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o, kNlLanes);
+            if (sub >= o) incl += v;
         }
-        const int excl = incl - nq, total = __shfl_sync(0xffffffffu, incl, 31);
-        for (int base = 0; base < total; base += 32) {
-            const int g = base + lane;
-            int owner = 0;  // the last lane whose queue starts at or before g
-            for (int step = 16; step > 0; step >>= 1) {
-                const int e = __shfl_sync(0xffffffffu, excl, owner + step);
-                if (e <= g) owner += step;
-            }
-            const int k = g - __shfl_sync(0xffffffffu, excl, owner);
-            const int row = __shfl_sync(0xffffffffu, stored, owner) + k;
-            if (g < total) {
-                const unsigned entry = queue[k * kB + wbase + owner];
-                const int j = (int)(entry & ~kNlWrapped);
-                const int po = blockIdx.x * kB + wbase + owner;
-                double a[3], b[3], disp[3];
-                pts(po, a[0], a[1], a[2]);
-                pts(j, b[0], b[1], b[2]);
-                for (int d = 0; d < 3; ++d) disp[d] = a[d] - b[d];
-                if (entry & kNlWrapped)
-                    for (int d = 0; d < 3; ++d) min_image(disp[d], prm.radius);
-                const double dd = disp[0] * disp[0] + disp[1] * disp[1] + disp[2] * disp[2];
-                const long at = (long)po * prm.nmax + row;
-                idx[at] = j;
-                vec[3 * at] = disp[0]; vec[3 * at + 1] = disp[1]; vec[3 * at + 2] = disp[2];
-                dist[at] = sqrt(dd);
+        int at = have + incl - cnt;
+        have += __shfl_sync(0xffffffffu, incl, kNlLanes - 1, kNlLanes);
+        for (int t0 = 0; t0 < total && at < prm.nmax; t0 += 32) {
+            if (t0) classify(t0, yes, wrapped);
+            for (; yes && at < prm.nmax; yes &= yes - 1, ++at) {
+                const int t = __ffs(yes) - 1;
+                idx[(long)pp * prm.nmax + at] = (int)((unsigned)candidate(t0 + t) | (wrapped >> t & 1 ? kNlWrapped : 0u));
             }
         }
-        stored += nq;
+        __syncwarp();
     }
-    // ---- the rest of each row is zero (resetNeighbors), written a row at a time by the warp
-    for (int o = 0; o < 32; ++o) {
-        const int s = __shfl_sync(0xffffffffu, stored, o);
-        const int po = blockIdx.x * kB + wbase + o;
-        if (po >= prm.np) break;
-        for (int k = s + lane; k < prm.nmax; k += 32) {
-            const long at = (long)po * prm.nmax + k;
-            idx[at] = 0;
-            vec[3 * at] = 0.; vec[3 * at + 1] = 0.; vec[3 * at + 2] = 0.;
-            dist[at] = 0.;
-        }
+    if (sub == 0) {
+        stored[row] = min(have, prm.nmax);
+        if (active) npp[pp] = (unsigned)have;
     }
-    if (active) npp[pp] = (unsigned)count;
-    count = __reduce_max_sync(0xffffffffu, count);  // one atomic per warp on the shared word
-    if (lane == 0 && count > 0) atomicMax(maxCount, count);
+    const int most = __reduce_max_sync(0xffffffffu, have);  // one atomic per warp on the shared word
+    if ((threadIdx.x & 31) == 0 && most > 0) atomicMax(maxCount, most);
+    __syncthreads();
+    // ---- phase 2, with the rest of each row zero (resetNeighbors)
+    const long entries = (long)min(kNlPoints, prm.np - p0) * prm.nmax;
+    for (long e = threadIdx.x; e < entries; e += kB) {
+        const int o = (int)(e / prm.nmax), k = (int)(e - (long)o * prm.nmax);
+        const long at = (long)p0 * prm.nmax + e;
+        int j = 0;
+        double disp[3] = {0., 0., 0.}, len = 0.;
+        if (k < stored[o]) {
+            j = idx[at];
+            const bool w = j < 0;
+            j &= (int)~kNlWrapped;
+            double b[3];
+            pts(j, b[0], b[1], b[2]);
+            for (int d = 0; d < 3; ++d) disp[d] = own[o][d] - b[d];
+            if (w)
+                for (int d = 0; d < 3; ++d) min_image(disp[d], prm.radius);
+            len = sqrt(disp[0] * disp[0] + disp[1] * disp[1] + disp[2] * disp[2]);
+        }
+        idx[at] = j;
+        vec[3 * at] = disp[0]; vec[3 * at + 1] = disp[1]; vec[3 * at + 2] = disp[2];
+        dist[at] = len;
+    }
 }
 }  // namespace
 
@@ -315,7 +360,6 @@ struct svm_neighbor_list {
     int* idx = nullptr;                 // [nPoints * nmax]
     double* vec = nullptr;              // [nPoints * nmax * 3]
     double* dist = nullptr;             // [nPoints * nmax]
-    int* maxCount = nullptr;
     float4* p32 = nullptr;              // [nPoints] FP32 copies for the candidate scan
 };
 
@@ -341,57 +385,34 @@ void nl_thresholds(NlParams& p) {
     p.thrLo = lo > 0 ? down(lo * lo) : -1.f;
 }
 
+// After the cell list's own launches: the points are binned and their FP32 copies written.
 template <typename P>
 int nl_compute(svm_neighbor_list* nl, P pts, int np) {
-    if (np != nl->nPoints) return SVM_ERR_ARG;
     svm_cell_list* cl = nl->cl;
-    const size_t nb = (np + kB - 1) / kB;
-    k_nl_pack<<<nb, kB, 0, cl->stream>>>(pts, np, nl->p32);
+    const int* sc = cl->hostScalars;
     for (int pass = 0; pass < 64; ++pass) {   // a third pass at most: slots widened, then nmax grown
         NlParams prm;
         prm.np = np; prm.cap = cl->cap; prm.nside = cl->nside; prm.K = nl->K; prm.nmax = nl->nmax;
-        prm.h = cl->h; prm.radius = cl->radius; prm.range = nl->range;
+        prm.radius = cl->radius; prm.range = nl->range;
         prm.range2Hi = nl->range * nl->range * (1.0 + 0x1p-48);
         nl_thresholds(prm);
-        cudaMemsetAsync(nl->maxCount, 0, sizeof(int), cl->stream);
-        k_nl<<<nb, kB, 0, cl->stream>>>(pts, nl->p32, prm, cl->counts, cl->slots, nl->mask, nl->npp, nl->idx, nl->vec,
-                                        nl->dist, nl->maxCount);
-        if (check_launch()) return SVM_ERR_CUDA;
-        int mc = 0, sc[4];
-        if (cudaMemcpyAsync(&mc, nl->maxCount, sizeof(int), cudaMemcpyDeviceToHost, cl->stream) != cudaSuccess ||
-            cudaMemcpyAsync(sc, cl->scalars, sizeof(sc), cudaMemcpyDeviceToHost, cl->stream) != cudaSuccess ||
-            cudaStreamSynchronize(cl->stream) != cudaSuccess)
-            return SVM_ERR_CUDA;
+        k_nl<<<(np + kNlPoints - 1) / kNlPoints, kB, 0, cl->stream>>>(pts, nl->p32, prm, cl->counts, cl->slots, cl->binOf,
+                                                                      nl->mask, nl->npp, nl->idx, nl->vec, nl->dist,
+                                                                      cl->scalars + 4);
+        if (check_launch() || read_scalars(cl)) return SVM_ERR_CUDA;
         if (sc[3]) return SVM_ERR_DEVICE;  // a point lay outside the grid (or was not finite)
         if (sc[2]) {                       // a bin overflowed its slots: widen them, bin again
-            if (cl_grow(cl, sc[0]) || compute(cl, pts, np)) return SVM_ERR_CUDA;
+            if (cl_grow(cl, sc[0]) || compute(cl, pts, np, nl->p32)) return SVM_ERR_CUDA;
             continue;
         }
-        if (mc <= nl->nmax) return SVM_OK;
-        nl->nmax = mc;  // grow-only, then recompute
+        const int longest = sc[4];         // (of the same points at any nmax: the next pass finds it again)
+        if (longest <= nl->nmax) return SVM_OK;
+        nl->nmax = longest;  // grow-only, then recompute
         if (nl_alloc(nl)) return SVM_ERR_CUDA;
     }
     return SVM_ERR_DEVICE;
 }
 }  // namespace
-
-namespace svm {
-int cell_list_bin(svm_cell_list* cl, const double* pts, int n, CellGrid* view) {
-    if (!cl || !pts || !view || n != cl->nPoints) return SVM_ERR_ARG;
-    for (int pass = 0; pass < 8; ++pass) {
-        if (compute(cl, AosPoints{pts}, n)) return SVM_ERR_CUDA;
-        int sc[4];
-        if (cudaMemcpyAsync(sc, cl->scalars, sizeof(sc), cudaMemcpyDeviceToHost, cl->stream) != cudaSuccess ||
-            cudaStreamSynchronize(cl->stream) != cudaSuccess)
-            return SVM_ERR_CUDA;
-        if (sc[3]) return SVM_ERR_DEVICE;
-        if (sc[2]) { if (cl_grow(cl, sc[0])) return SVM_ERR_CUDA; continue; }
-        *view = CellGrid{cl->counts, cl->slots, cl->cap, cl->nside, cl->h, cl->radius};
-        return SVM_OK;
-    }
-    return SVM_ERR_DEVICE;
-}
-}  // namespace svm
 
 extern "C" {
 
@@ -422,7 +443,6 @@ int svm_neighbor_list_create(double range, double radius, int subGridReduction, 
     nl->K = (int)mask.size() / 3;
     bool ok = cudaMalloc(&nl->mask, sizeof(int) * mask.size()) == cudaSuccess &&
               cudaMalloc(&nl->npp, sizeof(unsigned) * nPoints) == cudaSuccess &&
-              cudaMalloc(&nl->maxCount, sizeof(int)) == cudaSuccess &&
               cudaMalloc(&nl->p32, sizeof(float4) * nPoints) == cudaSuccess && nl_alloc(nl) == SVM_OK;
     if (ok) ok = cudaMemcpy(nl->mask, mask.data(), sizeof(int) * mask.size(), cudaMemcpyHostToDevice) == cudaSuccess;
     if (!ok) { svm_neighbor_list_destroy(nl); return SVM_ERR_CUDA; }
@@ -433,7 +453,7 @@ int svm_neighbor_list_create(double range, double radius, int subGridReduction, 
 int svm_neighbor_list_destroy(svm_neighbor_list* nl) {
     if (!nl) return SVM_ERR_ARG;
     if (nl->cl) svm_cell_list_destroy(nl->cl);
-    void* ptrs[] = {nl->mask, nl->npp, nl->idx, nl->vec, nl->dist, nl->maxCount, nl->p32};
+    void* ptrs[] = {nl->mask, nl->npp, nl->idx, nl->vec, nl->dist, nl->p32};
     for (void* p : ptrs) if (p) cudaFree(p);
     delete nl;
     return SVM_OK;
@@ -441,13 +461,13 @@ int svm_neighbor_list_destroy(svm_neighbor_list* nl) {
 
 int svm_neighbor_list_compute(svm_neighbor_list* nl, const double* pts, int n) {
     if (!nl || !pts) return SVM_ERR_ARG;
-    int rc = svm_cell_list_compute(nl->cl, pts, n);
+    int rc = compute(nl->cl, AosPoints{pts}, n, nl->p32);
     return rc ? rc : nl_compute(nl, AosPoints{pts}, n);
 }
 
 int svm_neighbor_list_compute_model(svm_neighbor_list* nl, svm_model* m) {
     if (!nl || !m) return SVM_ERR_ARG;
-    int rc = svm_cell_list_compute_model(nl->cl, m);
+    int rc = compute_model(nl->cl, m, nl->p32);
     if (rc) return rc;
     if (m->precision == SVM_PRECISION_MIXED) return nl_compute(nl, ModelPoints32{m->pos32[m->cur]}, m->nVertices);
     return nl_compute(nl, ModelPoints{m->pos[m->cur]}, m->nVertices);
@@ -487,11 +507,12 @@ int svm_cell_list_create(double a, double radius, int nPoints, int cap, void* st
               cudaMalloc(&cl->tmp, sizeof(int) * cl->total * cap) == cudaSuccess &&
               cudaMalloc(&cl->slots, sizeof(int) * cl->total * cap) == cudaSuccess &&
               cudaMalloc(&cl->binOf, sizeof(int) * nPoints) == cudaSuccess &&
-              cudaMalloc(&cl->scalars, sizeof(int) * 4) == cudaSuccess;
+              cudaMalloc(&cl->scalars, sizeof(int) * kClScalars) == cudaSuccess &&
+              cudaMallocHost(&cl->hostScalars, sizeof(int) * kClScalars) == cudaSuccess;
     if (!ok) { svm_cell_list_destroy(cl); return SVM_ERR_CUDA; }
     cudaMemsetAsync(cl->counts, 0, sizeof(unsigned) * cl->total, cl->stream);
     cudaMemsetAsync(cl->binOf, 0xff, sizeof(int) * nPoints, cl->stream);
-    const int init[4] = {0, 2, 0, 0};  // Nmax starts at 2 (hyperrectangularCellList.cpp:17,47)
+    const int init[kClScalars] = {0, 2};  // Nmax starts at 2 (hyperrectangularCellList.cpp:17,47)
     cudaMemcpyAsync(cl->scalars, init, sizeof(init), cudaMemcpyHostToDevice, cl->stream);
     if (cudaStreamSynchronize(cl->stream) != cudaSuccess) { svm_cell_list_destroy(cl); return SVM_ERR_CUDA; }
     *out = cl;
@@ -503,23 +524,14 @@ int svm_cell_list_destroy(svm_cell_list* cl) {
     if (cl->stream) cudaStreamSynchronize(cl->stream);
     void* ptrs[] = {cl->counts, cl->tmp, cl->slots, cl->binOf, cl->scalars};
     for (void* p : ptrs) if (p) cudaFree(p);
+    if (cl->hostScalars) cudaFreeHost(cl->hostScalars);
     if (cl->ownStream && cl->stream) cudaStreamDestroy(cl->stream);
     delete cl;
     return SVM_OK;
 }
 
 int svm_cell_list_compute_model(svm_cell_list* cl, svm_model* m) {
-    if (!cl || !m) return SVM_ERR_ARG;
-    if (cl->stream != m->stream) {
-        // order after the model's pending work
-        cudaEvent_t e;
-        cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
-        cudaEventRecord(e, m->stream);
-        cudaStreamWaitEvent(cl->stream, e, 0);
-        cudaEventDestroy(e);
-    }
-    if (m->precision == SVM_PRECISION_MIXED) return compute(cl, ModelPoints32{m->pos32[m->cur]}, m->nVertices);
-    return compute(cl, ModelPoints{m->pos[m->cur]}, m->nVertices);
+    return !cl || !m ? SVM_ERR_ARG : compute_model(cl, m);
 }
 
 int svm_cell_list_compute(svm_cell_list* cl, const double* pts, int n) {

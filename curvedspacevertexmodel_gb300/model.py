@@ -827,12 +827,11 @@ class neighborList:
             self._ensure(n)
             call("svm_neighbor_list_compute", self._h, C.c_void_p(points.data_ptr()), n)
         nm = C.c_int()
+        call("svm_neighbor_list_get", self._h, C.byref(nm), None, None, None, None, 0)
         if not fetch:
-            call("svm_neighbor_list_get", self._h, C.byref(nm), None, None, None, None, 0)
             self.Nmax = nm.value
             return
         npp = np.empty(self._n, dtype=np.uint32)
-        call("svm_neighbor_list_get", self._h, C.byref(nm), npp, None, None, None, 0)
         e = self._n * nm.value
         idx = np.empty(e, dtype=np.int32)
         vec = np.empty(3 * e)
