@@ -7,7 +7,7 @@
 //                  disp = dt v + dt^2/2 F, v += dt/2 F / m, move onto the sphere (in place), and
 //                  the moved vertex's norm for the corner pass
 //   corners + T1   unless motion is restricted: k_edges (edge terms and the T1 length test),
-//                  k_corner or k_corner_s, then the T1 pass (k_t1_parallel, k_t1_apply)
+//                  the corner kernels, then the T1 pass (k_t1_parallel)
 //   geometry       k_cells, k_fallback_fan (the corners too when motion is restricted)
 //   k_fire_force   per vertex: F, v += dt/2 F / m, block partials of F.v, F.F, v.v, max |F|^2;
 //                  the last block reduces them in a fixed order and runs the FIRE control

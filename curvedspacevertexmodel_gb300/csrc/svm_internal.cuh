@@ -496,15 +496,15 @@ constexpr int kT1CtlInts = sizeof(T1Ctl) / sizeof(int);
 
 struct T1Scratch {
     unsigned* bits = nullptr;      // one bit per (vertex, slot) position, 3*Nv bits
-    unsigned* summary = nullptr;   // one bit per word of `bits`: set only for k_t1_apply's replay
-    int* count = nullptr;          // positions a rolled-back segment left to k_t1_apply
+    unsigned* summary = nullptr;   // one bit per word of `bits`: set only for a replay
+    int* count = nullptr;          // positions that rolled-back segments left to the replay
     int* segCount = nullptr;       // per segment (the sphere, or each replica): positions the test flagged
     const int* segOff = nullptr;   // first vertex of each segment [segments + 1] (null: one sphere)
     int listPad = 0;               // list slack per segment
     int* flipLog = nullptr;        // (pass, position, v1, v2) per flip, capacity flipLogCap
     int* flipCount = nullptr;
     int* pass = nullptr;           // T1 passes so far (orders the flip log across passes)
-    int* touched = nullptr;        // cells whose rings changed (batches, and k_t1_apply's replay)
+    int* touched = nullptr;        // cells whose rings changed (batches, and replays)
     int nWords = 0, nSummary = 0, flipLogCap = 0, touchedCap = 0;
     // parallel pass (deterministic reservations), capacity `cap` pending positions
     int* listA = nullptr;          // pending positions of this round (the first: as the test flags them)
@@ -518,7 +518,7 @@ struct T1Scratch {
     int* comList = nullptr;        // footprints of executed positions (to clear comV/comC)
     UndoEntry* undo = nullptr;     // one entry per committed flip
     int* undoRings = nullptr;      // old rings of the four cells, 4*Wc ints per entry
-    int* ctr = nullptr;            // [0] pending, [1] next, [2] undo entries, [3] rollback, [4] executed
+    int* ctr = nullptr;            // [5] touched cells, [6] most rounds, [7] blocks finished (batches); then the T1Ctl
     int* stats = nullptr;          // svm_model_t1_stats counters
     unsigned long long* clocks = nullptr;  // svm_model_t1_clocks: SM cycles per phase (null: off)
     T1Ctl* ctl = nullptr;          // counters of a cooperative pass (inside the ctr allocation)
@@ -537,6 +537,12 @@ __device__ __forceinline__ void t1_footprint(int v1, int v2, const int4& n1, con
                                              int* f) {
     f[0] = v1; f[1] = v2; f[2] = n1.x; f[3] = n1.y; f[4] = n1.z; f[5] = n2.x; f[6] = n2.y; f[7] = n2.z;
     f[8] = c1.x; f[9] = c1.y; f[10] = c1.z; f[11] = c2.x; f[12] = c2.y; f[13] = c2.z;
+}
+// Before a T1 pass, by the test kernel (whose own work touches none of it): the touched cells, the most
+// rounds, the ticket, and the T1Ctl of a cooperative pass.
+__device__ __forceinline__ void t1_clear(const T1Scratch& t1) {
+    if (blockIdx.x != 0 || threadIdx.x >= 3 + kT1CtlInts) return;
+    t1.ctr[5 + threadIdx.x] = 0;
 }
 // The T1 test's record of a short edge (position p = 3 v + slot, neighbour u, replica seg): its flag, its
 // place in the pass's first list, its footprint, and its reservation of it -- so that the pass starts

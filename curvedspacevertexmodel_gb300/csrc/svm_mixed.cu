@@ -141,6 +141,7 @@ __global__ void k32_corners(const float4* __restrict__ pos, const int4* __restri
                             double2* __restrict__ corner, int Wc, int nV, const double* __restrict__ repR,
                             int t1test, float t1Threshold, T1Scratch t1) {
     step_begin();
+    if (t1test) t1_clear(t1);
     extern __shared__ double cornerSh[];
     const int bs = blockDim.x, t = threadIdx.x;
     double *cx = cornerSh, *cy = cx + bs, *cz = cy + bs, *nc = cz + bs, *val = nc + bs;

@@ -4,10 +4,11 @@
 // Kernel sequence of one Brownian timestep (invariant: `corner` and `vsph` describe the current
 // positions and topology when a step starts):
 //   k_cells         per cell: centroid, area (spherical excess), perimeter, total-area check
-//   k_fallback      per cell: triangle-fan areas, only when the total area is off by > 1e-6
+//   k_fallback_fan  per cell: triangle-fan areas, only when the total area is off by > 1e-6
 //   k_force_bd      per vertex: force, Brownian displacement, move onto the sphere (new buffer)
-//   k_corners       per vertex: spherical coordinates, per-corner arc and angle, T1 edge test
-//   k_t1_apply      one block: the CPU's sequential T1 order over the flagged edges; patches
+//   k_corners_few, or k_vnorm, k_edges and k_corner
+//                   per vertex: spherical coordinates, per-corner arc and angle, T1 edge test
+//   k_t1_parallel   the flagged edges' flips with the result of the CPU's sequential order; patches
 //                   corners of every cell whose ring changed
 // None of them synchronises with the host, so a run of steps is captured as one CUDA graph.
 #include <cstdio>
@@ -26,7 +27,6 @@ namespace svm {
 
 constexpr int kSplitCellsBelow = 20000;   // k_cells: two threads a cell
 constexpr int kBlock = 256;
-constexpr int kApplyThreads = 256;
 constexpr int kExtractCap = 1024;  // positions extracted per bitmap chunk (32 words)
 constexpr int kHeapCap = 512;
 
@@ -141,6 +141,7 @@ __global__ void k_edges(const double4_32a* __restrict__ pos, const double* __res
                         double4_32a* __restrict__ edgeC, double* __restrict__ edgeArc, int nV, double R, int t1test,
                         double t1Threshold, T1Scratch t1) {
     step_begin();
+    if (t1test) t1_clear(t1);
     const int v = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
     const bool live = v < nV;
     int4 nb = make_int4(-1, -1, -1, -1);
@@ -208,6 +209,7 @@ __global__ void __launch_bounds__(4 * kFewVerts) k_corners_few(
     const int4* __restrict__ vnbr, double2* __restrict__ corner, int Wc, int nV, double R, int t1test, double t1Threshold,
     T1Scratch t1) {
     step_begin();
+    if (t1test) t1_clear(t1);
     __shared__ double cx[3 * kFewVerts], cy[3 * kFewVerts], cz[3 * kFewVerts], nc[3 * kFewVerts];
     __shared__ double ux[3 * kFewVerts], uy[3 * kFewVerts], uz[3 * kFewVerts], arcs[3 * kFewVerts];
     __shared__ double val[4 * kFewVerts];
@@ -574,6 +576,7 @@ __global__ void k_t1_test(const double4_32a* __restrict__ pos, const float4* __r
                           const double* __restrict__ repR, const int4* __restrict__ vnbr,
                           const int4* __restrict__ vcell, int nV, double R, double t1Threshold, double cosLo, double cosHi, double s2Lo, double s2Hi, T1Scratch t1) {
     step_begin();
+    t1_clear(t1);
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nV) return;
     const int4 nb = vnbr[v];
@@ -1103,7 +1106,9 @@ __device__ bool t1_flip_warp(const ApplyArgs& A, int f, const WarpRings& W, int4
 // The cells are cellOf(i), i < count (-1: none), shared out round-robin over `blocks` blocks (cell i to
 // block i mod blocks, 32 of a block's at a time), and each block packs its cells' ring entries onto
 // consecutive threads: the few hundred cells of a pass then spread over many SMs, with every lane of a
-// busy warp on a real entry.  Every thread of the block calls it.
+// busy warp on a real entry.  The arc with the bookkeeping, the angle and the spherical coordinates of an
+// entry go to different warps: each is a chain of FP64 operations, and one after another they were two thirds of
+// the patch (FP64 form, 100k cells, 75 flips: 16.6 -> 10.9 us).  Every thread of the block calls it.
 template <class CellOf>
 __device__ __forceinline__ void patch_cells(const ApplyArgs& A, int count, int block, int blocks, bool hostOut, CellOf cellOf) {
     __shared__ int patchCell[32], patchOff[33];
@@ -1122,29 +1127,37 @@ __device__ __forceinline__ void patch_cells(const ApplyArgs& A, int count, int b
             if (threadIdx.x == 31) patchOff[32] = incl;
         }
         __syncthreads();
-        for (int e = threadIdx.x; e < patchOff[32]; e += blockDim.x) {
+        const int entries = patchOff[32], stride = (entries + 31) & ~31, roles = A.pos32 ? 2 : 3;
+        for (int x = threadIdx.x; x < roles * stride; x += blockDim.x) {
+            const int role = x >= 2 * stride ? 2 : (x >= stride ? 1 : 0), e = x - role * stride;
+            if (e >= entries) continue;
             int j = 0;
             while (patchOff[j + 1] <= e) ++j;
             const int cell = patchCell[j], k = e - patchOff[j];
             const int n = A.ringCount[cell];
             const int* rg = A.ring + (long)cell * A.Wc;
             const int u = rg[k];
-            const int last = rg[k == 0 ? n - 1 : k - 1], next = rg[k + 1 == n ? 0 : k + 1];
+            if (role == 2) {
+                A.vsph[u] = sph_coords<true>(apos(A, u));
+                continue;
+            }
+            const int last = rg[k == 0 ? n - 1 : k - 1];
+            const D3 pl = apos(A, last), p = apos(A, u);
+            double* cr = reinterpret_cast<double*>(A.corner + (long)cell * A.Wc + k);
+            if (role == 1) {
+                const D3 px = apos(A, rg[k + 1 == n ? 0 : k + 1]);
+                cr[1] = A.pos32 ? included_angle_clamped<true>(pl, p, px) : included_angle<true>(pl, p, px);
+                continue;
+            }
+            const int next = rg[k + 1 == n ? 0 : k + 1];
             for (int s = 0; s < 3; ++s)
                 if (compRef(A.vcell, u, s) == cell) {
                     compRef(A.vrpos, u, s) = k;
                     compRef(A.vlast, u, s) = last;
                     compRef(A.vnext, u, s) = next;
                 }
-            const D3 pl = apos(A, last), p = apos(A, u), px = apos(A, next);
             if (hostOut) { A.hostOut[3L * u] = p.x; A.hostOut[3L * u + 1] = p.y; A.hostOut[3L * u + 2] = p.z; }
-            if (A.pos32) {
-                A.corner[(long)cell * A.Wc + k] =
-                    make_double2((double)arc32(A.pos32[last], A.pos32[u], (float)aR(A, u)), included_angle_clamped<true>(pl, p, px));
-            } else {
-                A.corner[(long)cell * A.Wc + k] = make_double2(geodesic<true>(pl, p, A.R), included_angle<true>(pl, p, px));
-                A.vsph[u] = sph_coords<true>(p);
-            }
+            cr[0] = A.pos32 ? (double)arc32(A.pos32[last], A.pos32[u], (float)aR(A, u)) : geodesic<true>(pl, p, A.R);
         }
         __syncthreads();
     }
@@ -1154,7 +1167,7 @@ __device__ __forceinline__ void publish_ring_max(const ApplyArgs& A) {
     *(volatile int*)A.ringMaxOut = *(volatile int*)A.ringMax;
     __threadfence_system();
 }
-// The cells of the touched list (batches, and k_t1_apply's replay of a sphere's pass).  A host-buffer
+// The cells of the touched list (batches, and the replay of a sphere's pass).  A host-buffer
 // step's output: the force kernel wrote the moved positions; the flips moved vertices of the touched
 // cells, whose ring entries rewrite them.  A list that may have lost entries (full) rewrites every
 // vertex instead.  (Appends past the list's capacity roll the pass back; a pass cut short by an
@@ -1168,7 +1181,7 @@ __device__ __forceinline__ void patch_touched(const ApplyArgs& A, const T1Scratc
         }
     patch_cells(A, min(ntRaw, t1.touchedCap), block, blocks, A.hostOut && !hostAll, [&](int i) { return t1.touched[i]; });
 }
-// Batches: the patch over all replicas' touched cells, after k_t1_apply.
+// Batches: the patch over all replicas' touched cells, after k_t1_parallel.
 __global__ void k_t1_patch(ApplyArgs A, T1Scratch t1) {
     step_begin();
     if (blockIdx.x == 0 && threadIdx.x == 0) publish_ring_max(A);
@@ -1218,36 +1231,18 @@ __device__ __forceinline__ bool t1_candidate(const ApplyArgs& A, int q) {
 // Applies the flagged T1 flips in the order of the CPU loop (ascending vertex1, then slot),
 // re-testing each edge against the current state when it is reached and re-testing, after every
 // flip, the edges of the six vertices whose slots or positions the flip changed.  Flags ahead of
-// the extracted window live in the bitmap; flags inside it in a small heap.  Afterwards every
-// cell whose ring changed gets its ring bookkeeping (vrpos/vlast/vnext) and corners rebuilt (here for
-// one sphere, by k_t1_patch for a batch).  For one sphere it is the pass's last kernel and leaves the
-// counters of the next pass cleared.
-__device__ void t1_reset(const T1Scratch& t1) {
-    int* c = t1.ctr + 5;   // touched cells, round maximum, ticket, and the pass's T1Ctl
-    for (int k = 0; k < 3 + kT1CtlInts; ++k) c[k] = 0;
-}
-__global__ void __launch_bounds__(kApplyThreads) k_t1_apply(ApplyArgs A, T1Scratch t1, bool sphere) {
-    step_begin();
+// the extracted window live in the bitmap; flags inside it in a small heap.  The cells whose rings
+// changed are appended to the touched list, whose length is returned.  Run by one block of the parallel pass
+// (sphere: block 0; batch: the last block to finish) when a segment's flips were undone; every thread of
+// the block calls it.
+__device__ __noinline__ int t1_replay(const ApplyArgs& A, const T1Scratch& t1, int touched) {
     __shared__ int buf[kExtractCap];
     __shared__ int heap[kHeapCap];
     __shared__ int nbuf, head, nheap, extractWord, nTouched;
     __shared__ int nSummaryHit;
     const int tid = threadIdx.x;
-    const int total = *t1.count;
-    if (total == 0) {
-        if (tid == 0) {
-            *t1.pass += 1;
-            t1.stats[0] += 1;
-            if (A.bumpStep) *A.stepCounter += 1ull;
-            if (sphere) {
-                publish_ring_max(A);
-                t1_reset(t1);
-            }
-        }
-        return;
-    }
     // (a batch's touched cells are appended after those of the segments that succeeded)
-    if (tid == 0) { nbuf = 0; head = 0; nheap = 0; extractWord = 0; nTouched = t1.ctr[5]; t1.stats[6] = *t1.flipCount; }
+    if (tid == 0) { nbuf = 0; head = 0; nheap = 0; extractWord = 0; nTouched = touched; t1.stats[6] = *t1.flipCount; }
     __syncthreads();
     int lastProcessed = -1;
     while (true) {
@@ -1349,23 +1344,19 @@ __global__ void __launch_bounds__(kApplyThreads) k_t1_apply(ApplyArgs A, T1Scrat
         }
         __syncthreads();
     }
-    // ring bookkeeping and corners of the touched cells
-    __syncthreads();
-    if (sphere) patch_touched(A, t1, nTouched, 0, 1);
     if (tid == 0) {
-        t1.ctr[5] = nTouched;
-        if (sphere) {
-            publish_ring_max(A);
-            t1_reset(t1);
-        }
         *t1.count = 0;
-        *t1.pass += 1;
-        t1.stats[0] += 1;
         t1.stats[3] += *t1.flipCount - t1.stats[6];
-        if (A.bumpStep) *A.stepCounter += 1ull;
     }
+    __syncthreads();
+    return nTouched;
 }
-
+// The end of a pass, by one thread.
+__device__ __forceinline__ void t1_pass_done(const ApplyArgs& A, const T1Scratch& t1) {
+    *t1.pass += 1;
+    t1.stats[0] += 1;
+    if (A.bumpStep) *A.stepCounter += 1ull;
+}
 
 // ---- parallel T1 pass -------------------------------------------------------------------------
 // Footprint of the edge at position p.
@@ -1379,8 +1370,12 @@ __device__ __forceinline__ int pick_aff(int a, int v1, int v2, const int4& vs) {
     return a == 0 ? v1 : a == 1 ? v2 : a == 2 ? vs.x : a == 3 ? vs.y : a == 4 ? vs.z : vs.w;
 }
 
-constexpr int kParThreads = 512;        // one segment: the whole sphere
-constexpr int kParThreadsBatch = 128;   // one segment per replica (4 resident blocks per SM at 128 registers)
+// One segment a block, the whole sphere or a replica of a batch.  A batch's pass lasts as long as its hottest
+// replica's, whose flips go round the block's warps: 512 replicas at 100 to 5000 cells, 665 flips a pass,
+// 112 us with 128 threads (every block resident at once), 90 with 256, 81 with 512 -- but with three
+// batches on three streams, which fill the chip between them, four steps take 2373, 2385 and 2430 us (one
+// batch by itself 2940, 2835, 2783).
+constexpr int kParThreads = 512, kParThreadsBatch = 256;
 constexpr int kCoopThreads = 256;       // per block of a cooperative single-sphere pass
 
 // Barrier of all blocks of a cooperative launch (co-resident by construction): the last block
@@ -1422,26 +1417,28 @@ __device__ bool grid_barrier(T1Ctl* ctl, int spinLimit) {
 // running at once.  A position created by a re-test that overlaps a higher position which has already
 // run would need the CPU order broken; that is detected through the per-vertex/per-cell record of the
 // highest position that ran, and then every flip of the pass is undone and the bitmap restored for
-// k_t1_apply, which then applies the flips one by one (it finds nothing to do otherwise).
+// t1_replay, which applies the flips one by one.
 //
 // kCoop = false: one block per segment of the position space: the whole sphere, or one replica
 // of a batch (whose flagged edges share no vertex or cell with another replica's, and whose
 // positions are a contiguous range).  A block's lists, footprints, commit list and undo log are
 // its own slices of the scratch arrays; a batch's touched-cell list and the flip log are shared (atomic
 // appends).  A block whose pass is not the sequential order undoes its own flips, marks their log
-// entries invalid (pass -1) and restores its segment's flags, which k_t1_apply then replays.  The last
-// block to finish (ticket) folds the round count into the statistics.
+// entries invalid (pass -1) and restores its segment's flags.  The last block to finish (ticket) replays
+// what was undone, folds the round count into the statistics and ends the pass.
 // kCoop = true: one segment (the whole sphere) over all blocks of a cooperative launch, so that the
 // flips spread over many SMs instead of one: position i of a round runs on block i mod gridDim.x, the
 // phases are separated by grid barriers instead of block barriers, the counters live in global memory
-// (t1.ctl, cleared by the last pass's k_t1_apply), and block 0 alone finishes a rollback and the
-// statistics.  Same decisions, same results.
+// (t1.ctl, cleared by the T1 test: t1_clear), and block 0 alone finishes a rollback, its replay and the
+// statistics.  Same decisions, same results.  (The replay and the end of the pass were a kernel of their
+// own, which found nothing to do but for a rare rollback: 5 us by itself.)
 // A sphere's pass also rebuilds the corners of the cells its flips changed (patch_cells over the undo
 // entries): a batch leaves them to k_t1_patch, which spreads its hottest replicas' cells over all SMs.
 //
 // What bounds it is latency: a few tens of flips, each a chain of loads and the pair's FP64 rotation.  A
-// flip runs on a warp (t1_flip_warp).  100k cells, 1.3 rounds and 75 flips a pass on average: see the
-// figures at launch_t1_apply.
+// flip runs on a warp (t1_flip_warp), its atomics on their way while the tests run.  The pass, with 1.3 rounds
+// and 75 flips on average, 100k cells: 45 us, FP32 positions 42 (57 and 48 before the replay's kernel, the
+// patch's chain and the atomics' waits were taken out); 1M cells, 440 flips: 55 us (62).
 template <bool kCoop>
 __global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_parallel(ApplyArgs A, T1Scratch t1, int undoPer) {
     step_begin();
@@ -1464,13 +1461,22 @@ __global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_paral
     const int capB = (qHi - qLo) / 2 + t1.listPad;
     // The count is read by every block before the first grid barrier, so before block 0 can change it.
     const int nOrig = min(*(volatile int*)(t1.segCount + seg), capB);
+    auto sphere_done = [&]() {
+        if (tid != 0) return;
+        publish_ring_max(A);
+        t1_pass_done(A, t1);
+    };
     // one segment and nothing flagged: nothing to do.  (With several segments every block runs:
     // the last one to finish does the pass's cleanup.)
-    if (sphere && nOrig == 0) return;
+    if (sphere && nOrig == 0) {
+        if (leader) sphere_done();
+        return;
+    }
     auto group_sync = [&]() -> bool {
         if (!kCoop) { __syncthreads(); return true; }
         if (grid_barrier(ctl, A.barrierSpins)) return true;
         if (tid == 0) atomicOr(A.status, SVM_DEV_T1_TIMEOUT);
+        if (leader) sphere_done();
         return false;
     };
     int* cur = t1.listA + base;
@@ -1548,12 +1554,13 @@ __global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_paral
                 }
                 continue;
             }
-            // lanes 0 and 1 take the position's places in the commit and undo lists together
-            const bool isShort = v1 < v2 && t1_short(A, P1, P2);  // t1_candidate(A, p), on every lane alike
+            // lanes 0 and 1 take the position's places in the commit and undo lists together, while the test
+            // is evaluated (an undo place that stays empty is marked so)
             int got = 0;
-            if (lane == 0) got = atomicAdd(&ctl->exec, 1);
-            if (lane == 1 && isShort) got = atomicAdd(&ctl->undo, 1);
+            if (lane < 2) got = atomicAdd(lane == 0 ? &ctl->exec : &ctl->undo, 1);
+            const bool isShort = v1 < v2 && t1_short(A, P1, P2);  // t1_candidate(A, p), on every lane alike
             const int ci = __shfl_sync(kFull, got, 0), ui = __shfl_sync(kFull, got, 1);
+            if (lane == 0 && !isShort && ui < undoPer) undoB[ui].v1 = -1;
             if (ci >= capB) {
                 if (lane == 0) {
                     if (isShort && ui < undoPer) undoB[ui].v1 = -1;
@@ -1575,14 +1582,10 @@ __global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_paral
                 if (lane == 0) u->v1 = -1;  // nothing was written
                 continue;
             }
+            int fc = 0;   // this flip's place in the log, on its way while the re-tests run
             if (lane == 0) {
+                fc = atomicAdd(t1.flipCount, 1);
                 atomicAdd(&ctl->flips, 1);
-                const int fc = atomicAdd(t1.flipCount, 1);
-                u->logIdx = fc;
-                if (fc < t1.flipLogCap) {
-                    int* e = t1.flipLog + 4 * fc;
-                    e[0] = *t1.pass; e[1] = p; e[2] = v1; e[3] = v2;
-                }
             }
             if (lane == 1 && !sphere) {
                 const int tc = atomicAdd(t1.ctr + 5, 4);
@@ -1610,6 +1613,13 @@ __global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_paral
                     const int ni = atomicAdd(&ctl->next[par], 1);
                     if (ni < capB) nxt[ni] = r;
                     else atomicExch(&ctl->rollback, 1);
+                }
+            }
+            if (lane == 0) {
+                u->logIdx = fc;
+                if (fc < t1.flipLogCap) {
+                    int* e = t1.flipLog + 4 * fc;
+                    e[0] = *t1.pass; e[1] = p; e[2] = v1; e[3] = v2;
                 }
             }
             __syncwarp();
@@ -1720,7 +1730,7 @@ __global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_paral
         }
         __syncthreads();
         // the segment's flags back to the ones the test set: clear, then set the originals, with the
-        // summary bits that k_t1_apply finds them by
+        // summary bits that t1_replay finds them by
         const int wLo = qLo >> 5, wHi = (qHi + 31) >> 5;  // words [wLo, wHi)
         for (int w = wLo + tid; w < wHi; w += blockDim.x) {
             unsigned keep = 0u;  // bits of other segments in a shared boundary word
@@ -1736,12 +1746,14 @@ __global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_paral
         }
     }
     __syncthreads();
+    __shared__ int last;
     if (tid == 0) {
         t1.segCount[seg] = 0;   // (read by every block before the pass's first barrier)
         if (nOrig > 0) {
             atomicAdd(t1.stats + 1, nOrig);
             atomicAdd(t1.stats + 2, ne);
-            atomicMax(t1.ctr + 6, rounds);
+            if (sphere) t1.stats[4] += rounds;
+            else atomicMax(t1.ctr + 6, rounds);
             if (rollback) {
                 atomicAdd(t1.stats + 5, 1);
                 atomicAdd(t1.count, nOrig);
@@ -1749,10 +1761,31 @@ __global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_paral
                 atomicAdd(t1.stats + 3, *(volatile int*)&ctl->flips);
             }
         }
-        __threadfence();
-        if (sphere || atomicAdd(t1.ctr + 7, 1) == (int)gridDim.x - 1) t1.stats[4] += *(volatile int*)(t1.ctr + 6);
+        if (!sphere) {
+            __threadfence();
+            last = atomicAdd(t1.ctr + 7, 1) == (int)gridDim.x - 1;
+            __threadfence();
+        }
     }
     lap(4);
+    if (sphere) {
+        if (rollback) {
+            __syncthreads();
+            const int touched = t1_replay(A, t1, 0);
+            patch_touched(A, t1, touched, 0, 1);
+        }
+        sphere_done();
+        return;
+    }
+    __syncthreads();
+    if (!last) return;
+    if (tid == 0) t1.stats[4] += *(volatile int*)(t1.ctr + 6);
+    if (*(volatile int*)t1.count > 0) {
+        // (the touched cells are appended after those of the segments that succeeded)
+        const int touched = t1_replay(A, t1, *(volatile int*)(t1.ctr + 5));
+        if (tid == 0) t1.ctr[5] = touched;
+    }
+    if (tid == 0) t1_pass_done(A, t1);
 }
 
 // Ring bookkeeping for all vertices after a topology upload: for each cell and ring position,
@@ -2162,12 +2195,12 @@ static int mark_pass(svm_model* m) {
 int launch_t1_apply(svm_model* m, int bump) {
     if (int rc = ensure_ring_headroom(m)) return rc;
     const bool batch = m->nRep > 1;
-    PhaseTimer pt(m, SVM_PHASE_T1APPLY, batch ? 3 : 2);
+    PhaseTimer pt(m, SVM_PHASE_T1APPLY, batch ? 2 : 1);
     const int nSeg = batch ? m->nRep : 1;
     const int coop = batch ? 1 : t1_coop_blocks(m);
-    // a batch's touched-cell count (ctr[5]), per-pass round maximum (ctr[6]) and block ticket (ctr[7]);
-    // one sphere's k_t1_apply leaves them cleared
-    if (batch && cudaMemsetAsync(m->t1.ctr + 5, 0, 3 * sizeof(int), m->stream) != cudaSuccess) return SVM_ERR_CUDA;
+    // (restricted: no T1 test has cleared the batch's counters)
+    if (batch && m->restricted && cudaMemsetAsync(m->t1.ctr + 5, 0, 3 * sizeof(int), m->stream) != cudaSuccess)
+        return SVM_ERR_CUDA;
     if (coop > 1) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(coop);
@@ -2182,9 +2215,8 @@ int launch_t1_apply(svm_model* m, int bump) {
             return SVM_ERR_CUDA;
     } else {
         launch_next(m, k_t1_parallel<false>, nSeg, batch ? kParThreadsBatch : kParThreads, apply_args(m, bump), m->t1,
-                                                                                             m->t1.undoCap / nSeg);
+                    m->t1.undoCap / nSeg);
     }
-    launch_next(m, k_t1_apply, 1, kApplyThreads, apply_args(m, bump), m->t1, !batch);
     if (batch) launch_next(m, k_t1_patch, 2 * m->sms, 256, apply_args(m, bump), m->t1);
     if (int rc = check_launch()) return rc;
     return mark_pass(m);

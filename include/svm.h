@@ -246,7 +246,7 @@ int svm_model_stream(svm_model* m, void** stream);
 #define SVM_PHASE_CELLS 1      /* per-cell centroid, area, perimeter, total-area check */
 #define SVM_PHASE_FALLBACK 2   /* triangle-fan area fallback */
 #define SVM_PHASE_FORCE 3      /* forces (+ fused Brownian integrate and move, or FIRE half-kick) */
-#define SVM_PHASE_T1APPLY 4    /* ordered T1 flips (parallel pass, replay; a batch also patches: 2 or 3 kernels) */
+#define SVM_PHASE_T1APPLY 4    /* ordered T1 flips (one kernel; a batch also patches: two) */
 #define SVM_PHASE_MOVE 5       /* standalone moves and velocity-Verlet drift */
 #define SVM_PHASE_COUNT 6
 /* enable: 0 off, 1 every phase; SVM_PROFILE_ONLY | (1 << phase) | ... brackets only the phases named
