@@ -708,19 +708,38 @@ __device__ __forceinline__ void step_begin() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 template <class... Params, class... Args>
-inline void launch_next_smem(const svm_model* m, void (*kernel)(Params...), int grid, int block, int smem, Args&&... args) {
+inline void launch_next_with(const svm_model* m, void (*kernel)(Params...), int grid, int cluster, int block, int smem,
+                             Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = m->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (early_launch(m)) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = cluster;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = early_launch(m) ? 1 : 0;
+    cfg.numAttrs = n;
     // (an error stays with the runtime for check_launch)
     (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+template <class... Params, class... Args>
+inline void launch_next_smem(const svm_model* m, void (*kernel)(Params...), int grid, int block, int smem, Args&&... args) {
+    launch_next_with(m, kernel, grid, 1, block, smem, static_cast<Args&&>(args)...);
+}
+// One cluster or more of `cluster` blocks each.
+template <class... Params, class... Args>
+inline void launch_next_cluster(const svm_model* m, void (*kernel)(Params...), int grid, int cluster, int block, Args&&... args) {
+    launch_next_with(m, kernel, grid, cluster, block, 0, static_cast<Args&&>(args)...);
 }
 template <class... Params, class... Args>
 inline void launch_next(const svm_model* m, void (*kernel)(Params...), int grid, int block, Args&&... args) {

@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <atomic>
 #include <type_traits>
+#include <cooperative_groups.h>
 #include "svm_internal.cuh"
 #include "svm_force.cuh"
 #include "svm_hull.h"
@@ -1376,7 +1377,9 @@ __device__ __forceinline__ int pick_aff(int a, int v1, int v2, const int4& vs) {
 // batches on three streams, which fill the chip between them, four steps take 2373, 2385 and 2430 us (one
 // batch by itself 2940, 2835, 2783).
 constexpr int kParThreads = 512, kParThreadsBatch = 256;
-constexpr int kCoopThreads = 256;       // per block of a cooperative single-sphere pass
+constexpr int kCoopThreads = 256;       // per block of a single-sphere pass over several blocks
+constexpr int kT1ClusterBlocks = 8;
+enum T1Mode { kT1Block, kT1Cluster, kT1Grid };
 
 // Barrier of all blocks of a cooperative launch (co-resident by construction): the last block
 // to arrive resets the count and advances the generation; the others poll the generation, at most
@@ -1419,16 +1422,16 @@ __device__ bool grid_barrier(T1Ctl* ctl, int spinLimit) {
 // highest position that ran, and then every flip of the pass is undone and the bitmap restored for
 // t1_replay, which applies the flips one by one.
 //
-// kCoop = false: one block per segment of the position space: the whole sphere, or one replica
+// kT1Block: one block per segment of the position space: the whole sphere, or one replica
 // of a batch (whose flagged edges share no vertex or cell with another replica's, and whose
 // positions are a contiguous range).  A block's lists, footprints, commit list and undo log are
 // its own slices of the scratch arrays; a batch's touched-cell list and the flip log are shared (atomic
 // appends).  A block whose pass is not the sequential order undoes its own flips, marks their log
 // entries invalid (pass -1) and restores its segment's flags.  The last block to finish (ticket) replays
 // what was undone, folds the round count into the statistics and ends the pass.
-// kCoop = true: one segment (the whole sphere) over all blocks of a cooperative launch, so that the
+// kT1Cluster, kT1Grid: one segment (the whole sphere) over the blocks of a cluster or of a cooperative launch, so that the
 // flips spread over many SMs instead of one: position i of a round runs on block i mod gridDim.x, the
-// phases are separated by grid barriers instead of block barriers, the counters live in global memory
+// phases are separated by cluster or grid barriers instead of block barriers, the counters live in global memory
 // (t1.ctl, cleared by the T1 test: t1_clear), and block 0 alone finishes a rollback, its replay and the
 // statistics.  Same decisions, same results.  (The replay and the end of the pass were a kernel of their
 // own, which found nothing to do but for a rare rollback: 5 us by itself.)
@@ -1439,17 +1442,18 @@ __device__ bool grid_barrier(T1Ctl* ctl, int spinLimit) {
 // flip runs on a warp (t1_flip_warp), its atomics on their way while the tests run.  The pass, with 1.3 rounds
 // and 75 flips on average, 100k cells: 45 us, FP32 positions 42 (57 and 48 before the replay's kernel, the
 // patch's chain and the atomics' waits were taken out); 1M cells, 440 flips: 55 us (62).
-template <bool kCoop>
-__global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_parallel(ApplyArgs A, T1Scratch t1, int undoPer) {
+template <int kMode>
+__global__ void __launch_bounds__(kMode != kT1Block ? kCoopThreads : kParThreads)
+    k_t1_parallel(ApplyArgs A, T1Scratch t1, int undoPer) {
     step_begin();
+    constexpr bool kCoop = kMode != kT1Block;
     __shared__ T1Ctl sctl;
     T1Ctl* ctl = kCoop ? t1.ctl : &sctl;
     const int tid = threadIdx.x, seg = kCoop ? 0 : blockIdx.x;
     const bool leader = !kCoop || blockIdx.x == 0;  // finishes the pass
     const bool sphere = kCoop || t1.segOff == nullptr;
     // this thread's first position of a round and the stride (reserve and release phases), and
-    // this warp's (run phase: one warp per position).  Consecutive positions go to different
-    // blocks of a cooperative grid.
+    // this warp's (run phase: one warp per position).  Consecutive positions go to different blocks.
     const int lane = tid & 31, warps = blockDim.x >> 5;
     const int gi = kCoop ? blockIdx.x + gridDim.x * tid : tid;
     const int gs = kCoop ? gridDim.x * blockDim.x : blockDim.x;
@@ -1473,7 +1477,8 @@ __global__ void __launch_bounds__(kCoop ? kCoopThreads : kParThreads) k_t1_paral
         return;
     }
     auto group_sync = [&]() -> bool {
-        if (!kCoop) { __syncthreads(); return true; }
+        if (kMode == kT1Block) { __syncthreads(); return true; }
+        if (kMode == kT1Cluster) { cooperative_groups::this_cluster().sync(); return true; }
         if (grid_barrier(ctl, A.barrierSpins)) return true;
         if (tid == 0) atomicOr(A.status, SVM_DEV_T1_TIMEOUT);
         if (leader) sphere_done();
@@ -2101,9 +2106,8 @@ int launch_geometry(svm_model* m) {
     return launch_cells(m);
 }
 
-// Blocks of a single sphere's parallel T1 pass: one, or a cooperative grid of about one block per
-// 3000 vertices (from 20000 vertices on, at most the co-resident count), or the count set by
-// svm_model_set_t1_blocks.
+// Blocks of a sphere's T1 pass over a cooperative grid: about one per 3000 vertices, at most the co-resident
+// count, or the count set by svm_model_set_t1_blocks.
 static int t1_coop_blocks(svm_model* m) {
     // co-resident blocks of k_t1_parallel<true>, per device (computed on the model's device, which
     // is current while its calls run); atomics, as host threads may drive models concurrently
@@ -2115,13 +2119,24 @@ static int t1_coop_blocks(svm_model* m) {
     if (maxCoop == 0) {
         int sms = 0, perSm = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_t1_parallel<true>, kCoopThreads, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_t1_parallel<kT1Grid>, kCoopThreads, 0);
         maxCoop = std::max(1, sms * perSm);
         if (dev >= 0 && dev < kMaxDevices) maxCoopOf[dev].store(maxCoop, std::memory_order_relaxed);
     }
     int n = m->t1Blocks;
-    if (n == 0) n = m->nVertices < 20000 ? 1 : std::max(8, std::min(152, m->nVertices / 3000));
+    if (n == 0) n = std::max(8, std::min(152, m->nVertices / 3000));
     return std::min(n, maxCoop);
+}
+// How a pass's flips are spread (a flip and its patch take some 5 us of one SM's FP64 pipe, so a handful on
+// one SM already queue): a batch's replicas a block each; a sphere over one cluster, whose barrier is the
+// hardware's and which may start early like the other kernels; from kT1GridFrom vertices on, where eight SMs are too few,
+// over a cooperative grid.  A step, T = 0.01, one block / cluster / cooperative grid: 200 cells 41 / 41 / 41 us,
+// 2000 62 / 61 / 63, 5000 78 / 71 / 72, 10k 124 / 88 / 90, 20k 199 / 127 / 128, 40k 324 / 196 / 192, 60k 506 /
+// 285 / 260.
+constexpr int kT1GridFrom = 50000;
+static T1Mode t1_mode(const svm_model* m) {
+    if (m->nRep > 1 || m->t1Blocks == 1) return kT1Block;
+    return m->t1Blocks > 1 || m->nVertices >= kT1GridFrom ? kT1Grid : kT1Cluster;
 }
 
 // Copies the first ringCount[c] entries of every ring from stride Wc to stride Wn (the rest -1).
@@ -2197,11 +2212,15 @@ int launch_t1_apply(svm_model* m, int bump) {
     const bool batch = m->nRep > 1;
     PhaseTimer pt(m, SVM_PHASE_T1APPLY, batch ? 2 : 1);
     const int nSeg = batch ? m->nRep : 1;
-    const int coop = batch ? 1 : t1_coop_blocks(m);
     // (restricted: no T1 test has cleared the batch's counters)
     if (batch && m->restricted && cudaMemsetAsync(m->t1.ctr + 5, 0, 3 * sizeof(int), m->stream) != cudaSuccess)
         return SVM_ERR_CUDA;
-    if (coop > 1) {
+    const T1Mode mode = t1_mode(m);
+    const int coop = mode == kT1Grid ? t1_coop_blocks(m) : 1;
+    if (mode == kT1Cluster) {
+        launch_next_cluster(m, k_t1_parallel<kT1Cluster>, kT1ClusterBlocks, kT1ClusterBlocks, kCoopThreads,
+                            apply_args(m, bump), m->t1, m->t1.undoCap);
+    } else if (coop > 1) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(coop);
         cfg.blockDim = dim3(kCoopThreads);
@@ -2211,10 +2230,10 @@ int launch_t1_apply(svm_model* m, int bump) {
         attr[0].val.cooperative = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        if (cudaLaunchKernelEx(&cfg, k_t1_parallel<true>, apply_args(m, bump), m->t1, m->t1.undoCap) != cudaSuccess)
+        if (cudaLaunchKernelEx(&cfg, k_t1_parallel<kT1Grid>, apply_args(m, bump), m->t1, m->t1.undoCap) != cudaSuccess)
             return SVM_ERR_CUDA;
     } else {
-        launch_next(m, k_t1_parallel<false>, nSeg, batch ? kParThreadsBatch : kParThreads, apply_args(m, bump), m->t1,
+        launch_next(m, k_t1_parallel<kT1Block>, nSeg, batch ? kParThreadsBatch : kParThreads, apply_args(m, bump), m->t1,
                     m->t1.undoCap / nSeg);
     }
     if (batch) launch_next(m, k_t1_patch, 2 * m->sms, 256, apply_args(m, bump), m->t1);

@@ -190,8 +190,8 @@ int svm_model_t1_stats(svm_model* m, int* stats6);
  * (extraction of the flagged edges, reservation, flips, release, end), when cycles5 is non-NULL
  * and the counters are on; then (re)arms them (enable != 0) or turns them off. */
 int svm_model_t1_clocks(svm_model* m, int enable, unsigned long long* cycles5);
-/* Blocks of a single sphere's parallel T1 pass: 0 = automatic (a cooperative grid of about one
- * block per 3000 vertices from 20000 vertices on, else one block), 1 = one block, n > 1 = a
+/* Blocks of a single sphere's parallel T1 pass: 0 = automatic (one cluster of eight blocks, from
+ * 50000 vertices on a cooperative grid of about one block per 3000 vertices), 1 = one block, n > 1 = a
  * cooperative grid of n blocks (capped at the device's co-resident count).  Performance only:
  * the flips and every later value are the same for any count.  Ignored by batches. */
 int svm_model_set_t1_blocks(svm_model* m, int blocks);
