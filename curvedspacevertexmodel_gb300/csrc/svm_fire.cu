@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(slot_threads(kFireVerts), kForm == kFormVector
     __shared__ SlotShared<kFireVerts> slots;
     if (Sp->done) return;
     const double dt = Sp->dt;
-    const D3 fv = block_slot_force<kForm, kFireVerts>(A, nV, slots, NoSide());
+    const D3 fv = block_slot_force<kForm, false>(A, nV, slots, NoSide());
     const int i = blockIdx.x * kFireVerts + threadIdx.x;
     double P = 0.0, FF = 0.0, VV = 0.0;
     if (threadIdx.x < kFireVerts && i < nV) {

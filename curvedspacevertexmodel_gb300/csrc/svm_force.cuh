@@ -103,7 +103,7 @@ __device__ __forceinline__ bool det_negative(D3 p, D3 a, D3 b) {
 //   -pp (grad d(v, L) + grad d(v, X)) - aa (grad A(v, L, c) + grad A(v, c, X)), pp = 2 dP, aa = 2 Kr dA,
 // each term subtracted in the reference's order.  `side(q)` is work that does not depend on the force: one
 // call per slot, by role 1's threads while role 0 evaluates the edge gradients.  Every thread of the block calls it.
-template <int kVerts, class Side>
+template <bool kHwMul, int kVerts, class Side>
 __device__ __forceinline__ void slot_forces_reference(const ForceArgs& A, int nV, SlotShared<kVerts>& sh, Side side) {
     constexpr int kRole = slot_role_threads(kVerts);
     const bool role0 = threadIdx.x < kRole;
@@ -114,9 +114,9 @@ __device__ __forceinline__ void slot_forces_reference(const ForceArgs& A, int nV
     if (q.live) {
         sv = A.vsph[q.v];
         s2 = role0 ? A.vsph[q.L] : A.cellSph[q.c];
-        own = pair_terms(sv, s2);
+        own = pair_terms<kHwMul>(sv, s2);
         if (role0) {
-            gL = from_basis(sv, grad_geodesic(own, s2.y));
+            gL = from_basis(sv, grad_geodesic<kHwMul>(own, s2.y));
             put3<kVerts>(sh.g, q.at, gL);
         } else {
             side(q);
@@ -139,13 +139,13 @@ __device__ __forceinline__ void slot_forces_reference(const ForceArgs& A, int nV
             if (q.jx >= 0) gX = get3<kVerts>(sh.g, tx);
             else {
                 const double4_32a sx = A.vsph[q.X];
-                gX = from_basis(sv, grad_geodesic(pair_terms(sv, sx), sx.y));
+                gX = from_basis(sv, grad_geodesic<kHwMul>(pair_terms<kHwMul>(sv, sx), sx.y));
             }
             fs = sub3(scl3(-pp, gL), scl3(pp, gX));
         } else {
-            other = q.jx >= 0 ? get_pair<kVerts>(sh.l, tx) : pair_terms(sv, s3);
+            other = q.jx >= 0 ? get_pair<kVerts>(sh.l, tx) : pair_terms<kHwMul>(sv, s3);
         }
-        double2 g = grad_triangle(own, other, pair_cos(s2, s3), s2.y, s3.y, A.R);
+        double2 g = grad_triangle<kHwMul>(own, other, pair_cos<kHwMul>(s2, s3), s2.y, s3.y, A.R);
         const D3 p = ld3(A.pos, q.v), cp = ld3(A.cellPos, q.c), pn = ld3(A.pos, role0 ? q.L : q.X);
         if (det_negative(p, role0 ? pn : cp, role0 ? cp : pn)) g = make_double2(-g.x, -g.y);
         const D3 t = scl3(aa, from_basis(sv, g));
@@ -252,10 +252,10 @@ __device__ __forceinline__ void slot_forces_vector(const ForceArgs& A, int nV, S
 // The force of vertex threadIdx.x of the block's kVerts vertices (threads from kVerts on: zero).  The
 // slots' contributions are added in slot order, a NaN term skipped, as the reference's loop over the
 // three cells does.
-template <int kForm, int kVerts, class Side>
+template <int kForm, bool kHwMul, int kVerts, class Side>
 __device__ __forceinline__ D3 block_slot_force(const ForceArgs& A, int nV, SlotShared<kVerts>& sh, Side side) {
     if (kForm == kFormVector || (kForm == kFormAny && A.vec)) slot_forces_vector<kVerts>(A, nV, sh, side);
-    else slot_forces_reference<kVerts>(A, nV, sh, side);
+    else slot_forces_reference<kHwMul>(A, nV, sh, side);
     const int t = threadIdx.x;
     D3 f{0.0, 0.0, 0.0};
     if (t < kVerts && blockIdx.x * kVerts + t < nV) {

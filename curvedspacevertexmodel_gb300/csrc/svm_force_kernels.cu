@@ -37,11 +37,12 @@ __global__ void k_zig_init() {
 namespace {
 using namespace svm;
 
+template <bool kHwMul>
 __global__ void __launch_bounds__(slot_threads(kSlotVerts), kSlotMinBlocks)
     k_force(ForceArgs A, int nV, double4_32a* __restrict__ force) {
     step_begin();
     __shared__ SlotShared<> sh;
-    const D3 f = block_slot_force<kFormAny>(A, nV, sh, NoSide());
+    const D3 f = block_slot_force<kFormAny, kHwMul>(A, nV, sh, NoSide());
     const int v = blockIdx.x * kSlotVerts + threadIdx.x;
     if (threadIdx.x >= kSlotVerts || v >= nV) return;
     st3(force, v, f);
@@ -52,7 +53,7 @@ __global__ void __launch_bounds__(slot_threads(kSlotVerts), kSlotMinBlocks)
 // edge gradients.
 // (Writing the moved vertex's norm here as well, which would spare the corner pass its k_vnorm, made
 // this FP64-bound kernel as much slower as the corner pass got faster.)
-template <int kNoise>
+template <int kNoise, bool kHwMul>
 __global__ void __launch_bounds__(slot_threads(kSlotVerts), kSlotMinBlocks)
     k_force_bd(ForceArgs A, int nV, double4_32a* __restrict__ force, double4_32a* __restrict__ posNext,
                const double* __restrict__ noise, uint64_t seed, const unsigned long long* __restrict__ stepCounter,
@@ -60,7 +61,7 @@ __global__ void __launch_bounds__(slot_threads(kSlotVerts), kSlotMinBlocks)
     step_begin();
     __shared__ SlotShared<> sh;
     __shared__ double xi[3 * kSlotVerts];
-    const D3 f = block_slot_force<kFormAny>(A, nV, sh, [&](const SlotIndex& q) {
+    const D3 f = block_slot_force<kFormAny, kHwMul>(A, nV, sh, [&](const SlotIndex& q) {
         xi[q.at] = kNoise == SVM_NOISE_BUFFER ? noise[3 * q.v + q.s] : philox_normal(zig, seed, *stepCounter, q.v, q.s);
     });
     const int t = threadIdx.x, v = blockIdx.x * kSlotVerts + t;
@@ -80,8 +81,8 @@ int slot_blocks(int nV) { return (nV + kSlotVerts - 1) / kSlotVerts; }
 namespace svm {
 
 int launch_force_fp64(svm_model* m) {
-    launch_next(m, k_force, slot_blocks(m->nVertices), slot_threads(kSlotVerts), force_args(m, m->cur), m->nVertices,
-                                                                                  m->force);
+    launch_next(m, few_hw_mul(m) ? k_force<true> : k_force<false>, slot_blocks(m->nVertices), slot_threads(kSlotVerts),
+                force_args(m, m->cur), m->nVertices, m->force);
     return check_launch();
 }
 
@@ -111,7 +112,9 @@ int launch_force_bd_fp64(svm_model* m, double np, double fp, int noiseMode, cons
             force_args(m, m->cur), m->nVertices, m->force, m->pos[nxt], noise, seed, m->stepCounter, np, fp, zig,
             m->ioHostOut);
     };
-    noiseMode == SVM_NOISE_BUFFER ? go(k_force_bd<SVM_NOISE_BUFFER>) : go(k_force_bd<SVM_NOISE_PHILOX>);
+    const bool few = few_hw_mul(m);
+    if (noiseMode == SVM_NOISE_BUFFER) go(few ? k_force_bd<SVM_NOISE_BUFFER, true> : k_force_bd<SVM_NOISE_BUFFER, false>);
+    else go(few ? k_force_bd<SVM_NOISE_PHILOX, true> : k_force_bd<SVM_NOISE_PHILOX, false>);
     return check_launch();
 }
 

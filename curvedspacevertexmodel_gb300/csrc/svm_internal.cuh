@@ -122,7 +122,7 @@ __device__ __forceinline__ D3 cross3(D3 p1, D3 p2) {          // inc/functions.h
 // geometry's divisions and arccosines (corner phase 0.159 -> 0.151 ms at 100k cells when they moved), the
 // norms ahead of the centroids', vertices' and fan triangles' square roots (cells and fallback phases
 // 2-3% shorter).  The gradients' products are grad_mul.
-// (kHw: the hardware multiply, for the T1 pass's latency-bound chains.)
+// (kHw: the hardware multiply, for the T1 pass's latency-bound chains and for small models: kFewHwMul.)
 template <bool kHw = false>
 __device__ __forceinline__ double early_mul(double x, double y) {
     if constexpr (kHw) return __dmul_rn(x, y);
@@ -147,8 +147,9 @@ __device__ __forceinline__ double det3(D3 a, D3 b, D3 c) {    // a . (b x c), sp
 }
 
 // putInBoxReal (sphericalDomain.h:183-187): p <- R p / |p|
+template <bool kHwMul = false>
 __device__ __forceinline__ D3 renorm(D3 p, double R) {
-    double inv = f64_div_root(1.0, dot3e(p, p));
+    double inv = f64_div_root(1.0, dot3e<kHwMul>(p, p));
     return scl3(R, scl3(inv, p));
 }
 // move(p, v) (sphericalDomain.h:203-209): project v onto the tangent plane at p, add, renormalise
@@ -166,11 +167,12 @@ __device__ __forceinline__ double geodesic(D3 p1, D3 p2, double R) {
     return R * svm_acos(f64_div<kHw>(num, den));
 }
 // |p| as geodesic and sph_coords evaluate it (same operations, so the same value)
-template <bool kHw = false>
-__device__ __forceinline__ double pos_norm(D3 p) { return f64_sqrt<kHw>(dot3e<kHw>(p, p)); }
+template <bool kHw = false, bool kHwMul = kHw>
+__device__ __forceinline__ double pos_norm(D3 p) { return f64_sqrt<kHw>(dot3e<kHwMul>(p, p)); }
 // geodesic with the two norms given (n1 = pos_norm(p1), n2 = pos_norm(p2)): the same value
+template <bool kHwMul = false>
 __device__ __forceinline__ double geodesic_n(D3 p1, D3 p2, double n1, double n2, double R) {
-    return R * svm_acos(f64_div(dot3e(p1, p2), early_mul(n1, n2)));
+    return R * svm_acos(f64_div(dot3e<kHwMul>(p1, p2), early_mul<kHwMul>(n1, n2)));
 }
 // The T1 length test geodesic(p1, p2) < t, i.e. R acos(c) < t with c = p1.p2 / (|p1||p2|).  acos
 // is decreasing, so away from c = cos(t / R) the answer is c > cos(t / R); the formula itself is
@@ -252,9 +254,9 @@ __device__ __forceinline__ double included_angle(D3 p1, D3 p2, D3 p3) {
 __device__ __forceinline__ bool positive(double x) {   // x > 0
     return (unsigned long long)__double_as_longlong(x) - 1ull < 0x7ff0000000000000ull;
 }
-template <bool clamp = false>
+template <bool clamp = false, bool kHwMul = false>
 __device__ __forceinline__ double included_cos(D3 Cx, D3 Cl, double nx, double nl) {
-    double c = f64_div(dot3e(Cx, Cl), early_mul(nx, nl));
+    double c = f64_div(dot3e<kHwMul>(Cx, Cl), early_mul<kHwMul>(nx, nl));
     // fmin(1, fmax(-1, c)), a NaN to -1
     if (clamp) {
         const unsigned long long b = (unsigned long long)__double_as_longlong(c), m = b & 0x7fffffffffffffffull;
@@ -383,11 +385,11 @@ __host__ __device__ inline double mixed_area_limit(int nC, double R) {
 // Spherical coordinates of a point as the reference's gradients compute them
 // (sphericalDomain.h:218-232, 251-261): cos t = z/|p|, sin t = sqrt(1 - cos^2 t),
 // cos p = x / sqrt(x^2+y^2), sin p = y / sqrt(x^2+y^2).
-template <bool kHw = false>
+template <bool kHw = false, bool kHwMul = kHw>
 __device__ __forceinline__ double4_32a sph_coords_n(D3 p, double r) {  // r = pos_norm(p)
     double cosT = f64_div<kHw>(p.z, r);
     double sinT = f64_sqrt<kHw>(1. - cosT * cosT);
-    const double rxy2 = early_mul<kHw>(p.x, p.x) + early_mul<kHw>(p.y, p.y);
+    const double rxy2 = early_mul<kHwMul>(p.x, p.x) + early_mul<kHwMul>(p.y, p.y);
     if constexpr (kHw) {
         const double rxy = f64_sqrt<kHw>(rxy2);
         return make_double4_32a(cosT, sinT, f64_div<kHw>(p.x, rxy), f64_div<kHw>(p.y, rxy));
@@ -396,20 +398,25 @@ __device__ __forceinline__ double4_32a sph_coords_n(D3 p, double r) {  // r = po
         return make_double4_32a(cosT, sinT, f64_div(p.x, rxy), f64_div(p.y, rxy));
     }
 }
-template <bool kHw = false>
-__device__ __forceinline__ double4_32a sph_coords(D3 p) { return sph_coords_n<kHw>(p, pos_norm<kHw>(p)); }
+template <bool kHw = false, bool kHwMul = kHw>
+__device__ __forceinline__ double4_32a sph_coords(D3 p) { return sph_coords_n<kHw, kHwMul>(p, pos_norm<kHw, kHwMul>(p)); }
 
 // The gradients' products on the integer pipes, out of line: some sixty to a slot, whose inlined code
 // (56 KB for the Brownian force kernel) did not fit the instruction caches.
-__device__ __forceinline__ double grad_mul(double x, double y) { return sf::mul_call(x, y); }
+template <bool kHwMul = false>
+__device__ __forceinline__ double grad_mul(double x, double y) {
+    if constexpr (kHwMul) return __dmul_rn(x, y);
+    else return sf::mul_call(x, y);
+}
 
 // The terms of a pair of points (a, b), in spherical coordinates, that the gradients at a of both
 // gradientGeodesicDistance (sphericalDomain.h:248-273) and gradientTriangleArea (347-411) evaluate:
 // sin(phi_a - phi_b), s = cos of the arc, d = its derivative by theta_a, s s and s s - 1.  A pair is
 // evaluated once and serves its edge and both triangles it is a side of.
 struct PairTerms { double sP, s, d, ss, q; };
+template <bool kHwMul = false>
 __device__ __forceinline__ PairTerms pair_terms(const double4_32a& a, const double4_32a& b) {
-    const auto E = [](double x, double y) { return grad_mul(x, y); };
+    const auto E = [](double x, double y) { return grad_mul<kHwMul>(x, y); };
     PairTerms p;
     p.sP = E(a.w, b.z) - E(a.z, b.w);
     const double cP = E(a.z, b.z) + E(a.w, b.w);
@@ -420,17 +427,19 @@ __device__ __forceinline__ PairTerms pair_terms(const double4_32a& a, const doub
     return p;
 }
 // cos of the arc between b and c alone (the third side of a triangle at a)
+template <bool kHwMul = false>
 __device__ __forceinline__ double pair_cos(const double4_32a& b, const double4_32a& c) {
-    const auto E = [](double x, double y) { return grad_mul(x, y); };
+    const auto E = [](double x, double y) { return grad_mul<kHwMul>(x, y); };
     const double cP = E(b.z, c.z) + E(b.w, c.w);
     return E(b.x, c.x) + E(E(cP, b.y), c.y);
 }
 
 // gradientGeodesicDistance (sphericalDomain.h:248-273) in the (theta, phi) basis of v1, from the
 // pair's terms and sin(theta) of the other point: returns (d/dtheta, d/dphi) components.
+template <bool kHwMul = false>
 __device__ __forceinline__ double2 grad_geodesic(const PairTerms& p, double sinT2) {
     const double dinv = f64_div_root(1., -p.q);   // 1 - s s = -(s s - 1) exactly
-    return make_double2(-p.d * dinv, grad_mul(sinT2, p.sP) * dinv);
+    return make_double2(-p.d * dinv, grad_mul<kHwMul>(sinT2, p.sP) * dinv);
 }
 
 // grad_triangle's products that stay on the FP64 pipe, which balances the two: the roots' arguments
@@ -443,10 +452,11 @@ __device__ __forceinline__ double tri_mul(double x, double y) { return __dmul_rn
 // right, products first); equal subexpressions, and those that differ by an exact sign or a power
 // of two, are evaluated once.  Each denominator is a square root and divides two numerators: its
 // reciprocal comes with the root (f64_root_divisor) and serves both.
+template <bool kHwMul = false>
 __device__ __forceinline__ double2 grad_triangle(const PairTerms& p12, const PairTerms& p13, double s23, double sinT2,
                                                  double sinT3, double R) {
     const auto M = tri_mul;
-    const auto E = [](double x, double y) { return grad_mul(x, y); };
+    const auto E = [](double x, double y) { return grad_mul<kHwMul>(x, y); };
     const double s12s13 = E(p12.s, p13.s);
     // 2 s12 s13 s23 = 2 ((s12 s13) s23): the factor two is exact wherever it is applied
     const double g = ((-p12.q - p13.ss) - M(s23, s23)) + sf::twice(M(s12s13, s23));
@@ -762,6 +772,13 @@ inline int spread_block(const svm_model* m, long n) {
     while (bs > 32 && n < 4L * m->sms * bs) bs >>= 1;
     return bs;
 }
+// Small models' corner and force kernels take the hardware multiply in place of sf::mul (the same bits):
+// they wait on the chain of a thread's operations, not on the FP64 pipe, and the hardware's is the shorter.
+// A step, soft / hardware: 200 cells 40.6 / 35.1 us (force phase 20.8 / 18.0, corners 13.1 / 12.6), 1000
+// 55.6 / 50.0, 5000 70.6 / 70.4.  The line lies where three models on three streams, whose work adds up on the pipe,
+// are even; 8 steps: 150 cells 122 / 108 us, 1000 150 / 143, 1500 166 / 166, 2000 183 / 189, 5000 256 / 298.
+constexpr int kFewHwMul = 3000;   // vertices
+inline bool few_hw_mul(const svm_model* m) { return m->nVertices < kFewHwMul; }
 int ensure_ring_headroom(svm_model* m);
 int check_launch();
 void fire_detach(svm_fire* F);          // svm_fire.cu: the model is going away

@@ -204,6 +204,7 @@ __device__ __forceinline__ bool edge_terms(int v, int j, int u, const int4* __re
 // models running beside it get more done), 300k 317 -> 346: models from 50,000 vertices on keep the three.
 constexpr int kFewVerts = 32;                     // vertices per block: four whole warps
 constexpr int kFewCornersBelow = 50000;          // vertices
+template <bool kHwMul>
 __global__ void __launch_bounds__(4 * kFewVerts) k_corners_few(
     const double4_32a* __restrict__ pos, double4_32a* __restrict__ vsph, const int4* __restrict__ vcell,
     const int4* __restrict__ vlast, const int4* __restrict__ vnext, const int4* __restrict__ vrpos,
@@ -219,7 +220,7 @@ __global__ void __launch_bounds__(4 * kFewVerts) k_corners_few(
     const int t = threadIdx.x;
     if (t >= 3 * kFewVerts) {
         const int v = blockIdx.x * kFewVerts + t - 3 * kFewVerts;
-        if (v < nV) vsph[v] = sph_coords(ld3(pos, v));
+        if (v < nV) vsph[v] = sph_coords<false, kHwMul>(ld3(pos, v));
     }
     const int vi = t / 3, j = t - 3 * (t / 3), b = 3 * vi, v = blockIdx.x * kFewVerts + vi;
     const bool live = t < 3 * kFewVerts && v < nV;
@@ -228,9 +229,9 @@ __global__ void __launch_bounds__(4 * kFewVerts) k_corners_few(
         nb = vnbr[v];
         const int u = comp(nb, j);
         const D3 p = ld3(pos, v), U = ld3(pos, u);
-        const D3 C = cross3e(p, U);
-        const double arc = geodesic_n(U, p, pos_norm(U), pos_norm(p), R);
-        cx[t] = C.x; cy[t] = C.y; cz[t] = C.z; nc[t] = f64_sqrt(dot3e(C, C));
+        const D3 C = cross3e<kHwMul>(p, U);
+        const double arc = geodesic_n<kHwMul>(U, p, pos_norm<false, kHwMul>(U), pos_norm<false, kHwMul>(p), R);
+        cx[t] = C.x; cy[t] = C.y; cz[t] = C.z; nc[t] = f64_sqrt(dot3e<kHwMul>(C, C));
         ux[t] = U.x; uy[t] = U.y; uz[t] = U.z; arcs[t] = arc;
         if (t1test && v < u && arc < t1Threshold) t1_flag(t1, 3 * v + j, v, u, 0, vnbr, vcell);
     }
@@ -246,8 +247,8 @@ __global__ void __launch_bounds__(4 * kFewVerts) k_corners_few(
             const int l = b + jl, x = b + jx;
             const D3 X{cx[x], cy[x], cz[x]};
             arc = arcs[l];
-            flip = positive(dot3e(D3{ux[l], uy[l], uz[l]}, X));
-            cosine[0] = included_cos(X, D3{cx[l], cy[l], cz[l]}, nc[x], nc[l]);
+            flip = positive(dot3e<kHwMul>(D3{ux[l], uy[l], uz[l]}, X));
+            cosine[0] = included_cos<false, kHwMul>(X, D3{cx[l], cy[l], cz[l]}, nc[x], nc[l]);
         }
     }
     block_acos(cosine, val, src, warpHigh);
@@ -376,9 +377,9 @@ __global__ void k_cells(const PT* __restrict__ pos, const int* __restrict__ ring
                 for (int k = 0; k < kAhead; ++k) if (k < n) cp = add3(cp, q[k]);
             }
             for (int k = kAhead; k < n; ++k) cp = add3(cp, ld3(pos, rg[k]));
-            cp = renorm(cp, R);
+            cp = renorm<kSplit>(cp, R);
             st3(cellPos, c, cp);
-            if (cellSph) cellSph[c] = sph_coords(cp);
+            if (cellSph) cellSph[c] = sph_coords<false, kSplit>(cp);
         }
         if (!kSplit || second) {
             const double2* cr = corner + (long)c * Wc;
@@ -2022,7 +2023,7 @@ int launch_corners(svm_model* m, bool t1test, bool vnormReady) {
     }
     if (!m->edgeC) return SVM_ERR_ARG;  // FP64 corners exist for single spheres only
     if (m->nVertices < kFewCornersBelow) {
-        launch_next(m, k_corners_few, (m->nVertices + kFewVerts - 1) / kFewVerts, 4 * kFewVerts, m->pos[m->cur], m->vsph,
+        launch_next(m, few_hw_mul(m) ? k_corners_few<true> : k_corners_few<false>, (m->nVertices + kFewVerts - 1) / kFewVerts, 4 * kFewVerts, m->pos[m->cur], m->vsph,
                     m->vcell, m->vlast, m->vnext, m->vrpos, m->vnbr, m->corner, m->Wc, m->nVertices, m->R, t1test ? 1 : 0,
                     m->t1Threshold, m->t1);
         m->cornersValid = true;
