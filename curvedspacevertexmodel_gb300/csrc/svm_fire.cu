@@ -219,7 +219,11 @@ __device__ void fire_reduce_tail(FireState* __restrict__ Sp, double P, double FF
 // vertex.  One instantiation per force form, which lets each drop the other's registers: six blocks of
 // the vector form per SM.  FIRE iteration in the vector form against three threads a vertex and separate
 // products and sums: 20k cells 163 -> 121 us, 100k cells 432 us.
-template <int kForm>
+// Below kFireHwMul vertices the kernel takes the hardware multiply, as few_hw_mul's kernels do; the line
+// lies higher here because a minimisation waits for each iteration: vector form, integer pipes / hardware, 200
+// cells 41.9 / 39.2 us, 2000 44.4 / 41.5, 5000 54.0 / 55.0, 20k 105 / 113.
+constexpr int kFireHwMul = 8000;
+template <int kForm, bool kHwMul>
 __global__ void __launch_bounds__(slot_threads(kFireVerts), kForm == kFormVector ? 6 : kSlotMinBlocks)
     k_fire_force(ForceArgs A, FireState* __restrict__ Sp, int nV, double4_32a* __restrict__ force,
                  double4_32a* __restrict__ vel, double* __restrict__ partials, unsigned* __restrict__ ticket) {
@@ -229,7 +233,7 @@ __global__ void __launch_bounds__(slot_threads(kFireVerts), kForm == kFormVector
     __shared__ SlotShared<kFireVerts> slots;
     if (Sp->done) return;
     const double dt = Sp->dt;
-    const D3 fv = block_slot_force<kForm, false>(A, nV, slots, NoSide());
+    const D3 fv = block_slot_force<kForm, kHwMul>(A, nV, slots, NoSide());
     const int i = blockIdx.x * kFireVerts + threadIdx.x;
     double P = 0.0, FF = 0.0, VV = 0.0;
     if (threadIdx.x < kFireVerts && i < nV) {
@@ -291,12 +295,13 @@ int fire_iteration(svm_fire* F) {
     if (rc) return rc;
     PhaseTimer pt(m, SVM_PHASE_FORCE);
     const int nf = (m->nVertices + kFireVerts - 1) / kFireVerts;
-    if (m->precision == SVM_PRECISION_FP64_VECTOR)
-        launch_next(m, k_fire_force<kFormVector>, nf, slot_threads(kFireVerts), fargs(m), F->d, m->nVertices, m->force, m->vel,
-                                                                        F->partials, F->ticket);
-    else
-        launch_next(m, k_fire_force<kFormReference>, nf, slot_threads(kFireVerts), fargs(m), F->d, m->nVertices, m->force,
-                                                                           m->vel, F->partials, F->ticket);
+    const bool few = m->nVertices < kFireHwMul;
+    const auto go = [&](auto kernel) {
+        launch_next(m, kernel, nf, slot_threads(kFireVerts), fargs(m), F->d, m->nVertices, m->force, m->vel, F->partials,
+                    F->ticket);
+    };
+    if (m->precision == SVM_PRECISION_FP64_VECTOR) go(few ? k_fire_force<kFormVector, true> : k_fire_force<kFormVector, false>);
+    else go(few ? k_fire_force<kFormReference, true> : k_fire_force<kFormReference, false>);
     return check_launch();
 }
 

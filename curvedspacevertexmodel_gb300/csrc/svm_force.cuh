@@ -162,31 +162,43 @@ __device__ __forceinline__ void slot_forces_reference(const ForceArgs& A, int nV
 // The vector form (A.vec: the exact gradient as vectors, well conditioned where the reference's closed
 // forms lose digits -- short edges, thin fan triangles), the same way.  Products and sums contract to
 // multiply-adds here: the form's values are pinned to its formulas, not to the CPU's sequence of
-// roundings.
-__device__ __forceinline__ double dot3f(D3 a, D3 b) { return fma(a.z, b.z, fma(a.y, b.y, a.x * b.x)); }
+// roundings.  The products that are not part of a multiply-add run on the integer pipes, which the form
+// leaves idle (early_mul; kHwMul: on the FP64 pipe), a third of its FP64 instructions: a FIRE iteration of 20k cells
+// 115 -> 105 us, of 100k 391 -> 344.
+template <bool kHwMul>
+__device__ __forceinline__ double dot3f(D3 a, D3 b) { return fma(a.z, b.z, fma(a.y, b.y, early_mul<kHwMul>(a.x, b.x))); }
+template <bool kHwMul>
 __device__ __forceinline__ D3 cross3f(D3 a, D3 b) {
-    return D3{fma(a.y, b.z, -(a.z * b.y)), fma(a.z, b.x, -(a.x * b.z)), fma(a.x, b.y, -(a.y * b.x))};
+    return D3{fma(a.y, b.z, -early_mul<kHwMul>(a.z, b.y)), fma(a.z, b.x, -early_mul<kHwMul>(a.x, b.z)),
+              fma(a.x, b.y, -early_mul<kHwMul>(a.y, b.x))};
+}
+template <bool kHwMul>
+__device__ __forceinline__ D3 scl3f(double k, D3 a) {
+    return D3{early_mul<kHwMul>(k, a.x), early_mul<kHwMul>(k, a.y), early_mul<kHwMul>(k, a.z)};
 }
 __device__ __forceinline__ D3 axpy3f(double s, D3 x, D3 y) { return D3{fma(s, x.x, y.x), fma(s, x.y, y.y), fma(s, x.z, y.z)}; }
 // Unit tangent at a pointing away from the neighbour at v + d: gradient of the geodesic length
 // (any radius), from the raw position difference d.
+template <bool kHwMul>
 __device__ __forceinline__ D3 grad_geo_vec(D3 a, D3 d) {
-    const D3 t = axpy3f(-dot3f(d, a), a, d);
-    return scl3(f64_div_root(-1.0, dot3f(t, t)), t);
+    const D3 t = axpy3f(-dot3f<kHwMul>(d, a), a, d);
+    return scl3f<kHwMul>(f64_div_root(-1.0, dot3f<kHwMul>(t, t)), t);
 }
-// Gradient w.r.t. v = |v| a of the signed spherical triangle area R^2 E(a, a + beta, a + gamma), over R
-// and without its projection onto the tangent plane: tan(E/2) = N/D (Van Oosterom and Strackee, 1983)
-// differentiated, beta and gamma the raw differences to the other corners over |v|, ab = a x beta,
-// ag = a x gamma, and the squares of beta and gamma given.
-__device__ __forceinline__ D3 grad_tri_vec(D3 a, D3 beta, D3 gamma, D3 ab, D3 ag, double beta2, double gamma2) {
-    const D3 bg = cross3f(beta, gamma);
+// scale / 2 times the gradient w.r.t. v = |v| a of the signed spherical triangle area
+// R^2 E(a, a + beta, a + gamma), over R and without its projection onto the tangent plane: tan(E/2) = N/D (Van
+// Oosterom and Strackee, 1983) differentiated, beta and gamma the raw differences to the other corners over
+// |v|, ab = a x beta, ag = a x gamma, and the squares of beta and gamma given.
+template <bool kHwMul>
+__device__ __forceinline__ D3 grad_tri_vec(D3 a, D3 beta, D3 gamma, D3 ab, D3 ag, double beta2, double gamma2,
+                                              double scale) {
+    const D3 bg = cross3f<kHwMul>(beta, gamma);
     const D3 bxc = add3(sub3(ag, ab), bg);
-    const double N = dot3f(a, bg);
-    const double D = 4.0 - beta2 - gamma2 + dot3f(beta, gamma);
-    const double w = f64_div(2.0, fma(N, N, D * D));
-    return scl3(w, axpy3f(-N, add3(beta, gamma), scl3(D, bxc)));
+    const double N = dot3f<kHwMul>(a, bg);
+    const double D = fma(beta.z, gamma.z, fma(beta.y, gamma.y, fma(beta.x, gamma.x, 4.0 - beta2 - gamma2)));
+    const double w = f64_div(scale, fma(N, N, early_mul<kHwMul>(D, D)));
+    return scl3f<kHwMul>(w, axpy3f(-N, add3(beta, gamma), scl3f<kHwMul>(D, bxc)));
 }
-template <int kVerts, class Side>
+template <bool kHwMul, int kVerts, class Side>
 __device__ __forceinline__ void slot_forces_vector(const ForceArgs& A, int nV, SlotShared<kVerts>& sh, Side side) {
     constexpr int kRole = slot_role_threads(kVerts);
     const bool role0 = threadIdx.x < kRole;
@@ -195,17 +207,17 @@ __device__ __forceinline__ void slot_forces_vector(const ForceArgs& A, int nV, S
     double b2, inv;
     if (q.live) {
         const D3 P = ld3(A.pos, q.v), d = sub3(role0 ? ld3(A.pos, q.L) : ld3(A.cellPos, q.c), P);
-        inv = f64_div_root(1.0, dot3f(P, P));
-        a = scl3(inv, P);
-        b = scl3(inv, d);
-        ab = cross3f(a, b);
-        b2 = dot3f(b, b);
+        inv = f64_div_root(1.0, dot3f<kHwMul>(P, P));
+        a = scl3f<kHwMul>(inv, P);
+        b = scl3f<kHwMul>(inv, d);
+        ab = cross3f<kHwMul>(a, b);
+        b2 = dot3f<kHwMul>(b, b);
         double (*o)[3 * kVerts] = role0 ? sh.l : sh.c;
         put3<kVerts>(o, q.at, b);
         put3<kVerts>(o + 3, q.at, ab);
         o[6][q.at] = b2;
         if (role0) {
-            gL = grad_geo_vec(a, d);
+            gL = grad_geo_vec<kHwMul>(a, d);
             put3<kVerts>(sh.g, q.at, gL);
         } else {
             side(q);
@@ -226,15 +238,15 @@ __device__ __forceinline__ void slot_forces_vector(const ForceArgs& A, int nV, S
             ao = get3<kVerts>(p + 3, k);
             o2 = p[6][k];
         } else {  // inconsistent lists
-            o = scl3(inv, sub3(ld3(A.pos, q.X), ld3(A.pos, q.v)));
-            ao = cross3f(a, o);
-            o2 = dot3f(o, o);
+            o = scl3f<kHwMul>(inv, sub3(ld3(A.pos, q.X), ld3(A.pos, q.v)));
+            ao = cross3f<kHwMul>(a, o);
+            o2 = dot3f<kHwMul>(o, o);
         }
-        const D3 t = scl3(aaR, grad_tri_vec(a, b, o, ab, ao, b2, o2));
+        const D3 t = grad_tri_vec<kHwMul>(a, b, o, ab, ao, b2, o2, 2.0 * aaR);
         if (role0) {
             const double pp = 2.0 * (apc.y - pr.y);
-            gX = q.jx >= 0 ? get3<kVerts>(sh.g, tx) : grad_geo_vec(a, sub3(ld3(A.pos, q.X), ld3(A.pos, q.v)));
-            fs = sub3(scl3(-pp, add3(gL, gX)), t);
+            gX = q.jx >= 0 ? get3<kVerts>(sh.g, tx) : grad_geo_vec<kHwMul>(a, sub3(ld3(A.pos, q.X), ld3(A.pos, q.v)));
+            fs = sub3(scl3f<kHwMul>(-pp, add3(gL, gX)), t);
         } else {
             put3<kVerts>(sh.t, q.at, t);
         }
@@ -243,7 +255,7 @@ __device__ __forceinline__ void slot_forces_vector(const ForceArgs& A, int nV, S
     if (q.live) {
         if (role0) {   // the slot's sum, projected onto the tangent plane (the edge gradients lie in it)
             const D3 f = sub3(fs, get3<kVerts>(sh.t, q.at));
-            put3<kVerts>(sh.g, q.at, axpy3f(-dot3f(f, a), a, f));
+            put3<kVerts>(sh.g, q.at, axpy3f(-dot3f<kHwMul>(f, a), a, f));
         }
     }
     __syncthreads();
@@ -254,7 +266,7 @@ __device__ __forceinline__ void slot_forces_vector(const ForceArgs& A, int nV, S
 // three cells does.
 template <int kForm, bool kHwMul, int kVerts, class Side>
 __device__ __forceinline__ D3 block_slot_force(const ForceArgs& A, int nV, SlotShared<kVerts>& sh, Side side) {
-    if (kForm == kFormVector || (kForm == kFormAny && A.vec)) slot_forces_vector<kVerts>(A, nV, sh, side);
+    if (kForm == kFormVector || (kForm == kFormAny && A.vec)) slot_forces_vector<kHwMul>(A, nV, sh, side);
     else slot_forces_reference<kHwMul>(A, nV, sh, side);
     const int t = threadIdx.x;
     D3 f{0.0, 0.0, 0.0};
