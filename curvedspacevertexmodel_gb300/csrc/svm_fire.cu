@@ -72,17 +72,6 @@ __device__ double bmax(double v, double* sh, int live = 32) {
     return r;
 }
 
-__device__ __forceinline__ D3 move_exact_f(D3 p, D3 v, double R) {
-    const double vp = __dadd_rn(__dadd_rn(__dmul_rn(v.x, p.x), __dmul_rn(v.y, p.y)), __dmul_rn(v.z, p.z));
-    const double pp = __dadd_rn(__dadd_rn(__dmul_rn(p.x, p.x), __dmul_rn(p.y, p.y)), __dmul_rn(p.z, p.z));
-    const double s = f64_div(vp, pp);
-    D3 q{__dadd_rn(p.x, __dsub_rn(v.x, __dmul_rn(s, p.x))), __dadd_rn(p.y, __dsub_rn(v.y, __dmul_rn(s, p.y))),
-         __dadd_rn(p.z, __dsub_rn(v.z, __dmul_rn(s, p.z)))};
-    const double qq = __dadd_rn(__dadd_rn(__dmul_rn(q.x, q.x), __dmul_rn(q.y, q.y)), __dmul_rn(q.z, q.z));
-    const double inv = f64_div_root(1.0, qq);
-    return D3{__dmul_rn(R, __dmul_rn(inv, q.x)), __dmul_rn(R, __dmul_rn(inv, q.y)), __dmul_rn(R, __dmul_rn(inv, q.z))};
-}
-
 // FIRE velocity update of fireStepCPU (energyMinimizerFIRE.cpp:146-149, 168-172).
 __device__ __forceinline__ D3 fire_velocity(const FireState& S, D3 v, D3 f) {
     if (S.zeroV) return D3{0.0, 0.0, 0.0};
@@ -94,6 +83,11 @@ __device__ __forceinline__ D3 fire_velocity(const FireState& S, D3 v, D3 f) {
 // velocityVerlet::integrateEOMCPU's first loop for one vertex (velocityVerlet.cpp:14-20: unit
 // masses, the model's masses being 1): disp = dt v + (dt^2 / 2) F, v += (dt / 2) F, then the move
 // onto the sphere (moveParticles).  Products rounded before the sums, as on the CPU.
+// kHwMul: products on the FP64 pipe, or on the integer pipes; one thread a vertex leaves either half
+// empty until the model is large.  A FIRE iteration, hardware / integer pipes: 5000 cells 53.7 / 55.4 us, 20k 105.5 /
+// 105.3, 100k 342.8 / 336.3.
+constexpr int kDriftHwMul = 40000;   // vertices
+template <bool kHwMul>
 __device__ __forceinline__ void vv_drift(double4_32a* __restrict__ pos, double4_32a* __restrict__ vel,
                                          double* __restrict__ vnorm, int i, D3 v, D3 f, double dt, double R) {
     const double hv = (0.5 / 1.0) * dt, h2 = 0.5 * dt * dt;
@@ -101,9 +95,9 @@ __device__ __forceinline__ void vv_drift(double4_32a* __restrict__ pos, double4_
                __dadd_rn(__dmul_rn(dt, v.z), __dmul_rn(h2, f.z))};
     v = D3{__dadd_rn(v.x, __dmul_rn(hv, f.x)), __dadd_rn(v.y, __dmul_rn(hv, f.y)), __dadd_rn(v.z, __dmul_rn(hv, f.z))};
     st3(vel, i, v);
-    const D3 q = move_exact_f(ld3(pos, i), d, R);
+    const D3 q = move_exact<kHwMul>(ld3(pos, i), d, R);
     st3(pos, i, q);
-    vnorm[i] = pos_norm(q);  // k_vnorm's value, for the corner pass that follows
+    vnorm[i] = pos_norm<false, kHwMul>(q);  // k_vnorm's value, for the corner pass that follows
 }
 // gpu_update_velocity (velocityVerlet.cu): v += (dt / 2) F / m with unit masses.
 __device__ __forceinline__ D3 vv_kick(D3 v, D3 f, double dt) {
@@ -115,6 +109,7 @@ __device__ __forceinline__ D3 vv_kick(D3 v, D3 f, double dt) {
 // (k_fire_force's last block) sets it again before this kernel next reads it, and after the last
 // iteration k_fire_finish applies the update it stands for.  Once FIRE has stopped, the positions
 // stay and only their norms are written (the corner pass of a batch's remaining iterations reads them).
+template <bool kHwMul>
 __global__ void k_fire_vv1(const FireState* __restrict__ Sp, double4_32a* __restrict__ pos,
                            double4_32a* __restrict__ vel, const double4_32a* __restrict__ force,
                            double* __restrict__ vnorm, int nV, double R) {
@@ -129,17 +124,18 @@ __global__ void k_fire_vv1(const FireState* __restrict__ Sp, double4_32a* __rest
     const D3 f = ld3(force, i);
     D3 v = ld3(vel, i);
     if (S.pending) v = fire_velocity(S, v, f);
-    vv_drift(pos, vel, vnorm, i, v, f, S.dt, R);
+    vv_drift<kHwMul>(pos, vel, vnorm, i, v, f, S.dt, R);
 }
 
 // The standalone velocity-Verlet drift: vv_drift with the caller's dt.
+template <bool kHwMul>
 __global__ void k_vv_drift(double4_32a* __restrict__ pos, double4_32a* __restrict__ vel,
                            const double4_32a* __restrict__ force, double* __restrict__ vnorm, int nV, double dt,
                            double R) {
     step_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nV) return;
-    vv_drift(pos, vel, vnorm, i, ld3(vel, i), ld3(force, i), dt, R);
+    vv_drift<kHwMul>(pos, vel, vnorm, i, ld3(vel, i), ld3(force, i), dt, R);
 }
 __global__ void k_vv_half(double4_32a* __restrict__ vel, const double4_32a* __restrict__ force, int nV, double dt) {
     step_begin();
@@ -281,7 +277,7 @@ int fire_iteration(svm_fire* F) {
     const int bs = spread_block(m, m->nVertices), nb = (m->nVertices + bs - 1) / bs;
     {
         PhaseTimer pt(m, SVM_PHASE_MOVE);
-        launch_next(m, k_fire_vv1, nb, bs, F->d, m->pos[m->cur], m->vel, m->force, m->vnorm, m->nVertices, m->R);
+        launch_next(m, m->nVertices < kDriftHwMul ? k_fire_vv1<true> : k_fire_vv1<false>, nb, bs, F->d, m->pos[m->cur], m->vel, m->force, m->vnorm, m->nVertices, m->R);
     }
     m->cornersValid = false;
     int rc;
@@ -437,7 +433,7 @@ int svm_velocity_verlet_step(svm_model* m, double dt, int nSteps) {
     for (int k = 0; k < nSteps; ++k) {
         {
             PhaseTimer pt(m, SVM_PHASE_MOVE);
-            launch_next(m, k_vv_drift, nb, bs, m->pos[m->cur], m->vel, m->force, m->vnorm, m->nVertices, dt, m->R);
+            launch_next(m, m->nVertices < kDriftHwMul ? k_vv_drift<true> : k_vv_drift<false>, nb, bs, m->pos[m->cur], m->vel, m->force, m->vnorm, m->nVertices, dt, m->R);
         }
         m->cornersValid = false;
         int rc;

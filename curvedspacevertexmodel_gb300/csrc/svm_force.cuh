@@ -364,17 +364,27 @@ __device__ __forceinline__ double bd_disp(double xi, double np, double f, double
 }
 // sphericalDomain::move with every product and sum rounded separately (no contraction), so the
 // renormalised positions follow the CPU's sequence of roundings.
+// kHwMul: its products on the FP64 pipe (k_force_bd, whose force part already fills the integer pipes, and
+// small models), or on the integer pipes.
+template <bool kHwMul = true>
 __device__ __forceinline__ D3 move_exact(D3 p, D3 v, double R) {
-    const double vp = __dadd_rn(__dadd_rn(__dmul_rn(v.x, p.x), __dmul_rn(v.y, p.y)), __dmul_rn(v.z, p.z));
-    const double pp = __dadd_rn(__dadd_rn(__dmul_rn(p.x, p.x), __dmul_rn(p.y, p.y)), __dmul_rn(p.z, p.z));
-    const double s = f64_div(vp, pp);
-    D3 q{__dadd_rn(p.x, __dsub_rn(v.x, __dmul_rn(s, p.x))), __dadd_rn(p.y, __dsub_rn(v.y, __dmul_rn(s, p.y))),
-         __dadd_rn(p.z, __dsub_rn(v.z, __dmul_rn(s, p.z)))};
-    const double qq = __dadd_rn(__dadd_rn(__dmul_rn(q.x, q.x), __dmul_rn(q.y, q.y)), __dmul_rn(q.z, q.z));
-    const double inv = f64_div_root(1.0, qq);
-    return D3{__dmul_rn(R, __dmul_rn(inv, q.x)), __dmul_rn(R, __dmul_rn(inv, q.y)), __dmul_rn(R, __dmul_rn(inv, q.z))};
+    const auto M = [](double x, double y) { return early_mul<kHwMul>(x, y); };
+    const double s = f64_div(dot3e<kHwMul>(v, p), dot3e<kHwMul>(p, p));
+    D3 q{__dadd_rn(p.x, __dsub_rn(v.x, M(s, p.x))), __dadd_rn(p.y, __dsub_rn(v.y, M(s, p.y))),
+         __dadd_rn(p.z, __dsub_rn(v.z, M(s, p.z)))};
+    const double inv = f64_div_root(1.0, dot3e<kHwMul>(q, q));
+    return D3{M(R, M(inv, q.x)), M(R, M(inv, q.y)), M(R, M(inv, q.z))};
 }
-
+// a projected onto the tangent plane at p and normalised (projectToTangentPlaneAndNormalize,
+// sphericalDomain.h:173-177), every product and sum rounded.
+template <bool kHwMul>
+__device__ __forceinline__ D3 tangent_unit(D3 a, D3 p) {
+    const auto M = [](double x, double y) { return early_mul<kHwMul>(x, y); };
+    const double s = f64_div(dot3e<kHwMul>(a, p), dot3e<kHwMul>(p, p));
+    a = D3{__dsub_rn(a.x, M(s, p.x)), __dsub_rn(a.y, M(s, p.y)), __dsub_rn(a.z, M(s, p.z))};
+    const double inv = f64_div_root(1.0, dot3e<kHwMul>(a, a));
+    return D3{M(inv, a.x), M(inv, a.y), M(inv, a.z)};
+}
 
 inline ForceArgs force_args(svm_model* m, int buf) {
     ForceArgs A;

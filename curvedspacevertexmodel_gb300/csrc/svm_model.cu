@@ -1888,6 +1888,11 @@ __global__ void k_dynamics(const double4_32a* __restrict__ ref, const PT* __rest
 // src/updaters/sphericalSelfPropelledParticle.cpp:16-47) on the vertex model's directors ----------
 // The displacement dt (v0 n + mu F) and the move, in place, every product and sum rounded as on the
 // CPU (the director n as the previous step left it).
+// These kernels and the Vicsek pair below are FP64-bound from a few thousand vertices on: products and the
+// projections' divisions go to the integer pipes (kHwMul: the products stay, for small models, few_hw_mul), and a
+// sine and a cosine of one angle are evaluated together.  20k cells, with blocks spread over the SMs: a Vicsek
+// step 158 -> 143 us (k_vicsek_target was 35 us of it, 75% of the pipe).
+template <bool kHwMul>
 __global__ void k_spp_move(double4_32a* __restrict__ pos, const double4_32a* __restrict__ dir,
                            const double4_32a* __restrict__ force, double dt, double mu, double v0, int nV, double R) {
     step_begin();
@@ -1897,14 +1902,14 @@ __global__ void k_spp_move(double4_32a* __restrict__ pos, const double4_32a* __r
     const D3 d{__dmul_rn(dt, __dadd_rn(__dmul_rn(v0, n.x), __dmul_rn(mu, f.x))),
                __dmul_rn(dt, __dadd_rn(__dmul_rn(v0, n.y), __dmul_rn(mu, f.y))),
                __dmul_rn(dt, __dadd_rn(__dmul_rn(v0, n.z), __dmul_rn(mu, f.z)))};
-    st3(pos, v, move_exact(ld3(pos, v), d, R));
+    st3(pos, v, move_exact<kHwMul>(ld3(pos, v), d, R));
 }
 // After the move and its T1 flips: each director projected onto the tangent plane at its vertex and
 // normalised (projectToTangentPlaneAndNormalize, sphericalDomain.h:173-177), then rotated about the
 // vertex's position vector, unnormalised as the reference passes it (rodriguesRotation,
 // inc/functions.h:175-181), by theta = r amp, amp = sqrt(2 dt tau) and r uniform in [-1/2, 1/2):
 // injected (r[v]) or from Philox counter word 3 of (vertex, step).
-template <int kNoise>
+template <int kNoise, bool kHwMul>
 __global__ void k_spp_dirs(const double4_32a* __restrict__ pos, double4_32a* __restrict__ dir,
                            const double* __restrict__ r, uint64_t seed,
                            const unsigned long long* __restrict__ stepCounter, double amp, int nV) {
@@ -1912,11 +1917,7 @@ __global__ void k_spp_dirs(const double4_32a* __restrict__ pos, double4_32a* __r
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nV) return;
     const D3 p = ld3(pos, v);
-    D3 n = ld3(dir, v);
-    const double s = __ddiv_rn(dot3(n, p), dot3(p, p));
-    n = D3{__dsub_rn(n.x, __dmul_rn(s, p.x)), __dsub_rn(n.y, __dmul_rn(s, p.y)), __dsub_rn(n.z, __dmul_rn(s, p.z))};
-    const double inv = f64_div(1.0, f64_sqrt(dot3(n, n)));
-    n = D3{__dmul_rn(inv, n.x), __dmul_rn(inv, n.y), __dmul_rn(inv, n.z)};
+    const D3 n = tangent_unit<kHwMul>(ld3(dir, v), p);
     double rv;
     if (kNoise == SVM_NOISE_BUFFER) {
         rv = r[v];
@@ -1927,12 +1928,14 @@ __global__ void k_spp_dirs(const double4_32a* __restrict__ pos, double4_32a* __r
         rv = u53(q.x, q.y) - 0.5;
     }
     const double theta = __dmul_rn(rv, amp);
-    const double c = cos(theta), sn = sin(theta);
-    const D3 cp = cross3(p, n);
-    const double w = __dmul_rn(1.0 - c, dot3(p, n));
-    st3(dir, v, D3{__dadd_rn(__dadd_rn(__dmul_rn(c, n.x), __dmul_rn(sn, cp.x)), __dmul_rn(w, p.x)),
-                   __dadd_rn(__dadd_rn(__dmul_rn(c, n.y), __dmul_rn(sn, cp.y)), __dmul_rn(w, p.y)),
-                   __dadd_rn(__dadd_rn(__dmul_rn(c, n.z), __dmul_rn(sn, cp.z)), __dmul_rn(w, p.z))});
+    double c, sn;
+    sincos(theta, &sn, &c);
+    const D3 cp = cross3e<kHwMul>(p, n);
+    const auto M = [](double x, double y) { return early_mul<kHwMul>(x, y); };
+    const double w = M(1.0 - c, dot3e<kHwMul>(p, n));
+    st3(dir, v, D3{__dadd_rn(__dadd_rn(M(c, n.x), M(sn, cp.x)), M(w, p.x)),
+                   __dadd_rn(__dadd_rn(M(c, n.y), M(sn, cp.y)), M(w, p.y)),
+                   __dadd_rn(__dadd_rn(M(c, n.z), M(sn, cp.z)), M(w, p.z))});
 }
 
 // ---- vectorial Vicsek alignment (sphericalVectorialVicsek::integrateEOMCPU,
@@ -1941,7 +1944,7 @@ __global__ void k_spp_dirs(const double4_32a* __restrict__ pos, double4_32a* __r
 // unit vector (u, w: phi = 2 pi u, theta = acos(2 w - 1)) projected onto the tangent plane at the
 // vertex and normalised; the target (n_v + the three vertex neighbours' n) / 4 + eta point,
 // projected and normalised.  u, w injected (r[2v], r[2v + 1]) or from Philox counter word 4.
-template <int kNoise>
+template <int kNoise, bool kHwMul>
 __global__ void k_vicsek_target(const double4_32a* __restrict__ pos, const double4_32a* __restrict__ dir,
                                 const int4* __restrict__ vnbr, double4_32a* __restrict__ target,
                                 const double* __restrict__ r, uint64_t seed,
@@ -1960,12 +1963,11 @@ __global__ void k_vicsek_target(const double4_32a* __restrict__ pos, const doubl
     }
     const D3 p = ld3(pos, v);
     const double phi = __dmul_rn(2.0 * 3.141592653589793, u), theta = acos(__dsub_rn(__dmul_rn(2.0, w), 1.0));
-    const double st = sin(theta);
-    D3 sp{__dmul_rn(st, cos(phi)), __dmul_rn(st, sin(phi)), cos(theta)};
-    const double ps = __ddiv_rn(dot3(sp, p), dot3(p, p));
-    sp = D3{__dsub_rn(sp.x, __dmul_rn(ps, p.x)), __dsub_rn(sp.y, __dmul_rn(ps, p.y)), __dsub_rn(sp.z, __dmul_rn(ps, p.z))};
-    const double is = f64_div(1.0, f64_sqrt(dot3(sp, sp)));
-    sp = D3{__dmul_rn(sp.x, is), __dmul_rn(sp.y, is), __dmul_rn(sp.z, is)};
+    const auto M = [](double x, double y) { return early_mul<kHwMul>(x, y); };
+    double st, ct, sf, cf;
+    sincos(theta, &st, &ct);
+    sincos(phi, &sf, &cf);
+    const D3 sp = tangent_unit<kHwMul>(D3{M(st, cf), M(st, sf), ct}, p);
     const int4 nb = vnbr[v];
     D3 t = ld3(dir, v);
     const int nbs[3] = {nb.x, nb.y, nb.z};
@@ -1974,14 +1976,11 @@ __global__ void k_vicsek_target(const double4_32a* __restrict__ pos, const doubl
         t = D3{__dadd_rn(t.x, o.x), __dadd_rn(t.y, o.y), __dadd_rn(t.z, o.z)};
     }
     const double mi = 1.0 / 4.0;  // self plus three neighbours
-    t = D3{__dadd_rn(__dmul_rn(t.x, mi), __dmul_rn(sp.x, eta)), __dadd_rn(__dmul_rn(t.y, mi), __dmul_rn(sp.y, eta)),
-           __dadd_rn(__dmul_rn(t.z, mi), __dmul_rn(sp.z, eta))};
-    const double ts = __ddiv_rn(dot3(t, p), dot3(p, p));
-    t = D3{__dsub_rn(t.x, __dmul_rn(ts, p.x)), __dsub_rn(t.y, __dmul_rn(ts, p.y)), __dsub_rn(t.z, __dmul_rn(ts, p.z))};
-    const double it = f64_div(1.0, f64_sqrt(dot3(t, t)));
-    st3(target, v, D3{__dmul_rn(t.x, it), __dmul_rn(t.y, it), __dmul_rn(t.z, it)});
+    t = D3{__dadd_rn(M(t.x, mi), M(sp.x, eta)), __dadd_rn(M(t.y, mi), M(sp.y, eta)), __dadd_rn(M(t.z, mi), M(sp.z, eta))};
+    st3(target, v, tangent_unit<kHwMul>(t, p));
 }
 // n += (dt / tau)(target - n), projected onto the tangent plane and normalised.
+template <bool kHwMul>
 __global__ void k_vicsek_update(const double4_32a* __restrict__ pos, double4_32a* __restrict__ dir,
                                 const double4_32a* __restrict__ target, double rate, int nV) {
     step_begin();
@@ -1989,12 +1988,10 @@ __global__ void k_vicsek_update(const double4_32a* __restrict__ pos, double4_32a
     if (v >= nV) return;
     const D3 p = ld3(pos, v), t = ld3(target, v);
     D3 n = ld3(dir, v);
-    n = D3{__dadd_rn(n.x, __dmul_rn(rate, __dsub_rn(t.x, n.x))), __dadd_rn(n.y, __dmul_rn(rate, __dsub_rn(t.y, n.y))),
-           __dadd_rn(n.z, __dmul_rn(rate, __dsub_rn(t.z, n.z)))};
-    const double s = __ddiv_rn(dot3(n, p), dot3(p, p));
-    n = D3{__dsub_rn(n.x, __dmul_rn(s, p.x)), __dsub_rn(n.y, __dmul_rn(s, p.y)), __dsub_rn(n.z, __dmul_rn(s, p.z))};
-    const double inv = f64_div(1.0, f64_sqrt(dot3(n, n)));
-    st3(dir, v, D3{__dmul_rn(n.x, inv), __dmul_rn(n.y, inv), __dmul_rn(n.z, inv)});
+    const auto M = [](double x, double y) { return early_mul<kHwMul>(x, y); };
+    n = D3{__dadd_rn(n.x, M(rate, __dsub_rn(t.x, n.x))), __dadd_rn(n.y, M(rate, __dsub_rn(t.y, n.y))),
+           __dadd_rn(n.z, M(rate, __dsub_rn(t.z, n.z)))};
+    st3(dir, v, tangent_unit<kHwMul>(n, p));
 }
 
 // ---- launch helpers --------------------------------------------------------------------------
@@ -3087,19 +3084,21 @@ int svm_spp_step(svm_model* m, double dt, double mu, double v0, double tau, int 
                                  m->stream));
     int rc = svm::launch_geometry(m);
     if (rc || (rc = svm::launch_force_fp64(m))) return rc;
-    launch_next(m, k_spp_move, svm::blocksFor(m->nVertices), svm::kBlock, m->pos[m->cur], m->dir, m->force, dt, mu,
-                                                                            v0, m->nVertices, m->R);
+    const int bs = svm::spread_block(m, m->nVertices), nb = svm::blocksFor(m->nVertices, bs);
+    const bool few = svm::few_hw_mul(m);
+    launch_next(m, few ? k_spp_move<true> : k_spp_move<false>, nb, bs, m->pos[m->cur], m->dir, m->force, dt, mu, v0,
+                m->nVertices, m->R);
     if (svm::check_launch()) return SVM_ERR_CUDA;
     m->cornersValid = false;
     // moveParticles: the T1 pass unless restricted, as in the Brownian step
     if ((rc = svm::launch_corners(m, !m->restricted)) || (rc = svm::launch_t1_apply(m, 1))) return rc;
     const double amp = sqrt(2.0 * dt * tau);
-    if (noiseMode == SVM_NOISE_BUFFER)
-        launch_next(m, k_spp_dirs<SVM_NOISE_BUFFER>, svm::blocksFor(m->nVertices), svm::kBlock,
-            m->pos[m->cur], m->dir, m->noiseBuf, seed, m->stepCounter, amp, m->nVertices);
-    else
-        launch_next(m, k_spp_dirs<SVM_NOISE_PHILOX>, svm::blocksFor(m->nVertices), svm::kBlock,
-            m->pos[m->cur], m->dir, nullptr, seed, m->stepCounter, amp, m->nVertices);
+    const auto go = [&](auto kernel) {
+        launch_next(m, kernel, nb, bs, m->pos[m->cur], m->dir, noiseMode == SVM_NOISE_BUFFER ? m->noiseBuf : nullptr, seed,
+                    m->stepCounter, amp, m->nVertices);
+    };
+    if (noiseMode == SVM_NOISE_BUFFER) go(few ? k_spp_dirs<SVM_NOISE_BUFFER, true> : k_spp_dirs<SVM_NOISE_BUFFER, false>);
+    else go(few ? k_spp_dirs<SVM_NOISE_PHILOX, true> : k_spp_dirs<SVM_NOISE_PHILOX, false>);
     return svm::check_launch();
 }
 
@@ -3113,20 +3112,24 @@ int svm_vicsek_step(svm_model* m, double dt, double mu, double v0, double eta, d
                                  m->stream));
     int rc = svm::launch_geometry(m);
     if (rc || (rc = svm::launch_force_fp64(m))) return rc;
-    launch_next(m, k_spp_move, svm::blocksFor(m->nVertices), svm::kBlock, m->pos[m->cur], m->dir, m->force, dt, mu,
-                                                                            v0, m->nVertices, m->R);
+    const int bs = svm::spread_block(m, m->nVertices), nb = svm::blocksFor(m->nVertices, bs);
+    const bool few = svm::few_hw_mul(m);
+    launch_next(m, few ? k_spp_move<true> : k_spp_move<false>, nb, bs, m->pos[m->cur], m->dir, m->force, dt, mu, v0,
+                m->nVertices, m->R);
     if (svm::check_launch()) return SVM_ERR_CUDA;
     m->cornersValid = false;
     if ((rc = svm::launch_corners(m, !m->restricted)) || (rc = svm::launch_t1_apply(m, 1))) return rc;
+    const auto go = [&](auto kernel) {
+        launch_next(m, kernel, nb, bs, m->pos[m->cur], m->dir, m->vnbr, m->dirTarget,
+                    noiseMode == SVM_NOISE_BUFFER ? m->noiseBuf : nullptr, seed, m->stepCounter, eta, m->nVertices);
+    };
     if (noiseMode == SVM_NOISE_BUFFER)
-        launch_next(m, k_vicsek_target<SVM_NOISE_BUFFER>, svm::blocksFor(m->nVertices), svm::kBlock,
-            m->pos[m->cur], m->dir, m->vnbr, m->dirTarget, m->noiseBuf, seed, m->stepCounter, eta, m->nVertices);
+        go(few ? k_vicsek_target<SVM_NOISE_BUFFER, true> : k_vicsek_target<SVM_NOISE_BUFFER, false>);
     else
-        launch_next(m, k_vicsek_target<SVM_NOISE_PHILOX>, svm::blocksFor(m->nVertices), svm::kBlock,
-            m->pos[m->cur], m->dir, m->vnbr, m->dirTarget, nullptr, seed, m->stepCounter, eta, m->nVertices);
+        go(few ? k_vicsek_target<SVM_NOISE_PHILOX, true> : k_vicsek_target<SVM_NOISE_PHILOX, false>);
     if (svm::check_launch()) return SVM_ERR_CUDA;
-    launch_next(m, k_vicsek_update, svm::blocksFor(m->nVertices), svm::kBlock, m->pos[m->cur], m->dir, m->dirTarget,
-                                                                                 dt / tau, m->nVertices);
+    launch_next(m, few ? k_vicsek_update<true> : k_vicsek_update<false>, nb, bs, m->pos[m->cur], m->dir, m->dirTarget, dt / tau,
+                m->nVertices);
     return svm::check_launch();
 }
 
