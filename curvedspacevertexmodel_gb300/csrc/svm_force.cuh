@@ -23,14 +23,13 @@ struct ForceArgs {
     const double2* ap;
     const double2* pref;
     double Kr, R;
-    int vec;   // SVM_PRECISION_FP64_VECTOR: the exact gradient as vectors (grad_geo_vec, grad_tri_vec)
 };
 
 __device__ __forceinline__ int comp(const int4& a, int s) { return s == 0 ? a.x : (s == 1 ? a.y : a.z); }
 
-// The force form of a kernel: chosen per launch from A.vec (kFormAny), or fixed at compile time, which
-// lets a kernel that runs one form drop the other's registers.
-constexpr int kFormAny = 0, kFormVector = 1, kFormReference = 2;
+// The force form of a kernel (the closed forms of the reference, or SVM_PRECISION_FP64_VECTOR's exact gradient as
+// vectors: grad_geo_vec, grad_tri_vec), fixed at compile time, which lets each drop the other's registers.
+constexpr int kFormVector = 1, kFormReference = 2;
 
 // Block-level force of kVerts vertices by six threads a vertex: thread (role, vi, s) with s one of the
 // vertex's three cell slots and a role per triangle of the slot's fan.  Role 0 holds the slot's ring
@@ -159,7 +158,7 @@ __device__ __forceinline__ void slot_forces_reference(const ForceArgs& A, int nV
     __syncthreads();
 }
 
-// The vector form (A.vec: the exact gradient as vectors, well conditioned where the reference's closed
+// The vector form (the exact gradient as vectors, well conditioned where the reference's closed
 // forms lose digits -- short edges, thin fan triangles), the same way.  Products and sums contract to
 // multiply-adds here: the form's values are pinned to its formulas, not to the CPU's sequence of
 // roundings.  The products that are not part of a multiply-add run on the integer pipes, which the form
@@ -266,7 +265,7 @@ __device__ __forceinline__ void slot_forces_vector(const ForceArgs& A, int nV, S
 // three cells does.
 template <int kForm, bool kHwMul, int kVerts, class Side>
 __device__ __forceinline__ D3 block_slot_force(const ForceArgs& A, int nV, SlotShared<kVerts>& sh, Side side) {
-    if (kForm == kFormVector || (kForm == kFormAny && A.vec)) slot_forces_vector<kHwMul>(A, nV, sh, side);
+    if (kForm == kFormVector) slot_forces_vector<kHwMul>(A, nV, sh, side);
     else slot_forces_reference<kHwMul>(A, nV, sh, side);
     const int t = threadIdx.x;
     D3 f{0.0, 0.0, 0.0};
@@ -390,7 +389,6 @@ inline ForceArgs force_args(svm_model* m, int buf) {
     ForceArgs A;
     A.pos = m->pos[buf]; A.vsph = m->vsph; A.vcell = m->vcell; A.vlast = m->vlast; A.vnext = m->vnext;
     A.cellPos = m->cellPos; A.cellSph = m->cellSph; A.ap = m->ap; A.pref = m->pref; A.Kr = m->Kr; A.R = m->R;
-    A.vec = m->precision == SVM_PRECISION_FP64_VECTOR ? 1 : 0;
     return A;
 }
 }  // namespace svm

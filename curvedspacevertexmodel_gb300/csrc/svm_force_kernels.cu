@@ -5,6 +5,7 @@
 // rounding then differs from the CPU's only through acos), and the displacement and the move spell
 // out every product and sum with __dmul_rn / __dadd_rn.
 #include <mutex>
+#include <type_traits>
 
 #include "svm_force.cuh"
 
@@ -37,12 +38,15 @@ __global__ void k_zig_init() {
 namespace {
 using namespace svm;
 
-template <bool kHwMul>
-__global__ void __launch_bounds__(slot_threads(kSlotVerts), kSlotMinBlocks)
+// One instantiation per form (one that held both spilled more: 100k cells 231 -> 227 us, 200 cells 18 -> 17).
+constexpr int form_min_blocks(int form) { return form == kFormVector ? 6 : kSlotMinBlocks; }
+
+template <int kForm, bool kHwMul>
+__global__ void __launch_bounds__(slot_threads(kSlotVerts), form_min_blocks(kForm))
     k_force(ForceArgs A, int nV, double4_32a* __restrict__ force) {
     step_begin();
     __shared__ SlotShared<> sh;
-    const D3 f = block_slot_force<kFormAny, kHwMul>(A, nV, sh, NoSide());
+    const D3 f = block_slot_force<kForm, kHwMul>(A, nV, sh, NoSide());
     const int v = blockIdx.x * kSlotVerts + threadIdx.x;
     if (threadIdx.x >= kSlotVerts || v >= nV) return;
     st3(force, v, f);
@@ -53,15 +57,15 @@ __global__ void __launch_bounds__(slot_threads(kSlotVerts), kSlotMinBlocks)
 // edge gradients.
 // (Writing the moved vertex's norm here as well, which would spare the corner pass its k_vnorm, made
 // this FP64-bound kernel as much slower as the corner pass got faster.)
-template <int kNoise, bool kHwMul>
-__global__ void __launch_bounds__(slot_threads(kSlotVerts), kSlotMinBlocks)
+template <int kNoise, int kForm, bool kHwMul>
+__global__ void __launch_bounds__(slot_threads(kSlotVerts), form_min_blocks(kForm))
     k_force_bd(ForceArgs A, int nV, double4_32a* __restrict__ force, double4_32a* __restrict__ posNext,
                const double* __restrict__ noise, uint64_t seed, const unsigned long long* __restrict__ stepCounter,
                double np, double fp, const ZigTable* __restrict__ zig, double* __restrict__ hostOut) {
     step_begin();
     __shared__ SlotShared<> sh;
     __shared__ double xi[3 * kSlotVerts];
-    const D3 f = block_slot_force<kFormAny, kHwMul>(A, nV, sh, [&](const SlotIndex& q) {
+    const D3 f = block_slot_force<kForm, kHwMul>(A, nV, sh, [&](const SlotIndex& q) {
         xi[q.at] = kNoise == SVM_NOISE_BUFFER ? noise[3 * q.v + q.s] : philox_normal(zig, seed, *stepCounter, q.v, q.s);
     });
     const int t = threadIdx.x, v = blockIdx.x * kSlotVerts + t;
@@ -80,9 +84,25 @@ int slot_blocks(int nV) { return (nV + kSlotVerts - 1) / kSlotVerts; }
 
 namespace svm {
 
+// f(form, hwMul) with the two as compile-time constants
+template <class F>
+static void with_form(const svm_model* m, F f) {
+    using T = std::true_type;
+    using N = std::false_type;
+    if (m->precision == SVM_PRECISION_FP64_VECTOR) {
+        using V = std::integral_constant<int, kFormVector>;
+        few_hw_mul(m) ? f(V(), T()) : f(V(), N());
+    } else {
+        using R = std::integral_constant<int, kFormReference>;
+        few_hw_mul(m) ? f(R(), T()) : f(R(), N());
+    }
+}
+
 int launch_force_fp64(svm_model* m) {
-    launch_next(m, few_hw_mul(m) ? k_force<true> : k_force<false>, slot_blocks(m->nVertices), slot_threads(kSlotVerts),
-                force_args(m, m->cur), m->nVertices, m->force);
+    with_form(m, [&](auto form, auto hw) {
+        launch_next(m, k_force<form.value, hw.value>, slot_blocks(m->nVertices), slot_threads(kSlotVerts),
+                    force_args(m, m->cur), m->nVertices, m->force);
+    });
     return check_launch();
 }
 
@@ -112,9 +132,10 @@ int launch_force_bd_fp64(svm_model* m, double np, double fp, int noiseMode, cons
             force_args(m, m->cur), m->nVertices, m->force, m->pos[nxt], noise, seed, m->stepCounter, np, fp, zig,
             m->ioHostOut);
     };
-    const bool few = few_hw_mul(m);
-    if (noiseMode == SVM_NOISE_BUFFER) go(few ? k_force_bd<SVM_NOISE_BUFFER, true> : k_force_bd<SVM_NOISE_BUFFER, false>);
-    else go(few ? k_force_bd<SVM_NOISE_PHILOX, true> : k_force_bd<SVM_NOISE_PHILOX, false>);
+    with_form(m, [&](auto form, auto hw) {
+        if (noiseMode == SVM_NOISE_BUFFER) go(k_force_bd<SVM_NOISE_BUFFER, form.value, hw.value>);
+        else go(k_force_bd<SVM_NOISE_PHILOX, form.value, hw.value>);
+    });
     return check_launch();
 }
 
