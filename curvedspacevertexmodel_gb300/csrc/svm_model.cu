@@ -202,6 +202,7 @@ __device__ __forceinline__ bool edge_terms(int v, int j, int u, const int4* __re
 // and gather.  Corner pass, three kernels against this one: 200 cells 21.4 -> 13.0 us, 5k 39.7 -> 16.4,
 // 15k 41 -> 27, 30k 47.6 -> 43.5, 50k 67 -> 66, 100k 125 -> 123 (but less of the FP64 pipe with three: other
 // models running beside it get more done), 300k 317 -> 346: models from 50,000 vertices on keep the three.
+constexpr int kEdgeThreads = 128;                 // k_vnorm, k_edges
 constexpr int kFewVerts = 32;                     // vertices per block: four whole warps
 constexpr int kFewCornersBelow = 50000;          // vertices
 template <bool kHwMul>
@@ -264,56 +265,57 @@ __global__ void __launch_bounds__(4 * kFewVerts) k_corners_few(
 
 // Per vertex: for each of its three cells, the arc from the ring predecessor and the included
 // angle at the vertex (the per-corner terms of computeGeometryCPU, sphericalVertexModel.cpp:257-276)
-// from the edge terms of k_edges.  Compiled for six blocks of 128 per SM (80 registers, with some
-// spill).
-constexpr int kCornerThreads = 128;
-__global__ void __launch_bounds__(kCornerThreads, 6) k_corner(const double4_32a* __restrict__ pos, const int4* __restrict__ vcell,
+// from the edge terms of k_edges.  Three threads a vertex, as in the mixed form's pass: thread (v, j) fetches the
+// edge to neighbour j for the block, then evaluates the corner of cell slot j.  FP64-bound; the corner phase with
+// one thread a vertex (80 registers with some spill, 24 warps an SM) against this at 42 warps: 100k cells 101.1 ->
+// 99.0 us, 300k 249.5 -> 245.3 (six blocks an SM 101.3 and 251.7, eight 99.0 and 245.5).
+constexpr int kCornerThreads = 192, kCornerVerts = kCornerThreads / 3;
+__global__ void __launch_bounds__(kCornerThreads, 7) k_corner(const double4_32a* __restrict__ pos, const int4* __restrict__ vcell,
                          const int4* __restrict__ vlast, const int4* __restrict__ vnext, const int4* __restrict__ vrpos,
                          const int4* __restrict__ vnbr, const double4_32a* __restrict__ edgeC,
                          const double* __restrict__ edgeArc, double2* __restrict__ corner, int Wc, int nV, double R) {
     step_begin();
-    __shared__ double val[3 * kCornerThreads];
-    __shared__ unsigned short src[3 * kCornerThreads];
+    __shared__ double cx[kCornerThreads], cy[kCornerThreads], cz[kCornerThreads], nc[kCornerThreads], arcs[kCornerThreads];
+    __shared__ double val[kCornerThreads];
+    __shared__ unsigned short src[kCornerThreads];
     __shared__ int warpHigh[kCornerThreads / 32];
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = v < nV;
-    double cosine[3] = {-1.0, -1.0, -1.0}, arcs[3];
-    bool flip[3] = {false, false, false}, ok = true;
+    const int t = threadIdx.x, vi = t / 3, j = t - 3 * vi, v = blockIdx.x * kCornerVerts + vi;
+    const bool live = vi < kCornerVerts && v < nV;
+    int4 nb;
+    bool have = false;
+    if (live) {
+        nb = vnbr[v];
+        D3 C;
+        double nC, arc;
+        have = edge_terms(v, j, comp(nb, j), vnbr, edgeC, edgeArc, C, nC, arc);
+        cx[t] = C.x; cy[t] = C.y; cz[t] = C.z; nc[t] = nC;
+        arcs[t] = have ? arc : -1.0;   // (an arc is not negative, and a NaN not below zero)
+    }
+    __syncthreads();
+    double cosine[1] = {-1.0}, arc = 0.0;
+    bool flip = false, ok = false;
     int4 cells, lasts, nexts;
     if (live) {
-        const int4 nb = vnbr[v];
         cells = vcell[v]; lasts = vlast[v]; nexts = vnext[v];
-        D3 C[3], U[3];
-        double nC[3], arc[3];
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            const int u = comp(nb, j);
-            U[j] = ld3(pos, u);
-            ok &= edge_terms(v, j, u, vnbr, edgeC, edgeArc, C[j], nC[j], arc[j]);
-        }
-#pragma unroll
-        for (int s = 0; s < 3; ++s) {
-            const int jl = nbr_slot(nb, comp(lasts, s)), jx = nbr_slot(nb, comp(nexts, s));
-            ok &= jl >= 0 && jx >= 0;
-            if (ok) {
-                arcs[s] = pick3(arc, jl);
-                flip[s] = positive(dot3e(pick3(U, jl), pick3(C, jx)));
-                cosine[s] = included_cos(pick3(C, jx), pick3(C, jl), pick3(nC, jx), pick3(nC, jl));
-            }
+        const int last = comp(lasts, j), jl = nbr_slot(nb, last), jx = nbr_slot(nb, comp(nexts, j)), b = 3 * vi;
+        ok = jl >= 0 && jx >= 0 && !(arcs[b] < 0.0) && !(arcs[b + 1] < 0.0) && !(arcs[b + 2] < 0.0);
+        if (ok) {
+            const int l = b + jl, x = b + jx;
+            const D3 X{cx[x], cy[x], cz[x]};
+            arc = arcs[l];
+            flip = positive(dot3e(ld3(pos, last), X));
+            cosine[0] = included_cos(X, D3{cx[l], cy[l], cz[l]}, nc[x], nc[l]);
         }
     }
     block_acos(cosine, val, src, warpHigh);
     if (!live) return;
     const int4 rp = vrpos[v];
-#pragma unroll
-    for (int s = 0; s < 3; ++s) {
-        double2 cr = make_double2(arcs[s], included_finish(cosine[s], flip[s]));
-        if (!ok) {  // inconsistent lists: evaluate directly
-            const D3 p = ld3(pos, v), pl = ld3(pos, comp(lasts, s)), px = ld3(pos, comp(nexts, s));
-            cr = make_double2(geodesic(pl, p, R), included_angle(pl, p, px));
-        }
-        corner[(long)comp(cells, s) * Wc + comp(rp, s)] = cr;
+    double2 cr = make_double2(arc, included_finish(cosine[0], flip));
+    if (!ok) {  // inconsistent lists: evaluate directly
+        const D3 p = ld3(pos, v), pl = ld3(pos, comp(lasts, j)), px = ld3(pos, comp(nexts, j));
+        cr = make_double2(geodesic(pl, p, R), included_angle(pl, p, px));
     }
+    corner[(long)comp(cells, j) * Wc + comp(rp, j)] = cr;
 }
 
 // (n - 2) kPI and (n - 2) kPILo for rings of n entries up to kRingTable: the products as the reference
@@ -2027,12 +2029,12 @@ int launch_corners(svm_model* m, bool t1test, bool vnormReady) {
         return check_launch();
     }
     // (blocks of 256 leave the last wave short: 100k cells 133.7 against 124.7 us, 300k 322.6 against 317.4)
-    const int bv = std::min(kCornerThreads, spread_block(m, m->nVertices));
+    const int bv = std::min(kEdgeThreads, spread_block(m, m->nVertices));
     if (!vnormReady) launch_next(m, k_vnorm, blocksFor(m->nVertices, bv), bv, m->pos[m->cur], m->vnorm, m->nVertices);
     launch_next(m, k_edges, blocksFor(m->nVertices, bv), bv, m->pos[m->cur], m->vnorm, m->vsph, m->vnbr, m->vcell, m->edgeC,
                                                               m->edgeArc, m->nVertices, m->R, t1test ? 1 : 0,
                                                               m->t1Threshold, m->t1);
-    launch_next(m, k_corner, blocksFor(m->nVertices, bv), bv, m->pos[m->cur], m->vcell, m->vlast, m->vnext,
+    launch_next(m, k_corner, blocksFor(m->nVertices, kCornerVerts), kCornerThreads, m->pos[m->cur], m->vcell, m->vlast, m->vnext,
                 m->vrpos, m->vnbr, m->edgeC, m->edgeArc, m->corner, m->Wc, m->nVertices, m->R);
     m->cornersValid = true;
     return check_launch();
