@@ -147,10 +147,11 @@ __device__ __forceinline__ double det3(D3 a, D3 b, D3 c) {    // a . (b x c), sp
 }
 
 // putInBoxReal (sphericalDomain.h:183-187): p <- R p / |p|
-template <bool kHwMul = false>
+template <bool kHwMul = false, bool kHwScale = true>
 __device__ __forceinline__ D3 renorm(D3 p, double R) {
-    double inv = f64_div_root(1.0, dot3e<kHwMul>(p, p));
-    return scl3(R, scl3(inv, p));
+    const auto M = [](double x, double y) { return early_mul<kHwScale>(x, y); };
+    const double inv = f64_div_root(1.0, dot3e<kHwMul>(p, p));
+    return D3{M(R, M(inv, p.x)), M(R, M(inv, p.y)), M(R, M(inv, p.z))};
 }
 // move(p, v) (sphericalDomain.h:203-209): project v onto the tangent plane at p, add, renormalise
 __device__ __forceinline__ D3 sphere_move(D3 p, D3 v, double R) {

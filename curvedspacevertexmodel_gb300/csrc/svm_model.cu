@@ -334,16 +334,41 @@ __constant__ PolygonAngles kPolygon = polygon_angles();
 __device__ __forceinline__ double polygon_pi(int n) { return n <= kRingTable ? kPolygon.pi[n] : __dmul_rn((double)(n - 2), kPI); }
 __device__ __forceinline__ double polygon_lo(int n) { return n <= kRingTable ? kPolygon.lo[n] : __dmul_rn((double)(n - 2), kPILo); }
 
+// Exact sums of FP32 values on the integer pipes: f as a multiple of 2^(c - 150), in 64 bits.  `worst` collects
+// the shifts as unsigned numbers; the sum is exact if it stays at or below kFixedShift (a value too small for
+// the unit, zero, or too large, an infinity or NaN raises it).
+constexpr unsigned kFixedShift = 30;
+constexpr int kFixedRing = 64;   // |f| < 2^24 2^30 units: sums of 64 stay below 2^60
+__device__ __forceinline__ long long fixed32(int sign, int exponent, int m, int c, unsigned& worst) {
+    const int sh = exponent - c;
+    worst = max(worst, (unsigned)sh);
+    return (long long)(sign < 0 ? -m : m) * (int)(1u << (sh & 31));
+}
+__device__ __forceinline__ long long fixed32(float f, int c, unsigned& worst) {
+    const int b = __float_as_int(f);
+    return fixed32(b, (b >> 23) & 0xff, (b & 0x7fffff) | 0x800000, c, worst);
+}
+// ... of a double that holds an FP32 value (normal as one: the exponent is its own, rebased by the caller's c)
+__device__ __forceinline__ long long fixed32(double f, int c, unsigned& worst) {
+    const int h = __double2hiint(f);
+    return fixed32(h, (h >> 20) & 0x7ff, ((h & 0xfffff) << 3 | 0x800000) | (int)((unsigned)__double2loint(f) >> 29), c, worst);
+}
+
 // Per cell: centroid (sum of ring vertices in ring order, renormalised), perimeter and angle sum
 // in the CPU's order (ring positions n-2, n-1, 0, ..., n-3), area = (sum - (n-2) pi) wrapped
 // by floor(area / pi), times R^2 (sphericalVertexModel.cpp:228-303).  The last block to finish
 // totals the areas and raises the fallback flag when |sum A - 4 pi R^2| > 1e-6 (304-310; mixed form:
 // mixed_area_limit).
 //
+// FP32 positions, one thread a cell: the centroid and the perimeter are sums of FP32 values, whose FP64 sums
+// are exact but for values some 2^26 below the largest; they are summed in fixed point on the integer pipes
+// where that is exact (fixed32), else in FP64 as before: the same bits, without the widenings and with five of
+// eleven FP64 additions a corner gone.  1M cells 205 -> 111 us, 100k 31.8 -> 21.3, 512 replicas 140 -> 75.
+//
 // kSplit: two threads a cell, in the two halves of the block: the centroid, and the area and perimeter.
 // A cell's chain -- count, ring, positions or corners, sums, roots and divisions -- is latency at small N,
-// and the halves run theirs side by side (200 cells 16.8 -> 11.7 us; 100k cells 31 -> 33, FP32 positions at
-// 1M 212 -> 239: large models and batches keep one thread a cell).
+// and the halves run theirs side by side (200 cells 16.8 -> 11.7 us; 100k cells 31 -> 33: large models and
+// batches keep one thread a cell).
 //
 // Replicas (mixed form, repR non-null): the radius is the replica's, read through the first ring
 // vertex; with `ticket` null the area check is left to k_rep_check (per replica).
@@ -366,6 +391,8 @@ __global__ void k_cells(const PT* __restrict__ pos, const int* __restrict__ ring
         const double R = repR ? repR[rep_of(pos[rg[0]])] : R0;
         // split: the first kAhead ring entries' loads are all issued before their sums, which run in ring order
         constexpr int kAhead = kSplit ? 8 : 0;
+        constexpr bool kFixed = !kSplit && std::is_same<PT, float4>::value;
+        constexpr int kArcUnit = 1023 + 23 - 50;   // the perimeter in units of 2^-50: arcs in [2^-27, 16)
         if (!second) {
             D3 cp{0.0, 0.0, 0.0};
             if (kSplit) {
@@ -378,8 +405,26 @@ __global__ void k_cells(const PT* __restrict__ pos, const int* __restrict__ ring
 #pragma unroll
                 for (int k = 0; k < kAhead; ++k) if (k < n) cp = add3(cp, q[k]);
             }
-            for (int k = kAhead; k < n; ++k) cp = add3(cp, ld3(pos, rg[k]));
-            cp = renorm<kSplit>(cp, R);
+            bool summed = false;
+            if constexpr (kFixed) {
+                const int c0 = 98 - 1023 + ((__double2hiint(R) >> 20) & 0x7ff);   // |f| <= R: a shift of 30 at most
+                long long x = 0, y = 0, z = 0;
+                unsigned worst = n > kFixedRing ? kFixedShift + 1 : 0;
+                for (int k = 0; k < n; ++k) {
+                    const PT q = pos[rg[k]];
+                    x += fixed32(q.x, c0, worst);
+                    y += fixed32(q.y, c0, worst);
+                    z += fixed32(q.z, c0, worst);
+                }
+                // (in units of a power of two, which renorm takes out exactly)
+                if (worst <= kFixedShift) {
+                    cp = D3{__ll2double_rn(x), __ll2double_rn(y), __ll2double_rn(z)};
+                    summed = true;
+                }
+            }
+            if (!summed)
+                for (int k = kAhead; k < n; ++k) cp = add3(cp, ld3(pos, rg[k]));
+            cp = renorm<kSplit, kSplit || kFixed>(cp, R);
             st3(cellPos, c, cp);
             if (cellSph) cellSph[c] = sph_coords<false, kSplit>(cp);
         }
@@ -397,10 +442,23 @@ __global__ void k_cells(const PT* __restrict__ pos, const int* __restrict__ ring
                         ang += q[t].y;
                     }
             }
-            for (int t = kAhead; t < n; ++t) {
-                const double2 x = cr[t < 2 ? n - 2 + t : t - 2];
-                per += x.x;
-                ang += x.y;
+            if constexpr (kFixed) {
+                long long p = 0;
+                unsigned worst = n > kFixedRing ? kFixedShift + 1 : 0;
+                for (int t = 0; t < n; ++t) {
+                    const double2 x = cr[t < 2 ? n - 2 + t : t - 2];
+                    p += fixed32(x.x, kArcUnit, worst);
+                    ang += x.y;
+                }
+                if (worst <= kFixedShift) per = __dmul_rn(__ll2double_rn(p), 0x1p-50);
+                else
+                    for (int t = 0; t < n; ++t) per += cr[t < 2 ? n - 2 + t : t - 2].x;
+            } else {
+                for (int t = kAhead; t < n; ++t) {
+                    const double2 x = cr[t < 2 ? n - 2 + t : t - 2];
+                    per += x.x;
+                    ang += x.y;
+                }
             }
             area = __dsub_rn(ang, polygon_pi(n));
             // The mixed form also subtracts (n - 2) times the part of pi below the double kPI: the
