@@ -90,12 +90,13 @@ __device__ __forceinline__ void put3(double (*a)[3 * kVerts], int k, D3 p) { a[0
 template <int kVerts>
 __device__ __forceinline__ D3 get3(const double (*a)[3 * kVerts], int k) { return D3{a[0][k], a[1][k], a[2][k]}; }
 
+static __device__ __noinline__ bool det_negative_exact(D3 p, D3 a, D3 b) { return det3(p, a, b) < 0; }
 // det(p, a, b) < 0: in FP32 where that is certain (all but nearly flat triangles).
 __device__ __forceinline__ bool det_negative(D3 p, D3 a, D3 b) {
     const svm_det::F3 v32 = svm_det::near3(p.x, p.y, p.z);
     const int n = svm_det::below_zero(v32, svm_det::diff(svm_det::near3(a.x, a.y, a.z), v32),
                                       svm_det::diff(svm_det::near3(b.x, b.y, b.z), v32));
-    return n >= 0 ? n != 0 : det3(p, a, b) < 0;
+    return n >= 0 ? n != 0 : det_negative_exact(p, a, b);
 }
 
 // The slot forces of the reference form, left in sh.g for the block: per slot
@@ -146,7 +147,8 @@ __device__ __forceinline__ void slot_forces_reference(const ForceArgs& A, int nV
         }
         double2 g = grad_triangle<kHwMul>(own, other, pair_cos<kHwMul>(s2, s3), s2.y, s3.y, A.R);
         const D3 p = ld3(A.pos, q.v), cp = ld3(A.cellPos, q.c), pn = ld3(A.pos, role0 ? q.L : q.X);
-        if (det_negative(p, role0 ? pn : cp, role0 ? cp : pn)) g = make_double2(-g.x, -g.y);
+        const bool negative = det_negative(p, role0 ? pn : cp, role0 ? cp : pn);
+        g = make_double2(sf::negate_if(negative, g.x), sf::negate_if(negative, g.y));
         const D3 t = scl3(aa, from_basis(sv, g));
         if (role0) fs = sub3(fs, t);
         else put3<kVerts>(sh.t, q.at, t);
@@ -332,17 +334,17 @@ static __device__ __noinline__ double zig_slow(const ZigTable* __restrict__ Z, i
         // y < exp(-x^2 / 2) in FP32 where that is certain: the FP32 exponential is within 2e-6 of it
         const float xf = svm_det::near32(x), yf = svm_det::near32(y), ef = expf(-0.5f * xf * xf);
         const bool under = fabsf(yf - ef) > 2e-5f * ef ? yf < ef : y < exp(-0.5 * x * x);
-        if (under) return neg ? -x : x;
+        if (under) return sf::negate_if(neg, x);
         x = zig_draw(Z, r.z, r.w, i, neg);
-        if (x < __ldg(Z->x + i + 1)) return neg ? -x : x;
+        if (x < __ldg(Z->x + i + 1)) return sf::negate_if(neg, x);
     }
-    return neg ? -x : x;
+    return sf::negate_if(neg, x);
 }
 __device__ __forceinline__ double zig_normal(const ZigTable* __restrict__ Z, unsigned a, unsigned b, uint4 ctr, uint2 key) {
     int i;
     bool neg;
     const double x = zig_draw(Z, a, b, i, neg);
-    if (x < __ldg(Z->x + i + 1)) return neg ? -x : x;
+    if (x < __ldg(Z->x + i + 1)) return sf::negate_if(neg, x);
     return zig_slow(Z, i, x, neg, ctr, key);
 }
 // Component k of the three standard normals for (vertex, step): two Philox draws (counter words 0 and 1)

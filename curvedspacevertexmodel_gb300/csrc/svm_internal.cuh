@@ -267,7 +267,7 @@ __device__ __forceinline__ double included_cos(D3 Cx, D3 Cl, double nx, double n
 }
 // the angle from its arccosine a (in [0, pi], or NaN) and whether det(pl, p, px) > 0: a, or 2 pi - a
 __device__ __forceinline__ double included_finish(double a, bool detPositive) {
-    if (detPositive) a = positive(a) ? 2. * kPI - a : -a;
+    if (detPositive) a = positive(a) ? 2. * kPI - a : sf::negate_if(true, a);
     return a;
 }
 template <bool clamp = false>
@@ -480,8 +480,8 @@ __device__ __forceinline__ double2 grad_triangle(const PairTerms& p12, const Pai
 // (theta, phi) components to Cartesian with the basis of sphericalDomain.h:218-232:
 // thetaHat = (cos t cos p, cos t sin p, -sin t), phiHat = (-sin p, cos p, 0).
 __device__ __forceinline__ D3 from_basis(double4_32a s, double2 g) {
-    double z = g.x * (-s.y);   // + g.y * 0, which changes it only for an infinite or NaN g.y
-    if ((((unsigned)__double2hiint(g.y) >> 20) & 0x7ffu) == 0x7ffu) z += g.y * 0;
+    double z = g.x * (-s.y);   // + g.y * 0, which changes it only for an infinite or NaN g.y: to NaN
+    if ((((unsigned)__double2hiint(g.y) >> 20) & 0x7ffu) == 0x7ffu) z = __hiloint2double(0x7fffffff, -1);
     return D3{g.x * (s.x * s.z) + g.y * (-s.w), g.x * (s.x * s.w) + g.y * s.z, z};
 }
 

@@ -188,7 +188,7 @@ __device__ __forceinline__ bool edge_terms(int v, int j, int u, const int4* __re
         neg = true;
     }
     const double4_32a q = edgeC[e];
-    C = neg ? D3{-q.x, -q.y, -q.z} : D3{q.x, q.y, q.z};
+    C = D3{sf::negate_if(neg, q.x), sf::negate_if(neg, q.y), sf::negate_if(neg, q.z)};
     nC = q.w;
     arc = edgeArc[e];
     return true;

@@ -178,7 +178,7 @@ SF_SLOW double hw_mul(double a, double b) {
     return r;
 #endif
 }
-SF_HD double hw_add(double a, double b) {
+SF_SLOW double hw_add(double a, double b) {
 #if defined(__CUDA_ARCH__)
     return __dadd_rn(a, b);
 #else
@@ -237,6 +237,16 @@ SF_HD double mul(double a, double b) {
 
 // mul out of line, for kernels with dozens of products, whose code would not fit the instruction caches.
 SF_SLOW double mul_call(double a, double b) { return mul(a, b); }
+
+// -x and, if c, -x: a bit flip (the hardware's negation, where it is not an operand's modifier, is an
+// addition).
+SF_HD double negate_if(bool c, double x) {
+#if defined(__CUDA_ARCH__)
+    return __hiloint2double(__double2hiint(x) ^ (c ? (int)0x80000000u : 0), __double2loint(x));
+#else
+    return c ? -x : x;
+#endif
+}
 
 // 2 x (exact; zeros, subnormals, the largest binade, infinities and NaN take the hardware)
 SF_HD double twice(double x) {
@@ -394,7 +404,9 @@ SF_HD Divisor sqrt_divisor(double a) {
 // hardware conversion.
 SF_HD unsigned f32bits(float f) { return u32_of(f); }
 SF_HD float f32of(unsigned u) { return f32_of(u); }
-SF_HD double hw_widen(float f) {
+// (Out of line, as all fallbacks here: an inlined conversion or addition is evaluated on every call, beside
+// the fast path, and selected from.)
+SF_SLOW double hw_widen(float f) {
 #if defined(__CUDA_ARCH__)
     return (double)f;
 #else
@@ -402,7 +414,7 @@ SF_HD double hw_widen(float f) {
     return r;
 #endif
 }
-SF_HD float hw_narrow(double d) {
+SF_SLOW float hw_narrow(double d) {
 #if defined(__CUDA_ARCH__)
     return __double2float_rn(d);
 #else
