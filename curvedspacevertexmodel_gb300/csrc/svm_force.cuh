@@ -370,10 +370,10 @@ __device__ __forceinline__ double bd_disp(double xi, double np, double f, double
 template <bool kHwMul = true>
 __device__ __forceinline__ D3 move_exact(D3 p, D3 v, double R) {
     const auto M = [](double x, double y) { return early_mul<kHwMul>(x, y); };
-    const double s = f64_div(dot3e<kHwMul>(v, p), dot3e<kHwMul>(p, p));
+    const double s = f64_div(dot3e<kHwMul>(v, p), norm2e<kHwMul>(p));
     D3 q{__dadd_rn(p.x, __dsub_rn(v.x, M(s, p.x))), __dadd_rn(p.y, __dsub_rn(v.y, M(s, p.y))),
          __dadd_rn(p.z, __dsub_rn(v.z, M(s, p.z)))};
-    const double inv = f64_div_root(1.0, dot3e<kHwMul>(q, q));
+    const double inv = f64_div_root(1.0, norm2e<kHwMul>(q));
     return D3{M(R, M(inv, q.x)), M(R, M(inv, q.y)), M(R, M(inv, q.z))};
 }
 // a projected onto the tangent plane at p and normalised (projectToTangentPlaneAndNormalize,
@@ -381,9 +381,9 @@ __device__ __forceinline__ D3 move_exact(D3 p, D3 v, double R) {
 template <bool kHwMul>
 __device__ __forceinline__ D3 tangent_unit(D3 a, D3 p) {
     const auto M = [](double x, double y) { return early_mul<kHwMul>(x, y); };
-    const double s = f64_div(dot3e<kHwMul>(a, p), dot3e<kHwMul>(p, p));
+    const double s = f64_div(dot3e<kHwMul>(a, p), norm2e<kHwMul>(p));
     a = D3{__dsub_rn(a.x, M(s, p.x)), __dsub_rn(a.y, M(s, p.y)), __dsub_rn(a.z, M(s, p.z))};
-    const double inv = f64_div_root(1.0, dot3e<kHwMul>(a, a));
+    const double inv = f64_div_root(1.0, norm2e<kHwMul>(a));
     return D3{M(inv, a.x), M(inv, a.y), M(inv, a.z)};
 }
 

@@ -136,6 +136,20 @@ __device__ __forceinline__ double dot3e(D3 a, D3 b) {
     s += early_mul<kHw>(a.z, b.z);
     return s;
 }
+// dot3e(a, a)
+template <bool kHw = false>
+__device__ __forceinline__ double norm2e(D3 a) {
+    if constexpr (kHw) return dot3e<true>(a, a);
+    double s = sf::sqr(a.x);
+    s += sf::sqr(a.y);
+    s += sf::sqr(a.z);
+    return s;
+}
+// cross3 of FP32 points: the products are exact
+__device__ __forceinline__ D3 cross32(float4 a, float4 b) {
+    return D3{sf::mul32(a.y, b.z) - sf::mul32(a.z, b.y), sf::mul32(a.z, b.x) - sf::mul32(a.x, b.z),
+              sf::mul32(a.x, b.y) - sf::mul32(a.y, b.x)};
+}
 template <bool kHw = false>
 __device__ __forceinline__ D3 cross3e(D3 p1, D3 p2) {
     return D3{early_mul<kHw>(p1.y, p2.z) - early_mul<kHw>(p1.z, p2.y),
@@ -150,7 +164,7 @@ __device__ __forceinline__ double det3(D3 a, D3 b, D3 c) {    // a . (b x c), sp
 template <bool kHwMul = false, bool kHwScale = true>
 __device__ __forceinline__ D3 renorm(D3 p, double R) {
     const auto M = [](double x, double y) { return early_mul<kHwScale>(x, y); };
-    const double inv = f64_div_root(1.0, dot3e<kHwMul>(p, p));
+    const double inv = f64_div_root(1.0, norm2e<kHwMul>(p));
     return D3{M(R, M(inv, p.x)), M(R, M(inv, p.y)), M(R, M(inv, p.z))};
 }
 // move(p, v) (sphericalDomain.h:203-209): project v onto the tangent plane at p, add, renormalise
@@ -169,7 +183,7 @@ __device__ __forceinline__ double geodesic(D3 p1, D3 p2, double R) {
 }
 // |p| as geodesic and sph_coords evaluate it (same operations, so the same value)
 template <bool kHw = false, bool kHwMul = kHw>
-__device__ __forceinline__ double pos_norm(D3 p) { return f64_sqrt<kHw>(dot3e<kHwMul>(p, p)); }
+__device__ __forceinline__ double pos_norm(D3 p) { return f64_sqrt<kHw>(norm2e<kHwMul>(p)); }
 // geodesic with the two norms given (n1 = pos_norm(p1), n2 = pos_norm(p2)): the same value
 template <bool kHwMul = false>
 __device__ __forceinline__ double geodesic_n(D3 p1, D3 p2, double n1, double n2, double R) {
@@ -343,7 +357,7 @@ __device__ __forceinline__ double included_angle_clamped(D3 p1, D3 p2, D3 p3) {
 }
 // sphericalTriangleArea (sphericalDomain.h:135-166)
 // q / |q| as sphericalTriangleArea normalises each corner
-__device__ __forceinline__ D3 unit_corner(D3 q) { return scl3(f64_div_root(1.0, dot3e(q, q)), q); }
+__device__ __forceinline__ D3 unit_corner(D3 q) { return scl3(f64_div_root(1.0, norm2e(q)), q); }
 __device__ __forceinline__ double triangle_area_unit(D3 p1, D3 p2, D3 p3, double R);
 __device__ __forceinline__ double triangle_area(D3 q1, D3 q2, D3 q3, double R) {
     return triangle_area_unit(unit_corner(q1), unit_corner(q2), unit_corner(q3), R);
@@ -390,7 +404,7 @@ template <bool kHw = false, bool kHwMul = kHw>
 __device__ __forceinline__ double4_32a sph_coords_n(D3 p, double r) {  // r = pos_norm(p)
     double cosT = f64_div<kHw>(p.z, r);
     double sinT = f64_sqrt<kHw>(1. - cosT * cosT);
-    const double rxy2 = early_mul<kHwMul>(p.x, p.x) + early_mul<kHwMul>(p.y, p.y);
+    const double rxy2 = kHwMul ? __dadd_rn(__dmul_rn(p.x, p.x), __dmul_rn(p.y, p.y)) : __dadd_rn(sf::sqr(p.x), sf::sqr(p.y));
     if constexpr (kHw) {
         const double rxy = f64_sqrt<kHw>(rxy2);
         return make_double4_32a(cosT, sinT, f64_div<kHw>(p.x, rxy), f64_div<kHw>(p.y, rxy));

@@ -159,10 +159,10 @@ __global__ void k32_corners(const float4* __restrict__ pos, const int4* __restri
         nb = vnbr[v];
         const int u = comp(nb, j);
         const float4 q = pos[u];
-        const D3 C = cross3e(D3{sf::widen(p.x), sf::widen(p.y), sf::widen(p.z)}, D3{sf::widen(q.x), sf::widen(q.y), sf::widen(q.z)});
+        const D3 C = cross32(p, q);
         const float arc = arc32(q, p, R);
         cx[t] = C.x; cy[t] = C.y; cz[t] = C.z;
-        nc[t] = f64_sqrt(dot3e(C, C));
+        nc[t] = f64_sqrt(norm2e(C));
         arcs[t] = arc;
         if (t1test && v < u && arc < t1Threshold) t1_flag(t1, 3 * v + j, v, u, rep_of(p), vnbr, vcell);
     }

@@ -165,7 +165,7 @@ __global__ void k_edges(const double4_32a* __restrict__ pos, const double* __res
         const D3 C = cross3e(p, U);
         const double arc = geodesic_n(U, p, vnorm[u], vnorm[w], R);
         const int e = 3 * w + j;
-        edgeC[e] = make_double4_32a(C.x, C.y, C.z, f64_sqrt(dot3e(C, C)));
+        edgeC[e] = make_double4_32a(C.x, C.y, C.z, f64_sqrt(norm2e(C)));
         edgeArc[e] = arc;
         // geodesic(u, p) < t is the reference's test (sphericalVertexModel.cpp:475)
         if (t1test && arc < t1Threshold) t1_flag(t1, e, w, u, 0, vnbr, vcell);
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(4 * kFewVerts) k_corners_few(
         const D3 p = ld3(pos, v), U = ld3(pos, u);
         const D3 C = cross3e<kHwMul>(p, U);
         const double arc = geodesic_n<kHwMul>(U, p, pos_norm<false, kHwMul>(U), pos_norm<false, kHwMul>(p), R);
-        cx[t] = C.x; cy[t] = C.y; cz[t] = C.z; nc[t] = f64_sqrt(dot3e<kHwMul>(C, C));
+        cx[t] = C.x; cy[t] = C.y; cz[t] = C.z; nc[t] = f64_sqrt(norm2e<kHwMul>(C));
         ux[t] = U.x; uy[t] = U.y; uz[t] = U.z; arcs[t] = arc;
         if (t1test && v < u && arc < t1Threshold) t1_flag(t1, 3 * v + j, v, u, 0, vnbr, vcell);
     }

@@ -235,6 +235,25 @@ SF_HD double mul(double a, double b) {
     return hw_mul(a, b);
 }
 
+// x x
+SF_HD double sqr(double x) {
+    const unsigned long long ix = bits(x);
+    const unsigned hx = hi32(ix), ex = (hx >> 20) & 0x7ffu;
+    if (ex - 512u < 1023u) {   // 2 ex - 1023 in [1, 2045]
+        const unsigned xh = (hx & 0xfffffu) | 0x100000u, xl = lo32(ix);
+        const unsigned long long p0 = wide(xl, xl), c = wide(xh, xl);       // c < 2^53
+        const unsigned long long p1 = 2ull * c + (p0 >> 32);                // < 2^55
+        const unsigned long long p2 = wide_add(xh, xh, p1 >> 32);           // product in [2^104, 2^106)
+        const unsigned n = hi32(p2) >> 9, sh = 12u - n;
+        const unsigned mh = shl2(hi32(p2), lo32(p2), sh), ml = shl2(lo32(p2), lo32(p1), sh);
+        unsigned g = shl2(lo32(p1), lo32(p0), sh);
+        g |= (lo32(p0) << sh) != 0u ? 1u : 0u;
+        const unsigned up = hi32((unsigned long long)g + 0x7fffffffu + (ml & 1u));
+        const unsigned top = ((2u * ex - 1023u + n - 1u) << 20) + mh;
+        return dbl((((unsigned long long)top << 32) | ml) + up);
+    }
+    return hw_mul(x, x);
+}
 // mul out of line, for kernels with dozens of products, whose code would not fit the instruction caches.
 SF_SLOW double mul_call(double a, double b) { return mul(a, b); }
 
@@ -428,6 +447,19 @@ SF_HD double widen(float f) {
     // sign, exponent rebiased by 1023 - 127, the 23 significand bits on top of the double's 52
     return dbl(((unsigned long long)(u & 0x80000000u) << 32) | ((unsigned long long)(e + 896u) << 52) |
                ((unsigned long long)(u & 0x7fffffu) << 29));
+}
+// The product of two floats as a double: exact (48 bits).
+SF_SLOW double hw_mul32(float a, float b) { return hw_mul(hw_widen(a), hw_widen(b)); }
+SF_HD double mul32(float a, float b) {
+    const unsigned u = f32bits(a), w = f32bits(b);
+    const unsigned ea = (u >> 23) & 0xffu, eb = (w >> 23) & 0xffu;
+    if (ea - 1u < 254u && eb - 1u < 254u) {
+        const unsigned long long p = wide((u & 0x7fffffu) | 0x800000u, (w & 0x7fffffu) | 0x800000u);   // [2^46, 2^48)
+        const unsigned n = hi32(p) >> 15, sh = 6u - n;
+        const unsigned top = ((u ^ w) & 0x80000000u) + ((ea + eb + n + 768u) << 20) + shl2(hi32(p), lo32(p), sh);
+        return dbl(((unsigned long long)top << 32) | (lo32(p) << sh));
+    }
+    return hw_mul32(a, b);
 }
 SF_HD float narrow(double d) {
     const unsigned long long b = bits(d);
