@@ -290,6 +290,13 @@ __device__ __forceinline__ double included_angle_pre(D3 Cx, D3 Cl, double nx, do
     return included_finish(svm_acos(included_cos<clamp>(Cx, Cl, nx, nl)), dp);
 }
 
+// det(pl, p, px) > 0, the side of the corner (p x px = X): in FP32 where that is certain (svm_det), else as the
+// FP64 formula.  det(p, pl, px) is its negative.
+static __device__ __noinline__ bool det_positive_exact(D3 pl, D3 X) { return positive(dot3e(pl, X)); }
+__device__ __forceinline__ bool det_positive(svm_det::F3 pl, svm_det::F3 p, svm_det::F3 px, D3 pl64, D3 X) {
+    const int n = svm_det::below_zero(p, svm_det::diff(pl, p), svm_det::diff(px, p));
+    return n >= 0 ? n != 0 : det_positive_exact(pl64, X);
+}
 // Arccosines of a block's cosines with like magnitudes on the same warps.  An arccosine evaluates one of
 // two expansions by the magnitude of its argument, and the angles of a vertex model (60 to 180 degrees)
 // fall on both sides, so a warp of them in vertex order runs both: about 50 FP64 instructions instead of

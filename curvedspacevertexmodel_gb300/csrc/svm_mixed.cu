@@ -131,11 +131,13 @@ __device__ __forceinline__ F3 normals32(uint64_t seed, unsigned long long step, 
 // Three threads a vertex: thread (v, j) evaluates the edge to neighbour j (FP64 cross product with v and its
 // norm, FP32 arc, T1 test), then, after a block barrier, the corner of cell slot j.  A block of any size
 // takes blockDim.x / 3 vertices.  Dynamic shared memory: 46 bytes a thread (corner_smem).
-// What bounds it: the FP64 pipe (some 120 instructions per 32 vertices, more than half of them the
-// arccosines').  One thread a vertex took 106 registers (16 warps per SM, pipe 66% busy).  Corner phase
-// against that: 200 cells 21.4 -> 12.9 us, 20k 29.4 -> 22.1, 100k 73.4 -> 65.6, 1M 583 -> 562, 512 replicas
-// (646k cells) 383 -> 371.
-__global__ void k32_corners(const float4* __restrict__ pos, const int4* __restrict__ vcell,
+// What bounds it: the FP64 pipe, two thirds of whose 32 instructions a warp are the arccosines', next to some 1100
+// on the integer pipes.  Six blocks of 256 fit an SM at 40 registers.  The corner phase at 1M cells: 562 us as it
+// was with the inlined fallbacks of sf::widen and the general product, 507 with those out of line, 451 with sf::mul32
+// and sf::sqr, 436 with the corner's side found in FP32 (det_positive) and 48 registers, 429 with 40 (32: 416, but
+// 100k cells 53.5 against 52.0); 100k cells 65.6 -> 52.0, 512 replicas (646k cells) 371 -> 280.  One thread a vertex
+// took 106 registers (16 warps an SM).
+__global__ void __maxnreg__(40) k32_corners(const float4* __restrict__ pos, const int4* __restrict__ vcell,
                             const int4* __restrict__ vlast, const int4* __restrict__ vnext,
                             const int4* __restrict__ vrpos, const int4* __restrict__ vnbr,
                             double2* __restrict__ corner, int Wc, int nV, const double* __restrict__ repR,
@@ -179,7 +181,9 @@ __global__ void k32_corners(const float4* __restrict__ pos, const int4* __restri
             const int l = 3 * vi + jl, x = 3 * vi + jx;
             const D3 X{cx[x], cy[x], cz[x]};
             arc = arcs[l];
-            flip = positive(dot3e(ld3(pos, last), X));
+            const float4 L = pos[last], N = pos[comp(nexts, j)];
+            flip = det_positive(svm_det::F3{L.x, L.y, L.z}, svm_det::F3{p.x, p.y, p.z}, svm_det::F3{N.x, N.y, N.z},
+                                D3{sf::widen(L.x), sf::widen(L.y), sf::widen(L.z)}, X);
             cosine[0] = included_cos<true>(X, D3{cx[l], cy[l], cz[l]}, nc[x], nc[l]);
         }
     }

@@ -303,7 +303,9 @@ __global__ void __launch_bounds__(kCornerThreads, 7) k_corner(const double4_32a*
             const int l = b + jl, x = b + jx;
             const D3 X{cx[x], cy[x], cz[x]};
             arc = arcs[l];
-            flip = positive(dot3e(ld3(pos, last), X));
+            const D3 L = ld3(pos, last), N = ld3(pos, comp(nexts, j)), P = ld3(pos, v);
+            flip = det_positive(svm_det::near3(L.x, L.y, L.z), svm_det::near3(P.x, P.y, P.z), svm_det::near3(N.x, N.y, N.z),
+                                L, X);
             cosine[0] = included_cos(X, D3{cx[l], cy[l], cz[l]}, nc[x], nc[l]);
         }
     }
