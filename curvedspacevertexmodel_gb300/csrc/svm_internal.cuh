@@ -611,6 +611,7 @@ struct svm_model {
     int ringGrowths = 0;
     cudaEvent_t passEv[2] = {nullptr, nullptr};
     int passSlot = 0;
+    bool passChecks = true;            // false: the caller checks the headroom itself, between groups of passes
     double R = 1.0, Kr = 1.0, t1Threshold = 0.1;
     bool restricted = false;
     bool ownStream = false;

@@ -2245,6 +2245,7 @@ int grow_rings(svm_model* m, int Wn) {
 // maximum it reads lags at most two passes; a reading close to the capacity is confirmed after a
 // synchronisation.  (Graph launches check between replays instead.)
 int ensure_ring_headroom(svm_model* m) {
+    if (!m->passChecks) return SVM_OK;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(m->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return SVM_OK;
     cudaEvent_t& ev = m->passEv[m->passSlot];
@@ -2258,6 +2259,7 @@ int ensure_ring_headroom(svm_model* m) {
 }
 // Marks the end of a pass launched outside a capture (the wait of ensure_ring_headroom two passes on).
 static int mark_pass(svm_model* m) {
+    if (!m->passChecks) return SVM_OK;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(m->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return SVM_OK;
     cudaEvent_t& ev = m->passEv[m->passSlot];
