@@ -111,8 +111,12 @@ class ClockSampler:
         try:
             self.f = open(self.path, "w")
             self.proc = subprocess.Popen(["nvidia-smi", f"--id={self.gpu}", f"--query-gpu={self.QUERY}",
-                                          "--format=csv,noheader,nounits", "-lms", "200"], stdout=self.f,
+                                          "--format=csv,noheader,nounits", "-lms", "50"], stdout=self.f,
                                          stderr=subprocess.DEVNULL)
+            # its start holds the driver for some 0.2 s, in which launches of a timed step would wait
+            deadline = time.perf_counter() + 5.0
+            while os.path.getsize(self.path) == 0 and self.proc.poll() is None and time.perf_counter() < deadline:
+                time.sleep(0.01)
         except Exception:
             self.proc = None
         return self
@@ -168,9 +172,9 @@ def algorithmic_bytes_step(nv: int) -> int:
 # From an ncu --set full capture of one k_force_bd launch at N = 100k cells (bench.py --mode profile
 # --cells 100000 --stab 2 --steps 1; profiles/k_force_bd_n100k_full.md): DRAM bytes read + written
 # per vertex by one launch, and the FP64 and integer (ALU) pipes' busy fractions in that kernel.
-FORCE_BD_DRAM_BYTES_PER_VERTEX = (32.27776e6 + 0.608512e6) / 199_996
-FORCE_BD_FP64_PIPE_PCT = 67.7
-FORCE_BD_ALU_PIPE_PCT = 27.7
+FORCE_BD_DRAM_BYTES_PER_VERTEX = (33.1e6 + 1.3e6) / 199_996
+FORCE_BD_FP64_PIPE_PCT = 72.0
+FORCE_BD_ALU_PIPE_PCT = 50.0
 # FP64 arithmetic thread operations (DMUL + DFMA + DADD) per vertex in one k_force_bd launch of the
 # build whose divisions and square roots are the hardware sequences (ncu at N = 100k), and the FP64
 # issue rate they are bound by: 16 SM cycles per FP64 warp instruction (ncu:
@@ -387,7 +391,7 @@ def run_ours(args):
                      "fp64_pipe_busy_pct_ncu": FORCE_BD_FP64_PIPE_PCT,
                      "alu_pipe_busy_pct_ncu": FORCE_BD_ALU_PIPE_PCT,
                      "fp64": fp64_roofline(avg_launch_ms, nv) if names[dom] == "force" else None,
-                     "note": "FP64-issue and latency bound (ncu: FP64 pipe 68% and integer pipes 28% busy, DRAM "
+                     "note": "FP64-issue and latency bound (ncu: FP64 pipe 72% and integer pipes 50% busy, DRAM "
                              "under 1%; divisions, square roots and chain-starting products on the integer "
                              "pipes); HBM fraction is small by construction",
                      "algorithmic_bytes_per_launch": alg, "avg_launch_ms": avg_launch_ms},
