@@ -42,7 +42,8 @@ constexpr int kB = 256;
 constexpr int kClScalars = 5;
 
 __device__ __forceinline__ int bin_of(double x, double y, double z, double r, double h, int n, int* bad) {
-    int bx = (int)floor((x + r) / h), by = (int)floor((y + r) / h), bz = (int)floor((z + r) / h);
+    const F64Divisor H = kept_divisor(h);   // (the quotients on the integer pipes, the same bits)
+    int bx = (int)floor(f64_div(x + r, H)), by = (int)floor(f64_div(y + r, H)), bz = (int)floor(f64_div(z + r, H));
     if (bx < 0 || by < 0 || bz < 0 || bx >= n || by >= n || bz >= n) {
         atomicExch(bad, 1);
         bx = min(max(bx, 0), n - 1); by = min(max(by, 0), n - 1); bz = min(max(bz, 0), n - 1);
@@ -177,8 +178,10 @@ int cl_grow(svm_cell_list* cl, int cap) {
 // What bounds it: phase 1 is a chain of dependent loads (count, slot, position) per candidate, which
 // one thread a point walked for all ~25 candidates with 8 warps on an SM; eight threads a point walk
 // it for three or four candidates each, with 64 warps' loads in flight.  The call on the device, of
-// 39,996 points at two per unit area, range 1: 114 -> 69 us; of 300 points, where launches, clears and
-// the read-back of five scalars are all of it (eleven stream operations, now five): 100 -> 46 us.
+// 39,996 points at two per unit area, range 1: 114 -> 60 us; of 300 points, where launches, clears and
+// the read-back of five scalars are all of it (eleven stream operations, now five): 100 -> 37 us.  Longer rows
+// are bound by phase 2's FP64, whose roots and the bins' quotients run on the integer pipes: 199,996 vertices
+// with rows of 22 214 -> 164 us.
 // The minimum-image loops run at most kWrapIters times: points inside the grid need one, and a
 // point outside it is an error the host reports (the cell list's flag).
 constexpr int kNlLanes = 8;                 // threads a point
@@ -342,7 +345,7 @@ __global__ void __launch_bounds__(kB, 6) k_nl(P pts, const float4* __restrict__ 
             for (int d = 0; d < 3; ++d) disp[d] = own[o][d] - b[d];
             if (w)
                 for (int d = 0; d < 3; ++d) min_image(disp[d], prm.radius);
-            len = sqrt(disp[0] * disp[0] + disp[1] * disp[1] + disp[2] * disp[2]);
+            len = f64_sqrt(disp[0] * disp[0] + disp[1] * disp[1] + disp[2] * disp[2]);
         }
         idx[at] = j;
         vec[3 * at] = disp[0]; vec[3 * at + 1] = disp[1]; vec[3 * at + 2] = disp[2];

@@ -63,10 +63,12 @@ __device__ __forceinline__ double f64_sqrt(double a) {
 #ifdef SVM_NATIVE_FP64_DIV
 struct F64Divisor { double d; };
 __device__ __forceinline__ F64Divisor f64_root_divisor(double a) { return F64Divisor{__dsqrt_rn(a)}; }
+__device__ __forceinline__ F64Divisor kept_divisor(double b) { return F64Divisor{b}; }
 __device__ __forceinline__ double f64_div(double a, const F64Divisor& b) { return __ddiv_rn(a, b.d); }
 #else
 using F64Divisor = sf::Divisor;
 __device__ __forceinline__ F64Divisor f64_root_divisor(double a) { return sf::sqrt_divisor(a); }
+__device__ __forceinline__ F64Divisor kept_divisor(double b) { return sf::divisor(b); }
 __device__ __forceinline__ double f64_div(double a, const F64Divisor& b) { return sf::div(a, b); }
 #endif
 // a / sqrt(b)
