@@ -374,10 +374,11 @@ __device__ __forceinline__ double triangle_area(D3 q1, D3 q2, D3 q3, double R) {
 // the cosines of the three angles, from the normalised corners
 __device__ __forceinline__ void triangle_cosines(D3 p1, D3 p2, D3 p3, double (&c)[3]) {
     const double d12 = dot3e(p1, p2), d13 = dot3e(p1, p3), d23 = dot3e(p2, p3);
-    const double s12 = f64_sqrt(1 - d12 * d12), s13 = f64_sqrt(1 - d13 * d13), s23 = f64_sqrt(1 - d23 * d23);
-    c[0] = f64_div(d23 - d12 * d13, s12 * s13);
-    c[1] = f64_div(d12 - d13 * d23, s13 * s23);
-    c[2] = f64_div(d13 - d12 * d23, s12 * s23);
+    const auto M = [](double x, double y) { return early_mul(x, y); };
+    const double s12 = f64_sqrt(1 - sf::sqr(d12)), s13 = f64_sqrt(1 - sf::sqr(d13)), s23 = f64_sqrt(1 - sf::sqr(d23));
+    c[0] = f64_div(d23 - M(d12, d13), M(s12, s13));
+    c[1] = f64_div(d12 - M(d13, d23), M(s13, s23));
+    c[2] = f64_div(d13 - M(d12, d23), M(s12, s23));
 }
 // the area from the three angles
 __device__ __forceinline__ double triangle_sum(const double (&a)[3], double R) {
