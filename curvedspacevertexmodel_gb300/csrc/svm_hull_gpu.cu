@@ -154,9 +154,10 @@ struct BinGrid {
 // kMaxCand candidates, so that warps of the first launch do not wait on them.
 // What bounds it: issue slots and shared memory (about 1,700 FP32 instructions a warp to pivot six times
 // over 70 candidates); the FP64 pipe holds only the offsets x - p.  One centre per thread, candidates in
-// local memory: 4.5 ms at 100k centres.
+// local memory: 4.5 ms at 100k centres.  Seven and six blocks an SM: the whole build at 100k centres 1.30 -> 1.18
+// ms, 1M 10.8 -> 9.4 (93 registers, five blocks, before; eight blocks 1.20, ten 1.29).
 template <int kCap>
-__global__ void __launch_bounds__(kHB) k_hull_star(const double* __restrict__ P, const int* __restrict__ list,
+__global__ void __launch_bounds__(kHB, kCap == kFewCand ? 7 : 6) k_hull_star(const double* __restrict__ P, const int* __restrict__ list,
                                                   const int* __restrict__ countPtr, int n, int wFirst, int wLast, BinGrid g,
                                                   int* __restrict__ deg, int* __restrict__ star,
                                                   int* __restrict__ retry, int* __restrict__ retryCount,
@@ -172,14 +173,15 @@ __global__ void __launch_bounds__(kHB) k_hull_star(const double* __restrict__ P,
     int* st = stS[warp];
     const int count = list ? *countPtr : n;
     for (int t = blockIdx.x * kWarps + warp; t < count; t += gridDim.x * kWarps) {
-        const int p = list ? list[t] : t;
+        // (a queued centre: as ~p if it had too many candidates, else its first search cannot be certified)
+        const int entry = list ? list[t] : t, p = entry < 0 ? ~entry : entry;
         double pp[3];
         load3(P, p, pp);
         const float p32[3] = {(float)pp[0], (float)pp[1], (float)pp[2]};
         int c[3];
         for (int d = 0; d < 3; ++d) c[d] = max(0, min(g.nside - 1, (int)floor((pp[d] + g.radius) / g.h)));
-        bool hard = false, done = false;  // hard: a failure no wider search can repair
-        for (int w = wFirst; w <= wLast && !done && !hard; ++w) {
+        bool hard = false, done = false, full = false;  // hard: a failure no wider search can repair
+        for (int w = list && entry >= 0 ? wFirst + 1 : wFirst; w <= wLast && !done && !hard; ++w) {
             int lo[3], ext[3];
             bool whole = true;
             for (int d = 0; d < 3; ++d) {
@@ -230,7 +232,7 @@ __global__ void __launch_bounds__(kHB) k_hull_star(const double* __restrict__ P,
                 }
             }
             __syncwarp();
-            if (nc > kCap) { if (kCap == kMaxCand) hard = true; break; }
+            if (nc > kCap) { if (kCap == kMaxCand) hard = true; full = true; break; }
             if (nc < 3) { if (whole) hard = true; continue; }
             // the nearest in FP32 (squared length within 5 2^-24 relative of the exact one); a near tie: the
             // FP64 squared lengths of those near it, lowest index on ties
@@ -331,7 +333,7 @@ __global__ void __launch_bounds__(kHB) k_hull_star(const double* __restrict__ P,
         }
         if (!done && lane == 0) {
             deg[p] = 0;
-            if (retry && !hard) retry[atomicAdd(retryCount, 1)] = p;
+            if (retry && !hard) retry[atomicAdd(retryCount, 1)] = full ? ~p : p;
             else atomicOr(err, 1);
         }
     }
