@@ -683,11 +683,14 @@ struct svm_model {
     int maxPartialBlocks = 0;
     int sms = 152;                     // SMs of the model's device
     // graph cache for svm_brownian_run
-    cudaGraphExec_t bdGraph = nullptr;
+    // captured pairs of steps, one per role of the position buffers at its start (an odd run swaps them)
+    struct StepGraph {
+        cudaGraphExec_t exec = nullptr;
+        double T = 0, dt = 0, mu = 0;
+        uint64_t seed = 0;
+        unsigned version = ~0u;
+    } bdGraph[2];
     cudaEvent_t runEv[2] = {nullptr, nullptr};   // svm_brownian_run: ends of the last two chunks
-    double bdT = 0, bdDt = 0, bdMu = 0;
-    uint64_t bdSeed = 0;
-    int bdGraphCur = -1;
     // per-phase event timing (svm_model_profile)
     bool prof = false;
     int profMask = 0xff;               // phases bracketed by events while profiling (bit per phase)
@@ -698,7 +701,6 @@ struct svm_model {
     std::vector<int> profKernels[SVM_PHASE_COUNT];
     // bumped by every setter whose value a captured graph bakes in (Kr, threshold, restriction)
     unsigned paramsVersion = 0;
-    unsigned bdGraphVersion = ~0u;
     // graph cache for svm_brownian_step_io with pinned host buffers, one per position-buffer role
     struct IoGraph {
         cudaGraphExec_t exec = nullptr;

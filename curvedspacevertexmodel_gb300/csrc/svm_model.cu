@@ -2575,7 +2575,7 @@ int svm_model_destroy(svm_model* m) {
         if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : m->runEv)
         if (e) cudaEventDestroy(e);
-    if (m->bdGraph) cudaGraphExecDestroy(m->bdGraph);
+    for (auto& g : m->bdGraph) if (g.exec) cudaGraphExecDestroy(g.exec);
     for (auto& g : m->ioGraph)
         if (g.exec) cudaGraphExecDestroy(g.exec);
     if (m->ioEnergy) cudaFreeHost(m->ioEnergy);
@@ -3222,15 +3222,17 @@ int svm_brownian_run(svm_model* m, double T, double dt, double mu, uint64_t seed
     for (int chunk = 0; nSteps > 1; ++chunk) {
         if (chunk >= 2) SVM_CUDA(cudaEventSynchronize(m->runEv[chunk % 2]));
         if ((rc = svm::ensure_ring_headroom(m))) return rc;
-        const bool reuse = m->bdGraph && m->bdT == T && m->bdDt == dt && m->bdMu == mu && m->bdSeed == seed &&
-                           m->bdGraphCur == m->cur && m->bdGraphVersion == m->paramsVersion;
+        auto& graph = m->bdGraph[m->cur];
+        const bool reuse = graph.exec && graph.T == T && graph.dt == dt && graph.mu == mu && graph.seed == seed &&
+                           graph.version == m->paramsVersion;
         if (chunk == 0 || !reuse || !m->cornersValid) {
             rc = svm::launch_geometry(m);  // make corners valid outside the capture
             if (rc) return rc;
         }
         if (!reuse) {
-            if (m->bdGraph) { cudaGraphExecDestroy(m->bdGraph); m->bdGraph = nullptr; }
-            // a pair of steps returns the position buffers to their starting roles
+            if (graph.exec) { cudaGraphExecDestroy(graph.exec); graph.exec = nullptr; }
+            // a pair of steps returns the position buffers to their starting roles (each of which has its graph:
+            // with one graph, runs of an odd number of steps captured it anew each time, 50 us of host work)
             cudaGraph_t g;
             const int cur0 = m->cur;
             SVM_CUDA(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
@@ -3239,14 +3241,14 @@ int svm_brownian_run(svm_model* m, double T, double dt, double mu, uint64_t seed
             cudaError_t ce = cudaStreamEndCapture(m->stream, &g);
             m->cur = cur0;
             if (r2 || ce != cudaSuccess) { cudaGetLastError(); return SVM_ERR_CUDA; }
-            ce = cudaGraphInstantiate(&m->bdGraph, g, 0);
+            ce = cudaGraphInstantiate(&graph.exec, g, 0);
             cudaGraphDestroy(g);
-            if (ce != cudaSuccess) { m->bdGraph = nullptr; return SVM_ERR_CUDA; }
-            m->bdT = T; m->bdDt = dt; m->bdMu = mu; m->bdSeed = seed;
-            m->bdGraphCur = m->cur; m->bdGraphVersion = m->paramsVersion;
+            if (ce != cudaSuccess) { graph.exec = nullptr; return SVM_ERR_CUDA; }
+            graph.T = T; graph.dt = dt; graph.mu = mu; graph.seed = seed;
+            graph.version = m->paramsVersion;
         }
         const int pairs = std::min(nSteps / 2, 4);
-        for (int i = 0; i < pairs; ++i) SVM_CUDA(cudaGraphLaunch(m->bdGraph, m->stream));
+        for (int i = 0; i < pairs; ++i) SVM_CUDA(cudaGraphLaunch(graph.exec, m->stream));
         m->cornersValid = true;  // a replayed pair leaves the moved state's corners
         SVM_CUDA(cudaEventRecord(m->runEv[chunk % 2], m->stream));
         nSteps -= 2 * pairs;
