@@ -1310,9 +1310,11 @@ __device__ __noinline__ int t1_replay(const ApplyArgs& A, const T1Scratch& t1, i
     __syncthreads();
     int lastProcessed = -1;
     while (true) {
-        // Refill the window from the bitmap when both the window and the heap are empty.
-        if (head == nbuf && nheap == 0) {
-            __syncthreads();
+        // Refill the window from the bitmap when both the window and the heap are empty.  Every thread decides
+        // before thread 0 may go on to change either.
+        const bool empty = head == nbuf && nheap == 0;
+        __syncthreads();
+        if (empty) {
             if (tid == 0) { nSummaryHit = 0x7fffffff; }
             __syncthreads();
             const int sw0 = extractWord >> 5;
