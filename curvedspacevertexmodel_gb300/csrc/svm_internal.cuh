@@ -584,7 +584,8 @@ __device__ __forceinline__ void t1_clear(const T1Scratch& t1) {
 // with its first round's reservations made.  Short edges are a few in ten thousand.
 inline __device__ __noinline__ void t1_flag(const T1Scratch& t1, int p, int v, int u, int seg, const int4* __restrict__ vnbr,
                                      const int4* __restrict__ vcell) {
-    atomicOr(&t1.bits[p >> 5], 1u << (p & 31));
+    const unsigned bit = 1u << (p & 31);
+    if (atomicOr(&t1.bits[p >> 5], bit) & bit) return;   // listed by an earlier test whose pass did not run
     const int lo = t1.segOff ? 3 * t1.segOff[seg] : 0;
     const int i = atomicAdd(t1.segCount + seg, 1);
     const int at = lo / 2 + t1.listPad * seg + i;

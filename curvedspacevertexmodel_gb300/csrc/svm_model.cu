@@ -2074,7 +2074,17 @@ static ApplyArgs apply_args(svm_model* m, int bump) {
     return A;
 }
 
+// Before a T1 test: the ring capacity, whose growth may fail, so that no test is left without its pass (the
+// pass's list, reservations and footprints are the test's).
+static int ready_for_t1(svm_model* m) {
+    const int rc = ensure_ring_headroom(m);
+    if (rc) m->cornersValid = false;
+    return rc;
+}
+
 int launch_corners(svm_model* m, bool t1test, bool vnormReady) {
+    if (t1test)
+        if (int rc = ready_for_t1(m)) return rc;
     // FP64: k_corners_few, or k_vnorm (unless the moving kernel wrote the norms), k_edges and k_corner
     PhaseTimer pt(m, SVM_PHASE_CORNERS,
                   m->precision == SVM_PRECISION_MIXED || m->nVertices < kFewCornersBelow ? 1 : (vnormReady ? 2 : 3));
@@ -2242,7 +2252,7 @@ int grow_rings(svm_model* m, int Wn) {
     return SVM_OK;
 }
 
-// Before a T1 pass launched outside a capture: grows the ring capacity when ringHeadroom or fewer
+// Before a T1 test and its pass, launched outside a capture: grows the ring capacity when ringHeadroom or fewer
 // slots are free in the largest ring.  The host first waits for the pass before last, so the
 // maximum it reads lags at most two passes; a reading close to the capacity is confirmed after a
 // synchronisation.  (Graph launches check between replays instead.)
@@ -2272,7 +2282,8 @@ static int mark_pass(svm_model* m) {
 }
 
 int launch_t1_apply(svm_model* m, int bump) {
-    if (int rc = ensure_ring_headroom(m)) return rc;
+    if (m->restricted)   // (else ready_for_t1, ahead of the test)
+        if (int rc = ensure_ring_headroom(m)) return rc;
     const bool batch = m->nRep > 1;
     PhaseTimer pt(m, SVM_PHASE_T1APPLY, batch ? 2 : 1);
     const int nSeg = batch ? m->nRep : 1;
@@ -2308,6 +2319,7 @@ int launch_t1_apply(svm_model* m, int bump) {
 // The T1 edge test on its own (k_t1_test: the decisions of the test fused into the corner
 // kernels), for a state whose corners are not needed before the positions change again.
 int launch_t1_test(svm_model* m) {
+    if (int rc = ready_for_t1(m)) return rc;
     PhaseTimer pt(m, SVM_PHASE_CORNERS);
     double lo, hi, s2lo, s2hi;
     t1_bracket(m->t1Threshold, m->R, &lo, &hi);
