@@ -668,11 +668,12 @@ int svm_mlp_train(svm_mlp* M, const float* X, const float* Y, const int* order, 
     if (cudaMemsetAsync(M->loss, 0, sizeof(double), M->stream) != cudaSuccess) return SVM_ERR_CUDA;
     for (int first = 0; first < n; first += batch) {
         const int count = std::min(batch, n - first);
-        M->adamStep++;
+        const long step = M->adamStep + 1;
         AdamStep A{learningRate, M->beta1, M->beta2, M->eps, 0.f, 0.f};
-        A.c1 = 1.f - std::pow(M->beta1, (float)M->adamStep);
-        A.c2 = 1.f - std::pow(M->beta2, (float)M->adamStep);
+        A.c1 = 1.f - std::pow(M->beta1, (float)step);
+        A.c2 = 1.f - std::pow(M->beta2, (float)step);
         if (int rc = mlp_grad(M, X, Y, order, first, count, 1.f / count, &A)) return rc;
+        M->adamStep = step;
     }
     double total = 0.0;
     if (meanLoss && cudaMemcpyAsync(&total, M->loss, sizeof(double), cudaMemcpyDeviceToHost, M->stream) != cudaSuccess)

@@ -76,5 +76,35 @@ def growth(blocks):
     return rep
 
 
+def train(first, refused_samples):
+    """Two epochs of batches of 512 after a training call whose gradient sums found no room (and, with `first`, after an
+    epoch before it): losses and weights as without that call."""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3)
+    n = max(2000, refused_samples)
+    X, Y = torch.randn((n, 24), generator=g, device="cuda"), torch.randn((n, 2), generator=g, device="cuda")
+    order = torch.arange(n, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+
+    def epoch(net, samples, batch):
+        loss = C.c_double()
+        _lib.call("svm_mlp_train", net._h, C.c_void_p(X.data_ptr()), C.c_void_p(Y.data_ptr()), C.c_void_p(order.data_ptr()),
+                  samples, batch, C.c_float(1e-3), C.byref(loss))
+        return loss.value
+
+    rep, results = {}, []
+    for again in (False, True):
+        net = svm.warmStartNetwork(7)
+        losses = [epoch(net, 2000, 512)] if first else []
+        if again:
+            rep["refused"] = refused_call(lambda: epoch(net, refused_samples, refused_samples))
+        losses += [epoch(net, 2000, 512) for _ in range(2)]
+        results.append((losses, net.weights()))
+    rep["losses"] = results[0][0] == results[1][0]
+    rep["weights"] = bool(np.array_equal(results[0][1], results[1][1]))
+    return rep
+
+
 if __name__ == "__main__":
-    print(json.dumps({"growth": growth}[sys.argv[1]](*map(int, sys.argv[2:]))), flush=True)
+    print(json.dumps({"growth": growth, "train": train}[sys.argv[1]](*map(int, sys.argv[2:]))), flush=True)
