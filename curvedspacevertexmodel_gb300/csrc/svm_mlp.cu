@@ -511,14 +511,22 @@ struct svm_mlp {
     float beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f;
 };
 
+// (on failure both arrays are gone and maxBlocks is 0: the next call reserves again)
 static int mlp_reserve(svm_mlp* M, int blocks) {
     if (blocks <= M->maxBlocks) return SVM_OK;
-    if (M->partials) cudaFree(M->partials);
-    if (M->lossPartials) cudaFree(M->lossPartials);
-    M->partials = nullptr; M->lossPartials = nullptr;
+    const auto release = [&] {
+        cudaFree(M->partials);
+        cudaFree(M->lossPartials);
+        M->partials = nullptr; M->lossPartials = nullptr;
+        M->maxBlocks = 0;
+    };
+    release();
     if (cudaMalloc(&M->partials, sizeof(float) * (size_t)blocks * kParams) != cudaSuccess ||
-        cudaMalloc(&M->lossPartials, sizeof(double) * kTC * blocks) != cudaSuccess)
+        cudaMalloc(&M->lossPartials, sizeof(double) * kTC * blocks) != cudaSuccess) {
+        release();
+        cudaGetLastError();
         return SVM_ERR_CUDA;
+    }
     M->maxBlocks = blocks;
     return SVM_OK;
 }

@@ -37,6 +37,8 @@ def test_ring_growth_refused_before_a_pass(run, blocks):
     assert rep == dict(flips=True, neighbours=True, growths=1, status=0, step=True), rep
 
 
-def test_training_refused_room_for_its_sums(run):
-    """The refused call has taken no step: Adam's bias corrections go on from the last step taken."""
-    assert run("train", 0, 512) == dict(refused=True, losses=True, weights=True)
+@pytest.mark.parametrize("first,samples", [(0, 512), (1, 1500)])
+def test_training_refused_room_for_its_sums(run, first, samples):
+    """The refused call has taken no step: Adam's bias corrections go on from the last step taken, and a batch
+    that fitted before fits again."""
+    assert run("train", first, samples) == dict(refused=True, losses=True, weights=True)
