@@ -110,10 +110,33 @@ struct AosPoints {
     __device__ void operator()(int i, double& x, double& y, double& z) const { x = p[3 * i]; y = p[3 * i + 1]; z = p[3 * i + 2]; }
 };
 
+// A bin took more points than it has slots: give every bin `cap` slots, as the reference's cell
+// list widens its Nmax and bins again (hyperrectangularCellList.cpp:165-214).  The counts of the
+// overflowing call stay valid for the next call's incremental clear.
+// (On failure the list has no slots, and the next call allocates them.)
+int cl_grow(svm_cell_list* cl, int cap) {
+    if (cudaStreamSynchronize(cl->stream) != cudaSuccess) return SVM_ERR_CUDA;
+    const auto release = [&] {
+        cudaFree(cl->tmp); cudaFree(cl->slots);
+        cl->tmp = nullptr; cl->slots = nullptr;
+    };
+    release();
+    if (cudaMalloc(&cl->tmp, sizeof(int) * cl->total * cap) != cudaSuccess ||
+        cudaMalloc(&cl->slots, sizeof(int) * cl->total * cap) != cudaSuccess) {
+        release();
+        cudaGetLastError();
+        return SVM_ERR_CUDA;
+    }
+    cl->cap = cap;
+    return SVM_OK;
+}
+
 // `p32`: where to leave FP32 copies of the points, or null
 template <typename P>
 int compute(svm_cell_list* cl, P pts, int np, float4* p32 = nullptr) {
     if (np != cl->nPoints) return SVM_ERR_ARG;
+    if (!cl->slots)
+        if (int rc = cl_grow(cl, cl->cap)) return rc;
     const int nb = (np + kB - 1) / kB;
     k_cl_clear<<<nb, kB, 0, cl->stream>>>(cl->binOf, cl->counts, np, cl->scalars);
     k_cl_bin<<<nb, kB, 0, cl->stream>>>(pts, np, cl->radius, cl->h, cl->nside, cl->cap, cl->binOf, cl->counts, cl->tmp,
@@ -141,19 +164,6 @@ int read_scalars(svm_cell_list* cl) {
                    cudaStreamSynchronize(cl->stream) == cudaSuccess ? SVM_OK : SVM_ERR_CUDA;
 }
 
-// A bin took more points than it has slots: give every bin `cap` slots, as the reference's cell
-// list widens its Nmax and bins again (hyperrectangularCellList.cpp:165-214).  The counts of the
-// overflowing call stay valid for the next call's incremental clear.
-int cl_grow(svm_cell_list* cl, int cap) {
-    if (cudaStreamSynchronize(cl->stream) != cudaSuccess) return SVM_ERR_CUDA;
-    cudaFree(cl->tmp); cudaFree(cl->slots);
-    cl->tmp = nullptr; cl->slots = nullptr;
-    if (cudaMalloc(&cl->tmp, sizeof(int) * cl->total * cap) != cudaSuccess ||
-        cudaMalloc(&cl->slots, sizeof(int) * cl->total * cap) != cudaSuccess)
-        return SVM_ERR_CUDA;
-    cl->cap = cap;
-    return SVM_OK;
-}
 // neighborList (src/utilities/neighborList.cpp:6-18, 96-151; kernels neighborList.cu:108-357): per
 // point, over the adjacent bins of its (clamped) bin in the mask's order and each bin's points in
 // slot order, every other point whose minimum-image displacement (periodic box of side 2 radius,
@@ -367,13 +377,21 @@ struct svm_neighbor_list {
 };
 
 namespace {
-int nl_alloc(svm_neighbor_list* nl) {
-    cudaFree(nl->idx); cudaFree(nl->vec); cudaFree(nl->dist);
-    nl->idx = nullptr; nl->vec = nullptr; nl->dist = nullptr;
-    const size_t e = (size_t)nl->nPoints * nl->nmax;
+// Rows of nmax entries.  (On failure the list has no rows, and the next call allocates them.)
+int nl_alloc(svm_neighbor_list* nl, int nmax) {
+    const auto release = [&] {
+        cudaFree(nl->idx); cudaFree(nl->vec); cudaFree(nl->dist);
+        nl->idx = nullptr; nl->vec = nullptr; nl->dist = nullptr;
+    };
+    release();
+    const size_t e = (size_t)nl->nPoints * nmax;
     if (cudaMalloc(&nl->idx, sizeof(int) * e) != cudaSuccess || cudaMalloc(&nl->vec, sizeof(double) * 3 * e) != cudaSuccess ||
-        cudaMalloc(&nl->dist, sizeof(double) * e) != cudaSuccess)
+        cudaMalloc(&nl->dist, sizeof(double) * e) != cudaSuccess) {
+        release();
+        cudaGetLastError();
         return SVM_ERR_CUDA;
+    }
+    nl->nmax = nmax;
     return SVM_OK;
 }
 
@@ -393,6 +411,8 @@ template <typename P>
 int nl_compute(svm_neighbor_list* nl, P pts, int np) {
     svm_cell_list* cl = nl->cl;
     const int* sc = cl->hostScalars;
+    if (!nl->dist)
+        if (int rc = nl_alloc(nl, nl->nmax)) return rc;
     for (int pass = 0; pass < 64; ++pass) {   // a third pass at most: slots widened, then nmax grown
         NlParams prm;
         prm.np = np; prm.cap = cl->cap; prm.nside = cl->nside; prm.K = nl->K; prm.nmax = nl->nmax;
@@ -410,8 +430,7 @@ int nl_compute(svm_neighbor_list* nl, P pts, int np) {
         }
         const int longest = sc[4];         // (of the same points at any nmax: the next pass finds it again)
         if (longest <= nl->nmax) return SVM_OK;
-        nl->nmax = longest;  // grow-only, then recompute
-        if (nl_alloc(nl)) return SVM_ERR_CUDA;
+        if (nl_alloc(nl, longest)) return SVM_ERR_CUDA;   // grow-only, then recompute
     }
     return SVM_ERR_DEVICE;
 }
@@ -446,7 +465,7 @@ int svm_neighbor_list_create(double range, double radius, int subGridReduction, 
     nl->K = (int)mask.size() / 3;
     bool ok = cudaMalloc(&nl->mask, sizeof(int) * mask.size()) == cudaSuccess &&
               cudaMalloc(&nl->npp, sizeof(unsigned) * nPoints) == cudaSuccess &&
-              cudaMalloc(&nl->p32, sizeof(float4) * nPoints) == cudaSuccess && nl_alloc(nl) == SVM_OK;
+              cudaMalloc(&nl->p32, sizeof(float4) * nPoints) == cudaSuccess && nl_alloc(nl, nl->nmax) == SVM_OK;
     if (ok) ok = cudaMemcpy(nl->mask, mask.data(), sizeof(int) * mask.size(), cudaMemcpyHostToDevice) == cudaSuccess;
     if (!ok) { svm_neighbor_list_destroy(nl); return SVM_ERR_CUDA; }
     *out = nl;
@@ -482,6 +501,7 @@ int svm_neighbor_list_get(svm_neighbor_list* nl, int* nmax, unsigned* npp, int* 
     if (nmax) *nmax = nl->nmax;
     const size_t e = (size_t)nl->nPoints * nl->nmax;
     if ((idx || vec || dist) && (long)e > capacity) return SVM_ERR_ARG;
+    if ((idx || vec || dist) && !nl->dist) return SVM_ERR_CUDA;   // the last call found no room for its rows
     cudaStream_t s = nl->cl->stream;
     if (npp && cudaMemcpyAsync(npp, nl->npp, sizeof(unsigned) * nl->nPoints, cudaMemcpyDeviceToHost, s) != cudaSuccess)
         return SVM_ERR_CUDA;
@@ -556,6 +576,7 @@ int svm_cell_list_get(svm_cell_list* cl, int* nside, int* nmax, unsigned* counts
     }
     if (slots) {
         if (cap < cl->total * Nmax) return SVM_ERR_ARG;
+        if (!cl->slots) return SVM_ERR_CUDA;
         std::vector<unsigned> cnt(cl->total);
         std::vector<int> s((size_t)cl->total * cl->cap);
         if (cudaMemcpy(cnt.data(), cl->counts, sizeof(unsigned) * cl->total, cudaMemcpyDeviceToHost) != cudaSuccess ||

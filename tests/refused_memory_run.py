@@ -106,5 +106,25 @@ def train(first, refused_samples):
     return rep
 
 
+def lists(slots):
+    """A neighbour list whose bins (2 slots) or rows (64 slots: bins that hold all) are to grow, refused once."""
+    import torch
+    rng = np.random.default_rng(5)
+    p = rng.normal(size=(3000, 3))
+    p *= 8.0 / np.linalg.norm(p, axis=1)[:, None]
+    points = torch.from_numpy(p).cuda()
+    rep, results = {}, []
+    for again in (False, True):
+        nl = svm.neighborList(1.0, 10.5, slotCapacity=slots)
+        nl._ensure(len(p))
+        if again:
+            rep["refused"] = [refused_call(lambda: nl.computeNeighborLists(points)) for _ in range(2)]
+        nl.computeNeighborLists(points)
+        results.append((nl.neighborsPerParticle, nl.particleIndices, nl.neighborVectors, nl.neighborDistances))
+    rep["longest"] = int(results[0][0].max())
+    rep["same"] = all(a.shape == b.shape and np.array_equal(a, b) for a, b in zip(*results))
+    return rep
+
+
 if __name__ == "__main__":
-    print(json.dumps({"growth": growth, "train": train}[sys.argv[1]](*map(int, sys.argv[2:]))), flush=True)
+    print(json.dumps({"growth": growth, "train": train, "lists": lists}[sys.argv[1]](*map(int, sys.argv[2:]))), flush=True)

@@ -42,3 +42,9 @@ def test_training_refused_room_for_its_sums(run, first, samples):
     """The refused call has taken no step: Adam's bias corrections go on from the last step taken, and a batch
     that fitted before fits again."""
     assert run("train", first, samples) == dict(refused=True, losses=True, weights=True)
+
+
+@pytest.mark.parametrize("slots", [2, 64])
+def test_neighbour_list_refused_room_to_grow(run, slots):
+    rep = run("lists", slots)
+    assert rep.pop("longest") > 4 and rep == dict(refused=[True, True], same=True), rep
