@@ -109,7 +109,8 @@ __device__ __forceinline__ D3 vv_kick(D3 v, D3 f, double dt) {
 // The iteration's first kernel.  It leaves the pending flag as it is: the control of every iteration
 // (k_fire_force's last block) sets it again before this kernel next reads it, and after the last
 // iteration k_fire_finish applies the update it stands for.  Once FIRE has stopped, the positions
-// stay and only their norms are written (the corner pass of a batch's remaining iterations reads them).
+// stay and only their norms are written (the corner pass of a batch's remaining iterations reads them); that
+// pass's T1 test then flags nothing (T1Scratch::stop), so the state stays the last iteration's.
 template <bool kHwMul>
 __global__ void k_fire_vv1(const FireState* __restrict__ Sp, double4_32a* __restrict__ pos,
                            double4_32a* __restrict__ vel, const double4_32a* __restrict__ force,
@@ -283,7 +284,9 @@ int fire_iteration(svm_fire* F) {
     m->cornersValid = false;
     int rc;
     if (!m->restricted) {
+        m->t1.stop = &F->d->done;
         rc = launch_corners(m, true, /*vnormReady=*/true);
+        m->t1.stop = nullptr;
         if (rc) return rc;
         rc = launch_t1_apply(m, 0);
         if (rc) return rc;
@@ -364,10 +367,12 @@ int svm_fire_minimize(svm_fire* F, int criterion, int* iterations, double* value
     cudaMemcpyAsync(F->d, &S, sizeof(FireState), cudaMemcpyHostToDevice, m->stream);
     int rc = svm_model_compute_forces(m);  // sim->computeForces() before the loop (cpp:186)
     if (rc) return rc;
-    // Iterations in batches; kernels of a batch after convergence return at once.  Without a graph that fits the
-    // model's state the first batch is launched directly, and the graph of the following ones is captured while it
-    // runs: capturing ahead of the first cost 0.3 to 0.4 ms (32 iterations of 200 cells 1.80 -> 1.46 ms, of 20k cells
-    // 4.09 -> 3.85), and replays are the faster (200 cells 40.2 us an iteration against 42.5, 20k 112 against 115).
+    // Iterations in batches; after convergence the rest of a batch changes nothing (the moves and the forces return
+    // at once, the T1 test flags nothing, the corners and cells are evaluated to the same values).  Without a graph
+    // that fits the model's state the first batch is launched directly, and the graph of the following ones is
+    // captured while it runs: capturing ahead of the first cost 0.3 to 0.4 ms (32 iterations of 200 cells 1.80 ->
+    // 1.46 ms, of 20k cells 4.09 -> 3.85), and replays are the faster (200 cells 40.2 us an iteration against 42.5,
+    // 20k 112 against 115).
     const int batch = 32;
     auto have_graph = [&] {
         return F->graph && F->graphCriterion == criterion && F->graphIters == batch && F->graphCur == m->cur &&

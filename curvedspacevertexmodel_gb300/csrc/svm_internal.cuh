@@ -536,6 +536,7 @@ struct T1Scratch {
     int* segCount = nullptr;       // per segment (the sphere, or each replica): positions the test flagged
     const int* segOff = nullptr;   // first vertex of each segment [segments + 1] (null: one sphere)
     int listPad = 0;               // list slack per segment
+    const int* stop = nullptr;     // device flag: while it is set the test flags nothing (a minimisation that has ended)
     int* flipLog = nullptr;        // (pass, position, v1, v2) per flip, capacity flipLogCap
     int* flipCount = nullptr;
     int* pass = nullptr;           // T1 passes so far (orders the flip log across passes)
@@ -584,6 +585,7 @@ __device__ __forceinline__ void t1_clear(const T1Scratch& t1) {
 // with its first round's reservations made.  Short edges are a few in ten thousand.
 inline __device__ __noinline__ void t1_flag(const T1Scratch& t1, int p, int v, int u, int seg, const int4* __restrict__ vnbr,
                                      const int4* __restrict__ vcell) {
+    if (t1.stop && *t1.stop) return;
     const unsigned bit = 1u << (p & 31);
     if (atomicOr(&t1.bits[p >> 5], bit) & bit) return;   // listed by an earlier test whose pass did not run
     const int lo = t1.segOff ? 3 * t1.segOff[seg] : 0;
