@@ -542,7 +542,7 @@ struct Arena {
 }  // namespace
 
 // The arrays stay on the device, where they were computed, until svm_topology_get copies them straight
-// into the caller's.
+// into the caller's; the workspace they were computed with is given back when the build returns.
 struct svm::DeviceTopology {
     void* base = nullptr;
     const double* vpos = nullptr;
@@ -591,15 +591,14 @@ extern "C" int svm_topology_from_points_gpu(const double* pts, int n, void* stre
     g.h = 2.0 * gridR / g.nside;
     g.radius = gridR;
     const size_t bins = (size_t)g.nside * g.nside * g.nside, nf = 2 * (size_t)n - 4;
-    // one allocation: what svm_topology_get copies (kept), and the workspace
+    // the workspace, one allocation
     Arena A;
-    double *P, *vpos;
-    int *deg, *star, *own, *ctl, *retry, *F, *vcells, *vnbrs, *ringOff, *ring, *off, *cursor, *binOf, *list, *tmp, *sums;
+    double* P;
+    int *deg, *star, *own, *ctl, *retry, *F, *ringOff, *ring, *off, *cursor, *binOf, *list, *tmp, *sums;
     const auto lay = [&] {
         A.used = 0;
-        vpos = A.cut<double>(3 * nf);
-        vcells = A.cut<int>(3 * nf); vnbrs = A.cut<int>(3 * nf); deg = A.cut<int>(n);
-        star = A.cut<int>((size_t)n * kMaxDeg);   // the stars, then the ring rows
+        deg = A.cut<int>(n);
+        star = A.cut<int>((size_t)n * kMaxDeg);
         P = A.cut<double>(3 * (size_t)n);
         own = A.cut<int>((size_t)n + 1); retry = A.cut<int>(n); F = A.cut<int>(3 * nf);
         ringOff = A.cut<int>((size_t)n + 1); ring = A.cut<int>(3 * nf);
@@ -612,10 +611,9 @@ extern "C" int svm_topology_from_points_gpu(const double* pts, int n, void* stre
     const size_t bytes = A.used;
     svm_topology* t = new svm_topology();
     t->dev = new DeviceTopology();
-    if (cudaMalloc(&t->dev->base, bytes) != cudaSuccess) { cudaGetLastError(); delete t; return SVM_ERR_CUDA; }
-    A.base = (char*)t->dev->base;
+    if (cudaMalloc((void**)&A.base, bytes) != cudaSuccess) { cudaGetLastError(); delete t; return SVM_ERR_CUDA; }
     lay();
-    const auto fail = [&](int rc) { cudaStreamSynchronize(s); delete t; return rc; };
+    const auto fail = [&](int rc) { cudaStreamSynchronize(s); cudaFree(A.base); delete t; return rc; };
     if (cudaMemcpyAsync(P, pts, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, s) != cudaSuccess ||
         cudaMemsetAsync(ctl, 0, (char*)A.base + bytes - (char*)ctl, s) != cudaSuccess ||
         cudaMemsetAsync(own + n, 0, sizeof(int), s) != cudaSuccess)
@@ -643,16 +641,31 @@ extern "C" int svm_topology_from_points_gpu(const double* pts, int n, void* stre
         return fail(SVM_ERR_CUDA);
     if (got[0] & kOutside) return fail(SVM_ERR_DEVICE);
     if (got[0] || (size_t)facets != nf) return fail(SVM_ERR_HULL);
+    // what svm_topology_get copies, in an allocation of its own
+    const int W = got[2];
+    double* vpos;
+    int *vcells, *vnbrs, *counts, *rows;
+    Arena K;
+    const auto keep = [&] {
+        K.used = 0;
+        vpos = K.cut<double>(3 * nf);
+        vcells = K.cut<int>(3 * nf); vnbrs = K.cut<int>(3 * nf); counts = K.cut<int>(n);
+        rows = K.cut<int>((size_t)n * W);
+    };
+    keep();
+    if (cudaMalloc(&t->dev->base, K.used) != cudaSuccess) { cudaGetLastError(); return fail(SVM_ERR_CUDA); }
+    K.base = (char*)t->dev->base;
+    keep();
     const double radius = std::sqrt(pts[0] * pts[0] + pts[1] * pts[1] + pts[2] * pts[2]);
     k_hull_emit<<<nb, kB, 0, s>>>(star, deg, n, own, F);
     k_hull_vertex<<<((int)nf + kB - 1) / kB, kB, 0, s>>>(P, F, (int)nf, own, star, deg, radius, vpos, vcells, vnbrs, ctl);
-    if (check_launch() || cudaMemcpyAsync(ringOff, deg, sizeof(int) * n, cudaMemcpyDeviceToDevice, s) != cudaSuccess ||
+    if (check_launch() || cudaMemcpyAsync(counts, deg, sizeof(int) * n, cudaMemcpyDeviceToDevice, s) != cudaSuccess ||
+        cudaMemcpyAsync(ringOff, deg, sizeof(int) * n, cudaMemcpyDeviceToDevice, s) != cudaSuccess ||
         cudaMemsetAsync(ringOff + n, 0, sizeof(int), s) != cudaSuccess || exclusive_scan(ringOff, n + 1, s, sums))
         return fail(SVM_ERR_CUDA);
     // (a triangulated sphere of nf facets has rings of 3 nf entries)
     k_hull_ring<<<nb, kB, 0, s>>>(star, deg, n, own, F, ringOff, ring, ctl);
-    const int W = got[2];
-    k_hull_rows<<<(int)(((long)n * W + kB - 1) / kB), kB, 0, s>>>(ringOff, ring, n, W, star);
+    k_hull_rows<<<(int)(((long)n * W + kB - 1) / kB), kB, 0, s>>>(ringOff, ring, n, W, rows);
     int e = 0, nr = 0;
     if (check_launch() || cudaMemcpyAsync(&e, ctl, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaMemcpyAsync(&nr, ringOff + n, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
@@ -662,7 +675,8 @@ extern "C" int svm_topology_from_points_gpu(const double* pts, int n, void* stre
     t->t.nCells = n;
     t->t.nVertices = (int)nf;
     t->t.maxRing = W;
-    t->dev->vpos = vpos; t->dev->vcells = vcells; t->dev->vnbrs = vnbrs; t->dev->rows = star; t->dev->deg = deg;
+    t->dev->vpos = vpos; t->dev->vcells = vcells; t->dev->vnbrs = vnbrs; t->dev->rows = rows; t->dev->deg = counts;
+    cudaFree(A.base);
     *out = t;
     return SVM_OK;
 }
