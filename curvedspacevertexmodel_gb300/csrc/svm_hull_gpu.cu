@@ -33,7 +33,6 @@
 // double-double evaluation where the filter cannot decide (the host uses long double there).
 #include <algorithm>
 #include <cmath>
-#include <vector>
 #include "svm_internal.cuh"
 #include "svm_hull.h"
 
@@ -543,11 +542,26 @@ struct Arena {
 
 // The arrays stay on the device, where they were computed, until svm_topology_get copies them straight
 // into the caller's; the workspace they were computed with is given back when the build returns.
+// Fetching and freeing them take no part in what other threads have under way: the copies run on a stream of
+// the handle's own, which the default stream's work and captures do not order, and the thread's calls are not
+// counted among those that another thread's capture forbids.
+namespace {
+struct OutsideCaptures {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    OutsideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~OutsideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+}  // namespace
 struct svm::DeviceTopology {
     void* base = nullptr;
+    cudaStream_t stream = nullptr;
     const double* vpos = nullptr;
     const int *vcells = nullptr, *vnbrs = nullptr, *rows = nullptr, *deg = nullptr;
-    ~DeviceTopology() { cudaFree(base); }
+    ~DeviceTopology() {
+        OutsideCaptures guard;
+        cudaFree(base);
+        if (stream) cudaStreamDestroy(stream);
+    }
 };
 svm_topology::~svm_topology() { delete dev; }
 
@@ -556,18 +570,17 @@ namespace svm {
 int device_topology_get(const svm_topology* t, double* vp, int* rings, int stride, unsigned* counts, int* vc, int* vn) {
     const DeviceTopology& D = *t->dev;
     const size_t nC = t->t.nCells, nV = t->t.nVertices, W = t->t.maxRing;
-    const auto copy = [](void* dst, const void* src, size_t bytes) {
-        return cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost) == cudaSuccess;
+    OutsideCaptures guard;
+    const auto copy = [&](void* dst, const void* src, size_t bytes) {
+        return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, D.stream) == cudaSuccess;
     };
     bool ok = (!vp || copy(vp, D.vpos, sizeof(double) * 3 * nV)) && (!vc || copy(vc, D.vcells, sizeof(int) * 3 * nV)) &&
-              (!vn || copy(vn, D.vnbrs, sizeof(int) * 3 * nV)) && (!counts || copy(counts, D.deg, sizeof(int) * nC));
-    if (ok && rings && (size_t)stride == W) ok = copy(rings, D.rows, sizeof(int) * nC * W);
-    else if (ok && rings) {   // wider rows than the rings need
-        std::vector<int> rows(nC * W);
-        ok = copy(rows.data(), D.rows, sizeof(int) * rows.size());
-        for (size_t c = 0; c < nC; ++c)
-            for (size_t k = 0; k < (size_t)stride; ++k) rings[c * stride + k] = k < W ? rows[c * W + k] : -1;
-    }
+              (!vn || copy(vn, D.vnbrs, sizeof(int) * 3 * nV)) && (!counts || copy(counts, D.deg, sizeof(int) * nC)) &&
+              (!rings || copy(rings, D.rows, sizeof(int) * nC * W));
+    ok = cudaStreamSynchronize(D.stream) == cudaSuccess && ok;
+    if (ok && rings && (size_t)stride > W)   // wider rows than the rings need: spread them, the last first
+        for (size_t c = nC; c-- > 0;)
+            for (size_t k = stride; k-- > 0;) rings[c * stride + k] = k < W ? rings[c * W + k] : -1;
     return ok ? SVM_OK : SVM_ERR_CUDA;
 }
 }  // namespace svm
@@ -611,7 +624,12 @@ extern "C" int svm_topology_from_points_gpu(const double* pts, int n, void* stre
     const size_t bytes = A.used;
     svm_topology* t = new svm_topology();
     t->dev = new DeviceTopology();
-    if (cudaMalloc((void**)&A.base, bytes) != cudaSuccess) { cudaGetLastError(); delete t; return SVM_ERR_CUDA; }
+    if (cudaStreamCreateWithFlags(&t->dev->stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaMalloc((void**)&A.base, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        delete t;
+        return SVM_ERR_CUDA;
+    }
     lay();
     const auto fail = [&](int rc) { cudaStreamSynchronize(s); cudaFree(A.base); delete t; return rc; };
     if (cudaMemcpyAsync(P, pts, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, s) != cudaSuccess ||

@@ -1,4 +1,5 @@
-"""A device-built topology's handle (svm_topology_*), as a C caller keeps one: what it holds on the device."""
+"""A device-built topology's handle (svm_topology_*), as a C caller keeps one: what it holds on the device, and what the
+calls on it wait for."""
 import ctypes as C
 
 import numpy as np
@@ -42,3 +43,83 @@ def test_handle_holds_its_results_only(svm_lib):
     results = 8 * 3 * nv.value + 4 * (2 * 3 * nv.value + n + n * w.value)
     assert held <= results + (8 << 20), (held, results)   # (the driver hands memory out in pages of 2 MB)
     assert before - torch.cuda.mem_get_info()[0] <= 0
+
+
+def fetch(h):
+    from curvedspacevertexmodel_gb300 import _lib
+    nc, nv, w = C.c_int(), C.c_int(), C.c_int()
+    _lib.call("svm_topology_sizes", h, C.byref(nc), C.byref(nv), C.byref(w))
+    out = [np.empty(3 * nv.value), np.empty(nc.value * (w.value + 3), np.int32), np.empty(nc.value, np.uint32),
+           np.empty(3 * nv.value, np.int32), np.empty(3 * nv.value, np.int32)]
+    _lib.call("svm_topology_get", h, out[0], out[1], w.value + 3, out[2], out[3], out[4])
+    return out
+
+
+def host(svm, pts):
+    """The arrays of the host's hull, in rows three entries wider than its rings."""
+    t = svm.Topology(pts)
+    rows = np.full((len(pts), t.rings.shape[1] + 3), -1, np.int32)
+    for c, k in enumerate(t.ringCounts):
+        rows[c, :k] = t.rings[c, :k]
+    return [t.vertexPositions.reshape(-1), rows.reshape(-1), t.ringCounts, t.vertexCells.reshape(-1), t.vertexNeighbors.reshape(-1)]
+
+
+def same(a, b):
+    return all(np.array_equal(x, y) for x, y in zip(a, b))
+
+
+def test_fetched_while_another_thread_captures(svm_lib):
+    """Fetching and freeing a handle takes no part in a capture that another thread has under way, whatever its mode."""
+    import threading
+    import torch
+    from curvedspacevertexmodel_gb300 import _lib
+    svm = svm_lib
+    if svm.device_count() < 1:
+        pytest.fail("no CUDA device: the GPU tests need a GB300")
+    pts = centres(500)
+    h, expect, got = build(svm, pts), host(svm, pts), []
+
+    def other():
+        try:
+            got.append(fetch(h))
+            _lib.lib().svm_topology_free(h)
+        except Exception as e:
+            got.append(e)
+
+    x = torch.zeros(1000, device="cuda")
+    x += 1
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, capture_error_mode="global"):
+        x += 1
+        t = threading.Thread(target=other)
+        t.start()
+        t.join()
+        x += 1
+    g.replay()
+    torch.cuda.synchronize()
+    assert float(x[0]) == 3.0 and float(x[-1]) == 3.0
+    assert len(got) == 1 and not isinstance(got[0], Exception), got
+    assert same(got[0], expect)
+
+
+def test_fetched_while_the_device_is_busy(svm_lib):
+    """Fetching does not wait for work on the default stream."""
+    import torch
+    from curvedspacevertexmodel_gb300 import _lib
+    svm = svm_lib
+    if svm.device_count() < 1:
+        pytest.fail("no CUDA device: the GPU tests need a GB300")
+    pts = centres(500)
+    h, expect = build(svm, pts), host(svm, pts)
+    fetch(h)
+    done = torch.cuda.Event()
+    torch.cuda._sleep(1000)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(1 << 30)   # half a second
+    done.record()
+    got = fetch(h)
+    early = not done.query()
+    torch.cuda.synchronize()
+    _lib.lib().svm_topology_free(h)
+    assert early and same(got, expect)
