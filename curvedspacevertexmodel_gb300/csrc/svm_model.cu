@@ -338,9 +338,10 @@ __device__ __forceinline__ double polygon_lo(int n) { return n <= kRingTable ? k
 
 // Exact sums of FP32 values on the integer pipes: f as a multiple of 2^(c - 150), in 64 bits.  `worst` collects
 // the shifts as unsigned numbers; the sum is exact if it stays at or below kFixedShift (a value too small for
-// the unit, zero, or too large, an infinity or NaN raises it).
-constexpr unsigned kFixedShift = 30;
-constexpr int kFixedRing = 64;   // |f| < 2^24 2^30 units: sums of 64 stay below 2^60
+// the unit, zero, or too large, an infinity or NaN raises it).  |f| < 2^24 2^25 units: sums of 16 and their
+// partial sums stay within 2^53, so FP64 additions in any order are exact too, and give the same bits.
+constexpr unsigned kFixedShift = 25;
+constexpr int kFixedRing = 16;
 __device__ __forceinline__ long long fixed32(int sign, int exponent, int m, int c, unsigned& worst) {
     const int sh = exponent - c;
     worst = max(worst, (unsigned)sh);
@@ -363,8 +364,8 @@ __device__ __forceinline__ long long fixed32(double f, int c, unsigned& worst) {
 // mixed_area_limit).
 //
 // FP32 positions, one thread a cell: the centroid and the perimeter are sums of FP32 values, whose FP64 sums
-// are exact but for values some 2^26 below the largest; they are summed in fixed point on the integer pipes
-// where that is exact (fixed32), else in FP64 as before: the same bits, without the widenings and with five of
+// are exact but for values some 2^25 below the largest; where they are, they are summed in fixed point on the
+// integer pipes (fixed32), else in FP64 as before: the same bits, without the widenings and with five of
 // eleven FP64 additions a corner gone.  1M cells 205 -> 111 us, 100k 31.8 -> 21.3, 512 replicas 140 -> 75.
 //
 // kSplit: two threads a cell, in the two halves of the block: the centroid, and the area and perimeter.
@@ -394,7 +395,7 @@ __global__ void k_cells(const PT* __restrict__ pos, const int* __restrict__ ring
         // split: the first kAhead ring entries' loads are all issued before their sums, which run in ring order
         constexpr int kAhead = kSplit ? 8 : 0;
         constexpr bool kFixed = !kSplit && std::is_same<PT, float4>::value;
-        constexpr int kArcUnit = 1023 + 23 - 50;   // the perimeter in units of 2^-50: arcs in [2^-27, 16)
+        constexpr int kArcUnit = 1023 + 23 - 45;   // the perimeter in units of 2^-45: arcs in [2^-22, 16)
         if (!second) {
             D3 cp{0.0, 0.0, 0.0};
             if (kSplit) {
@@ -409,7 +410,7 @@ __global__ void k_cells(const PT* __restrict__ pos, const int* __restrict__ ring
             }
             bool summed = false;
             if constexpr (kFixed) {
-                const int c0 = 98 - 1023 + ((__double2hiint(R) >> 20) & 0x7ff);   // |f| <= R: a shift of 30 at most
+                const int c0 = 103 - 1023 + ((__double2hiint(R) >> 20) & 0x7ff);   // |f| <= R: a shift of 25 at most
                 long long x = 0, y = 0, z = 0;
                 unsigned worst = n > kFixedRing ? kFixedShift + 1 : 0;
                 for (int k = 0; k < n; ++k) {
@@ -452,7 +453,7 @@ __global__ void k_cells(const PT* __restrict__ pos, const int* __restrict__ ring
                     p += fixed32(x.x, kArcUnit, worst);
                     ang += x.y;
                 }
-                if (worst <= kFixedShift) per = __dmul_rn(__ll2double_rn(p), 0x1p-50);
+                if (worst <= kFixedShift) per = __dmul_rn(__ll2double_rn(p), 0x1p-45);
                 else
                     for (int t = 0; t < n; ++t) per += cr[t < 2 ? n - 2 + t : t - 2].x;
             } else {
