@@ -652,28 +652,37 @@ extern "C" int svm_topology_from_points_gpu(const double* pts, int n, void* stre
     if (check_launch() || exclusive_scan(own, n + 1, s, sums)) return fail(SVM_ERR_CUDA);
     // the stars have to close into one triangulated sphere before facets are numbered from them
     k_hull_max<<<nb, kB, 0, s>>>(deg, n, ctl + 2);
+    // what svm_topology_get copies, in an allocation of its own: made while the device works, with rows for rings of up
+    // to kKeptRow
+    constexpr int kKeptRow = 16;
+    double* vpos;
+    int *vcells, *vnbrs, *counts, *rows;
+    const auto keep = [&](int row) {
+        Arena K;
+        const auto cut = [&] {
+            K.used = 0;
+            vpos = K.cut<double>(3 * nf);
+            vcells = K.cut<int>(3 * nf); vnbrs = K.cut<int>(3 * nf); counts = K.cut<int>(n);
+            rows = K.cut<int>((size_t)n * row);
+        };
+        cut();
+        cudaFree(t->dev->base);
+        t->dev->base = nullptr;
+        if (cudaMalloc(&t->dev->base, K.used) != cudaSuccess) { cudaGetLastError(); return false; }
+        K.base = (char*)t->dev->base;
+        cut();
+        return true;
+    };
+    if (check_launch() || !keep(kKeptRow)) return fail(SVM_ERR_CUDA);
     int got[3], facets = 0;
-    if (check_launch() || cudaMemcpyAsync(got, ctl, sizeof(got), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+    if (cudaMemcpyAsync(got, ctl, sizeof(got), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaMemcpyAsync(&facets, own + n, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess)
         return fail(SVM_ERR_CUDA);
     if (got[0] & kOutside) return fail(SVM_ERR_DEVICE);
     if (got[0] || (size_t)facets != nf) return fail(SVM_ERR_HULL);
-    // what svm_topology_get copies, in an allocation of its own
     const int W = got[2];
-    double* vpos;
-    int *vcells, *vnbrs, *counts, *rows;
-    Arena K;
-    const auto keep = [&] {
-        K.used = 0;
-        vpos = K.cut<double>(3 * nf);
-        vcells = K.cut<int>(3 * nf); vnbrs = K.cut<int>(3 * nf); counts = K.cut<int>(n);
-        rows = K.cut<int>((size_t)n * W);
-    };
-    keep();
-    if (cudaMalloc(&t->dev->base, K.used) != cudaSuccess) { cudaGetLastError(); return fail(SVM_ERR_CUDA); }
-    K.base = (char*)t->dev->base;
-    keep();
+    if (W > kKeptRow && !keep(W)) return fail(SVM_ERR_CUDA);
     const double radius = std::sqrt(pts[0] * pts[0] + pts[1] * pts[1] + pts[2] * pts[2]);
     k_hull_emit<<<nb, kB, 0, s>>>(star, deg, n, own, F);
     k_hull_vertex<<<((int)nf + kB - 1) / kB, kB, 0, s>>>(P, F, (int)nf, own, star, deg, radius, vpos, vcells, vnbrs, ctl);

@@ -83,7 +83,7 @@ int svm_topology_from_points(const double* cellCentres, int nCells, svm_topology
  * SVM_ERR_HULL when the stars do not close into one triangulated sphere, or when a centre would need
  * more than 512 candidates (a local density roughly 7x the mean): svm_topology_from_points then
  * builds the same topology on the host.  The handle keeps its arrays on the device that was current (about
- * 144 bytes a cell) until svm_topology_free, which may wait for the device as cudaFree does;
+ * 164 bytes a cell) until svm_topology_free, which may wait for the device as cudaFree does;
  * svm_topology_get copies them from there and returns when they have arrived, without waiting for other
  * streams' work.  Neither disturbs a capture that another thread has under way. */
 int svm_topology_from_points_gpu(const double* cellCentres, int nCells, void* stream, svm_topology** out);
