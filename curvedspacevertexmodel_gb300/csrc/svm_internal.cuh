@@ -286,11 +286,6 @@ __device__ __forceinline__ double included_finish(double a, bool detPositive) {
     if (detPositive) a = positive(a) ? 2. * kPI - a : sf::negate_if(true, a);
     return a;
 }
-template <bool clamp = false>
-__device__ __forceinline__ double included_angle_pre(D3 Cx, D3 Cl, double nx, double nl, D3 pl) {
-    const bool dp = positive(dot3e(pl, Cx));
-    return included_finish(svm_acos(included_cos<clamp>(Cx, Cl, nx, nl)), dp);
-}
 
 // det(pl, p, px) > 0, the side of the corner (p x px = X): in FP32 where that is certain (svm_det), else as the
 // FP64 formula.  det(p, pl, px) is its negative.

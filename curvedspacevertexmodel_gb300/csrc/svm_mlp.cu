@@ -531,9 +531,8 @@ static int mlp_reserve(svm_mlp* M, int blocks) {
     return SVM_OK;
 }
 
-// forward + backward over samples [first, first + count) of `order` (or of X directly): the gradient
-// of sum (y - t)^2 * invBatch into M->g and the loss sum into M->loss, or, with an Adam step, the
-// step taken and the loss added to M->loss
+// A launch on `stream`; with `early` its blocks may be set up while the previous kernel of the stream ends (programmatic
+// stream serialisation: the kernel waits for it in step_begin).
 template <class... Params, class... Args>
 static void launch_early(cudaStream_t stream, bool early, void (*kernel)(Params...), int grid, int block, size_t smem,
                          Args... args) {
@@ -550,6 +549,9 @@ static void launch_early(cudaStream_t stream, bool early, void (*kernel)(Params.
     (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);   // (an error stays for check_launch)
 }
 
+// forward + backward over samples [first, first + count) of `order` (or of X directly): the gradient
+// of sum (y - t)^2 * invBatch into M->g and the loss sum into M->loss, or, with an Adam step, the
+// step taken and the loss added to M->loss
 static int mlp_grad(svm_mlp* M, const float* X, const float* Y, const int* order, int first, int count,
                     float invBatch, const AdamStep* adam) {
     const int blocks = (count + kTB - 1) / kTB;

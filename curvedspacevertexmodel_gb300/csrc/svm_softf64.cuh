@@ -68,13 +68,6 @@ SF_HD double dbl(unsigned long long u) {
     return x;
 #endif
 }
-SF_HD unsigned long long mulhi(unsigned long long a, unsigned long long b) {
-#if defined(__CUDA_ARCH__)
-    return __umul64hi(a, b);
-#else
-    return (unsigned long long)(((unsigned __int128)a * b) >> 64);
-#endif
-}
 SF_HD int clz64(unsigned long long x) {
 #if defined(__CUDA_ARCH__)
     return __clzll((long long)x);
@@ -83,8 +76,8 @@ SF_HD int clz64(unsigned long long x) {
 #endif
 }
 // FP32 seeds: the approximate reciprocal (1 ulp) and reciprocal square root (2 ulp) instructions.  Any
-// seed within kSeedUlps ulp gives the same results; the host build's are moved by SF_HOST_SEED_ULPS
-// (0 unless a test sets it) to check that.
+// seed within 4 ulp gives the same results; the host build's are moved by SF_HOST_SEED_ULPS (0 unless a test
+// sets it, to -4 or 4) to check that.
 #ifndef SF_HOST_SEED_ULPS
 #define SF_HOST_SEED_ULPS 0
 #endif
