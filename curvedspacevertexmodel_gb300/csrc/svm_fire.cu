@@ -98,7 +98,7 @@ __device__ __forceinline__ void vv_drift(double4_32a* __restrict__ pos, double4_
     st3(vel, i, v);
     const D3 q = move_exact<kHwMul>(ld3(pos, i), d, R);
     st3(pos, i, q);
-    vnorm[i] = pos_norm<false, kHwMul>(q);  // k_vnorm's value, for the corner pass that follows
+    vnorm[i] = pos_norm<false, kHwMul>(q);  // k_vnorm's value, for k_edges (models that k_corners_few does not serve)
 }
 // gpu_update_velocity (velocityVerlet.cu): v += (dt / 2) F / m with unit masses.
 __device__ __forceinline__ D3 vv_kick(D3 v, D3 f, double dt) {
@@ -109,8 +109,8 @@ __device__ __forceinline__ D3 vv_kick(D3 v, D3 f, double dt) {
 // The iteration's first kernel.  It leaves the pending flag as it is: the control of every iteration
 // (k_fire_force's last block) sets it again before this kernel next reads it, and after the last
 // iteration k_fire_finish applies the update it stands for.  Once FIRE has stopped, the positions
-// stay and only their norms are written (the corner pass of a batch's remaining iterations reads them); that
-// pass's T1 test then flags nothing (T1Scratch::stop), so the state stays the last iteration's.
+// stay and only their norms are written (k_edges reads them in a batch's remaining iterations); the T1 test then
+// flags nothing (T1Scratch::stop), so the state stays the last iteration's.
 template <bool kHwMul>
 __global__ void k_fire_vv1(const FireState* __restrict__ Sp, double4_32a* __restrict__ pos,
                            double4_32a* __restrict__ vel, const double4_32a* __restrict__ force,
@@ -246,7 +246,8 @@ __global__ void __launch_bounds__(slot_threads(kFireVerts), kForm == kFormVector
 
 // fireStep (energyMinimizerFIRE.h:56, fireStepCPU cpp:122-174) on the current forces and
 // velocities: the sums and the control, in blocks whose first kFireVerts threads hold one vertex each,
-// which is k_fire_force's layout, so the sums are bitwise those of a minimize iteration.  With kControl false: the four totals to out4 (gpu_dVec_dot_products).
+// which is k_fire_force's layout, so the sums are bitwise those of a minimize iteration.  With kControl false:
+// the four totals to out4 (gpu_dVec_dot_products).
 template <bool kControl>
 __global__ void __launch_bounds__(slot_threads(kFireVerts)) k_fire_sums(FireState* __restrict__ Sp, int nV,
                                                               const double4_32a* __restrict__ force,
@@ -279,7 +280,8 @@ int fire_iteration(svm_fire* F) {
     const int bs = spread_block(m, m->nVertices), nb = (m->nVertices + bs - 1) / bs;
     {
         PhaseTimer pt(m, SVM_PHASE_MOVE);
-        launch_next(m, m->nVertices < kDriftHwMul ? k_fire_vv1<true> : k_fire_vv1<false>, nb, bs, F->d, m->pos[m->cur], m->vel, m->force, m->vnorm, m->nVertices, m->R);
+        launch_next(m, m->nVertices < kDriftHwMul ? k_fire_vv1<true> : k_fire_vv1<false>, nb, bs, F->d, m->pos[m->cur],
+                    m->vel, m->force, m->vnorm, m->nVertices, m->R);
     }
     m->cornersValid = false;
     int rc;
@@ -452,7 +454,8 @@ int svm_velocity_verlet_step(svm_model* m, double dt, int nSteps) {
     for (int k = 0; k < nSteps; ++k) {
         {
             PhaseTimer pt(m, SVM_PHASE_MOVE);
-            launch_next(m, m->nVertices < kDriftHwMul ? k_vv_drift<true> : k_vv_drift<false>, nb, bs, m->pos[m->cur], m->vel, m->force, m->vnorm, m->nVertices, dt, m->R);
+            launch_next(m, m->nVertices < kDriftHwMul ? k_vv_drift<true> : k_vv_drift<false>, nb, bs, m->pos[m->cur],
+                        m->vel, m->force, m->vnorm, m->nVertices, dt, m->R);
         }
         m->cornersValid = false;
         int rc;

@@ -392,11 +392,14 @@ __device__ __forceinline__ double triangle_area_unit(D3 p1, D3 p2, D3 p3, double
 
 // The total-area check of the mixed form (sphericalVertexModel.cpp:304-310 compares with 1e-6): the areas
 // of nC cells on a sphere of radius R sum to 4 pi R^2 plus whole turns of R^2 -- what the check is after --
-// plus the rounding of 6 nC angles, up to half an ulp of pi each if it has a bias.  That rounding passes
-// 1e-6 at about 137,000 cells, and at 1M the check failed on nearly every state and replaced the areas by
-// the triangle fan's, which there are the less accurate ones (1e-5 each: the fan's cosines cancel) and
-// took 2.1 ms of a 3.4 ms step.  The limit is therefore never below that rounding; up to 137,000 cells it
-// is the reference's.
+// plus the rounding of 6 nC angles, which grows with nC R^2.  At 1M cells of unit density the check failed by
+// rounding alone on nearly every state and replaced the areas by the triangle fan's, which there are the less
+// accurate ones (1e-5 each: the fan's cosines cancel) and took 2.1 ms of a 3.4 ms step.  The limit is therefore
+// 2^-53 R^2 an angle where that is above 1e-6: for nC R^2 above 1.5e9, which at unit density is 137,000
+// cells; below, it is the reference's.  It is an empirical limit, not a bound (roundings that all erred one way,
+// an ulp of the angle and more each, would pass it): sheets of 20k to 1M cells in steps at T = 0.01 and of up to
+// 900 times the unit density's area sum to 0 to 0.07 of it as a rule and to 0.45 at most, and a turn of one
+// angle is pi R^2 or more, nine orders above.
 __host__ __device__ inline double mixed_area_limit(int nC, double R) {
     const double rounding = 6.0 * nC * R * R * 0x1p-53;
     return rounding > 1e-6 ? rounding : 1e-6;

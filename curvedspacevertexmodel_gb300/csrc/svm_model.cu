@@ -4,7 +4,8 @@
 // Kernel sequence of one Brownian timestep (invariant: `corner` and `vsph` describe the current
 // positions and topology when a step starts):
 //   k_cells         per cell: centroid, area (spherical excess), perimeter, total-area check
-//   k_fallback_fan  per cell: triangle-fan areas, only when the total area is off by > 1e-6
+//   k_fallback_fan  per cell: triangle-fan areas, only when the total area is off by > 1e-6 (mixed form:
+//                   mixed_area_limit)
 //   k_force_bd      per vertex: force, Brownian displacement, move onto the sphere (new buffer)
 //   k_corners_few, or k_vnorm, k_edges and k_corner
 //                   per vertex: spherical coordinates, per-corner arc and angle, T1 edge test
@@ -104,12 +105,11 @@ __device__ double block_sum(double v) {
 }
 
 // ---- geometry ------------------------------------------------------------------------------
+// The corner pass (k_corners_few, or k_vnorm, k_edges and k_corner): per vertex, spherical coordinates and,
+// for each of its three cells, the arc from the ring predecessor and the included angle at the vertex (the
+// per-corner terms of computeGeometryCPU, sphericalVertexModel.cpp:257-276).  With `t1test`, also flags
+// every edge (v, u), v < u, shorter than the T1 threshold (sphericalVertexModel.cpp:469-481).
 
-// Per vertex: spherical coordinates and, for each of its three cells, the arc from the ring
-// predecessor and the included angle at the vertex (the per-corner terms of
-// computeGeometryCPU, sphericalVertexModel.cpp:257-276).  With `t1test`, also marks every edge
-// (v, u), v < u, shorter than the T1 threshold (sphericalVertexModel.cpp:469-481).
-// One thread per vertex (large vertex counts: keeps each vertex's shared values in registers).
 // |p| of every vertex, once per corner pass: each is read by the vertex and its three neighbours.
 __global__ void k_vnorm(const double4_32a* __restrict__ pos, double* __restrict__ vnorm, int nV) {
     step_begin();
@@ -639,7 +639,8 @@ __global__ void k_move(double4_32a* __restrict__ pos, const double* __restrict__
 // Standalone T1 edge test (gpu_vm_test_edges_for_T1, sphericalVertexModel.cu:225-273).
 __global__ void k_t1_test(const double4_32a* __restrict__ pos, const float4* __restrict__ pos32,
                           const double* __restrict__ repR, const int4* __restrict__ vnbr,
-                          const int4* __restrict__ vcell, int nV, double R, double t1Threshold, double cosLo, double cosHi, double s2Lo, double s2Hi, T1Scratch t1) {
+                          const int4* __restrict__ vcell, int nV, double R, double t1Threshold, double cosLo, double cosHi,
+                          double s2Lo, double s2Hi, T1Scratch t1) {
     step_begin();
     t1_clear(t1);
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
@@ -674,9 +675,9 @@ struct ApplyArgs {
     int bumpStep;
     int barrierSpins;      // polls of a grid-barrier wait before it gives up
     int* ringMax;          // largest ring count produced (atomicMax by the commits)
-    int* ringMaxOut;       // host-visible copy, written once per pass by k_t1_patch
-    double* hostOut;       // a host-buffer step's mapped AoS output (FP64 form), else null: k_t1_patch
-                           // rewrites the vertices the pass may have moved
+    int* ringMaxOut;       // host-visible copy, written once per pass (publish_ring_max)
+    double* hostOut;       // a host-buffer step's mapped AoS output (FP64 form), else null: the pass's patch
+                           // rewrites the vertices that it may have moved
 };
 
 __device__ __forceinline__ int& compRef(int4* a, int v, int s) { return reinterpret_cast<int*>(a + v)[s]; }
@@ -1561,7 +1562,7 @@ __global__ void __launch_bounds__(kMode != kT1Block ? kCoopThreads : kParThreads
         if (tid == 0) { sctl.undo = 0; sctl.rollback = 0; sctl.exec = 0; sctl.flips = 0; sctl.next[0] = 0; sctl.next[1] = 0; sctl.late = 0; }
         __syncthreads();
     }
-    // phase clocks (block 0, thread 0; svm_model_t1_clocks): (none), reserve, run, release, end
+    // phase clocks (block 0, thread 0; svm_model_t1_clocks): (slot 0 unused), reserve, run, release, end
     const bool clk = t1.clocks && seg == 0 && blockIdx.x == 0 && tid == 0;
     long long c0 = clk ? clock64() : 0, c1 = c0;
     auto lap = [&](int slot) {
@@ -2095,8 +2096,9 @@ int launch_corners(svm_model* m, bool t1test, bool vnormReady) {
     }
     if (!m->edgeC) return SVM_ERR_ARG;  // FP64 corners exist for single spheres only
     if (m->nVertices < kFewCornersBelow) {
-        launch_next(m, few_hw_mul(m) ? k_corners_few<true> : k_corners_few<false>, (m->nVertices + kFewVerts - 1) / kFewVerts, 4 * kFewVerts, m->pos[m->cur], m->vsph,
-                    m->vcell, m->vlast, m->vnext, m->vrpos, m->vnbr, m->corner, m->Wc, m->nVertices, m->R, t1test ? 1 : 0,
+        launch_next(m, few_hw_mul(m) ? k_corners_few<true> : k_corners_few<false>,
+                    (m->nVertices + kFewVerts - 1) / kFewVerts, 4 * kFewVerts, m->pos[m->cur], m->vsph, m->vcell,
+                    m->vlast, m->vnext, m->vrpos, m->vnbr, m->corner, m->Wc, m->nVertices, m->R, t1test ? 1 : 0,
                     m->t1Threshold, m->t1);
         m->cornersValid = true;
         return check_launch();
@@ -2182,7 +2184,7 @@ int launch_geometry(svm_model* m) {
 // Blocks of a sphere's T1 pass over a cooperative grid: about one per 3000 vertices, at most the co-resident
 // count, or the count set by svm_model_set_t1_blocks.
 static int t1_coop_blocks(svm_model* m) {
-    // co-resident blocks of k_t1_parallel<true>, per device (computed on the model's device, which
+    // co-resident blocks of k_t1_parallel<kT1Grid>, per device (computed on the model's device, which
     // is current while its calls run); atomics, as host threads may drive models concurrently
     constexpr int kMaxDevices = 64;
     static std::atomic<int> maxCoopOf[kMaxDevices];

@@ -335,8 +335,8 @@ class sphericalVertexModel:
         call("svm_model_set_t1_wait_limit", self._h, int(polls))
 
     def t1Clocks(self, enable: bool = True):
-        """SM cycles of the parallel T1 pass's phases since the last call (extraction, reserve,
-        flips, release, end) and re-arms the counters (or turns them off)."""
+        """SM cycles of the parallel T1 pass's phases since the last call (extraction, which is 0 as
+        the edges come listed from the test, reserve, flips, release, end) and re-arms the counters (or turns them off)."""
         out = np.zeros(5, dtype=np.uint64)
         call("svm_model_t1_clocks", self._h, int(enable), out)
         return dict(zip(("extract", "reserve", "flip", "release", "end"), map(int, out)))

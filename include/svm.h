@@ -174,8 +174,8 @@ int svm_model_get_vertex_cells(svm_model* m, int* out);
 int svm_model_get_vertex_neighbors(svm_model* m, int* out);
 /* The last geometry pass's total-area check (sphericalVertexModel.cpp:304-310): sum of cell
  * areas, its excess over 4 pi R^2, and whether the triangle-fan fallback replaced the areas: when the
- * excess is above 1e-6 or, in the mixed form from about 137,000 cells on, above what the rounding of
- * the angles can add up to (6 nCells R^2 2^-53). */
+ * excess is above 1e-6 or, in the mixed form for nCells R^2 above 1.5e9 (137,000 cells at unit density),
+ * above 6 nCells R^2 2^-53 (empirical: the rounding of the angles was measured to add up to half of it at most). */
 int svm_model_area_check(svm_model* m, double* totalArea, double* excess, int* fallbackTaken);
 /* Geometry passes of a single sphere that took the triangle-fan fallback since the last call
  * (read and cleared). */
@@ -190,8 +190,8 @@ int svm_model_take_flips(svm_model* m, int* pairs, int capacity, int* count);
  * at a time after a rollback.  (The reference's T1 loop keeps no such counters.) */
 int svm_model_t1_stats(svm_model* m, int* stats6);
 /* SM cycles spent by the first segment of the parallel T1 pass in its phases since the last call
- * (extraction of the flagged edges, reservation, flips, release, end), when cycles5 is non-NULL
- * and the counters are on; then (re)arms them (enable != 0) or turns them off. */
+ * (always 0: the flagged edges come listed from the test; reservation, flips, release, end), when cycles5 is
+ * non-NULL and the counters are on; then (re)arms them (enable != 0) or turns them off. */
 int svm_model_t1_clocks(svm_model* m, int enable, unsigned long long* cycles5);
 /* Blocks of a single sphere's parallel T1 pass: 0 = automatic (one cluster of eight blocks, from
  * 50000 vertices on a cooperative grid of about one block per 3000 vertices), 1 = one block, n > 1 = a
