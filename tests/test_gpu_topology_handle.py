@@ -123,3 +123,20 @@ def test_fetched_while_the_device_is_busy(svm_lib):
     torch.cuda.synchronize()
     _lib.lib().svm_topology_free(h)
     assert early and same(got, expect)
+
+
+@pytest.mark.parametrize("spokes", [15, 16, 17, 24])
+def test_rings_wider_than_the_rows_made_ahead(svm_lib, spokes):
+    """A centre with up to 24 neighbours: rows of 16 entries are allocated before the rings are known."""
+    from curvedspacevertexmodel_gb300 import _lib
+    svm = svm_lib
+    if svm.device_count() < 1:
+        pytest.fail("no CUDA device: the GPU tests need a GB300")
+    rng = np.random.default_rng(spokes)
+    theta = np.concatenate([[0.0], 0.8 + 0.01 * rng.standard_normal(spokes), np.arccos(rng.uniform(-1, np.cos(1.2), 60))])
+    phi = np.concatenate([[0.0], 2 * np.pi * (np.arange(spokes) + 0.2 * rng.random(spokes)) / spokes, rng.uniform(0, 2 * np.pi, 60)])
+    pts = 2.5 * np.stack([np.sin(theta) * np.cos(phi), np.sin(theta) * np.sin(phi), np.cos(theta)], 1)
+    h, expect = build(svm, pts), host(svm, pts)
+    assert int(expect[2][0]) == expect[2].max() == spokes
+    assert same(fetch(h), expect)
+    _lib.lib().svm_topology_free(h)
